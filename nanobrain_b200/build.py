@@ -1,7 +1,8 @@
-"""Builds the C-ABI shared library ``libnb_attn.so`` next to this package with nvcc for sm_100a.
+"""Builds the C-ABI shared library ``libnb_attn.so`` with nvcc for sm_100a and the PyTorch binding
+``_nb_torch.so`` (the custom ops' native bodies, linked to the former) next to this package.
 
-The library is compiled in-tree (not into a JIT cache) so that the built file sits beside the
-sources it came from. ``python -m nanobrain_b200.build`` rebuilds it.
+Both are compiled in-tree (not into a JIT cache) so that the built files sit beside the sources they
+came from. ``python -m nanobrain_b200.build`` rebuilds them.
 """
 
 from __future__ import annotations
@@ -30,6 +31,11 @@ NVCC_FLAGS = [
 ]
 
 
+TORCH_LIB_PATH = PKG_DIR / "_nb_torch.so"
+TORCH_SOURCES = [CSRC / "torch_ops.cpp"]
+TORCH_HEADERS = [PKG_DIR.parent / "include" / "nb_attn.h"]
+
+
 def find_nvcc() -> str:
     nvcc = shutil.which("nvcc") or os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "bin", "nvcc")
     if not os.path.exists(nvcc):
@@ -37,26 +43,60 @@ def find_nvcc() -> str:
     return nvcc
 
 
-def is_stale() -> bool:
-    if not LIB_PATH.exists():
+def _stale(lib: Path, sources) -> bool:
+    if not lib.exists():
         return True
-    built = LIB_PATH.stat().st_mtime
-    return any(src.stat().st_mtime > built for src in SOURCES + HEADERS)
+    built = lib.stat().st_mtime
+    return any(src.stat().st_mtime > built for src in sources)
 
 
-def build(force: bool = False, verbose: bool = False) -> Path:
-    """Compile ``libnb_attn.so`` if it is missing or older than its sources."""
-    if not force and not is_stale():
-        return LIB_PATH
-    cmd = [find_nvcc(), *NVCC_FLAGS]
-    if verbose:
-        cmd += ["-Xptxas", "-v"]
-    cmd += ["-o", str(LIB_PATH), *map(str, SOURCES)]
+def is_stale() -> bool:
+    return _stale(LIB_PATH, SOURCES + HEADERS) or _stale(TORCH_LIB_PATH, TORCH_SOURCES + TORCH_HEADERS)
+
+
+def _run(cmd, what: str, verbose: bool) -> None:
     proc = subprocess.run(cmd, capture_output=True, text=True)
     if verbose:
         sys.stderr.write(proc.stdout + proc.stderr)
     if proc.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + proc.stdout + proc.stderr)
+        raise RuntimeError(f"{what} failed:\n" + proc.stdout + proc.stderr)
+
+
+def _build_abi(verbose: bool) -> None:
+    cmd = [find_nvcc(), *NVCC_FLAGS]
+    if verbose:
+        cmd += ["-Xptxas", "-v"]
+    _run(cmd + ["-o", str(LIB_PATH), *map(str, SOURCES)], "nvcc", verbose)
+
+
+def _build_torch(verbose: bool) -> None:
+    """The binding has no device code: a host compiler, torch's headers and libraries, and a run path
+    that finds ``libnb_attn.so`` beside it."""
+    import sysconfig
+
+    import torch
+
+    root = Path(torch.__file__).resolve().parent
+    cuda = Path(find_nvcc()).resolve().parent.parent
+    includes = [root / "include", root / "include" / "torch" / "csrc" / "api" / "include", cuda / "include",
+                Path(sysconfig.get_paths()["include"])]
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-DTORCH_API_INCLUDE_EXTENSION_H",
+           f"-DTORCH_EXTENSION_NAME={TORCH_LIB_PATH.stem}"]
+    for inc in includes:
+        cmd += ["-isystem", str(inc)]
+    cmd += ["-o", str(TORCH_LIB_PATH), *map(str, TORCH_SOURCES), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda",
+            "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python", f"-L{PKG_DIR}", f"-l:{LIB_PATH.name}",
+            "-Wl,-rpath,$ORIGIN"]
+    _run(cmd, "the binding's compilation", verbose)
+
+
+def build(force: bool = False, verbose: bool = False) -> Path:
+    """Compile what is missing or older than its sources; returns the C-ABI library's path."""
+    if force or _stale(LIB_PATH, SOURCES + HEADERS):
+        _build_abi(verbose)
+    if force or _stale(TORCH_LIB_PATH, TORCH_SOURCES + TORCH_HEADERS):
+        _build_torch(verbose)
     return LIB_PATH
 
 

@@ -28,7 +28,10 @@ using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                    CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
+using CtxGetCurrentFn = CUresult (*)(CUcontext*);
+
 EncodeTiledFn g_encode = nullptr;
+CtxGetCurrentFn g_ctx_get_current = nullptr;
 std::once_flag g_encode_once;
 
 EncodeTiledFn get_encode() {
@@ -39,8 +42,22 @@ EncodeTiledFn get_encode() {
         qres == cudaDriverEntryPointSuccess) {
       g_encode = reinterpret_cast<EncodeTiledFn>(fn);
     }
+    if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &fn, cudaEnableDefault, &qres) == cudaSuccess &&
+        qres == cudaDriverEntryPointSuccess) {
+      g_ctx_get_current = reinterpret_cast<CtxGetCurrentFn>(fn);
+    }
   });
   return g_encode;
+}
+
+// Encoding a tensor map is a driver call and needs a current context. A thread whose first CUDA call
+// this is (autograd's device thread, when the allocator serves the scratch from its cache) has none
+// yet: the runtime would bind it at its first launch.
+int bind_context(int dev) {
+  if (get_encode() == nullptr || g_ctx_get_current == nullptr) return NB_ATTN_ERR_TENSOR_MAP;
+  CUcontext ctx = nullptr;
+  if (g_ctx_get_current(&ctx) == CUDA_SUCCESS && ctx != nullptr) return NB_ATTN_OK;
+  return cudaSetDevice(dev) == cudaSuccess ? NB_ATTN_OK : NB_ATTN_ERR_LAUNCH;
 }
 
 constexpr int kMaxDevices = 64;
@@ -48,11 +65,13 @@ std::mutex g_dev_mutex;
 int g_dev_state[kMaxDevices];  // 0 = not set up, 1 = ready, <0 = error code (negated)
 int g_dev_sms[kMaxDevices];    // SM count, valid once the device is ready
 
-// Once per device: check the architecture and opt the kernels into their dynamic shared memory.
+// Bind the thread's context, and once per device: check the architecture and opt the kernels into
+// their dynamic shared memory.
 int ensure_device_ready() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return NB_ATTN_ERR_LAUNCH;
   if (dev < 0 || dev >= kMaxDevices) return NB_ATTN_ERR_DEVICE;
+  if (const int rc = bind_context(dev)) return rc;
   std::lock_guard<std::mutex> lock(g_dev_mutex);
   if (g_dev_state[dev] == 1) return NB_ATTN_OK;
   if (g_dev_state[dev] < 0) return -g_dev_state[dev];

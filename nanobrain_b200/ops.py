@@ -14,16 +14,19 @@ Two public entry points:
     ``[cu_seqlens[i], cu_seqlens[i+1])``. ``max_seqlen_*`` are host integers, so the call never
     synchronises with the device.
 
-Anything outside that subset raises; there is no fallback and no backend dispatch. Both ops
-carry fake (meta) kernels and autograd formulas, so they trace under ``torch.compile`` and
-``loss.backward()`` reaches the CUDA backward (``src/nanobrain/misc.py:368-371``).
+Anything outside that subset raises; there is no fallback and no backend dispatch. The four ops
+(forward and backward of both) have their CUDA and autograd kernels in native code
+(``csrc/torch_ops.cpp``) and their schemas and fake (meta) kernels here, so they trace under
+``torch.compile`` and ``loss.backward()`` reaches the CUDA backward
+(``src/nanobrain/misc.py:368-371``).
 """
 
 from __future__ import annotations
 
 import ctypes as C
+import importlib.machinery
+import importlib.util
 import math
-import os
 from typing import Optional
 
 import torch
@@ -32,9 +35,27 @@ from torch import Tensor
 from . import _lib
 
 HEAD_DIM = 64
-_DEBUG = os.environ.get("NB_ATTN_DEBUG", "0") == "1"
+BINDING_PATH = _lib.LIB_PATH.with_name("_nb_torch.so")
 
-_status_words: dict[int, Tensor] = {}
+_native = None  # the binding, once loaded
+
+
+def _load_native():
+    """Load the binding (which registers the ops' CUDA and autograd kernels)."""
+    global _native
+    if _native is None:
+        _lib.load()
+        if not BINDING_PATH.exists():
+            raise RuntimeError(
+                f"{BINDING_PATH} is missing: build it with `python -m nanobrain_b200.build` "
+                "(there is no CPU or PyTorch fallback for this operator)"
+            )
+        loader = importlib.machinery.ExtensionFileLoader(BINDING_PATH.stem, str(BINDING_PATH))
+        spec = importlib.util.spec_from_file_location(BINDING_PATH.stem, str(BINDING_PATH), loader=loader)
+        module = importlib.util.module_from_spec(spec)
+        loader.exec_module(module)
+        _native = module
+    return _native
 
 
 def _status_word(device: torch.device) -> Tensor:
@@ -43,11 +64,7 @@ def _status_word(device: torch.device) -> Tensor:
     The word lives in pinned host memory, which the GPU addresses directly: a kernel's rare write
     goes over the bus, and the host can look at the word at any time without synchronising."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
-    t = _status_words.get(idx)
-    if t is None:
-        t = torch.zeros(1, dtype=torch.int32).pin_memory()
-        _status_words[idx] = t
-    return t
+    return _load_native().status_word(idx)
 
 
 def _raise_for_status(word: Tensor) -> None:
@@ -60,7 +77,7 @@ def _raise_for_status(word: Tensor) -> None:
 
 def poll_status(device: Optional[torch.device] = None) -> None:
     """Raise if a kernel that has already finished reported a problem. Never synchronises: every
-    op calls this before it launches, so a failed step surfaces at the next attention call."""
+    op does this before it launches, so a failed step surfaces at the next attention call."""
     device = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     _raise_for_status(_status_word(device))
 
@@ -78,49 +95,25 @@ def _require(cond: bool, msg: str) -> None:
         raise RuntimeError("nanobrain_b200.sdpa: " + msg)
 
 
-def _check_qkv(q: Tensor, k: Tensor, v: Tensor, ndim: int) -> None:
-    for name, t in (("query", q), ("key", k), ("value", v)):
-        _require(t.is_cuda, f"{name} must be a CUDA tensor (there is no CPU path)")
-        _require(t.dtype == torch.bfloat16, f"{name} must be bfloat16, got {t.dtype}")
-        _require(t.dim() == ndim, f"{name} must have {ndim} dimensions, got {t.dim()}")
-        _require(t.shape[-1] == HEAD_DIM, f"head_dim must be {HEAD_DIM}, got {t.shape[-1]}")
-    _require(q.device == k.device == v.device, "query, key and value must be on the same device")
-    _require(k.shape == v.shape, "key and value must have the same shape")
+# ------------------------------------------------------------------------------------------
+# The ops: schemas and fake kernels (same shapes and strides as the real results)
+# ------------------------------------------------------------------------------------------
+_library = torch.library.Library("nanobrain_b200", "DEF")
+for _schema in (
+    "sdpa_fwd(Tensor q, Tensor k, Tensor v, float scale) -> (Tensor, Tensor)",
+    "sdpa_bwd(Tensor d_out, Tensor q, Tensor k, Tensor v, Tensor out, Tensor lse, float scale)"
+    " -> (Tensor, Tensor, Tensor)",
+    "sdpa_varlen_fwd(Tensor q, Tensor k, Tensor v, Tensor cu_seqlens_q, Tensor cu_seqlens_k, SymInt max_seqlen_q,"
+    " SymInt max_seqlen_k, float scale) -> (Tensor, Tensor)",
+    "sdpa_varlen_bwd(Tensor d_out, Tensor q, Tensor k, Tensor v, Tensor out, Tensor lse, Tensor cu_seqlens_q,"
+    " Tensor cu_seqlens_k, SymInt max_seqlen_q, SymInt max_seqlen_k, float scale) -> (Tensor, Tensor, Tensor)",
+):
+    _library.define(_schema, tags=(torch.Tag.pt2_compliant_tag,))
 
-
-def _strides_ok(t: Tensor) -> bool:
-    if t.stride(-1) != 1 or t.data_ptr() % 16 != 0:
-        return False
-    for size, stride in zip(t.shape[:-1], t.stride()[:-1]):
-        if size > 1 and (stride <= 0 or stride % 8 != 0):
-            return False
-    return True
-
-
-def _dense_layout(t: Tensor) -> Tensor:
-    """Return ``t`` (logical [B,H,L,64]) if the kernels can address it, else a [B,L,H,64]-memory copy."""
-    if _strides_ok(t):
-        return t
-    return t.transpose(1, 2).contiguous().transpose(1, 2)
-
-
-def _packed_layout(t: Tensor) -> Tensor:
-    return t if _strides_ok(t) else t.contiguous()
-
-
-def _dense_desc(t: Tensor) -> _lib.Tensor:
-    b, h, l, d = t.shape
-    sb = t.stride(0) if b > 1 else h * l * d
-    sh = t.stride(1) if h > 1 else d
-    st = t.stride(2) if l > 1 else h * d
-    return _lib.Tensor(t.data_ptr(), sb, st, sh)
-
-
-def _packed_desc(t: Tensor) -> _lib.Tensor:
-    n, h, d = t.shape
-    st = t.stride(0) if n > 1 else h * d
-    sh = t.stride(1) if h > 1 else d
-    return _lib.Tensor(t.data_ptr(), 0, st, sh)
+sdpa_fwd = torch.ops.nanobrain_b200.sdpa_fwd.default
+sdpa_bwd = torch.ops.nanobrain_b200.sdpa_bwd.default
+sdpa_varlen_fwd = torch.ops.nanobrain_b200.sdpa_varlen_fwd.default
+sdpa_varlen_bwd = torch.ops.nanobrain_b200.sdpa_varlen_bwd.default
 
 
 def _new_dense(like: Tensor) -> Tensor:
@@ -128,202 +121,30 @@ def _new_dense(like: Tensor) -> Tensor:
     return like.new_empty((b, l, h, d)).transpose(1, 2)
 
 
-def _stream_ptr() -> C.c_void_p:
-    return C.c_void_p(torch.cuda.current_stream().cuda_stream)
-
-
-def _before_launch(device: torch.device) -> None:
-    poll_status(device)
-
-
-def _after_launch(device: torch.device) -> None:
-    if _DEBUG:
-        check_status(device)
-
-
-# ------------------------------------------------------------------------------------------
-# Dense ops
-# ------------------------------------------------------------------------------------------
-@torch.library.custom_op("nanobrain_b200::sdpa_fwd", mutates_args=(), device_types="cuda")
-def sdpa_fwd(q: Tensor, k: Tensor, v: Tensor, scale: float) -> tuple[Tensor, Tensor]:
-    _check_qkv(q, k, v, 4)
-    b, h, lq, d = q.shape
-    _require(k.shape[0] == b and k.shape[1] == h, "query and key must agree on batch and heads (no GQA)")
-    lk = k.shape[2]
-    _require(b > 0 and h > 0 and lq > 0 and lk > 0, "empty tensors are not supported")
-    q, k, v = _dense_layout(q), _dense_layout(k), _dense_layout(v)
-    out = _new_dense(q)
-    lse = torch.empty((b, h, lq), dtype=torch.float32, device=q.device)
-    lib = _lib.load()
-    _before_launch(q.device)
-    with torch.cuda.device(q.device):
-        args = _lib.FwdArgs(
-            _lib.Shape(b, h, d, lq, lk, b * lq, b * lk, None, None, scale),
-            _dense_desc(q), _dense_desc(k), _dense_desc(v), _dense_desc(out),
-            lse.data_ptr(), _status_word(q.device).data_ptr(), None, 0,
-        )
-        _lib.check(lib.nb_attn_fwd(C.byref(args), _stream_ptr()), "nb_attn_fwd")
-    _after_launch(q.device)
-    return out, lse
-
-
-@sdpa_fwd.register_fake
+@torch.library.register_fake("nanobrain_b200::sdpa_fwd", lib=_library)
 def _(q, k, v, scale):
     b, h, lq, d = q.shape
     return _new_dense(q), q.new_empty((b, h, lq), dtype=torch.float32)
 
 
-@torch.library.custom_op("nanobrain_b200::sdpa_bwd", mutates_args=(), device_types="cuda")
-def sdpa_bwd(
-    d_out: Tensor, q: Tensor, k: Tensor, v: Tensor, out: Tensor, lse: Tensor, scale: float
-) -> tuple[Tensor, Tensor, Tensor]:
-    _check_qkv(q, k, v, 4)
-    b, h, lq, d = q.shape
-    lk = k.shape[2]
-    q, k, v = _dense_layout(q), _dense_layout(k), _dense_layout(v)
-    out, d_out = _dense_layout(out), _dense_layout(d_out)
-    _require(d_out.dtype == torch.bfloat16 and out.dtype == torch.bfloat16, "out and d_out must be bfloat16")
-    lse = lse.contiguous()
-    dq, dk, dv = _new_dense(q), _new_dense(k), _new_dense(v)
-    lib = _lib.load()
-    _before_launch(q.device)
-    shape = _lib.Shape(b, h, d, lq, lk, b * lq, b * lk, None, None, scale)
-    ws_bytes = _lib.bwd_workspace_bytes(shape)
-    workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-    with torch.cuda.device(q.device):
-        args = _lib.BwdArgs(
-            shape,
-            _dense_desc(q), _dense_desc(k), _dense_desc(v), _dense_desc(out), _dense_desc(d_out),
-            _dense_desc(dq), _dense_desc(dk), _dense_desc(dv),
-            lse.data_ptr(), workspace.data_ptr(), ws_bytes, _status_word(q.device).data_ptr(),
-        )
-        _lib.check(lib.nb_attn_bwd(C.byref(args), _stream_ptr()), "nb_attn_bwd")
-    _after_launch(q.device)
-    return dq, dk, dv
-
-
-@sdpa_bwd.register_fake
+@torch.library.register_fake("nanobrain_b200::sdpa_bwd", lib=_library)
 def _(d_out, q, k, v, out, lse, scale):
     return _new_dense(q), _new_dense(k), _new_dense(v)
 
 
-def _sdpa_setup(ctx, inputs, output):
-    q, k, v, scale = inputs
-    out, lse = output
-    ctx.save_for_backward(q, k, v, out, lse)
-    ctx.scale = scale
-
-
-def _sdpa_backward(ctx, d_out, d_lse):
-    q, k, v, out, lse = ctx.saved_tensors
-    dq, dk, dv = sdpa_bwd(d_out, q, k, v, out, lse, ctx.scale)
-    return dq, dk, dv, None
-
-
-sdpa_fwd.register_autograd(_sdpa_backward, setup_context=_sdpa_setup)
-
-
-# ------------------------------------------------------------------------------------------
-# Varlen ops
-# ------------------------------------------------------------------------------------------
-def _check_cu(cu: Tensor, name: str, device: torch.device) -> None:
-    _require(cu.dtype == torch.int32 and cu.dim() == 1 and cu.numel() >= 2, f"{name} must be int32 [B+1]")
-    _require(cu.device == device, f"{name} must live on the same device as the tokens")
-    _require(cu.is_contiguous(), f"{name} must be contiguous")
-
-
-@torch.library.custom_op("nanobrain_b200::sdpa_varlen_fwd", mutates_args=(), device_types="cuda")
-def sdpa_varlen_fwd(
-    q: Tensor, k: Tensor, v: Tensor, cu_seqlens_q: Tensor, cu_seqlens_k: Tensor,
-    max_seqlen_q: int, max_seqlen_k: int, scale: float,
-) -> tuple[Tensor, Tensor]:
-    _check_qkv(q, k, v, 3)
-    _check_cu(cu_seqlens_q, "cu_seqlens_q", q.device)
-    _check_cu(cu_seqlens_k, "cu_seqlens_k", q.device)
-    _require(cu_seqlens_q.numel() == cu_seqlens_k.numel(), "cu_seqlens_q and cu_seqlens_k must have the same length")
-    tq, h, d = q.shape
-    tk = k.shape[0]
-    _require(k.shape[1] == h, "query and key must agree on heads (no GQA)")
-    _require(tq > 0 and tk > 0 and max_seqlen_q > 0 and max_seqlen_k > 0, "empty tensors are not supported")
-    nseq = cu_seqlens_q.numel() - 1
-    q, k, v = _packed_layout(q), _packed_layout(k), _packed_layout(v)
-    out = torch.empty((tq, h, d), dtype=q.dtype, device=q.device)
-    lse = torch.empty((h, tq), dtype=torch.float32, device=q.device)
-    lib = _lib.load()
-    _before_launch(q.device)
-    shape = _lib.Shape(nseq, h, d, max_seqlen_q, max_seqlen_k, tq, tk,
-                       cu_seqlens_q.data_ptr(), cu_seqlens_k.data_ptr(), scale)
-    ws_bytes = _lib.fwd_workspace_bytes(shape)  # the scheduler's work list
-    workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-    with torch.cuda.device(q.device):
-        args = _lib.FwdArgs(
-            shape, _packed_desc(q), _packed_desc(k), _packed_desc(v), _packed_desc(out),
-            lse.data_ptr(), _status_word(q.device).data_ptr(), workspace.data_ptr(), ws_bytes,
-        )
-        _lib.check(lib.nb_attn_fwd(C.byref(args), _stream_ptr()), "nb_attn_fwd")
-    _after_launch(q.device)
-    return out, lse
-
-
-@sdpa_varlen_fwd.register_fake
+@torch.library.register_fake("nanobrain_b200::sdpa_varlen_fwd", lib=_library)
 def _(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, scale):
     tq, h, d = q.shape
     return q.new_empty((tq, h, d)), q.new_empty((h, tq), dtype=torch.float32)
 
 
-@torch.library.custom_op("nanobrain_b200::sdpa_varlen_bwd", mutates_args=(), device_types="cuda")
-def sdpa_varlen_bwd(
-    d_out: Tensor, q: Tensor, k: Tensor, v: Tensor, out: Tensor, lse: Tensor,
-    cu_seqlens_q: Tensor, cu_seqlens_k: Tensor, max_seqlen_q: int, max_seqlen_k: int, scale: float,
-) -> tuple[Tensor, Tensor, Tensor]:
-    _check_qkv(q, k, v, 3)
-    tq, h, d = q.shape
-    tk = k.shape[0]
-    nseq = cu_seqlens_q.numel() - 1
-    q, k, v = _packed_layout(q), _packed_layout(k), _packed_layout(v)
-    out, d_out = _packed_layout(out), _packed_layout(d_out)
-    _require(d_out.dtype == torch.bfloat16 and out.dtype == torch.bfloat16, "out and d_out must be bfloat16")
-    lse = lse.contiguous()
-    dq = torch.empty((tq, h, d), dtype=q.dtype, device=q.device)
-    dk = torch.empty((tk, h, d), dtype=q.dtype, device=q.device)
-    dv = torch.empty((tk, h, d), dtype=q.dtype, device=q.device)
-    lib = _lib.load()
-    _before_launch(q.device)
-    shape = _lib.Shape(nseq, h, d, max_seqlen_q, max_seqlen_k, tq, tk,
-                       cu_seqlens_q.data_ptr(), cu_seqlens_k.data_ptr(), scale)
-    ws_bytes = _lib.bwd_workspace_bytes(shape)
-    workspace = torch.empty(ws_bytes, dtype=torch.uint8, device=q.device)
-    with torch.cuda.device(q.device):
-        args = _lib.BwdArgs(
-            shape,
-            _packed_desc(q), _packed_desc(k), _packed_desc(v), _packed_desc(out), _packed_desc(d_out),
-            _packed_desc(dq), _packed_desc(dk), _packed_desc(dv),
-            lse.data_ptr(), workspace.data_ptr(), ws_bytes, _status_word(q.device).data_ptr(),
-        )
-        _lib.check(lib.nb_attn_bwd(C.byref(args), _stream_ptr()), "nb_attn_bwd")
-    _after_launch(q.device)
-    return dq, dk, dv
-
-
-@sdpa_varlen_bwd.register_fake
+@torch.library.register_fake("nanobrain_b200::sdpa_varlen_bwd", lib=_library)
 def _(d_out, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, scale):
-    return torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    return q.new_empty(q.shape), k.new_empty(k.shape), k.new_empty(k.shape)
 
 
-def _varlen_setup(ctx, inputs, output):
-    q, k, v, cu_q, cu_k, max_q, max_k, scale = inputs
-    out, lse = output
-    ctx.save_for_backward(q, k, v, out, lse, cu_q, cu_k)
-    ctx.max_q, ctx.max_k, ctx.scale = max_q, max_k, scale
-
-
-def _varlen_backward(ctx, d_out, d_lse):
-    q, k, v, out, lse, cu_q, cu_k = ctx.saved_tensors
-    dq, dk, dv = sdpa_varlen_bwd(d_out, q, k, v, out, lse, cu_q, cu_k, ctx.max_q, ctx.max_k, ctx.scale)
-    return dq, dk, dv, None, None, None, None, None
-
-
-sdpa_varlen_fwd.register_autograd(_varlen_backward, setup_context=_varlen_setup)
+if _lib.LIB_PATH.exists() and BINDING_PATH.exists():
+    _load_native()  # a tree that has not been built yet can still be imported, traced and inspected
 
 
 # ------------------------------------------------------------------------------------------
@@ -382,8 +203,9 @@ def sdpa(
     _require(not is_causal, "is_causal=True is not supported (the reference's blocks are bidirectional)")
     _require(not enable_gqa, "enable_gqa is not supported")
     scale = 1.0 / math.sqrt(query.shape[-1]) if scale is None else float(scale)
-    out, _ = sdpa_fwd(query, key, value, scale)
-    return out
+    if torch.compiler.is_compiling():  # tracing sees the op itself
+        return sdpa_fwd(query, key, value, scale)[0]
+    return (_native or _load_native()).sdpa(query, key, value, scale)
 
 
 def sdpa_varlen(
@@ -398,8 +220,10 @@ def sdpa_varlen(
 ) -> Tensor:
     """Bidirectional attention over packed ``[T, H, 64]`` tokens addressed by ``cu_seqlens``."""
     scale = 1.0 / math.sqrt(q.shape[-1]) if scale is None else float(scale)
-    out, _ = sdpa_varlen_fwd(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k), scale)
-    return out
+    if torch.compiler.is_compiling():  # tracing sees the op itself
+        return sdpa_varlen_fwd(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k), scale)[0]
+    return (_native or _load_native()).sdpa_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q),
+                                                   int(max_seqlen_k), scale)
 
 
 def selftest_mma(mode: int, a: Tensor, b: Tensor) -> Tensor:
@@ -412,7 +236,8 @@ def selftest_mma(mode: int, a: Tensor, b: Tensor) -> Tensor:
     with torch.cuda.device(a.device):
         _lib.check(
             lib.nb_attn_selftest_mma(mode, a.data_ptr(), b.data_ptr(), d.data_ptr(),
-                                     _status_word(a.device).data_ptr(), _stream_ptr()),
+                                     _status_word(a.device).data_ptr(),
+                                     C.c_void_p(torch.cuda.current_stream().cuda_stream)),
             "nb_attn_selftest_mma",
         )
     return d
