@@ -5,13 +5,21 @@
 //   attn_bwd_kernel          : a work unit is one 128-row K/V tile of one (sequence, head), walked
 //                              over the sequence's queries in 128-row steps. Everything is computed
 //                              transposed so that a thread owns a key row (tensor-memory lane):
-//                                S^T  = K Q^T                       (tcgen05, smem x smem)
-//                                dP^T = V dO^T                      (tcgen05, smem x smem)
+//                                S^T  = K Q^T                       (A = K from tensor memory)
+//                                dP^T = V dO^T                      (A = V from tensor memory)
 //                                P^T  = exp2(S^T*scale_log2 - lse)  (recomputed from the saved LSE)
 //                                dS^T = P^T o (dP^T - delta)
 //                                dV  += P^T dO                      (A = P^T from tensor memory)
-//                                dK  += dS^T Q                      (A = dS^T from shared memory)
-//                                dQ   = dS K                        (same dS bytes read MN-major)
+//                                dK  += dS^T Q                      (A = dS^T from tensor memory)
+//                                dQ   = dS K                        (A = dS from shared memory)
+//                              What bounds it: the SM's shared-memory port (operand reads of the MMAs,
+//                              128 B per clock), the compute warps' dependent chain and the board's
+//                              power limit (at 1 kW the SMs run at 1.65-1.75 GHz of 1.965). So operands
+//                              come from tensor memory wherever they can: K and V are copied there once
+//                              per work unit (tcgen05.cp) and P^T and dS^T are written over the scores
+//                              they came from; only dQ reads both operands from shared memory. Per step
+//                              the port then carries 896 clocks of operand reads where A operands from
+//                              shared memory need 1408.
 //                              dQ tiles are added into the fp32 accumulator with TMA add-reductions
 //                              because every K/V tile of a sequence contributes to every dQ row.
 //                              CTAs are persistent (one per SM): each walks its share of the work
@@ -22,11 +30,10 @@
 //                              and tail (a third of a CTA's life on ~800-token sequences) overlap
 //                              its neighbours' steps.
 //                              Warp roles (640 threads): warps 0-7 are two compute warpgroups that
-//                              split the 128 query columns of a step (64 each); warps 8-11 are
-//                              four MMA issuers (S^T/dP^T, dV, dK, dQ: one elected thread each --
-//                              a single thread can issue a tcgen05.mma only every ~55 cycles, so
-//                              the 32 MMAs of a step need several issuers to keep the tensor pipe
-//                              fed); warps 12-15 drain the dQ tiles (one tensor-memory lane
+//                              split the 128 query columns of a step (64 each); warps 8, 10, 11 are
+//                              three MMA issuers (dV and the next S^T; dK and the next dP^T; dQ: one
+//                              elected thread each, so that a wait of one does not hold back the
+//                              others); warps 12-15 drain the dQ tiles (one tensor-memory lane
 //                              quadrant each) into the accumulator and, at the end of a unit, dV
 //                              and dK into their tensors; warp 16 drives TMA; warp 17 stages the
 //                              steps' LSE/delta rows and control words (warps 18-19 only complete
@@ -37,8 +44,12 @@
 //                              the same time and have to share the SM's instruction cache (at
 //                              67 KB of code its hit rate was 68 % and instruction fetch was the
 //                              top stall; at 48 KB it is above 93 %). Hence the compact wait loop,
-//                              rolled MMA-issue loops, divisions by multiply-high, and the compute
-//                              role as a function that is not inlined.
+//                              divisions by multiply-high, and the compute role as a function that is
+//                              not inlined. (The MMA-issue loops are unrolled: rolled, a thread issues
+//                              an N = 64 MMA every 45-58 clocks instead of every 32.)
+//                              Measured (dense 32 x 8 x 4096, repeated for 0.3 s, at the power limit;
+//                              whole backward): A operands from shared memory, one row per thread
+//                              3.82 ms; this form 3.37 ms.
 //   attn_bwd_epilogue_kernel : dQ = bf16(scale * accumulator). HBM-bound.
 //
 // Packed mode: block 0 of the prologue also builds the scheduler's work list of key tiles
@@ -204,8 +215,9 @@ constexpr int kBwdOutStageBytes = 8192;  // dK/dV read-out: 2 KB per drain warp
 // K (two buffers), V, 3x(Q, dO), dS (two 64-column halves), fp32 dQ staging (two 32-column halves),
 // the dK/dV read-out staging, LSE/delta stages, the steps' control words and alignment slack
 constexpr int kBwdSmemBytes =
-    (3 + 2 * kBwdStages + 4) * kTileBytes + kBwdOutStageBytes + kBwdStages * 2 * kTile * 4 + 32 + 1024;
-constexpr int kBwdTmemCols = 512;  // S^T 0, dP^T 128, P^T 256, dV 320, dK 384, dQ 448
+    (3 + 2 * kBwdStages + 4) * kTileBytes + kBwdOutStageBytes + kBwdStages * 2 * kTile * 4 + 64 + 1024;
+// Tensor memory: S^T 0 (P^T over it), dP^T 128 (dS^T over it), dV 256, dK 320, dQ 384, K 448, V 480
+constexpr int kBwdTmemCols = 512;
 // Register re-partitioning. The CTA launches with 640 threads x 96 registers (the most the
 // register file allows); setmaxnreg only moves registers inside that allocation, so the budget
 // must balance exactly or the growing warps would wait for ever:
@@ -224,17 +236,16 @@ enum BwdBar : int {
   kBarKFull = 0,                            // [2] K is double-buffered across a CTA's work items
   kBarKFree = 2,                            // [2] the item's last dQ MMA has read K
   kBarVFull = 4,
-  kBarVFree,                                // the item's last dP^T MMA has read V
+  kBarVFree,                                // the item's V has been copied into tensor memory
   kBarQdoFull,                              // [kBwdStages] TMA issue + LSE/delta staged
-  kBarQdoEmpty = kBarQdoFull + kBwdStages,  // [kBwdStages], 3 arrivals: S/dP, dV and dK issuers
+  kBarQdoEmpty = kBarQdoFull + kBwdStages,  // [kBwdStages], 2 arrivals: both issuers
+  // [2]: one per half of the step's query columns (= per compute warpgroup)
   kBarSFull = kBarQdoEmpty + kBwdStages,
-  kBarSFree,    // 8 arrivals (one per compute warp)
-  kBarDpFull,
-  kBarDpFree,   // 8
-  kBarPFull,    // 8
-  kBarPtFree,   // dV MMAs of the step have consumed P^T
-  kBarDsFull,   // 8 arrivals
-  kBarDsFree,   // 2 arrivals: dK and dQ issuers
+  kBarDpFull = kBarSFull + 2,
+  kBarPFull = kBarDpFull + 2,    // 4 arrivals (one per compute warp): P^T is in tensor memory
+  kBarDstFull = kBarPFull + 2,   // 4: dS^T is in tensor memory
+  kBarDsFull = kBarDstFull + 2,  // 4: dS is in shared memory
+  kBarDsFree = kBarDsFull + 2,   // the step's dQ MMAs have read dS from shared memory
   kBarDqFull,
   kBarDqFree,   // 4 (dQ drain warps)
   kBarDvDone,   // the item's last dV MMA is complete
@@ -312,7 +323,7 @@ enum BwdCtrl : uint32_t {
   kCtrlLast = 2u,   // last step of a work item
   kCtrlKb = 4u,     // which K buffer the item uses
   kCtrlStop = 8u,   // no step: the CTA's work has ended
-  // bits 8-15: live query columns of the step's tile (1..128); bits 16-23: live key rows of the item's tile
+  // bits 8 and up: live key rows of the item's tile (1..128)
 };
 
 // The compute warps' role: for every step of the CTA, P^T from S^T, then dS^T from dP^T.
@@ -321,133 +332,140 @@ enum BwdCtrl : uint32_t {
 // whenever the code around it changed).
 __device__ __noinline__ void bwd_compute_role(const uint32_t bar0, int* abort_flag, int32_t* status,
                                               const uint32_t tmem_base, const float* sLse, const float* sDelta,
-                                              const volatile uint32_t* sCtrl, uint8_t* sDS_ptr,
+                                              const volatile uint32_t* sCtrl, const uint32_t ds_smem,
                                               const float scale_log2) {
   const int warp = threadIdx.x >> 5;
   const int w = warp >> 2;                       // warpgroup: query columns [64w, 64w+64)
-  const int krow_in_tile = threadIdx.x & 127;    // key row of this thread = tensor-memory lane
-  const uint32_t tm_lane = tmem_base + (uint32_t((warp & 3) * 32) << 16);
-  uint8_t* ds_half = sDS_ptr + w * kTileBytes;
+  const int t = threadIdx.x & 31, quad = warp & 3;
+  const uint32_t tm_lane = tmem_base + (uint32_t(quad * 32) << 16);
+  // This warpgroup's score columns; its P^T (dS^T) takes the first half of the S^T (dP^T) columns it
+  // has just read.
+  const uint32_t tm_s = tm_lane + 64 * w, tm_dp = tm_lane + 128 + 64 * w;
+  // A thread owns key rows row0 + {0, 8, 16, 24} of the tile and query columns 8i + col0 + {0, 1} of its
+  // warpgroup's 64 (the register layout of the 16-lane tensor-memory loads below): it needs 16 values
+  // of -lse and of -delta per step where a thread owning a whole row would need 64.
+  const int row0 = quad * 32 + (t >> 2), col0 = 2 * (t & 3);
+  const uint32_t lane0 = t == 0;
+  const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
+  auto bar = [&](int i) { return bar0 + 8u * uint32_t(i); };
+  // stmatrix: this lane's row of the 8x8 block it addresses (blocks: column block 0 / 1 x row half).
+  const uint32_t st_row = uint32_t(quad * 32 + ((t >> 3) & 1) * 8 + (t & 7)), st_chunk = uint32_t(t >> 4);
+  const uint32_t st_base = ds_smem + w * kTileBytes + st_row * 128u, st_xor = st_row & 7u;
   BwdStepPos pos;
   for (;; pos.advance()) {
-  const uint32_t s = pos.s, qs = pos.qs, qph = pos.qph;
-  auto bar = [&](int i) { return bar0 + 8u * uint32_t(i); };
-  const int lane = threadIdx.x & 31;
-  const uint32_t tm_s = tm_lane, tm_dp = tm_lane + 128, tm_pt = tm_lane + 256;
-  const uint64_t scale2 = pack_f32x2(scale_log2, scale_log2);
-  const float4* lse4 = reinterpret_cast<const float4*>(sLse + qs * kTile + 64 * w);   // -lse (log2)
-  const float4* dl4 = reinterpret_cast<const float4*>(sDelta + qs * kTile + 64 * w);  // -delta
-  uint64_t pf[32];  // P^T values of this thread as packed fp32 pairs
+    const uint32_t s = pos.s, qs = pos.qs;
+    const float2* lse2 = reinterpret_cast<const float2*>(sLse + qs * kTile + 64 * w + col0);   // -lse (log2)
+    const float2* dl2 = reinterpret_cast<const float2*>(sDelta + qs * kTile + 64 * w + col0);  // -delta
+    uint64_t pf[32];  // P^T values of this thread as packed fp32 pairs: [16 * lane half + 2 * block + row half]
 
-  bool pt_ok, dp_ok;
-  // ---- phase A: P^T = exp2(S^T * scale_log2 - lse) ----
-  mbar_wait2(bar(kBarQdoFull + qs), qph, bar(kBarSFull), s & 1, abort_flag, status);
-  const uint32_t ctrl = sCtrl[qs];
-  if ((ctrl & kCtrlStop) || *reinterpret_cast<volatile int*>(abort_flag)) break;
-  // Key rows past the end of the sequence must not contribute to dQ; on the ragged last query tile
-  // this warpgroup's half has fewer than 64 live columns.
-  const bool zero_row = krow_in_tile >= int((ctrl >> 16) & 0xFFu);
-  const int valid_cols = int((ctrl >> 8) & 0xFFu) - 64 * w;
-  tc_fence_after();
-  {
-    uint32_t ra[32], rb[32];
-    tmem_ld32(tm_s + 64 * w, ra);
-    tmem_ld32(tm_s + 64 * w + 32, rb);
-    tmem_wait_ld();
-    tc_fence_before();
+    // ---- phase A: P^T = exp2(S^T * scale_log2 - lse) ----
+    if (!mbar_wait2(bar(kBarQdoFull + qs), pos.qph, bar(kBarSFull + w), s & 1, abort_flag, status)) break;
+    const uint32_t ctrl = sCtrl[qs];
     __syncwarp();
-    if (lane == 0) mbar_arrive(bar(kBarSFree));
-    // Poll the barriers needed after the exponentials now; the polls' latency overlaps them.
-    pt_ok = s > 0 ? mbar_try_wait(bar(kBarPtFree), (s - 1) & 1) : true;
-    dp_ok = mbar_try_wait(bar(kBarDpFull), s & 1);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const uint32_t* src = i < 8 ? &ra[4 * i] : &rb[4 * (i - 8)];
-      const float4 l = lse4[i];
-      float x0, x1, x2, x3;
-      unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(src[0]), __uint_as_float(src[1])), scale2,
-                             pack_f32x2(l.x, l.y)), x0, x1);
-      unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(src[2]), __uint_as_float(src[3])), scale2,
-                             pack_f32x2(l.z, l.w)), x2, x3);
-      pf[2 * i] = pack_f32x2(fast_exp2(x0), fast_exp2(x1));
-      // Every other second pair goes to the FMA pipe: the exponentials are this phase's
-      // bottleneck (both warps of an SM sub-partition run it together on one MUFU unit).
-      if (i & 1) pf[2 * i + 1] = exp2_poly_f32x2(pack_f32x2(x2, x3));
-      else pf[2 * i + 1] = pack_f32x2(fast_exp2(x2), fast_exp2(x3));
-    }
-  }
-  if (zero_row) {
-    // Key rows past the end of the sequence must not contribute to dQ.
-#pragma unroll
-    for (int i = 0; i < 32; ++i) pf[i] = 0ull;
-  }
-  if (valid_cols < 64) {
-    // Query columns past the end of the sequence: the hardware exponential already gave exactly 0
-    // for their -inf argument, but the polynomial's clamp gave 2^-126. Zero those too (the second
-    // pair of every odd group of four columns), so that nothing at all is added to the dQ rows of
-    // the next packed sequence.
-#pragma unroll
-    for (int i = 1; i < 16; i += 2) {
-      float a0, a1;
-      unpack_f32x2(pf[2 * i + 1], a0, a1);
-      pf[2 * i + 1] = pack_f32x2(4 * i + 2 < valid_cols ? a0 : 0.f, 4 * i + 3 < valid_cols ? a1 : 0.f);
-    }
-  }
-  if (s > 0) {
-    if (!pt_ok) mbar_wait(bar(kBarPtFree), (s - 1) & 1, abort_flag, status);
     tc_fence_after();
-  }
-  {
-    uint32_t pk[16];
+    bool dp_ok;
+    {
+      uint32_t ra[2][32];
+      tmem_ld_16x256b_x8(tm_s, ra[0]);
+      tmem_ld_16x256b_x8(tm_s + (16u << 16), ra[1]);
+      uint64_t l[8];
 #pragma unroll
-    for (int c = 0; c < 2; ++c) {
+      for (int i = 0; i < 8; ++i) {
+        const float2 v = lse2[4 * i];
+        l[i] = pack_f32x2(v.x, v.y);
+      }
+      tmem_wait_ld();
+      // Look at the barrier needed after the exponentials now; the latency overlaps them.
+      dp_ok = mbar_test_wait(bar(kBarDpFull + w), s & 1);
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {  // pair i: column block i >> 1, row half i & 1
+          const uint64_t x = fma_f32x2(
+              pack_f32x2(__uint_as_float(ra[half][2 * i]), __uint_as_float(ra[half][2 * i + 1])), scale2, l[i >> 1]);
+          // All on the MUFU unit: with a quarter of them evaluated as a polynomial on the FMA pipe the
+          // kernel takes 5 % longer (issue slots and power, not the MUFU unit, are what is short).
+          // Query columns past the end of the sequence have -lse = -inf and come out as exactly 0.
+          float x0, x1;
+          unpack_f32x2(x, x0, x1);
+          pf[16 * half + i] = pack_f32x2(fast_exp2(x0), fast_exp2(x1));
+        }
+    }
+    if (ctrl & kCtrlStop) {
+      // The dQ issuer learns of the end here -- once it has seen the step before (a barrier must never
+      // run two phases ahead of a waiter that tests by parity).
+      if (s > 0) mbar_wait(bar(kBarDsFree), (s - 1) & 1, abort_flag, status);
+      __syncwarp();
+      mbar_arrive_if(bar(kBarDsFull + w), lane0);
+      break;
+    }
+    const int rows_live = int(ctrl >> 8);
+    if (rows_live < kTile) {
+      // Key rows past the end of the sequence must not contribute to dQ.
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          if (row0 + 16 * half + 8 * (i & 1) >= rows_live) pf[16 * half + i] = 0ull;
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      uint32_t pk[16];
 #pragma unroll
       for (int i = 0; i < 16; ++i) {
         float a0, a1;
-        unpack_f32x2(pf[16 * c + i], a0, a1);
+        unpack_f32x2(pf[16 * half + i], a0, a1);
         pk[i] = pack_bf16(a0, a1);
       }
-      tmem_st16(tm_pt + 32 * w + 16 * c, pk);
+      tmem_st_16x128b_x8(tm_s + (uint32_t(16 * half) << 16), pk);
     }
-  }
+    tmem_wait_st();
+    tc_fence_before();
+    __syncwarp();
+    mbar_arrive_if(bar(kBarPFull + w), lane0);
 
-  // ---- middle: pull dP^T of this tile out of tensor memory ----
-  uint32_t ra[32], rb[32];
-  if (!dp_ok) mbar_wait(bar(kBarDpFull), s & 1, abort_flag, status);
-  tc_fence_after();
-  const bool ds_ok = s > 0 ? mbar_try_wait(bar(kBarDsFree), (s - 1) & 1) : true;
-  tmem_ld32(tm_dp + 64 * w, ra);
-  tmem_ld32(tm_dp + 64 * w + 32, rb);
-  tmem_wait_ld();
-  tmem_wait_st();
-  tc_fence_before();
-  __syncwarp();
-  if (lane == 0) {
-    mbar_arrive(bar(kBarPFull));
-    mbar_arrive(bar(kBarDpFree));
-  }
-
-  // ---- phase B: dS^T = P^T o (dP^T - delta) -> shared memory ----
-  if (!ds_ok) mbar_wait(bar(kBarDsFree), (s - 1) & 1, abort_flag, status);
+    // ---- phase B: dS^T = P^T o (dP^T - delta) -> tensor memory (for dK) and shared memory (for dQ) ----
+    uint32_t ra[2][32];
+    uint64_t nd[8];
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {  // 16-byte chunk c = query columns [8c, 8c+8) of this half
-    const uint32_t* src = c < 4 ? &ra[8 * c] : &rb[8 * (c - 4)];
-    const float4 d0 = dl4[2 * c], d1 = dl4[2 * c + 1];
-    const uint64_t nd[4] = {pack_f32x2(d0.x, d0.y), pack_f32x2(d0.z, d0.w), pack_f32x2(d1.x, d1.y),
-                            pack_f32x2(d1.z, d1.w)};
-    uint32_t o[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint64_t dp2 = pack_f32x2(__uint_as_float(src[2 * i]), __uint_as_float(src[2 * i + 1]));
-      float a0, a1;
-      unpack_f32x2(mul_f32x2(pf[4 * c + i], add_f32x2(dp2, nd[i])), a0, a1);
-      o[i] = pack_bf16(a0, a1);
+    for (int i = 0; i < 8; ++i) {
+      const float2 v = dl2[4 * i];
+      nd[i] = pack_f32x2(v.x, v.y);
     }
-    *reinterpret_cast<uint4*>(ds_half + swz128(krow_in_tile, c)) = make_uint4(o[0], o[1], o[2], o[3]);
-  }
-  fence_proxy_async_smem();
-  __syncwarp();
-  if (lane == 0) mbar_arrive(bar(kBarDsFull));
+    if (!dp_ok) mbar_wait(bar(kBarDpFull + w), s & 1, abort_flag, status);
+    __syncwarp();
+    tc_fence_after();
+    tmem_ld_16x256b_x8(tm_dp, ra[0]);
+    tmem_ld_16x256b_x8(tm_dp + (16u << 16), ra[1]);
+    tmem_wait_ld();
+    const bool ds_ok = s == 0 || mbar_test_wait(bar(kBarDsFree), (s - 1) & 1);
+    uint32_t ds[2][16];
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const uint64_t dp2 = pack_f32x2(__uint_as_float(ra[half][2 * i]), __uint_as_float(ra[half][2 * i + 1]));
+        float a0, a1;
+        unpack_f32x2(mul_f32x2(pf[16 * half + i], add_f32x2(dp2, nd[i >> 1])), a0, a1);
+        ds[half][i] = pack_bf16(a0, a1);
+      }
+      tmem_st_16x128b_x8(tm_dp + (uint32_t(16 * half) << 16), ds[half]);
+    }
+    tmem_wait_st();
+    tc_fence_before();
+    __syncwarp();
+    mbar_arrive_if(bar(kBarDstFull + w), lane0);
+    if (!ds_ok) mbar_wait(bar(kBarDsFree), (s - 1) & 1, abort_flag, status);
+    __syncwarp();  // lanes leave a wait one by one; the aligned instructions below need the whole warp
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+#pragma unroll
+      for (int c = 0; c < 8; c += 2)  // two 16-byte chunks (column blocks c, c + 1) of 16 key rows
+        stmatrix_x4(st_base + half * (16 * 128) + (((c + st_chunk) ^ st_xor) << 4), ds[half][2 * c], ds[half][2 * c + 1],
+                    ds[half][2 * c + 2], ds[half][2 * c + 3]);
+    fence_proxy_async_smem();
+    __syncwarp();
+    mbar_arrive_if(bar(kBarDsFull + w), lane0);
   }
 }
 
@@ -476,13 +494,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   auto sDO = [&](uint32_t s) { return smem_base + (4 + 2 * s) * kTileBytes; };
   constexpr int kDsTile0 = 3 + 2 * kBwdStages;
   const uint32_t sDS = smem_base + kDsTile0 * kTileBytes;  // 32 KB bf16: q columns 0..63 | 64..127
-  uint8_t* sDS_ptr = smem_al + kDsTile0 * kTileBytes;
   uint8_t* sDQ_ptr = smem_al + (kDsTile0 + 2) * kTileBytes;  // 32 KB fp32: d columns 0..31 | 32..63
   uint8_t* sOut_ptr = smem_al + (kDsTile0 + 4) * kTileBytes;  // dK/dV read-out staging
   float* sLse = reinterpret_cast<float*>(sOut_ptr + kBwdOutStageBytes);  // [stages][128], log2 domain
   float* sDelta = sLse + kBwdStages * kTile;                             // [stages][128]
   uint32_t* sCtrl = reinterpret_cast<uint32_t*>(sDelta + kBwdStages * kTile);  // [stages], see BwdCtrl
-  uint32_t* sCtrlQ = sCtrl + 4;  // [4], indexed by step & 3: the dQ issuer's copy (it does not hold the stage)
+  uint32_t* sCtrlQ = sCtrl + 4;  // [8], indexed by step & 7: the dQ issuer's copy (it does not hold the stage)
 
   const uint32_t bar0 = smem_u32(&bars[0]);
   auto bar = [&](int i) { return bar0 + 8u * uint32_t(i); };
@@ -496,10 +513,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     for (int i = 0; i < kBwdNumBars; ++i) {
       uint32_t count = 1;
       if (i >= kBarQdoFull && i < kBarQdoFull + kBwdStages) count = 2;  // TMA issue + LSE/delta staged
-      if (i >= kBarQdoEmpty && i < kBarQdoEmpty + kBwdStages) count = 3;
-      if (i == kBarSFree || i == kBarDpFree || i == kBarPFull || i == kBarDsFull) count = 8;
+      if (i >= kBarQdoEmpty && i < kBarQdoEmpty + kBwdStages) count = 2;
+      if (i >= kBarPFull && i < kBarDsFull + 2) count = 4;
       if (i == kBarDqFree || i == kBarDvOut || i == kBarDkOut) count = 4;
-      if (i == kBarDsFree) count = 2;
       mbar_init(bar(i), count);
     }
     fence_mbar_init();
@@ -512,10 +528,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
-  const uint32_t tm_s = tmem_base, tm_dp = tmem_base + 128, tm_pt = tmem_base + 256;
-  const uint32_t tm_dv = tmem_base + 320, tm_dk = tmem_base + 384, tm_dq = tmem_base + 448;
+  const uint32_t tm_s = tmem_base, tm_dp = tmem_base + 128;
+  const uint32_t tm_dv = tmem_base + 256, tm_dk = tmem_base + 320, tm_dq = tmem_base + 384;
+  const uint32_t tm_k = tmem_base + 448, tm_v = tmem_base + 480;
 
-  constexpr uint32_t kIdescS = make_idesc(128, 128, 0, 0);   // K-major x K-major, N = 128
+  constexpr uint32_t kIdescSH = make_idesc(128, 64, 0, 0);   // K-major x K-major, N = 64
   constexpr uint32_t kIdescKN = make_idesc(128, 64, 0, 1);   // A K-major / tensor memory, B MN-major
   constexpr uint32_t kIdescNN = make_idesc(128, 64, 1, 1);   // A MN-major, B MN-major
   const bool packed = p.cu_q != nullptr;
@@ -600,12 +617,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             sDelta[pos.qs * kTile + r4 * 32 + lane] = dl[r4];
           }
           if (lane == 0) {
-            const int cols_live = min(wk.lq - jt * kTile, kTile);
             const uint32_t ctrl = (j == 0 ? kCtrlFirst : 0u) | (j == wk.n_q - 1 ? kCtrlLast : 0u) |
-                                  ((ni & 1u) ? kCtrlKb : 0u) | (uint32_t(cols_live) << 8) |
-                                  (uint32_t(rows_live) << 16);
+                                  ((ni & 1u) ? kCtrlKb : 0u) | (uint32_t(rows_live) << 8);
             sCtrl[pos.qs] = ctrl;
-            sCtrlQ[pos.s & 3u] = ctrl;
+            sCtrlQ[pos.s & 7u] = ctrl;
           }
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(kBarQdoFull + pos.qs));
@@ -617,7 +632,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       if (lane == 0) {
         if (pos.s >= uint32_t(kBwdStages)) mbar_wait(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u, &abort_flag, p.status);
         sCtrl[pos.qs] = kCtrlStop;
-        sCtrlQ[pos.s & 3u] = kCtrlStop;
+        sCtrlQ[pos.s & 7u] = kCtrlStop;
         mbar_arrive(bar(kBarQdoFull + pos.qs));
       }
     }
@@ -754,120 +769,162 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     if (lane == 0) bulk_wait_group_read0();  // the staging rows must outlive the TMA engine's reads
   } else if (warp >= 8) {
     setmaxnreg_dec<kBwdIssuerRegs>();
-    // Each issuer is one elected thread that walks the CTA's steps by their control words.
-    if (elect_one()) {
+    // Three issuers, one elected thread each, that walk the CTA's steps by their control words. The two
+    // halves of a step's query columns (one per compute warpgroup) run half a step apart, so one
+    // warpgroup's exponentials overlap the other's dS arithmetic and the MMAs of both. P^T takes the
+    // columns of the S^T it came from and dS^T those of its dP^T, so the next S^T (dP^T) may only be
+    // written after the dV (dK) MMAs have read them: each pair is issued by one thread in that order, and
+    // MMAs of one thread execute in order.
+    if (warp != 9 && elect_one()) {
       BwdStepPos pos;
       uint32_t ni = 0;  // items started
       volatile uint32_t* ctrl_ring = sCtrl;
+      uint32_t ctrl = 0;
       if (warp == 8) {
-        // ---------------- MMA issuer: S^T = K Q^T and dP^T = V dO^T ----------------
-        const uint64_t vd = make_sdesc(sV, 16, 1024);
-        uint64_t kd = 0;
+        // ---------------- S^T = K Q^T of step s+1 after dV += P^T dO of step s, half by half ----------------
+        // K goes into tensor memory once per item, so S^T takes its A operand from there and the
+        // shared-memory port carries only Q.
+        auto copy_k = [&](uint32_t c) {
+          const uint32_t kb = (c & kCtrlKb) ? 1u : 0u;
+          const uint64_t kd = make_sdesc(sK(kb), 16, 1024);
+          mbar_wait(bar(kBarKFull + kb), (ni >> 1) & 1, &abort_flag, p.status);
+          ++ni;
 #pragma unroll 1
-        for (;; pos.advance()) {
-          if (!mbar_wait(bar(kBarQdoFull + pos.qs), pos.qph, &abort_flag, p.status)) break;
-          const uint32_t ctrl = ctrl_ring[pos.qs];
-          if (ctrl & kCtrlStop) {
-            // The compute warps wait for the stage and for S^T together, so the stop mark needs an
-            // arrival on the S^T barrier -- once they have consumed the previous step's phase (a
-            // barrier must never run two phases ahead of a waiter that tests by parity).
-            if (pos.s > 0) mbar_wait(bar(kBarSFree), (pos.s - 1) & 1, &abort_flag, p.status);
-            mbar_arrive(bar(kBarSFull));
-            break;
-          }
-          if (ctrl & kCtrlFirst) {
-            const uint32_t kb = (ctrl & kCtrlKb) ? 1u : 0u;
-            kd = make_sdesc(sK(kb), 16, 1024);
-            mbar_wait(bar(kBarKFull + kb), (ni >> 1) & 1, &abort_flag, p.status);
-          }
-          if (pos.s > 0) mbar_wait(bar(kBarSFree), (pos.s - 1) & 1, &abort_flag, p.status);
-          tc_fence_after();
-          const uint64_t qd = make_sdesc(sQ(pos.qs), 16, 1024), gd = make_sdesc(sDO(pos.qs), 16, 1024);
-#pragma unroll 1
-          for (int k = 0; k < 4; ++k) mma_ss(tm_s, kd + 2 * k, qd + 2 * k, kIdescS, k > 0);
-          tc_commit(bar(kBarSFull));
-          if (ctrl & kCtrlFirst) mbar_wait(bar(kBarVFull), ni & 1, &abort_flag, p.status);
-          if (pos.s > 0) mbar_wait(bar(kBarDpFree), (pos.s - 1) & 1, &abort_flag, p.status);
-          tc_fence_after();
-#pragma unroll 1
-          for (int k = 0; k < 4; ++k) mma_ss(tm_dp, vd + 2 * k, gd + 2 * k, kIdescS, k > 0);
-          tc_commit(bar(kBarDpFull));
-          tc_commit(bar(kBarQdoEmpty + pos.qs));
-          if (ctrl & kCtrlLast) {
-            tc_commit(bar(kBarVFree));
-            ++ni;
-          }
+          for (int k = 0; k < 4; ++k) tmem_copy_128x256b(tm_k + 8 * k, kd + 2 * k);
+        };
+        auto issue_s = [&](uint32_t stage, int h) {
+          const uint64_t qd = make_sdesc(sQ(stage) + h * (kTileBytes / 2), 16, 1024);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) mma_ts(tm_s + 64 * h, tm_k + 8 * k, qd + 2 * k, kIdescSH, k > 0);
+          tc_commit(bar(kBarSFull + h));
+        };
+        mbar_wait(bar(kBarQdoFull), 0, &abort_flag, p.status);
+        ctrl = ctrl_ring[0];
+        if (!(ctrl & kCtrlStop)) {
+          copy_k(ctrl);
+          issue_s(0, 0);
+        } else {
+          mbar_arrive(bar(kBarSFull));
+          mbar_arrive(bar(kBarSFull + 1));
         }
-      } else if (warp == 9) {
-        // ---------------- MMA issuer: dV += P^T dO ----------------
 #pragma unroll 1
-        for (;; pos.advance()) {
-          if (!mbar_wait(bar(kBarQdoFull + pos.qs), pos.qph, &abort_flag, p.status)) break;
-          const uint32_t ctrl = ctrl_ring[pos.qs];
-          if (ctrl & kCtrlStop) break;
+        while (!(ctrl & kCtrlStop)) {
           const bool first = (ctrl & kCtrlFirst) != 0;
+          BwdStepPos next = pos;
+          next.advance();
           // The previous item's dV has to be out of tensor memory before this one's first MMA.
-          if (first && ni > 0) mbar_wait(bar(kBarDvOut), (ni - 1) & 1, &abort_flag, p.status);
-          mbar_wait(bar(kBarPFull), pos.s & 1, &abort_flag, p.status);
-          tc_fence_after();
+          if (first && ni > 1) mbar_wait(bar(kBarDvOut), (ni - 2) & 1, &abort_flag, p.status);
           const uint64_t gd_mn = make_sdesc(sDO(pos.qs), 1024, 1024);
+          uint32_t next_ctrl = 0;
 #pragma unroll 1
-          for (int k = 0; k < 8; ++k) mma_ts(tm_dv, tm_pt + 8 * k, gd_mn + 128 * k, kIdescKN, !first || (k > 0));
-          tc_commit(bar(kBarPtFree));
-          tc_commit(bar(kBarQdoEmpty + pos.qs));
-          if (ctrl & kCtrlLast) {
-            tc_commit(bar(kBarDvDone));
-            ++ni;
+          for (int h = 0; h < 2; ++h) {
+            if (!mbar_wait(bar(kBarPFull + h), pos.s & 1, &abort_flag, p.status)) next_ctrl = kCtrlStop;
+            tc_fence_after();
+#pragma unroll
+            for (int k = 0; k < 4; ++k)  // A: P^T of query columns [64h + 16k, +16)
+              mma_ts(tm_dv, tm_s + 64 * h + 8 * k, gd_mn + 512 * h + 128 * k, kIdescKN, !first || (h + k > 0));
+            if (h == 0) {
+              if (pos.s == 0) issue_s(0, 1);  // the second half starts later: see above
+              mbar_wait(bar(kBarQdoFull + next.qs), next.qph, &abort_flag, p.status);
+              next_ctrl |= ctrl_ring[next.qs];
+              if ((next_ctrl & (kCtrlFirst | kCtrlStop)) == kCtrlFirst) {
+                // The MMAs that read the previous item's K must be complete.
+                mbar_wait(bar(kBarSFull + 1), pos.s & 1, &abort_flag, p.status);
+                tc_fence_after();
+                copy_k(next_ctrl);
+              }
+            } else {
+              tc_commit(bar(kBarQdoEmpty + pos.qs));
+              if (ctrl & kCtrlLast) tc_commit(bar(kBarDvDone));
+            }
+            // The compute warps wait for the stage and for S^T together, so the stop mark needs an
+            // arrival on the S^T barrier (they have consumed the phase before: P^T was full).
+            if (next_ctrl & kCtrlStop) mbar_arrive(bar(kBarSFull + h));
+            else issue_s(next.qs, h);
           }
+          ctrl = next_ctrl;
+          pos = next;
         }
       } else if (warp == 10) {
-        // ---------------- MMA issuer: dK += dS^T Q ----------------
+        // ---------------- dP^T = V dO^T of step s+1 after dK += dS^T Q of step s, half by half ----------------
+        const uint64_t vd = make_sdesc(sV, 16, 1024);
+        auto copy_v = [&] {
+          mbar_wait(bar(kBarVFull), ni & 1, &abort_flag, p.status);
+          ++ni;
 #pragma unroll 1
-        for (;; pos.advance()) {
-          if (!mbar_wait(bar(kBarQdoFull + pos.qs), pos.qph, &abort_flag, p.status)) break;
-          const uint32_t ctrl = ctrl_ring[pos.qs];
-          if (ctrl & kCtrlStop) break;
+          for (int k = 0; k < 4; ++k) tmem_copy_128x256b(tm_v + 8 * k, vd + 2 * k);
+          tc_commit(bar(kBarVFree));
+        };
+        auto issue_dp = [&](uint32_t stage, int h) {
+          const uint64_t gd = make_sdesc(sDO(stage) + h * (kTileBytes / 2), 16, 1024);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) mma_ts(tm_dp + 64 * h, tm_v + 8 * k, gd + 2 * k, kIdescSH, k > 0);
+          tc_commit(bar(kBarDpFull + h));
+        };
+        mbar_wait(bar(kBarQdoFull), 0, &abort_flag, p.status);
+        ctrl = ctrl_ring[0];
+        if (!(ctrl & kCtrlStop)) {
+          copy_v();
+          issue_dp(0, 0);
+          issue_dp(0, 1);
+        }
+#pragma unroll 1
+        while (!(ctrl & kCtrlStop)) {
           const bool first = (ctrl & kCtrlFirst) != 0;
-          if (first && ni > 0) mbar_wait(bar(kBarDkOut), (ni - 1) & 1, &abort_flag, p.status);
-          mbar_wait(bar(kBarDsFull), pos.s & 1, &abort_flag, p.status);
-          tc_fence_after();
+          BwdStepPos next = pos;
+          next.advance();
+          if (first && ni > 1) mbar_wait(bar(kBarDkOut), (ni - 2) & 1, &abort_flag, p.status);
           const uint64_t qd_mn = make_sdesc(sQ(pos.qs), 1024, 1024);
+          uint32_t next_ctrl = 0;
 #pragma unroll 1
-          for (int k = 0; k < 8; ++k) {
-            // A: K-major view of the dS buffer; one K step = 16 query columns.
-            const uint64_t ad = make_sdesc(sDS + (k >> 2) * kTileBytes, 16, 1024) + 2 * (k & 3);
-            mma_ss(tm_dk, ad, qd_mn + 128 * k, kIdescKN, !first || (k > 0));
+          for (int h = 0; h < 2; ++h) {
+            if (!mbar_wait(bar(kBarDstFull + h), pos.s & 1, &abort_flag, p.status)) next_ctrl = kCtrlStop;
+            tc_fence_after();
+#pragma unroll
+            for (int k = 0; k < 4; ++k)  // A: dS^T of query columns [64h + 16k, +16)
+              mma_ts(tm_dk, tm_dp + 64 * h + 8 * k, qd_mn + 512 * h + 128 * k, kIdescKN, !first || (h + k > 0));
+            if (h == 0) {
+              mbar_wait(bar(kBarQdoFull + next.qs), next.qph, &abort_flag, p.status);
+              next_ctrl |= ctrl_ring[next.qs];
+              if ((next_ctrl & (kCtrlFirst | kCtrlStop)) == kCtrlFirst) {
+                // The MMAs that read the previous item's V must be complete.
+                mbar_wait(bar(kBarDpFull + 1), pos.s & 1, &abort_flag, p.status);
+                tc_fence_after();
+                copy_v();
+              }
+            } else {
+              tc_commit(bar(kBarQdoEmpty + pos.qs));
+              if (ctrl & kCtrlLast) tc_commit(bar(kBarDkDone));
+            }
+            if (!(next_ctrl & kCtrlStop)) issue_dp(next.qs, h);
           }
-          tc_commit(bar(kBarDsFree));
-          tc_commit(bar(kBarQdoEmpty + pos.qs));
-          if (ctrl & kCtrlLast) {
-            tc_commit(bar(kBarDkDone));
-            ++ni;
-          }
+          ctrl = next_ctrl;
+          pos = next;
         }
       } else {
-        // ---------------- MMA issuer: dQ = dS K ----------------
-        // A: MN-major view of the same dS bytes; one K step = 16 key rows.
+        // ---------------- dQ = dS K ----------------
+        // A: MN-major view of the dS bytes in shared memory; one K step = 16 key rows.
         const uint64_t ds_mn = make_sdesc(sDS, kTileBytes, 1024);
         uint64_t kd_mn = 0;
         uint32_t kb = 0;
 #pragma unroll 1
         for (;; pos.advance()) {
-          if (!mbar_wait(bar(kBarQdoFull + pos.qs), pos.qph, &abort_flag, p.status)) break;
           // This issuer does not hold the stage (the path from a stage becoming free to becoming full
-          // again is the tightest in the pipeline), so it reads a copy that is overwritten four steps
-          // later: that write comes after the dK MMA of step s+1, which follows this step's dQ MMA.
-          const uint32_t ctrl = (reinterpret_cast<volatile uint32_t*>(sCtrlQ))[pos.s & 3u];
+          // again is the tightest in the pipeline), so it reads a copy of the control word from a ring of
+          // eight: the word of step s+8 is written after step s+5 has freed its stage, hence after the
+          // dQ MMAs of step s+3. The compute warps have seen the word before they arrive here.
+          if (!mbar_wait(bar(kBarDsFull), pos.s & 1, &abort_flag, p.status)) break;
+          ctrl = (reinterpret_cast<volatile uint32_t*>(sCtrlQ))[pos.s & 7u];
           if (ctrl & kCtrlStop) break;
           if (ctrl & kCtrlFirst) {
             kb = (ctrl & kCtrlKb) ? 1u : 0u;
             kd_mn = make_sdesc(sK(kb), 1024, 1024);
             mbar_wait(bar(kBarKFull + kb), (ni >> 1) & 1, &abort_flag, p.status);
           }
-          mbar_wait(bar(kBarDsFull), pos.s & 1, &abort_flag, p.status);
           if (pos.s > 0) mbar_wait(bar(kBarDqFree), (pos.s - 1) & 1, &abort_flag, p.status);
+          mbar_wait(bar(kBarDsFull + 1), pos.s & 1, &abort_flag, p.status);
           tc_fence_after();
-#pragma unroll 1
+#pragma unroll
           for (int k = 0; k < 8; ++k) mma_ss(tm_dq, ds_mn + 128 * k, kd_mn + 128 * k, kIdescNN, k > 0);
           tc_commit(bar(kBarDqFull));
           tc_commit(bar(kBarDsFree));
@@ -881,7 +938,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   } else {
     // ---------------- compute warpgroups: w = 0 / 1 owns query columns [64w, 64w+64) ----------------
     setmaxnreg_inc<kBwdComputeRegs>();
-    bwd_compute_role(bar0, &abort_flag, p.status, tmem_base, sLse, sDelta, sCtrl, sDS_ptr, p.scale_log2);
+    bwd_compute_role(bar0, &abort_flag, p.status, tmem_base, sLse, sDelta, sCtrl, sDS, p.scale_log2);
   }
 
   tc_fence_before();

@@ -72,6 +72,18 @@ __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// Arrive where `pred` is non-zero, without a branch (an `if (lane == 0)` around an arrival costs the
+// warp its divergence and reconvergence).
+__device__ __forceinline__ void mbar_arrive_if(uint32_t bar, uint32_t pred) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "@p mbarrier.arrive.shared::cta.b64 _, [%0];\n\t"
+      "}\n" ::"r"(bar), "r"(pred)
+      : "memory");
+}
+
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
                : "memory");
@@ -129,6 +141,31 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   if (status_word)
     asm volatile("st.volatile.global.u32 [%0], %1;" ::"l"(status_word), "r"((int)kStatusWaitTimeout) : "memory");
   return false;
+}
+
+// One look at a barrier that never suspends the thread.
+__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+// The same wait for a single thread on a latency-critical path: it polls without being suspended for
+// a while first (a suspended thread wakes about 250 cycles after its barrier completes).
+__device__ __forceinline__ bool mbar_spin_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                               int* status_word) {
+#pragma unroll 1
+  for (int i = 0; i < 64; ++i)
+    if (mbar_test_wait(bar, parity)) return true;
+  return mbar_wait(bar, parity, abort_flag, status_word);
 }
 
 // ----------------------------------------------------------------------------------------
@@ -235,7 +272,15 @@ __device__ __forceinline__ void tmem_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
-// Arrive on an mbarrier once every tcgen05.mma issued so far by this thread has finished.
+// Copies 128 rows x 32 bytes from shared memory into 128 lanes x 8 columns (the data of one K step of a
+// K-major bf16 A operand; the descriptor is the one an MMA would take). Executed in order with later
+// MMAs of the same thread.
+__device__ __forceinline__ void tmem_copy_128x256b(uint32_t taddr, uint64_t s_desc) {
+  asm volatile("tcgen05.cp.cta_group::1.128x256b [%0], %1;" ::"r"(taddr), "l"(s_desc) : "memory");
+}
+
+// Arrive on an mbarrier once every tcgen05.mma and tcgen05.cp issued so far by this
+// thread has finished.
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
                : "memory");
@@ -293,25 +338,37 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
       : "memory");
 }
 
-// 16 lanes x 256 bit, repeated 4 times along columns (32 columns): thread t of the warp receives,
-// for column block i (8 columns each), r[4i+0..1] = row (lane_base + t/4), columns 8i + 2(t%4) + {0,1}
-// and r[4i+2..3] = row (lane_base + 8 + t/4), same columns. Four neighbouring threads thus hold
-// 32 contiguous bytes of one row, which makes a warp-wide vector store or reduction hit whole
-// 32-byte sectors.
-__device__ __forceinline__ void tmem_ld_16x256b_x4(uint32_t taddr, uint32_t (&r)[16]) {
+// 16 lanes x 256 bit, repeated 8 times along columns (64 columns): thread t of the warp receives, for
+// column block i (8 columns each), r[4i+0..1] = row (lane_base + t/4), columns 8i + 2(t%4) + {0,1} and
+// r[4i+2..3] = row (lane_base + 8 + t/4), same columns: a thread meets only 16 of the 64 columns, so
+// per-column data costs it a quarter of what the one-row-per-thread shape needs.
+__device__ __forceinline__ void tmem_ld_16x256b_x8(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
-      "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]),
-        "=r"(r[15])
+      "tcgen05.ld.sync.aligned.16x256b.x8.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
       : "r"(taddr)
       : "memory");
 }
 
-// Fire-and-forget fp32 vector reduction into global memory (two adjacent floats).
-__device__ __forceinline__ void red_add_v2(float* addr, float a, float b) {
-  asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(addr), "f"(a), "f"(b) : "memory");
+// 16 lanes x 128 bit, repeated 8 times along columns (32 columns): r[2i] goes to row (lane_base + t/4),
+// column 4i + t%4 and r[2i+1] to row (lane_base + 8 + t/4). With two bf16 per register this is the
+// layout of the load above after packing column pairs.
+__device__ __forceinline__ void tmem_st_16x128b_x8(uint32_t taddr, const uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.16x128b.x8.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
+      :
+      : "r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
+      : "memory");
+}
+
+// Four 8x8 blocks of 16-bit values from the same register layout to shared memory: lane l gives the
+// address of row l%8 (16 bytes) of block l/8.
+__device__ __forceinline__ void stmatrix_x4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b),
+               "r"(c), "r"(d)
+               : "memory");
 }
 
 // Register re-partitioning between warpgroups (all four warps of an aligned warpgroup execute it).
@@ -325,12 +382,12 @@ __device__ __forceinline__ void setmaxnreg_dec() {
 }
 
 // Waits for two barriers with the two polls in flight together (their latencies overlap).
-__device__ __forceinline__ void mbar_wait2(uint32_t bar_a, uint32_t par_a, uint32_t bar_b, uint32_t par_b,
+__device__ __forceinline__ bool mbar_wait2(uint32_t bar_a, uint32_t par_a, uint32_t bar_b, uint32_t par_b,
                                            volatile int* abort_flag, int* status_word) {
   const bool a = mbar_try_wait(bar_a, par_a);
   const bool b = mbar_try_wait(bar_b, par_b);
-  if (!a) mbar_wait(bar_a, par_a, abort_flag, status_word);
-  if (!b) mbar_wait(bar_b, par_b, abort_flag, status_word);
+  if (!a && !mbar_wait(bar_a, par_a, abort_flag, status_word)) return false;
+  return b || mbar_wait(bar_b, par_b, abort_flag, status_word);
 }
 
 // ----------------------------------------------------------------------------------------
