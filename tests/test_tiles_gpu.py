@@ -1,0 +1,53 @@
+"""The kernels at the edges of their tiles: key and query counts around the 64-column halves and the
+128-row tiles the main kernels work in, one and several of them, against the CPU oracle."""
+
+import numpy as np
+import pytest
+import torch
+
+import nanobrain_b200
+from nanobrain_b200 import ops
+from oracle import attn_oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def check(names, got, want):
+    for name, a, b in zip(names, got, want):
+        b = np.asarray(b, dtype=np.float32)
+        err = np.abs(a.detach().float().cpu().numpy() - b)
+        assert np.isfinite(err).all(), name
+        assert err.max() <= 2e-2 * max(1.0, np.abs(b).max()) and err.mean() <= 2e-3 * max(1.0, np.abs(b).max()), name
+
+
+@pytest.mark.parametrize("lk", [1, 15, 16, 17, 63, 64, 65, 127, 128, 129, 191, 192, 193, 320, 321])
+@pytest.mark.parametrize("lq", [1, 129])
+def test_half_tile_edges(lq, lk):
+    g = torch.Generator().manual_seed(1000 * lq + lk)
+    q, d_out = (torch.randn(2, 2, lq, 64, generator=g).to(torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(2, 2, lk, 64, generator=g).to(torch.bfloat16) for _ in range(2))
+    want = O.sdpa_fwd_bwd(*(t.float().numpy() for t in (q, k, v, d_out)))
+    qd, kd, vd = (t.to(DEV).requires_grad_(True) for t in (q, k, v))
+    out = nanobrain_b200.sdpa(qd, kd, vd)
+    out.backward(d_out.to(DEV))
+    ops.check_status()
+    check(("out", "dq", "dk", "dv"), (out, qd.grad, kd.grad, vd.grad), (want[0], *want[2:5]))
+
+
+@pytest.mark.parametrize("lk", [129, 192, 200, 256, 321])
+def test_second_pass_over_the_keys(lk):
+    # Scores that rise by far more than 2^60 after the first half tile: the forward walks the keys a
+    # second time with a running max. The last tile has one or two halves, ragged or full.
+    g = torch.Generator().manual_seed(lk)
+    q = torch.randn(1, 2, 140, 64, generator=g)
+    k = torch.randn(1, 2, lk, 64, generator=g)
+    v = torch.randn(1, 2, lk, 64, generator=g).to(torch.bfloat16)
+    k[:, :, 70:] *= 20.0
+    k[:, :, 128:] *= 2.0
+    q, k = q.to(torch.bfloat16), k.to(torch.bfloat16)
+    want, lse = O.sdpa_forward(*(t.float().numpy() for t in (q, k, v)))[:2]
+    out, got_lse = ops.sdpa_fwd(q.to(DEV), k.to(DEV), v.to(DEV), 0.125)
+    ops.check_status()
+    check(("out",), (out,), (want,))
+    np.testing.assert_allclose(got_lse.cpu().numpy(), lse, rtol=2e-3, atol=2e-3)
