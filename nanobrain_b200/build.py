@@ -16,8 +16,8 @@ from pathlib import Path
 PKG_DIR = Path(__file__).resolve().parent
 CSRC = PKG_DIR / "csrc"
 LIB_PATH = PKG_DIR / "libnb_attn.so"
-SOURCES = [CSRC / "nb_attn.cu"]
-HEADERS = sorted(CSRC.glob("*.cuh")) + [PKG_DIR.parent / "include" / "nb_attn.h"]
+SOURCES = [CSRC / "nb_attn.cu", CSRC / "encoder.cu"]
+HEADERS = sorted(CSRC.glob("*.cuh")) + sorted((PKG_DIR.parent / "include").glob("nb_*.h"))
 
 NVCC_FLAGS = [
     "-gencode",
@@ -32,8 +32,8 @@ NVCC_FLAGS = [
 
 
 TORCH_LIB_PATH = PKG_DIR / "_nb_torch.so"
-TORCH_SOURCES = [CSRC / "torch_ops.cpp"]
-TORCH_HEADERS = [PKG_DIR.parent / "include" / "nb_attn.h"]
+TORCH_SOURCES = [CSRC / "torch_ops.cpp", CSRC / "torch_encoder.cpp"]
+TORCH_HEADERS = [CSRC / "torch_common.h"] + sorted((PKG_DIR.parent / "include").glob("nb_*.h"))
 
 
 def find_nvcc() -> str:

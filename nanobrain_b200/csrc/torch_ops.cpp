@@ -26,6 +26,7 @@
 #include <tuple>
 
 #include "../../include/nb_attn.h"
+#include "torch_common.h"
 
 namespace {
 
@@ -59,6 +60,10 @@ Tensor status_word(int64_t device) {
   return *g_status_tensors[device];
 }
 
+}  // namespace
+
+namespace nbt {
+
 volatile int32_t* status_ptr(int64_t device) {
   volatile int32_t* p = g_status_ptrs[device].load(std::memory_order_acquire);
   if (p == nullptr) {
@@ -81,7 +86,6 @@ void raise_for_status(volatile int32_t* word) {
                         : "unknown code");
 }
 
-// NB_ATTN_DEBUG=1: synchronise and look at the status word after every call.
 void after_launch(volatile int32_t* word) {
   static const bool debug = [] {
     const char* v = std::getenv("NB_ATTN_DEBUG");
@@ -96,6 +100,15 @@ void after_launch(volatile int32_t* word) {
 void check_rc(int rc, const char* what) {
   TORCH_CHECK(rc == NB_ATTN_OK, what, " failed: ", nb_attn_strerror(rc), " (code ", rc, ")");
 }
+
+}  // namespace nbt
+
+namespace {
+
+using nbt::after_launch;
+using nbt::check_rc;
+using nbt::raise_for_status;
+using nbt::status_ptr;
 
 // ------------------------------------------------------------------------------------------
 // Argument checks and layouts
@@ -404,4 +417,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("sdpa", &sdpa, py::call_guard<py::gil_scoped_release>());
   m.def("sdpa_varlen", &sdpa_varlen, py::call_guard<py::gil_scoped_release>());
   m.def("status_word", &status_word);
+  nbt::bind_encoder(m);
 }

@@ -31,8 +31,9 @@ import torch.nn as nn
 import torch.nn.functional as F
 from torch import Tensor
 
+from . import ops
 from . import token_prep as T
-from .modules import Block, LayerNorm, SeparablePosEmbed3D
+from .modules import Attention, Block, LayerNorm, Mlp, SeparablePosEmbed3D
 
 
 def patchify3d(x: Tensor, patch_size: int = 8) -> Tensor:
@@ -293,6 +294,9 @@ class ViTMAE3D(nn.Module):
         single varlen attention call. Outputs follow ``model.py:271-285``: the mean of the patch
         tokens (class tokens dropped) and, on request, the tokens scattered back on the patch grid."""
         device = self.coord_grid.device
+        encoder = self._native_encoder(samples)
+        if encoder is not None:
+            return self._embed_native(samples, return_dense, *encoder)
         lengths = [int(m.sum()) for _, m in samples]
         if min(lengths) <= 0:
             raise ValueError("every image needs at least one in-mask patch")
@@ -320,3 +324,73 @@ class ViTMAE3D(nn.Module):
                 out["dense_mask"] = m.reshape(grid)
             outputs.append(out)
         return outputs
+
+    # ------------------------------------------------------------------ native inference encoder
+    def _native_encoder(self, samples):
+        """The encoder's parameters as ``csrc/torch_encoder.cpp`` takes them, or None where that does
+        not apply: CPU, other types than fp32 parameters and patches, modules that are not the ones this
+        file builds (or carry hooks), active stochastic depth."""
+        stem = (self.patch_embed, self.pos_embed, self.norm)
+        wx = self.pos_embed.weight_x if type(self.pos_embed) is SeparablePosEmbed3D else None
+        if wx is None or not wx.is_cuda or len(samples) == 0 or len(self.blocks) == 0 or self.pos_embed.unit != 1.0:
+            return None
+        if type(self.patch_embed) is not nn.Linear or type(self.norm) is not nn.LayerNorm or _hooked(self, *stem):
+            return None
+        dim, patch_dim = wx.shape[1], self.patch_embed.in_features
+        if dim % 64 or dim > 1024 or patch_dim % 4:
+            return None
+        blocks, eps = [], []
+        heads = None
+        for blk in self.blocks:
+            sub = blk._modules
+            n1, attn, n2, mlp = sub.get("norm1"), sub.get("attn"), sub.get("norm2"), sub.get("mlp")
+            if (type(blk) is not Block or type(attn) is not Attention or type(mlp) is not Mlp or blk.training and
+                    not (type(blk.drop_path1) is nn.Identity and type(blk.drop_path2) is nn.Identity)):
+                return None
+            am, mm = attn._modules, mlp._modules
+            linears = (am["q"], am["k"], am["v"], am["proj"], mm["fc1"], mm["fc2"])
+            if type(mm["act"]) is not nn.GELU or mm["act"].approximate != "none":
+                return None
+            if any(type(m) is not nn.Linear for m in linears) or type(n1) is not nn.LayerNorm or type(n2) is not nn.LayerNorm:
+                return None
+            if _hooked(blk, n1, attn, n2, mlp, mm["act"], *linears) or heads not in (None, attn.num_heads):
+                return None
+            heads = attn.num_heads
+            for m in (n1, *linears[:4], n2, *linears[4:]):
+                blocks += [m._parameters["weight"], m._parameters["bias"]]
+            eps += [n1.eps, n2.eps]
+        eps.append(self.norm.eps)
+        pos = self.pos_embed
+        head = [self.patch_embed.weight, self.patch_embed.bias, wx, pos.weight_y, pos.weight_z, self.cls_token,
+                self.norm.weight, self.norm.bias]
+        for t in head + blocks:
+            if t is not None and (t.dtype != torch.float32 or t.device != wx.device or not t.is_contiguous()):
+                return None
+        patches_per_image = self.coord_grid.shape[1]
+        for pt, m in samples:
+            if (pt.dtype != torch.float32 or m.dtype != torch.bool or tuple(pt.shape) != (patches_per_image, patch_dim)
+                    or m.numel() != patches_per_image):
+                return None
+        return head, blocks, eps, heads
+
+    def _embed_native(self, samples, return_dense, head, blocks, eps, heads) -> List[dict]:
+        device = head[2].device
+        patches = [pt.to(device).contiguous() for pt, _ in samples]
+        masks = [m.to(device).contiguous() for _, m in samples]
+        means, dense = ops._load_native().encode_images(patches, masks, self.coord_grid[0].contiguous(), head, blocks,
+                                                        eps, heads, return_dense)
+        grid = [size // self.patch_size[0] for size in self.grid_size]
+        outputs = []
+        for i, m in enumerate(masks):
+            out = {"global_embedding": means[i], "dense_embedding": None, "dense_mask": None}
+            if return_dense:
+                out["dense_embedding"] = dense[i].reshape(*grid, self.embed_dim)
+                out["dense_mask"] = m.reshape(grid)
+            outputs.append(out)
+        return outputs
+
+
+def _hooked(*modules: nn.Module) -> bool:
+    """Does any forward hook want to see one of these modules run?"""
+    return bool(nn.modules.module._global_forward_hooks or nn.modules.module._global_forward_pre_hooks) or any(
+        m._forward_hooks or m._forward_pre_hooks for m in modules)

@@ -1,0 +1,79 @@
+"""The native inference encoder behind ``embed_packed`` against the module-by-module path of the same
+model (``forward_encoder`` per image under bf16 autocast), at row widths and patch counts where its
+kernels have remainders, and the cases it has to leave to the modules."""
+
+import pytest
+import torch
+
+from nanobrain_b200 import model as M
+from nanobrain_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def build(heads, class_tokens, bias=True, grid=(24, 16, 20), patch=4, depth=2):
+    torch.manual_seed(heads)
+    model = M.ViTMAE3D(grid_size=grid, patch_size=patch, depth=depth, embed_dim=64 * heads, num_heads=heads,
+                       decoder_depth=0, decoder_embed_dim=64, decoder_num_heads=1, qkv_bias=bias, proj_bias=bias,
+                       class_tokens=class_tokens)
+    for p in model.parameters():
+        if p.dim() == 1:
+            torch.nn.init.normal_(p, std=0.1)
+    return model.to(DEV).eval()
+
+
+def images(model, counts, seed=0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    p, d = model.coord_grid.shape[1], model.patch_embed.in_features
+    out = []
+    for n in counts:
+        m = torch.zeros(p, dtype=torch.bool, device=DEV)
+        m[torch.randperm(p, generator=g, device=DEV)[:n]] = True
+        out.append((torch.randn(p, d, generator=g, device=DEV), m))
+    return out
+
+
+@pytest.mark.parametrize("heads,class_tokens,bias", [(1, 1, True), (2, 0, True), (3, 2, False), (11, 1, True), (16, 4, True)])
+def test_native_encoder_matches_the_modules(heads, class_tokens, bias):
+    model = build(heads, class_tokens, bias)
+    samples = images(model, [1, 120, 63, 65, 7])
+    assert model._native_encoder(samples) is not None
+    outs = model.embed_packed(samples, return_dense=True)
+    plain = model.embed_packed(samples)
+    ops.check_status()
+    for (patches, mask), out, short in zip(samples, outs, plain):
+        with torch.inference_mode(), torch.autocast("cuda", dtype=torch.bfloat16):
+            tokens = model.forward_encoder(patches[mask][None], model.coord_grid[:, mask])[0, class_tokens:].float()
+        dense = out["dense_embedding"].reshape(-1, model.embed_dim)
+        scale = tokens.abs().max()
+        assert (dense[mask] - tokens).abs().max() <= 3e-2 * scale
+        assert (dense[mask] - tokens).norm() <= 1e-2 * tokens.norm()
+        assert bool((dense[~mask] == 0).all()) and torch.equal(out["dense_mask"].reshape(-1), mask)
+        assert (out["global_embedding"] - dense[mask].mean(dim=0)).abs().max() <= 1e-4 * scale
+        assert torch.equal(short["global_embedding"], out["global_embedding"]) and short["dense_embedding"] is None
+
+
+def test_many_images_and_an_empty_one():
+    model = build(1, 1, grid=(8, 8, 8))
+    samples = images(model, [1 + i % 8 for i in range(70)])      # more than one call's worth of images
+    outs = model.embed_packed(samples)
+    for i in (0, 63, 64, 69):
+        alone = model.embed_packed([samples[i]])[0]["global_embedding"]
+        assert (alone - outs[i]["global_embedding"]).abs().max() <= 2e-2 * alone.abs().max()
+    with pytest.raises(ValueError, match="in-mask"):
+        model.embed_packed(samples[:2] + images(model, [0]))
+
+
+def test_what_the_native_encoder_leaves_to_the_modules():
+    model = build(2, 1)
+    samples = images(model, [30, 40])
+    want = [o["global_embedding"] for o in model.embed_packed(samples)]
+    seen = []
+    handle = model.blocks[0].attn.register_forward_hook(lambda *a: seen.append(1))
+    assert model._native_encoder(samples) is None
+    got = [o["global_embedding"] for o in model.embed_packed(samples)]
+    handle.remove()
+    assert seen and all((a - b).abs().max() <= 2e-2 * b.abs().max() for a, b in zip(got, want))
+    assert model._native_encoder([(p.half(), m) for p, m in samples]) is None
+    assert model.double()._native_encoder(samples) is None
