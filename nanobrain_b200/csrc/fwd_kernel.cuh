@@ -77,8 +77,10 @@ enum FwdBar : int {
   kFwdVEmpty = kFwdVFull + kFwdStages,    // [stages]
   kFwdSFull = kFwdVEmpty + kFwdStages,    // [2]: per half of a key tile
   kFwdPFull = kFwdSFull + 2,              // [2], 4 arrivals (one per softmax warp)
-  kFwdPvDone = kFwdPFull + 2,             // one phase per half
-  kFwdVerdict,                            // 4 arrivals: the first pass is judged
+  // [2]: P V of the half is complete. One barrier per half: the softmax warps hand over two halves
+  // before they look, and a barrier must never be two phases behind a waiter that tests by parity.
+  kFwdPvDone = kFwdPFull + 2,
+  kFwdVerdict = kFwdPvDone + 2,           // 4 arrivals: the first pass is judged
   kFwdNumBars
 };
 
@@ -277,7 +279,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
                 for (int k = 0; k < ksteps; ++k)
                   mma_ts(tm_o, tm_s + 64 * hf + 8 * k, vd + 512 * hf + 128 * k, kIdescPV, (i | hf | k) > 0);
               }
-              tc_commit(bar(kFwdPvDone));
+              tc_commit(bar(kFwdPvDone + hf));
               if (hf == nh - 1) tc_commit(bar(kFwdVEmpty + s));
               if (hf < nh1) {
                 if (hf == 0) {
@@ -345,7 +347,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             } else if (__any_sync(0xffffffffu, need)) {
               // Second pass: refresh the offset of the rows that need it, rescale their running sum and
               // their row of the O accumulator (complete up to the previous half).
-              mbar_wait(bar(kFwdPvDone), (t[0] + t[1] - 1) & 1, &abort_flag, p.status);
+              mbar_wait(bar(kFwdPvDone + (hf ^ 1)), ((hf ? t[0] : t[1]) - 1) & 1, &abort_flag, p.status);
               __syncwarp();
               tc_fence_after();
               const float alpha = need ? fast_exp2((m_run - m_new) * p.scale_log2) : 1.f;
@@ -390,7 +392,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
 
       // Epilogue: O / l -> bf16, natural-log LSE.
-      mbar_wait(bar(kFwdPvDone), (t[0] + t[1] - 1) & 1, &abort_flag, p.status);
+      const int last_half = ((lk - 1) >> 6) & 1;  // MMAs complete in order
+      mbar_wait(bar(kFwdPvDone + last_half), ((last_half ? t[1] : t[0]) - 1) & 1, &abort_flag, p.status);
       __syncwarp();
       tc_fence_after();
       const volatile int* meta = epi_meta;
