@@ -35,9 +35,9 @@
  *    lengths in cu_seqlens (they size tensor maps and the work list); the kernels verify this on
  *    the device and report NB_ATTN_STATUS_BAD_SEQLENS instead of dropping tiles.
  *  - Varlen scheduling: every call turns cu_seqlens into a work list of (sequence, 128-row tile)
- *    items on the device, most expensive items first and ragged last tiles at the end; the forward
- *    launches one CTA per item and head, the backward one persistent CTA per SM that takes the
- *    (item, head) pairs in list order. The list lives in the call's workspace.
+ *    items on the device, most expensive items first and ragged last tiles at the end; persistent CTAs
+ *    (two per SM in the forward, one in the backward) take the (item, head) pairs in list order. The
+ *    list lives in the call's workspace.
  *  - Varlen padding: cu_seqlens[batch] may be smaller than total_q / total_k (tokens packed into
  *    a buffer of fixed capacity). The rows past the last sequence belong to no sequence; the
  *    kernels write zeros to them in o, dq, dk and dv (and -inf in lse), so every output row is
@@ -99,7 +99,7 @@ typedef struct nb_attn_shape {
  * src/nanobrain/modules.py:62. Writes o (bf16) and lse (fp32, saved for backward).
  * Varlen mode needs `workspace`: caller-owned scratch of at least
  * nb_attn_fwd_workspace_bytes(&shape) bytes, 256-byte aligned, for the work list (contents on
- * entry do not matter). Dense mode ignores it. */
+ * entry do not matter). In dense mode it is optional, see nb_attn_fwd_split_workspace_bytes. */
 typedef struct nb_attn_fwd_args {
   nb_attn_shape shape;
   nb_attn_tensor q, k, v; /* inputs */
@@ -114,6 +114,11 @@ int nb_attn_fwd(const nb_attn_fwd_args* args, void* stream);
 
 /* Scratch bytes nb_attn_fwd needs: the work list of query tiles in varlen mode, 0 in dense mode. */
 size_t nb_attn_fwd_workspace_bytes(const nb_attn_shape* shape);
+
+/* Scratch bytes that let a dense nb_attn_fwd divide few query tiles evenly over the SMs of the current
+ * device (a tile's keys are then walked by more than one CTA and the parts added up); 0 where that would
+ * not pay. Optional: with less scratch the call gives the same results from whole tiles. */
+size_t nb_attn_fwd_split_workspace_bytes(const nb_attn_shape* shape);
 
 /* Backward: replaces the autograd backward of the same call (reached from
  * src/nanobrain/misc.py:368-371). Reads q, k, v, o, d_o, lse; writes dq, dk, dv (bf16).

@@ -37,9 +37,9 @@
 //                              quadrant each) into the accumulator and, at the end of a unit, dV
 //                              and dK into their tensors; warp 16 drives TMA; warp 17 stages the
 //                              steps' LSE/delta rows and control words (warps 18-19 only complete
-//                              its warpgroup for the register re-partitioning). The loaders and
-//                              the drain warps read the work list; the compute warps and the
-//                              issuers learn about a step from its control word alone.
+//                              its warpgroup for the register re-partitioning). Warp 16 fetches the
+//                              units and publishes them to warp 17 and the drain warps; the compute
+//                              warps and the issuers learn about a step from its control word alone.
 //                              Code size is a first-order concern here: five roles' loops run at
 //                              the same time and have to share the SM's instruction cache (at
 //                              67 KB of code its hit rate was 68 % and instruction fetch was the
@@ -54,7 +54,7 @@
 //
 // Packed mode: block 0 of the prologue also builds the scheduler's work list of key tiles
 // (sched_kernel.cuh); the main kernel's work units are list entries x heads (the heads of one entry
-// adjacent), dealt to the CTAs in the list's order of decreasing cost.
+// adjacent), taken by the CTAs in the list's order of decreasing cost.
 // A ragged tile is computed at full width and masked: rows of the NEXT packed sequence that it
 // brings into shared memory are
 // multiplied by exact zeros of P^T / dS^T. For finite data that is exact; if the next sequence's
@@ -68,26 +68,6 @@
 #include "ptx.cuh"
 
 namespace nb {
-
-// Division of a number below 2^31 by a fixed divisor as a multiply-high and a shift (the divisor's
-// magic numbers come from the host). The work-index split is inlined in four warp roles, and an
-// integer division routine in each of them is code the instruction cache has no room for.
-struct FastDiv {
-  uint32_t mul, shr, div;
-  __device__ __forceinline__ uint32_t quot(uint32_t n) const { return div == 1u ? n : __umulhi(n, mul) >> shr; }
-};
-inline FastDiv make_fast_div(uint32_t d) {
-  FastDiv f;
-  f.div = d, f.mul = 0, f.shr = 0;
-  if (d > 1) {
-    uint32_t lg = 0;
-    while ((1ull << lg) < d) ++lg;  // ceil(log2 d)
-    const uint64_t p = 31 + lg;
-    f.mul = uint32_t(((1ull << p) + d - 1) / d);
-    f.shr = uint32_t(p - 32);
-  }
-  return f;
-}
 
 #ifndef NB_BWD_L2_HINTS
 #define NB_BWD_L2_HINTS 1
@@ -221,16 +201,18 @@ constexpr int kBwdTmemCols = 512;
 // Register re-partitioning. The CTA launches with 640 threads x 96 registers (the most the
 // register file allows); setmaxnreg only moves registers inside that allocation, so the budget
 // must balance exactly or the growing warps would wait for ever:
-//   2 compute warpgroups x 128 x 168 + issuers 128 x 56 + dQ drainers 128 x 56 + loader group 128 x 32
-//   = 43008 + 7168 + 7168 + 4096 = 61440 = 640 x 96.
+//   2 compute warpgroups x 128 x 152 + issuers 128 x 64 + drainers 128 x 64 + loader group 128 x 48
+//   = 38912 + 8192 + 8192 + 6144 = 61440 = 640 x 96 (the compute role needs 144).
 // Every warp of an aligned warpgroup executes the same setmaxnreg instruction.
 constexpr int kBwdLaunchRegs = 96;
-constexpr int kBwdComputeRegs = 168;
-constexpr int kBwdIssuerRegs = 56;
-constexpr int kBwdDrainRegs = 56;
-constexpr int kBwdLoaderRegs = 32;
+constexpr int kBwdComputeRegs = 152;
+constexpr int kBwdIssuerRegs = 64;
+constexpr int kBwdDrainRegs = 64;
+constexpr int kBwdLoaderRegs = 48;
 static_assert(256 * kBwdComputeRegs + 128 * (kBwdIssuerRegs + kBwdDrainRegs + kBwdLoaderRegs) ==
                   kBwdThreads * kBwdLaunchRegs, "register budget");
+
+constexpr int kBwdWorkSlots = 4;
 
 enum BwdBar : int {
   kBarKFull = 0,                            // [2] K is double-buffered across a CTA's work items
@@ -252,7 +234,9 @@ enum BwdBar : int {
   kBarDkDone,
   kBarDvOut,    // 4: the drain warps have read the item's dV accumulator
   kBarDkOut,    // 4
-  kBwdNumBars
+  kBarWorkFull,                                  // [kBwdWorkSlots] the ring of published units
+  kBarWorkEmpty = kBarWorkFull + kBwdWorkSlots,  // [kBwdWorkSlots], 5: LSE/delta warp and drain warps
+  kBwdNumBars = kBarWorkEmpty + kBwdWorkSlots
 };
 
 // One unit of a CTA's work: a 128-row K/V tile of one (sequence, head).
@@ -262,18 +246,12 @@ struct BwdWork {
   int k_begin, lk, q_begin, lq;
 };
 
-// CTAs are persistent: CTA c of G takes the work units c, 2G-1-c, 2G+c, ... ("snake" order over
-// rounds of G). The list is ordered by decreasing cost, so this hands every CTA nearly the same
-// total, without a shared counter: every warp role of a CTA walks the same sequence on its own.
-__device__ __forceinline__ uint32_t bwd_work_index(uint32_t round) {
-  const uint32_t c = (round & 1u) ? gridDim.x - 1u - blockIdx.x : blockIdx.x;
-  return round * gridDim.x + c;
-}
-
-__device__ __forceinline__ BwdWork bwd_work(const BwdParams& p, uint32_t round) {
+// Unit g of the call; n_q = -1 past the last one. The loader fetches a CTA's units and publishes them to
+// the other roles through a small ring. Dense units all cost the same: CTA c of G takes c, G + c, ...
+// Packed units are taken from the list's counter, most expensive first.
+__device__ __forceinline__ BwdWork bwd_work(const BwdParams& p, uint32_t g) {
   BwdWork w;
   w.n_q = -1, w.kt = 0, w.h = 0, w.b = 0, w.bcoord = 0, w.k_begin = 0, w.lk = 0, w.q_begin = 0, w.lq = 0;
-  const uint32_t g = bwd_work_index(round);
   if (g >= uint32_t(p.n_work)) return w;
   if (p.cu_q != nullptr) {
     // One 32-byte read tells all about the item (the sequence index `batch` stands for the rows past
@@ -477,6 +455,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __shared__ __align__(8) uint64_t bars[kBwdNumBars];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
+  __shared__ BwdWork work_ring[kBwdWorkSlots];
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -516,6 +495,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       if (i >= kBarQdoEmpty && i < kBarQdoEmpty + kBwdStages) count = 2;
       if (i >= kBarPFull && i < kBarDsFull + 2) count = 4;
       if (i == kBarDqFree || i == kBarDvOut || i == kBarDkOut) count = 4;
+      if (i >= kBarWorkEmpty) count = 5;
       mbar_init(bar(i), count);
     }
     fence_mbar_init();
@@ -537,6 +517,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   constexpr uint32_t kIdescNN = make_idesc(128, 64, 1, 1);   // A MN-major, B MN-major
   const bool packed = p.cu_q != nullptr;
 
+  // The CTA's unit number `round`, read by a whole warp from the loader's ring.
+  auto next_work = [&](uint32_t round) {
+    const uint32_t slot = round % kBwdWorkSlots;
+    BwdWork w;
+    w.n_q = -1;
+    if (mbar_wait(bar(kBarWorkFull + slot), (round / kBwdWorkSlots) & 1, &abort_flag, p.status)) w = work_ring[slot];
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar(kBarWorkEmpty + slot));
+    return w;
+  };
+
   if (warp >= 16) {
     setmaxnreg_dec<kBwdLoaderRegs>();
     if (warp == 16) {
@@ -546,10 +537,17 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       if (lane == 0) {
         BwdStepPos pos;
         uint32_t ni = 0;  // items with queries so far
+        uint32_t g = packed ? sched_next(p.items) : blockIdx.x;
 #pragma unroll 1
         for (uint32_t round = 0;; ++round) {
-          const BwdWork wk = bwd_work(p, round);
+          const BwdWork wk = bwd_work(p, g);
+          const uint32_t slot = round % kBwdWorkSlots;
+          if (round >= uint32_t(kBwdWorkSlots))
+            mbar_wait(bar(kBarWorkEmpty + slot), ((round / kBwdWorkSlots) - 1) & 1, &abort_flag, p.status);
+          work_ring[slot] = wk;
+          mbar_arrive(bar(kBarWorkFull + slot));
           if (wk.n_q < 0) break;
+          g = packed ? sched_next(p.items) : g + gridDim.x;  // in flight during this unit's loads
           if (wk.n_q == 0) continue;
           const uint32_t kb = ni & 1u;
           const int krow = wk.k_begin + wk.kt * kTile;
@@ -589,7 +587,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       uint32_t ni = 0;
 #pragma unroll 1
       for (uint32_t round = 0;; ++round) {
-        const BwdWork wk = bwd_work(p, round);
+        const BwdWork wk = next_work(round);
         if (wk.n_q < 0) break;
         if (wk.n_q == 0) continue;
         const int rows_live = min(wk.lk - wk.kt * kTile, kTile);
@@ -659,21 +657,21 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #endif
 #pragma unroll 1
     for (uint32_t round = 0;; ++round) {
-      const BwdWork wk = bwd_work(p, round);
+      const BwdWork wk = next_work(round);
       const int n_q = wk.n_q;
       if (n_q < 0) break;
       const int h = wk.h;
       const int rows_live = wk.lk - wk.kt * kTile - quad * 32;  // this warp's rows below that exist
-      const int64_t out_row = int64_t(wk.k_begin + wk.kt * kTile + quad * 32);
-      const int64_t dv_off = int64_t(wk.bcoord) * p.dv_sb + int64_t(h) * p.dv_sh + out_row * p.dv_st;
-      const int64_t dk_off = int64_t(wk.bcoord) * p.dk_sb + int64_t(h) * p.dk_sh + out_row * p.dk_st;
+      const int out_row = wk.k_begin + wk.kt * kTile + quad * 32, bcoord = wk.bcoord;
+      auto dv_rows = [&] { return p.dv + (int64_t(bcoord) * p.dv_sb + int64_t(h) * p.dv_sh + out_row * p.dv_st); };
+      auto dk_rows = [&] { return p.dk + (int64_t(bcoord) * p.dk_sb + int64_t(h) * p.dk_sh + out_row * p.dk_st); };
       if (n_q == 0) {
         // No queries at all: dK = dV = 0.
         if (lane < rows_live) {
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
-            reinterpret_cast<uint4*>(p.dv + dv_off + int64_t(lane) * p.dv_st)[c] = make_uint4(0, 0, 0, 0);
-            reinterpret_cast<uint4*>(p.dk + dk_off + int64_t(lane) * p.dk_st)[c] = make_uint4(0, 0, 0, 0);
+            reinterpret_cast<uint4*>(dv_rows() + int64_t(lane) * p.dv_st)[c] = make_uint4(0, 0, 0, 0);
+            reinterpret_cast<uint4*>(dk_rows() + int64_t(lane) * p.dk_st)[c] = make_uint4(0, 0, 0, 0);
           }
         }
         continue;
@@ -689,8 +687,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           tc_fence_after();
           const uint32_t tm_acc = (is_dk ? tm_dk : tm_dv) + lane_off;
           const float out_scale = is_dk ? p.scale : 1.f;
-          __nv_bfloat16* out = is_dk ? p.dk + dk_off : p.dv + dv_off;
-          const int64_t out_st = is_dk ? p.dk_st : p.dv_st;
           // The whole 64-column row of this lane becomes 32 packed registers (four 16-column loads)
           // and the accumulator is handed back at once. The rows then go out 32 columns at a time
           // through a 2 KB scratch area, four lanes per 64-byte half row (a row per lane straight
@@ -709,6 +705,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(is_dk ? kBarDkOut : kBarDvOut));  // the accumulator is free
+          __nv_bfloat16* out = is_dk ? dk_rows() : dv_rows();
+          const int64_t out_st = is_dk ? p.dk_st : p.dv_st;
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
             // Row `lane` of the scratch holds 32 bf16 = four 16-byte chunks, XOR-ed with the row

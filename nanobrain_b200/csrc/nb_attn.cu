@@ -123,8 +123,10 @@ int check_shape(const nb_attn_shape& s) {
   if (s.cu_seqlens_q == nullptr) {
     if (s.total_q != int64_t(s.batch) * s.max_seqlen_q || s.total_k != int64_t(s.batch) * s.max_seqlen_k)
       return NB_ATTN_ERR_SHAPE;
-    // The backward kernel counts its work units (key tiles x heads x sequences) in 32 bits.
-    if ((int64_t(s.max_seqlen_k) + nb::kTile - 1) / nb::kTile * s.heads * s.batch > INT32_MAX) return NB_ATTN_ERR_SHAPE;
+    // The kernels count their work units (query or key tiles x heads x sequences) in 32 bits.
+    if ((int64_t(s.max_seqlen_k) + nb::kTile - 1) / nb::kTile * s.heads * s.batch > INT32_MAX ||
+        (int64_t(s.max_seqlen_q) + nb::kTile - 1) / nb::kTile * s.heads * s.batch > INT32_MAX)
+      return NB_ATTN_ERR_SHAPE;
   } else {
     if (s.total_q > INT32_MAX || s.total_k > INT32_MAX) return NB_ATTN_ERR_SHAPE;
     // The grid is items x heads.
@@ -205,6 +207,7 @@ nb::SchedParams make_sched(const nb_attn_shape& s, int side, nb::SchedItem* item
   sp.items = items;
   sp.n_items = int32_t(n_items);
   sp.status = status;
+  sp.merged = 0;
   return sp;
 }
 
@@ -236,6 +239,33 @@ int builtin_scratch_address(void** out) {
   }
   *out = g_builtin_scratch_addr[dev];
   return NB_ATTN_OK;
+}
+
+// Should a dense forward cut its units (query tiles) between CTAs, and into how many CTAs? Whole units
+// leave SMs idle where the last round over the SMs is short or there is not even one round: one image of
+// 3476 tokens and 12 heads has 336 units for 148 SMs of two CTAs each. In key tiles per CTA, with k
+// units on the busiest SM whole units take about (k/2 rounded down, plus 0.9 where k is odd: a CTA that
+// has the SM for itself is only a little faster) x tiles; cut ones take an equal share plus about four
+// tiles' time for the parts and the kernel that puts them together. An eighth has to be gained, because
+// at the power limit SMs that wait let the others run faster (1024 units of 32 tiles: 186 us whole, 189
+// cut; the image: 68 whole, 57 cut). A CTA gets at least four tiles.
+struct FwdSplit {
+  unsigned ctas = 0;  // 0: whole units
+  size_t bytes = 0;
+};
+FwdSplit fwd_split(const nb_attn_shape& s) {
+  FwdSplit r;
+  if (s.cu_seqlens_q != nullptr) return r;
+  const int64_t n_kt = ceil_div(s.max_seqlen_k, nb::kTile);
+  const int64_t units = int64_t(ceil_div(s.max_seqlen_q, nb::kFwdQRows)) * s.heads * s.batch;
+  const int64_t slots = 2 * int64_t(device_sm_count()), steps = units * n_kt;
+  const int64_t ctas = steps / 4 < slots ? steps / 4 : slots;
+  if (ctas < 2 || steps > INT32_MAX) return r;
+  const int64_t k = (units + slots / 2 - 1) / (slots / 2);
+  if ((k / 2 * 10 + (k & 1) * 9) * n_kt * 8 <= 90 * ((steps + ctas - 1) / ctas + 4)) return r;
+  r.ctas = unsigned(ctas);
+  r.bytes = 2 * size_t(ctas) * nb::kFwdPartFloats * sizeof(float);
+  return r;
 }
 
 // Everything about a backward call that can be checked without touching CUDA.
@@ -314,6 +344,7 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
         reinterpret_cast<nb::SchedItem*>(static_cast<unsigned char*>(workspace) + bwd_items_offset(s));
     p.items = items;
     p.sched = make_sched(s, 1, items, n_items, a->status);
+    p.sched.merged = 1;
     n_work = n_items * s.heads;
   }
   p.n_work = int32_t(n_work);
@@ -374,6 +405,11 @@ size_t nb_attn_fwd_workspace_bytes(const nb_attn_shape* shape) {
   return size_t(nb::sched_capacity(shape->total_q, shape->batch)) * sizeof(nb::SchedItem);
 }
 
+size_t nb_attn_fwd_split_workspace_bytes(const nb_attn_shape* shape) {
+  if (shape == nullptr || check_shape(*shape) != NB_ATTN_OK || ensure_device_ready() != NB_ATTN_OK) return 0;
+  return fwd_split(*shape).bytes;
+}
+
 int nb_attn_fwd(const nb_attn_fwd_args* a, void* stream) {
   if (a == nullptr) return NB_ATTN_ERR_NULL;
   int rc = check_shape(a->shape);
@@ -413,19 +449,40 @@ int nb_attn_fwd(const nb_attn_fwd_args* a, void* stream) {
   p.status = a->status;
 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  dim3 grid(ceil_div(s.max_seqlen_q, nb::kFwdQRows), s.heads, s.batch);
   bool ok = true;
   p.items = nullptr;
-  if (!dense) {
-    // The scheduler's list of query tiles, then one CTA per item and head.
+  p.parts = nullptr;
+  p.n_qt = ceil_div(s.max_seqlen_q, nb::kFwdQRows);
+  p.n_kt = ceil_div(s.max_seqlen_k, nb::kTile);
+  int64_t n_units = int64_t(p.n_qt) * s.heads * s.batch;
+  unsigned slots = 2 * unsigned(device_sm_count());  // CTAs are persistent, two per SM
+  if (dense) {
+    const FwdSplit split = fwd_split(s);
+    if (split.ctas > 0 && a->workspace != nullptr && a->workspace_bytes >= split.bytes &&
+        (reinterpret_cast<uintptr_t>(a->workspace) & 255u) == 0) {
+      const uint32_t steps = uint32_t(n_units * p.n_kt);
+      p.parts = static_cast<float*>(a->workspace);
+      slots = split.ctas;
+      p.split_base = steps / split.ctas, p.split_extra = steps % split.ctas;
+    }
+  } else {
+    // The scheduler's list of query tiles; a unit is an entry and a head.
     const int64_t n_items = nb::sched_capacity(s.total_q, s.batch);
     nb::SchedItem* items = static_cast<nb::SchedItem*>(a->workspace);
-    const nb::SchedParams sp = make_sched(s, 0, items, n_items, a->status);
+    nb::SchedParams sp = make_sched(s, 0, items, n_items, a->status);
+    sp.merged = 1;
     ok = launch(nb::attn_sched_kernel, dim3(1), dim3(nb::kSchedThreads), 0, st, sp) == cudaSuccess;
     p.items = items;
-    grid = dim3(unsigned(n_items * s.heads), 1, 1);
+    n_units = n_items * s.heads;
   }
+  p.n_units = int32_t(n_units);
+  p.div_heads = nb::make_fast_div(uint32_t(s.heads));
+  p.div_n_qt = nb::make_fast_div(uint32_t(p.n_qt));
+  p.div_n_kt = nb::make_fast_div(uint32_t(p.n_kt));
+  const dim3 grid(p.parts != nullptr || n_units > int64_t(slots) ? slots : unsigned(n_units), 1, 1);
   ok = ok && launch(nb::attn_fwd_kernel, grid, dim3(nb::kFwdThreads), nb::kFwdSmemBytes, st, tq, tk, tv, p) == cudaSuccess;
+  if (p.parts != nullptr)
+    ok = ok && launch(nb::attn_fwd_combine_kernel, dim3(slots - 1, 2), dim3(256), 0, st, p) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
     return NB_ATTN_ERR_LAUNCH;

@@ -192,8 +192,9 @@ void launch_fwd(nb_attn_fwd_args& a, const Tensor& q, Tensor& workspace) {
   volatile int32_t* word = status_ptr(q.get_device());
   raise_for_status(word);
   a.status = const_cast<int32_t*>(word);
-  a.workspace_bytes = nb_attn_fwd_workspace_bytes(&a.shape);
-  if (a.workspace_bytes > 0) {  // the scheduler's work list
+  a.workspace_bytes = a.shape.cu_seqlens_q != nullptr ? nb_attn_fwd_workspace_bytes(&a.shape)  // the work list
+                                                      : nb_attn_fwd_split_workspace_bytes(&a.shape);
+  if (a.workspace_bytes > 0) {
     workspace = at::empty({int64_t(a.workspace_bytes)}, q.options().dtype(at::kByte));
     a.workspace = workspace.data_ptr();
   }

@@ -143,8 +143,10 @@ def _(d_out, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_se
     return q.new_empty(q.shape), k.new_empty(k.shape), k.new_empty(k.shape)
 
 
-if _lib.LIB_PATH.exists() and BINDING_PATH.exists():
-    _load_native()  # a tree that has not been built yet can still be imported, traced and inspected
+try:
+    _load_native()
+except (RuntimeError, OSError, ImportError, AttributeError):
+    pass  # not built yet, or older than these sources: import (to build it) works, the first use raises
 
 
 # ------------------------------------------------------------------------------------------

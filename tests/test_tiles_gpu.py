@@ -51,3 +51,25 @@ def test_second_pass_over_the_keys(lk):
     ops.check_status()
     check(("out",), (out,), (want,))
     np.testing.assert_allclose(got_lse.cpu().numpy(), lse, rtol=2e-3, atol=2e-3)
+
+
+@pytest.mark.parametrize("batch,heads,lq,lk,rising", [
+    (1, 1, 130, 2000, False), (1, 1, 1, 2500, False), (1, 2, 300, 1537, False), (2, 1, 64, 4096, False),
+    (1, 6, 900, 2500, False), (1, 1, 200, 1900, True),
+])
+def test_query_tiles_cut_between_ctas(batch, heads, lq, lk, rising):
+    # Few query tiles and many keys: the dense forward gives every CTA an equal run of key tiles and
+    # puts the parts of a query tile together afterwards; `rising` scores need the second walk as well.
+    g = torch.Generator().manual_seed(lq + lk)
+    q = torch.randn(batch, heads, lq, 64, generator=g)
+    k, v = (torch.randn(batch, heads, lk, 64, generator=g) for _ in range(2))
+    if rising:
+        k[:, :, 300:] *= 20.0
+        k[:, :, 1000:] *= 2.0
+    q, k, v = (t.to(torch.bfloat16) for t in (q, k, v))
+    want, lse = O.sdpa_forward(*(t.float().numpy() for t in (q, k, v)))[:2]
+    for _ in range(2):
+        out, got_lse = ops.sdpa_fwd(q.to(DEV), k.to(DEV), v.to(DEV), 0.125)
+        ops.check_status()
+        check(("out",), (out,), (want,))
+        np.testing.assert_allclose(got_lse.cpu().numpy(), lse, rtol=2e-3, atol=2e-3)
