@@ -145,6 +145,10 @@ int nb_attn_bwd(const nb_attn_bwd_args* args, void* stream);
  * dO.O dot products [heads * total_q] and, in varlen mode, the work list of key tiles. */
 size_t nb_attn_bwd_workspace_bytes(const nb_attn_shape* shape);
 
+/* The larger workspace with which a dense nb_attn_bwd divides few key tiles evenly over the SMs of the
+ * current device (see nb_attn_fwd_split_workspace_bytes); 0 where that would not pay. Optional. */
+size_t nb_attn_bwd_split_workspace_bytes(const nb_attn_shape* shape);
+
 /* Backward for callers that cannot allocate device memory (no counterpart in the reference).
  *
  * Who needs it: code that runs where a device allocation is forbidden or unavailable -- inside a

@@ -23,6 +23,7 @@ EXPORTED_SYMBOLS = (
     "nb_attn_bwd_builtin_scratch",
     "nb_attn_fwd_workspace_bytes",
     "nb_attn_fwd_split_workspace_bytes",
+    "nb_attn_bwd_split_workspace_bytes",
     "nb_attn_selftest_wait",
     "nb_attn_schedule_capacity",
     "nb_attn_schedule_build",
@@ -123,6 +124,8 @@ def load() -> C.CDLL:
     lib.nb_attn_fwd_workspace_bytes.argtypes = [C.POINTER(Shape)]
     lib.nb_attn_fwd_split_workspace_bytes.restype = C.c_size_t
     lib.nb_attn_fwd_split_workspace_bytes.argtypes = [C.POINTER(Shape)]
+    lib.nb_attn_bwd_split_workspace_bytes.restype = C.c_size_t
+    lib.nb_attn_bwd_split_workspace_bytes.argtypes = [C.POINTER(Shape)]
     lib.nb_attn_selftest_wait.restype = C.c_int
     lib.nb_attn_selftest_wait.argtypes = [C.c_uint64, C.c_void_p, C.c_void_p, C.c_void_p]
     lib.nb_attn_schedule_capacity.restype = C.c_int64

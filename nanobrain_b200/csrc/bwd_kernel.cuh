@@ -73,6 +73,8 @@ namespace nb {
 #define NB_BWD_L2_HINTS 1
 #endif
 
+constexpr int kBwdPartFloats = 2 * kTile * kHeadDim;  // a cut unit's dV and dK
+
 struct BwdParams {
   const __nv_bfloat16 *o, *d_o;
   int64_t o_sb, o_st, o_sh, do_sb, do_st, do_sh;
@@ -90,6 +92,13 @@ struct BwdParams {
   int32_t n_work;  // work units of the main kernel: key tiles x heads x sequences, or list entries x heads
   int32_t n_kt;    // dense mode: key tiles per (sequence, head)
   FastDiv div_heads, div_n_kt;  // the main kernel splits a work index without a division routine
+  // Dense mode with few units: a CTA takes an equal run of (unit, query tile) steps, units are cut between
+  // CTAs (see bwd_work) and the epilogue adds their parts up. NULL: whole units.
+  float* parts;  // [2 * CTAs][kBwdPartFloats]
+  uint32_t split_base, split_extra;  // CTA c starts at step c * base + min(c, extra)
+  int32_t n_qt;                      // dense mode: query tiles per sequence
+  FastDiv div_n_qt;
+  int32_t row_blocks;  // blocks of the epilogue that convert dQ; the ones after them add up parts
   int64_t total_q, total_k;
   float scale, scale_log2;
   int32_t* status;
@@ -150,19 +159,57 @@ __global__ void __launch_bounds__(256) attn_bwd_prologue_kernel(const BwdParams 
   }
 }
 
+__device__ __forceinline__ uint32_t bwd_split_start(const BwdParams& p, uint32_t c) {
+  return c * p.split_base + min(c, p.split_extra);
+}
+
+// dV and dK of a cut unit from its parts, in each of them 16 groups of four columns x 128 rows of fp32.
+// Four blocks look after the unit in which CTA b's run starts, if that is the first cut in it: dV / dK
+// times two halves of the rows; thread = (row, four groups).
+__device__ __forceinline__ void bwd_combine(const BwdParams& p, uint32_t block) {
+  const uint32_t b = (block >> 2) + 1, s0 = bwd_split_start(p, b);
+  const uint32_t u = p.div_n_qt.quot(s0), first = u * uint32_t(p.n_qt), end = first + uint32_t(p.n_qt);
+  if (s0 == first || bwd_split_start(p, b - 1) > first) return;
+  const bool is_dk = (block & 1u) != 0;
+  const int row = int(block >> 1 & 1u) * 64 + int(threadIdx.x & 63), g0 = int(threadIdx.x >> 6) * 4;
+  const uint32_t t = p.div_n_kt.quot(u), seq = p.div_heads.quot(t), h = t - seq * uint32_t(p.heads);
+  const int tok = int(u - t * uint32_t(p.n_kt)) * kTile + row;
+  if (tok >= p.lk) return;
+  float4 o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) o[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+  for (uint32_t c = b - 1; bwd_split_start(p, c) < end; ++c) {
+    const float* part = p.parts + int64_t(2 * c + (c == b - 1)) * kBwdPartFloats + (is_dk ? kTile * kHeadDim : 0);
+    const float4* src = reinterpret_cast<const float4*>(part) + g0 * kTile + row;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 a = src[j * kTile];
+      o[j].x += a.x, o[j].y += a.y, o[j].z += a.z, o[j].w += a.w;
+    }
+  }
+  __nv_bfloat16* out = is_dk ? p.dk + int64_t(seq) * p.dk_sb + int64_t(h) * p.dk_sh + int64_t(tok) * p.dk_st
+                             : p.dv + int64_t(seq) * p.dv_sb + int64_t(h) * p.dv_sh + int64_t(tok) * p.dv_st;
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    reinterpret_cast<uint4*>(out)[g0 / 2 + j] =
+        make_uint4(pack_bf16(o[2 * j].x, o[2 * j].y), pack_bf16(o[2 * j].z, o[2 * j].w),
+                   pack_bf16(o[2 * j + 1].x, o[2 * j + 1].y), pack_bf16(o[2 * j + 1].z, o[2 * j + 1].w));
+}
+
 // ----------------------------------------------------------------------------------------
-// Epilogue: dQ = bf16(scale * accumulator), 8 lanes per (token, head) row.
+// Epilogue: dQ = bf16(scale * accumulator), 8 lanes per (token, head) row; dK and dV of cut units.
 // ----------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) attn_bwd_epilogue_kernel(const BwdParams p) {
   pdl_wait();  // the accumulator is complete when the main kernel is
   pdl_launch_dependents();
+  if (int(blockIdx.x) >= p.row_blocks) return bwd_combine(p, blockIdx.x - uint32_t(p.row_blocks));
 #if NB_BWD_L2_HINTS
   const uint64_t drop = l2_policy_evict_first();
 #endif
   const int64_t n_rows = p.total_q * p.heads;
   const int lane8 = threadIdx.x & 7;
   int64_t row = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 3;
-  const int64_t row_step = (int64_t(gridDim.x) * blockDim.x) >> 3;
+  const int64_t row_step = (int64_t(p.row_blocks) * blockDim.x) >> 3;
   for (; row < n_rows; row += row_step) {
     const int64_t t = row / p.heads;
     const int h = int(row - t * p.heads);
@@ -246,14 +293,54 @@ struct BwdWork {
   int k_begin, lk, q_begin, lq;
 };
 
+// Query tile an item starts at. Concurrent CTAs work on the key tiles of one (sequence, head) and
+// all add into the same dQ tiles, so they start at different ones: key tile kt at query tile kt,
+// and where there are more key tiles than query tiles at a tile picked by a multiplicative hash
+// (a multiply-high maps it into [0, n_q) without a division routine).
+__device__ __forceinline__ int bwd_first_tile(int kt, int n_q) {
+  return kt < n_q ? kt : int(__umulhi(uint32_t(kt) * 0x9E3779B9u, uint32_t(n_q)));
+}
+
+// The same where units may be cut between CTAs. The two forms are separate instantiations of the kernel:
+// with the extra fields and the drain warps' second way out in one kernel, calls without cut units took
+// 1.5 % (long sequences) to 7 % (short ones) longer.
+struct BwdCutWork : BwdWork {
+  int jt0, n_qt;  // first query tile of the walk, query tiles of the sequence
+  int part;       // >= 0: the unit is cut; where this CTA's dV and dK go
+};
+__device__ __forceinline__ int bwd_start(const BwdWork& w) { return bwd_first_tile(w.kt, w.n_q); }
+__device__ __forceinline__ int bwd_start(const BwdCutWork& w) { return w.jt0; }
+__device__ __forceinline__ int bwd_tiles(const BwdWork& w) { return w.n_q; }
+__device__ __forceinline__ int bwd_tiles(const BwdCutWork& w) { return w.n_qt; }
+__device__ __forceinline__ int bwd_part(const BwdWork&) { return -1; }
+__device__ __forceinline__ int bwd_part(const BwdCutWork& w) { return w.part; }
+template <bool kCut>
+using BwdWorkOf = std::conditional_t<kCut, BwdCutWork, BwdWork>;
+
 // Unit g of the call; n_q = -1 past the last one. The loader fetches a CTA's units and publishes them to
 // the other roles through a small ring. Dense units all cost the same: CTA c of G takes c, G + c, ...
-// Packed units are taken from the list's counter, most expensive first.
-__device__ __forceinline__ BwdWork bwd_work(const BwdParams& p, uint32_t g) {
-  BwdWork w;
+// Packed units are taken from the list's counter, most expensive first. Where whole dense units would
+// leave CTAs idle, CTA c takes an equal run of (unit, query tile) steps; g then counts the units that run
+// touches, and at most two of them are cut: the one the run starts in and the one it ends in.
+template <bool kCut>
+__device__ __forceinline__ BwdWorkOf<kCut> bwd_work(const BwdParams& p, uint32_t g) {
+  BwdWorkOf<kCut> w;
   w.n_q = -1, w.kt = 0, w.h = 0, w.b = 0, w.bcoord = 0, w.k_begin = 0, w.lk = 0, w.q_begin = 0, w.lq = 0;
-  if (g >= uint32_t(p.n_work)) return w;
-  if (p.cu_q != nullptr) {
+  if constexpr (kCut) {
+    w.jt0 = w.n_qt = 0, w.part = -1;
+    const int s0 = int(bwd_split_start(p, blockIdx.x)), s1 = int(bwd_split_start(p, blockIdx.x + 1));
+    const uint32_t u = p.div_n_qt.quot(uint32_t(s0)) + g;
+    const int first = int(u) * p.n_qt;
+    const int tile0 = g == 0 ? s0 - first : 0;
+    if (first + tile0 >= s1) return w;
+    const int tile1 = min(s1 - first, p.n_qt);
+    if (tile0 > 0 || tile1 < p.n_qt) w.part = 2 * int(blockIdx.x) + (tile0 == 0);
+    w.jt0 = tile0, w.n_q = tile1 - tile0, w.n_qt = p.n_qt;
+    g = u;
+  } else if (g >= uint32_t(p.n_work)) {
+    return w;
+  }
+  if (!kCut && p.cu_q != nullptr) {
     // One 32-byte read tells all about the item (the sequence index `batch` stands for the rows past
     // the last sequence: keys without queries). Unused entries sit at the end of the list.
     const uint32_t idx = p.div_heads.quot(g);
@@ -270,16 +357,12 @@ __device__ __forceinline__ BwdWork bwd_work(const BwdParams& p, uint32_t g) {
     w.h = int(t - uint32_t(w.b) * uint32_t(p.heads));
     w.lk = p.lk, w.lq = p.lq;
   }
-  w.n_q = (w.lq + kTile - 1) / kTile;
+  if constexpr (kCut) {
+    if (w.part < 0) w.jt0 = bwd_first_tile(w.kt, w.n_qt);
+  } else {
+    w.n_q = (w.lq + kTile - 1) / kTile;
+  }
   return w;
-}
-
-// Query tile an item starts at. Concurrent CTAs work on the key tiles of one (sequence, head) and
-// all add into the same dQ tiles, so they start at different ones: key tile kt at query tile kt,
-// and where there are more key tiles than query tiles at a tile picked by a multiplicative hash
-// (a multiply-high maps it into [0, n_q) without a division routine).
-__device__ __forceinline__ int bwd_first_tile(int kt, int n_q) {
-  return kt < n_q ? kt : int(__umulhi(uint32_t(kt) * 0x9E3779B9u, uint32_t(n_q)));
 }
 
 // Running position of a role in the CTA's stream of steps: step count, Q/dO stage and the phase of
@@ -447,6 +530,7 @@ __device__ __noinline__ void bwd_compute_role(const uint32_t bar0, int* abort_fl
   }
 }
 
+template <bool kCut>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
@@ -455,7 +539,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __shared__ __align__(8) uint64_t bars[kBwdNumBars];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
-  __shared__ BwdWork work_ring[kBwdWorkSlots];
+  __shared__ BwdWorkOf<kCut> work_ring[kBwdWorkSlots];
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -515,12 +599,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   constexpr uint32_t kIdescSH = make_idesc(128, 64, 0, 0);   // K-major x K-major, N = 64
   constexpr uint32_t kIdescKN = make_idesc(128, 64, 0, 1);   // A K-major / tensor memory, B MN-major
   constexpr uint32_t kIdescNN = make_idesc(128, 64, 1, 1);   // A MN-major, B MN-major
-  const bool packed = p.cu_q != nullptr;
+  const bool packed = !kCut && p.cu_q != nullptr;
 
   // The CTA's unit number `round`, read by a whole warp from the loader's ring.
   auto next_work = [&](uint32_t round) {
     const uint32_t slot = round % kBwdWorkSlots;
-    BwdWork w;
+    BwdWorkOf<kCut> w;
     w.n_q = -1;
     if (mbar_wait(bar(kBarWorkFull + slot), (round / kBwdWorkSlots) & 1, &abort_flag, p.status)) w = work_ring[slot];
     __syncwarp();
@@ -537,24 +621,25 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       if (lane == 0) {
         BwdStepPos pos;
         uint32_t ni = 0;  // items with queries so far
-        uint32_t g = packed ? sched_next(p.items) : blockIdx.x;
+        uint32_t g = packed ? sched_next(p.items) : kCut ? 0u : blockIdx.x;
 #pragma unroll 1
         for (uint32_t round = 0;; ++round) {
-          const BwdWork wk = bwd_work(p, g);
+          const BwdWorkOf<kCut> wk = bwd_work<kCut>(p, g);
           const uint32_t slot = round % kBwdWorkSlots;
           if (round >= uint32_t(kBwdWorkSlots))
             mbar_wait(bar(kBarWorkEmpty + slot), ((round / kBwdWorkSlots) - 1) & 1, &abort_flag, p.status);
           work_ring[slot] = wk;
           mbar_arrive(bar(kBarWorkFull + slot));
           if (wk.n_q < 0) break;
-          g = packed ? sched_next(p.items) : g + gridDim.x;  // in flight during this unit's loads
+          // (The counter's answer is in flight during this unit's loads.)
+          g = packed ? sched_next(p.items) : kCut ? g + 1 : g + gridDim.x;
           if (wk.n_q == 0) continue;
           const uint32_t kb = ni & 1u;
           const int krow = wk.k_begin + wk.kt * kTile;
           if (ni >= 2) mbar_wait(bar(kBarKFree + kb), ((ni >> 1) - 1) & 1, &abort_flag, p.status);
           mbar_arrive_expect_tx(bar(kBarKFull + kb), kTileBytes);
           tma_load_4d(sK(kb), &tmap_k, bar(kBarKFull + kb), 0, krow, wk.h, wk.bcoord);
-          int jt = bwd_first_tile(wk.kt, wk.n_q);
+          int jt = bwd_start(wk);
 #pragma unroll 1
           for (int j = 0; j < wk.n_q; ++j) {
             if (pos.s >= uint32_t(kBwdStages))
@@ -569,7 +654,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
               tma_load_4d(sV, &tmap_v, bar(kBarVFull), 0, krow, wk.h, wk.bcoord);
             }
             pos.advance();
-            jt = jt + 1 == wk.n_q ? 0 : jt + 1;
+            jt = jt + 1 == bwd_tiles(wk) ? 0 : jt + 1;
           }
           ++ni;
         }
@@ -587,13 +672,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       uint32_t ni = 0;
 #pragma unroll 1
       for (uint32_t round = 0;; ++round) {
-        const BwdWork wk = next_work(round);
+        const BwdWorkOf<kCut> wk = next_work(round);
         if (wk.n_q < 0) break;
         if (wk.n_q == 0) continue;
         const int rows_live = min(wk.lk - wk.kt * kTile, kTile);
         const int64_t stat_base =
             packed ? int64_t(wk.h) * p.total_q + wk.q_begin : (int64_t(wk.b) * p.heads + wk.h) * p.lq;
-        int jt = bwd_first_tile(wk.kt, wk.n_q);
+        int jt = bwd_start(wk);
 #pragma unroll 1
         for (int j = 0; j < wk.n_q; ++j) {
           float l2[4], dl[4];
@@ -623,7 +708,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           __syncwarp();
           if (lane == 0) mbar_arrive(bar(kBarQdoFull + pos.qs));
           pos.advance();
-          jt = jt + 1 == wk.n_q ? 0 : jt + 1;
+          jt = jt + 1 == bwd_tiles(wk) ? 0 : jt + 1;
         }
         ++ni;
       }
@@ -657,7 +742,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #endif
 #pragma unroll 1
     for (uint32_t round = 0;; ++round) {
-      const BwdWork wk = next_work(round);
+      const BwdWorkOf<kCut> wk = next_work(round);
       const int n_q = wk.n_q;
       if (n_q < 0) break;
       const int h = wk.h;
@@ -676,8 +761,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
         continue;
       }
-      int row = (packed ? 0 : wk.b * p.lq) + wk.q_begin + quad * 32 + bwd_first_tile(wk.kt, n_q) * kTile;
-      const int row_end = (packed ? 0 : wk.b * p.lq) + wk.q_begin + quad * 32 + n_q * kTile;
+      const int n_qt = bwd_tiles(wk), part = bwd_part(wk);
+      int row = (packed ? 0 : wk.b * p.lq) + wk.q_begin + quad * 32 + bwd_start(wk) * kTile;
+      const int row_end = (packed ? 0 : wk.b * p.lq) + wk.q_begin + quad * 32 + n_qt * kTile;
       // Events of an item, in order: the dQ tiles of steps 0 .. n_q-2, dV, the last dQ tile, dK.
 #pragma unroll 1
       for (int e = 0; e < n_q + 2; ++e) {
@@ -691,6 +777,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           // and the accumulator is handed back at once. The rows then go out 32 columns at a time
           // through a 2 KB scratch area, four lanes per 64-byte half row (a row per lane straight
           // from the registers was measured slower: 32 separate lines per store instruction).
+          if (kCut && part >= 0) {
+            // A cut unit: the fp32 rows go to the workspace (the layout bwd_combine reads).
+            float4* dst = reinterpret_cast<float4*>(p.parts + int64_t(part) * kBwdPartFloats) +
+                          (is_dk ? 16 * kTile : 0) + quad * 32 + lane;
+#pragma unroll 1
+            for (int q4 = 0; q4 < 4; ++q4) {
+              uint32_t r[16];
+              tmem_ld16(tm_acc + 16 * q4, r);
+              tmem_wait_ld();
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                dst[(4 * q4 + i) * kTile] =
+                    make_float4(__uint_as_float(r[4 * i]) * out_scale, __uint_as_float(r[4 * i + 1]) * out_scale,
+                                __uint_as_float(r[4 * i + 2]) * out_scale, __uint_as_float(r[4 * i + 3]) * out_scale);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(is_dk ? kBarDkOut : kBarDvOut));
+            continue;
+          }
           uint32_t pk[32];
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
@@ -760,7 +866,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
         ++s;
         row += kTile;
-        if (row == row_end) row -= n_q * kTile;
+        if (row == row_end) row -= n_qt * kTile;
       }
       ++ni;
     }

@@ -85,7 +85,9 @@ int ensure_device_ready() {
     rc = NB_ATTN_ERR_DEVICE;
   } else if (cudaFuncSetAttribute(nb::attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   nb::kFwdSmemBytes) != cudaSuccess ||
-             cudaFuncSetAttribute(nb::attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+             cudaFuncSetAttribute(nb::attn_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  nb::kBwdSmemBytes) != cudaSuccess ||
+             cudaFuncSetAttribute(nb::attn_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   nb::kBwdSmemBytes) != cudaSuccess ||
              cudaFuncSetAttribute(nb::mma_selftest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   nb::kSelftestSmemBytes) != cudaSuccess) {
@@ -268,6 +270,28 @@ FwdSplit fwd_split(const nb_attn_shape& s) {
   return r;
 }
 
+// The same question for a dense backward (units are key tiles, steps are query tiles, one CTA per SM).
+// Whole units take ceil(units / SMs) x tiles steps; cut ones an equal share plus about three steps' time
+// for the parts. At least a twelfth has to be gained, and a CTA gets at least two steps.
+struct BwdSplit {
+  unsigned ctas = 0;
+  size_t parts_offset = 0, bytes = 0;  // of the whole workspace
+};
+BwdSplit bwd_split(const nb_attn_shape& s) {
+  BwdSplit r;
+  if (s.cu_seqlens_q != nullptr) return r;
+  const int64_t n_qt = ceil_div(s.max_seqlen_q, nb::kTile);
+  const int64_t units = int64_t(ceil_div(s.max_seqlen_k, nb::kTile)) * s.heads * s.batch;
+  const int64_t sms = device_sm_count(), steps = units * n_qt;
+  const int64_t ctas = steps / 2 < sms ? steps / 2 : sms;
+  if (ctas < 2 || steps > INT32_MAX) return r;
+  if ((units + sms - 1) / sms * n_qt * 12 <= 13 * ((steps + ctas - 1) / ctas + 3)) return r;
+  r.ctas = unsigned(ctas);
+  r.parts_offset = align_up(bwd_accum_bytes(s) + bwd_delta_bytes(s), 256);
+  r.bytes = r.parts_offset + 2 * size_t(ctas) * nb::kBwdPartFloats * sizeof(float);
+  return r;
+}
+
 // Everything about a backward call that can be checked without touching CUDA.
 int validate_bwd(const nb_attn_bwd_args* a) {
   if (a == nullptr) return NB_ATTN_ERR_NULL;
@@ -333,10 +357,20 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
   // (key tiles x heads x sequences, or work-list entries x heads).
   int64_t n_work = 0;
   p.n_kt = ceil_div(s.max_seqlen_k, nb::kTile);
+  p.n_qt = ceil_div(s.max_seqlen_q, nb::kTile);
+  p.parts = nullptr;
+  unsigned ctas = unsigned(device_sm_count());
   if (dense) {
     p.items = nullptr;
     p.sched = nb::SchedParams{};
     n_work = int64_t(p.n_kt) * s.heads * s.batch;
+    const BwdSplit split = bwd_split(s);
+    if (split.ctas > 0 && workspace_bytes >= split.bytes) {
+      const uint32_t steps = uint32_t(n_work * p.n_qt);
+      p.parts = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + split.parts_offset);
+      ctas = split.ctas;
+      p.split_base = steps / ctas, p.split_extra = steps % ctas;
+    }
   } else {
     // Block 0 of the prologue builds the list of key tiles; the main kernel runs items x heads CTAs.
     const int64_t n_items = nb::sched_capacity(s.total_k, s.batch);
@@ -350,19 +384,21 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
   p.n_work = int32_t(n_work);
   p.div_heads = nb::make_fast_div(uint32_t(s.heads));
   p.div_n_kt = nb::make_fast_div(uint32_t(p.n_kt));
-  const int sms = device_sm_count();
-  const dim3 grid(unsigned(n_work < sms ? n_work : sms), 1, 1);
+  p.div_n_qt = nb::make_fast_div(uint32_t(p.n_qt));
+  const dim3 grid(p.parts == nullptr && n_work < int64_t(ctas) ? unsigned(n_work) : ctas, 1, 1);
 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t rows = s.total_q * s.heads;
   const int64_t want_blocks = (rows * 8 + 255) / 256;
   const int aux_blocks = int(want_blocks < 148 * 16 ? want_blocks : 148 * 16);
+  p.row_blocks = aux_blocks;
+  const int combine_blocks = p.parts != nullptr ? 4 * (int(ctas) - 1) : 0;
   bool ok = launch(nb::attn_bwd_prologue_kernel, dim3(aux_blocks), dim3(256), 0, st, p) == cudaSuccess;
   if (a->event_main_begin) cudaEventRecord(static_cast<cudaEvent_t>(a->event_main_begin), st);
-  ok = ok && launch(nb::attn_bwd_kernel, grid, dim3(nb::kBwdThreads), nb::kBwdSmemBytes, st, tq, tk, tv, tg, tdq, p) ==
+  ok = ok && launch(p.parts != nullptr ? nb::attn_bwd_kernel<true> : nb::attn_bwd_kernel<false>, grid, dim3(nb::kBwdThreads), nb::kBwdSmemBytes, st, tq, tk, tv, tg, tdq, p) ==
                  cudaSuccess;
   if (a->event_main_end) cudaEventRecord(static_cast<cudaEvent_t>(a->event_main_end), st);
-  ok = ok && launch(nb::attn_bwd_epilogue_kernel, dim3(aux_blocks), dim3(256), 0, st, p) == cudaSuccess;
+  ok = ok && launch(nb::attn_bwd_epilogue_kernel, dim3(aux_blocks + combine_blocks), dim3(256), 0, st, p) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();  // leave no sticky "last error" behind for the caller's own checks
     return NB_ATTN_ERR_LAUNCH;
@@ -398,6 +434,11 @@ size_t nb_attn_bwd_workspace_bytes(const nb_attn_shape* shape) {
   const nb_attn_shape& s = *shape;
   if (s.cu_seqlens_q == nullptr) return bwd_accum_bytes(s) + bwd_delta_bytes(s);
   return bwd_items_offset(s) + size_t(nb::sched_capacity(s.total_k, s.batch)) * sizeof(nb::SchedItem);
+}
+
+size_t nb_attn_bwd_split_workspace_bytes(const nb_attn_shape* shape) {
+  if (shape == nullptr || check_shape(*shape) != NB_ATTN_OK || ensure_device_ready() != NB_ATTN_OK) return 0;
+  return bwd_split(*shape).bytes;
 }
 
 size_t nb_attn_fwd_workspace_bytes(const nb_attn_shape* shape) {

@@ -207,7 +207,8 @@ void launch_bwd(nb_attn_bwd_args& a, const Tensor& q, const Tensor& lse) {
   raise_for_status(word);
   a.lse = lse.data_ptr<float>();
   a.status = const_cast<int32_t*>(word);
-  a.workspace_bytes = nb_attn_bwd_workspace_bytes(&a.shape);
+  a.workspace_bytes =
+      std::max(nb_attn_bwd_workspace_bytes(&a.shape), nb_attn_bwd_split_workspace_bytes(&a.shape));
   Tensor workspace = at::empty({int64_t(a.workspace_bytes)}, q.options().dtype(at::kByte));
   a.workspace = workspace.data_ptr();
   check_rc(nb_attn_bwd(&a, at::cuda::getCurrentCUDAStream().stream()), "nb_attn_bwd");

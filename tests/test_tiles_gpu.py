@@ -73,3 +73,20 @@ def test_query_tiles_cut_between_ctas(batch, heads, lq, lk, rising):
         ops.check_status()
         check(("out",), (out,), (want,))
         np.testing.assert_allclose(got_lse.cpu().numpy(), lse, rtol=2e-3, atol=2e-3)
+
+
+@pytest.mark.parametrize("batch,heads,lq,lk", [
+    (1, 1, 600, 130), (1, 1, 1000, 1), (2, 1, 1537, 300), (1, 2, 4096, 64), (1, 12, 900, 1500), (2, 12, 820, 820),
+])
+def test_key_tiles_cut_between_ctas(batch, heads, lq, lk):
+    # Few key tiles and many queries: the dense backward gives every CTA an equal run of query tiles and
+    # the epilogue adds up the parts of a key tile's dK and dV.
+    g = torch.Generator().manual_seed(lq + lk)
+    q, d_out = (torch.randn(batch, heads, lq, 64, generator=g).to(torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(batch, heads, lk, 64, generator=g).to(torch.bfloat16) for _ in range(2))
+    want = O.sdpa_fwd_bwd(*(t.float().numpy() for t in (q, k, v, d_out)))
+    for _ in range(2):
+        qd, kd, vd = (t.to(DEV).requires_grad_(True) for t in (q, k, v))
+        nanobrain_b200.sdpa(qd, kd, vd).backward(d_out.to(DEV))
+        ops.check_status()
+        check(("dq", "dk", "dv"), (qd.grad, kd.grad, vd.grad), want[2:5])
