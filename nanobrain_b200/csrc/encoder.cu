@@ -10,6 +10,7 @@
 #include <type_traits>
 
 #include "../../include/nb_attn.h"
+#include "ptx.cuh"
 
 namespace {
 
@@ -97,6 +98,22 @@ struct Row {
       }
   }
 };
+
+// Launch with programmatic stream serialization: the kernel's blocks may be resident while its
+// predecessor drains; every kernel launched this way begins with griddepcontrol.wait.
+template <typename... KArgs, typename... Args>
+void launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, void* stream, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
 
 // f(integral_constant<kChunks>) for the smallest kChunks that holds a row of `dim` values.
 template <typename F>
@@ -251,6 +268,8 @@ __global__ void __launch_bounds__(kThreads)
 template <int kChunks>
 __global__ void __launch_bounds__(kThreads)
     add_norm_kernel(float* x, const __nv_bfloat16* add, int64_t rows, int dim, nb_enc_norm norm, __nv_bfloat16* y) {
+  nb::pdl_wait();
+  nb::pdl_launch_dependents();
   const int64_t row = int64_t(blockIdx.x) * kWarps + (threadIdx.x >> 5);
   if (row >= rows) return;
   Row<kChunks> r;
@@ -261,17 +280,43 @@ __global__ void __launch_bounds__(kThreads)
   r.store(y + row * dim, dim);
 }
 
-__device__ __forceinline__ float gelu(float v) { return 0.5f * v * (1.f + erff(v * 0.70710678118654752f)); }
+// v * Phi(v) of two bf16 values, Phi the normal distribution function, by Abramowitz and Stegun's 7.1.26:
+// erfc(z) = (a1 t + ... + a5 t^5) exp(-z^2) with t = 1 / (1 + 0.3275911 z), z >= 0, absolute error
+// 1.5e-7. With z = |v| / sqrt(2), v Phi(v) = max(v, 0) - (z / sqrt(2)) erfc(z): the tail keeps its own
+// relative accuracy because nothing is taken from 1. The kernel is bound by its instructions: 14 000 x
+// 3072 values took 47 us with erff, 40 us with this formula one value at a time, 33 us on packed pairs
+// (26 us of memory traffic).
+__device__ __forceinline__ uint32_t gelu2(uint32_t v) {
+  auto both = [](float c) { return nb::pack_f32x2(c, c); };
+  const uint32_t mag = __vminu2(v & 0x7fff7fffu, 0x7f7f7f7fu);  // infinities as the largest finite value
+  const uint64_t z = nb::mul_f32x2(nb::pack_f32x2(__uint_as_float(mag << 16), __uint_as_float(mag & 0xffff0000u)),
+                                   both(0.70710678118654752f));
+  float d0, d1;
+  nb::unpack_f32x2(nb::fma_f32x2(z, both(0.3275911f), both(1.f)), d0, d1);
+  const uint64_t t = nb::pack_f32x2(__fdividef(1.f, d0), __fdividef(1.f, d1));
+  // The coefficients times -1 / sqrt(2).
+  uint64_t poly = nb::fma_f32x2(t, both(-0.75054333f), both(1.02753367f));
+  poly = nb::fma_f32x2(poly, t, both(-1.00509670f));
+  poly = nb::fma_f32x2(poly, t, both(0.20116957f));
+  poly = nb::fma_f32x2(poly, t, both(-0.18018894f));
+  float e0, e1;
+  nb::unpack_f32x2(nb::mul_f32x2(z, nb::mul_f32x2(z, both(-1.4426950408889634f))), e0, e1);
+  const uint64_t scaled = nb::mul_f32x2(nb::mul_f32x2(z, t), nb::pack_f32x2(nb::fast_exp2(e0), nb::fast_exp2(e1)));
+  const __nv_bfloat162 hv = *reinterpret_cast<const __nv_bfloat162*>(&v);
+  const float2 pos = __bfloat1622float2(__hmax2_nan(hv, __floats2bfloat162_rn(0.f, 0.f)));
+  float r0, r1;
+  nb::unpack_f32x2(nb::fma_f32x2(poly, scaled, nb::pack_f32x2(pos.x, pos.y)), r0, r1);
+  return pack2(r0, r1);
+}
 __global__ void __launch_bounds__(256) gelu_kernel(__nv_bfloat16* v, int64_t n) {
+  nb::pdl_wait();
+  nb::pdl_launch_dependents();
   const int64_t i = (int64_t(blockIdx.x) * 256 + threadIdx.x) * 8;
   if (i >= n) return;
   uint4 u = *reinterpret_cast<const uint4*>(v + i);
   uint32_t* w = reinterpret_cast<uint32_t*>(&u);
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const float2 f = unpack2(w[k]);
-    w[k] = pack2(gelu(f.x), gelu(f.y));
-  }
+  for (int k = 0; k < 4; ++k) w[k] = gelu2(w[k]);
   *reinterpret_cast<uint4*>(v + i) = u;
 }
 
@@ -326,11 +371,19 @@ __global__ void __launch_bounds__(kThreads)
     __syncthreads();
   }
 }
-__global__ void mean_kernel(const float* partial, int blocks, int dim, const int32_t* counts, int first, float* means) {
+// One block per image and 64 columns: four threads per column share the partial sums.
+__global__ void __launch_bounds__(256) mean_kernel(const float* partial, int blocks, int dim, const int32_t* counts,
+                                                   int first, float* means) {
+  __shared__ float sums[4][64];
   const int64_t image = first + blockIdx.x;
-  for (int d = threadIdx.x; d < dim; d += blockDim.x) {
-    float s = 0.f;
-    for (int b = 0; b < blocks; ++b) s += partial[(int64_t(blockIdx.x) * blocks + b) * dim + d];
+  const int d = blockIdx.y * 64 + (threadIdx.x & 63), part = threadIdx.x >> 6;
+  float s = 0.f;
+#pragma unroll 8
+  for (int b = part; b < blocks; b += 4) s += partial[(int64_t(blockIdx.x) * blocks + b) * dim + d];
+  sums[part][threadIdx.x & 63] = s;
+  __syncthreads();
+  if (part == 0) {
+    s = (sums[0][threadIdx.x] + sums[1][threadIdx.x]) + (sums[2][threadIdx.x] + sums[3][threadIdx.x]);
     means[image * dim + d] = s / float(counts[image] > 1 ? counts[image] : 1);
   }
 }
@@ -416,8 +469,8 @@ int nb_enc_add_norm(float* x, const void* add, int64_t rows, int dim, const nb_e
   if (x == nullptr || add == nullptr || norm == nullptr || y == nullptr) return NB_ATTN_ERR_NULL;
   if (!dim_ok(dim) || rows <= 0) return NB_ATTN_ERR_SHAPE;
   return with_chunks(dim, [&](auto c) {
-    add_norm_kernel<decltype(c)::value><<<row_blocks(rows), kThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        x, static_cast<const __nv_bfloat16*>(add), rows, dim, *norm, static_cast<__nv_bfloat16*>(y));
+    launch(add_norm_kernel<decltype(c)::value>, dim3(row_blocks(rows)), dim3(kThreads), stream, x,
+           static_cast<const __nv_bfloat16*>(add), rows, dim, *norm, static_cast<__nv_bfloat16*>(y));
   });
 }
 
@@ -425,8 +478,7 @@ int nb_enc_gelu(void* v, int64_t n, void* stream) {
   if (v == nullptr) return NB_ATTN_ERR_NULL;
   if (!aligned16(v)) return NB_ATTN_ERR_ALIGN;
   if (n <= 0 || n % 8 != 0) return NB_ATTN_ERR_SHAPE;
-  gelu_kernel<<<unsigned((n / 8 + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<__nv_bfloat16*>(v), n);
+  launch(gelu_kernel, dim3(unsigned((n / 8 + 255) / 256)), dim3(256), stream, static_cast<__nv_bfloat16*>(v), n);
   return launched();
 }
 
@@ -453,7 +505,7 @@ int nb_enc_finish(const float* x, const void* add, const int32_t* rank, const in
         x, static_cast<const __nv_bfloat16*>(add), rank, cu_r, first, patches, class_tokens, dim, *norm, t, partial);
   });
   if (rc) return rc;
-  mean_kernel<<<n, 256, 0, st>>>(partial, blocks, dim, counts, first, means);
+  mean_kernel<<<dim3(n, dim / 64), 256, 0, st>>>(partial, blocks, dim, counts, first, means);
   return launched();
 }
 
