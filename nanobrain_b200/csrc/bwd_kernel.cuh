@@ -631,14 +631,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           work_ring[slot] = wk;
           mbar_arrive(bar(kBarWorkFull + slot));
           if (wk.n_q < 0) break;
-          // (The counter's answer is in flight during this unit's loads.)
-          g = packed ? sched_next(p.items) : kCut ? g + 1 : g + gridDim.x;
-          if (wk.n_q == 0) continue;
           const uint32_t kb = ni & 1u;
           const int krow = wk.k_begin + wk.kt * kTile;
-          if (ni >= 2) mbar_wait(bar(kBarKFree + kb), ((ni >> 1) - 1) & 1, &abort_flag, p.status);
-          mbar_arrive_expect_tx(bar(kBarKFull + kb), kTileBytes);
-          tma_load_4d(sK(kb), &tmap_k, bar(kBarKFull + kb), 0, krow, wk.h, wk.bcoord);
+          if (wk.n_q > 0) {
+            if (ni >= 2) mbar_wait(bar(kBarKFree + kb), ((ni >> 1) - 1) & 1, &abort_flag, p.status);
+            mbar_arrive_expect_tx(bar(kBarKFull + kb), kTileBytes);
+            tma_load_4d(sK(kb), &tmap_k, bar(kBarKFull + kb), 0, krow, wk.h, wk.bcoord);
+          }
           int jt = bwd_start(wk);
 #pragma unroll 1
           for (int j = 0; j < wk.n_q; ++j) {
@@ -656,7 +655,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             pos.advance();
             jt = jt + 1 == bwd_tiles(wk) ? 0 : jt + 1;
           }
-          ++ni;
+          if (wk.n_q > 0) ++ni;
+          // The next unit is taken as late as can be: this thread is about three steps ahead of the MMAs,
+          // which covers the counter's and the list's latency, and a unit taken earlier would wait behind a
+          // long one while other CTAs run dry.
+          g = packed ? sched_next(p.items) : kCut ? g + 1 : g + gridDim.x;
         }
         // One more stage carries the stop mark (no data).
         if (pos.s >= uint32_t(kBwdStages)) mbar_wait(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u, &abort_flag, p.status);
