@@ -41,7 +41,7 @@ NOMINAL_BF16_TFLOPS = 2250.0
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
 # dram__bytes_read.sum + dram__bytes_write.sum of one attn_bwd_kernel launch, from an ncu capture of
 # this workload (only known for that workload; not measured by the run itself).
-NCU_DRAM_BYTES_BWD_MAIN = {"vitb_encoder_varlen": 600.6e6}
+NCU_DRAM_BYTES_BWD_MAIN = {"vitb_encoder_varlen": 510.6e6}
 
 
 def parse_args():

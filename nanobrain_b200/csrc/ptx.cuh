@@ -158,16 +158,6 @@ __device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
   return ok != 0;
 }
 
-// The same wait for a single thread on a latency-critical path: it polls without being suspended for
-// a while first (a suspended thread wakes about 250 cycles after its barrier completes).
-__device__ __forceinline__ bool mbar_spin_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                               int* status_word) {
-#pragma unroll 1
-  for (int i = 0; i < 64; ++i)
-    if (mbar_test_wait(bar, parity)) return true;
-  return mbar_wait(bar, parity, abort_flag, status_word);
-}
-
 // ----------------------------------------------------------------------------------------
 // TMA: tiled 4-D load global -> shared, completion on an mbarrier (CTA-local).
 // ----------------------------------------------------------------------------------------
