@@ -112,6 +112,11 @@ typedef struct nb_attn_fwd_args {
 
 int nb_attn_fwd(const nb_attn_fwd_args* args, void* stream);
 
+/* The same for further calls with the shape, cu_seqlens and `workspace` of an nb_attn_fwd call that comes
+ * before it in the order of `stream` (the layers of a network): the work list in `workspace` is used again
+ * instead of built again. Calls that share a workspace must not run at the same time. */
+int nb_attn_fwd_again(const nb_attn_fwd_args* args, void* stream);
+
 /* Scratch bytes nb_attn_fwd needs: the work list of query tiles in varlen mode, 0 in dense mode. */
 size_t nb_attn_fwd_workspace_bytes(const nb_attn_shape* shape);
 

@@ -15,6 +15,7 @@ ABI_VERSION = 2
 # Every symbol include/nb_attn.h declares.
 EXPORTED_SYMBOLS = (
     "nb_attn_fwd",
+    "nb_attn_fwd_again",
     "nb_attn_bwd",
     "nb_attn_bwd_workspace_bytes",
     "nb_attn_strerror",
@@ -135,8 +136,9 @@ def load() -> C.CDLL:
     lib.nb_attn_schedule_host.restype = C.c_int
     lib.nb_attn_schedule_host.argtypes = [C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int64,
                                           C.c_int64, C.c_int, C.c_void_p, C.c_int64]
-    lib.nb_attn_fwd.restype = C.c_int
-    lib.nb_attn_fwd.argtypes = [C.POINTER(FwdArgs), C.c_void_p]
+    for fn in (lib.nb_attn_fwd, lib.nb_attn_fwd_again):
+        fn.restype = C.c_int
+        fn.argtypes = [C.POINTER(FwdArgs), C.c_void_p]
     lib.nb_attn_bwd.restype = C.c_int
     lib.nb_attn_bwd.argtypes = [C.POINTER(BwdArgs), C.c_void_p]
     lib.nb_attn_bwd_builtin_scratch.restype = C.c_int

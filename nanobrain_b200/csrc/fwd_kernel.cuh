@@ -360,6 +360,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       units[u & 1u].lk = -1;
       mbar_arrive(bar(kFwdQFull + (u & 1u)));
+      if (packed) sched_leave(p.items, gridDim.x);
     }
   } else if (warp == 4) {
     // ---------------- MMA issuer ----------------

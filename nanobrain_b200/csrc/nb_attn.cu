@@ -406,52 +406,8 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
   return cudaGetLastError() == cudaSuccess ? NB_ATTN_OK : NB_ATTN_ERR_LAUNCH;
 }
 
-}  // namespace
-
-extern "C" {
-
-int nb_attn_abi_version(void) { return NB_ATTN_ABI_VERSION; }
-
-const char* nb_attn_strerror(int code) {
-  switch (code) {
-    case NB_ATTN_OK: return "ok";
-    case NB_ATTN_ERR_NULL: return "a required pointer is NULL";
-    case NB_ATTN_ERR_HEAD_DIM: return "head_dim must be 64";
-    case NB_ATTN_ERR_SHAPE: return "invalid or inconsistent sizes";
-    case NB_ATTN_ERR_ALIGN: return "pointers must be 16-byte aligned and strides positive multiples of 8 elements";
-    case NB_ATTN_ERR_WORKSPACE: return "workspace missing, misaligned or too small";
-    case NB_ATTN_ERR_TENSOR_MAP: return "could not encode a TMA tensor map";
-    case NB_ATTN_ERR_LAUNCH: return "a CUDA runtime call failed";
-    case NB_ATTN_ERR_DEVICE: return "the current device is not an sm_100 GPU";
-    case NB_ATTN_ERR_TOO_LARGE:
-      return "total_q * heads exceeds NB_ATTN_BUILTIN_SCRATCH_ROWS; use nb_attn_bwd with a caller workspace";
-    default: return "unknown error code";
-  }
-}
-
-size_t nb_attn_bwd_workspace_bytes(const nb_attn_shape* shape) {
-  if (shape == nullptr || check_shape(*shape) != NB_ATTN_OK) return 0;
-  const nb_attn_shape& s = *shape;
-  if (s.cu_seqlens_q == nullptr) return bwd_accum_bytes(s) + bwd_delta_bytes(s);
-  return bwd_items_offset(s) + size_t(nb::sched_capacity(s.total_k, s.batch)) * sizeof(nb::SchedItem);
-}
-
-size_t nb_attn_bwd_split_workspace_bytes(const nb_attn_shape* shape) {
-  if (shape == nullptr || check_shape(*shape) != NB_ATTN_OK || ensure_device_ready() != NB_ATTN_OK) return 0;
-  return bwd_split(*shape).bytes;
-}
-
-size_t nb_attn_fwd_workspace_bytes(const nb_attn_shape* shape) {
-  if (shape == nullptr || check_shape(*shape) != NB_ATTN_OK || shape->cu_seqlens_q == nullptr) return 0;
-  return size_t(nb::sched_capacity(shape->total_q, shape->batch)) * sizeof(nb::SchedItem);
-}
-
-size_t nb_attn_fwd_split_workspace_bytes(const nb_attn_shape* shape) {
-  if (shape == nullptr || check_shape(*shape) != NB_ATTN_OK || ensure_device_ready() != NB_ATTN_OK) return 0;
-  return fwd_split(*shape).bytes;
-}
-
-int nb_attn_fwd(const nb_attn_fwd_args* a, void* stream) {
+// `listed`: the workspace holds the list of an earlier call.
+int run_fwd(const nb_attn_fwd_args* a, bool listed, void* stream) {
   if (a == nullptr) return NB_ATTN_ERR_NULL;
   int rc = check_shape(a->shape);
   if (rc) return rc;
@@ -510,9 +466,11 @@ int nb_attn_fwd(const nb_attn_fwd_args* a, void* stream) {
     // The scheduler's list of query tiles; a unit is an entry and a head.
     const int64_t n_items = nb::sched_capacity(s.total_q, s.batch);
     nb::SchedItem* items = static_cast<nb::SchedItem*>(a->workspace);
-    nb::SchedParams sp = make_sched(s, 0, items, n_items, a->status);
-    sp.merged = 1;
-    ok = launch(nb::attn_sched_kernel, dim3(1), dim3(nb::kSchedThreads), 0, st, sp) == cudaSuccess;
+    if (!listed) {
+      nb::SchedParams sp = make_sched(s, 0, items, n_items, a->status);
+      sp.merged = 1;
+      ok = launch(nb::attn_sched_kernel, dim3(1), dim3(nb::kSchedThreads), 0, st, sp) == cudaSuccess;
+    }
     p.items = items;
     n_units = n_items * s.heads;
   }
@@ -530,6 +488,55 @@ int nb_attn_fwd(const nb_attn_fwd_args* a, void* stream) {
   }
   return cudaGetLastError() == cudaSuccess ? NB_ATTN_OK : NB_ATTN_ERR_LAUNCH;
 }
+
+}  // namespace
+
+extern "C" {
+
+int nb_attn_abi_version(void) { return NB_ATTN_ABI_VERSION; }
+
+const char* nb_attn_strerror(int code) {
+  switch (code) {
+    case NB_ATTN_OK: return "ok";
+    case NB_ATTN_ERR_NULL: return "a required pointer is NULL";
+    case NB_ATTN_ERR_HEAD_DIM: return "head_dim must be 64";
+    case NB_ATTN_ERR_SHAPE: return "invalid or inconsistent sizes";
+    case NB_ATTN_ERR_ALIGN: return "pointers must be 16-byte aligned and strides positive multiples of 8 elements";
+    case NB_ATTN_ERR_WORKSPACE: return "workspace missing, misaligned or too small";
+    case NB_ATTN_ERR_TENSOR_MAP: return "could not encode a TMA tensor map";
+    case NB_ATTN_ERR_LAUNCH: return "a CUDA runtime call failed";
+    case NB_ATTN_ERR_DEVICE: return "the current device is not an sm_100 GPU";
+    case NB_ATTN_ERR_TOO_LARGE:
+      return "total_q * heads exceeds NB_ATTN_BUILTIN_SCRATCH_ROWS; use nb_attn_bwd with a caller workspace";
+    default: return "unknown error code";
+  }
+}
+
+size_t nb_attn_bwd_workspace_bytes(const nb_attn_shape* shape) {
+  if (shape == nullptr || check_shape(*shape) != NB_ATTN_OK) return 0;
+  const nb_attn_shape& s = *shape;
+  if (s.cu_seqlens_q == nullptr) return bwd_accum_bytes(s) + bwd_delta_bytes(s);
+  return bwd_items_offset(s) + size_t(nb::sched_capacity(s.total_k, s.batch)) * sizeof(nb::SchedItem);
+}
+
+size_t nb_attn_bwd_split_workspace_bytes(const nb_attn_shape* shape) {
+  if (shape == nullptr || check_shape(*shape) != NB_ATTN_OK || ensure_device_ready() != NB_ATTN_OK) return 0;
+  return bwd_split(*shape).bytes;
+}
+
+size_t nb_attn_fwd_workspace_bytes(const nb_attn_shape* shape) {
+  if (shape == nullptr || check_shape(*shape) != NB_ATTN_OK || shape->cu_seqlens_q == nullptr) return 0;
+  return size_t(nb::sched_capacity(shape->total_q, shape->batch)) * sizeof(nb::SchedItem);
+}
+
+size_t nb_attn_fwd_split_workspace_bytes(const nb_attn_shape* shape) {
+  if (shape == nullptr || check_shape(*shape) != NB_ATTN_OK || ensure_device_ready() != NB_ATTN_OK) return 0;
+  return fwd_split(*shape).bytes;
+}
+
+int nb_attn_fwd(const nb_attn_fwd_args* a, void* stream) { return run_fwd(a, false, stream); }
+
+int nb_attn_fwd_again(const nb_attn_fwd_args* a, void* stream) { return run_fwd(a, true, stream); }
 
 int nb_attn_bwd(const nb_attn_bwd_args* a, void* stream) {
   int rc = validate_bwd(a);

@@ -47,7 +47,7 @@ struct __align__(16) SchedItem {
   int32_t own_len;      // its length there
   int32_t other_begin;  // the same on the side the item's inner loop walks
   int32_t other_len;
-  int32_t reserved[2];  // zero in a new list; the first entry's first word counts the units taken
+  int32_t reserved[2];  // zero in a new list; the first entry's count the units taken and the CTAs done
 };
 static_assert(sizeof(SchedItem) == 32, "two 16-byte loads");
 
@@ -64,6 +64,12 @@ __device__ __forceinline__ SchedItem sched_load(const SchedItem* items, uint32_t
 // Takes the next unit of a list.
 __device__ __forceinline__ uint32_t sched_next(const SchedItem* items) {
   return uint32_t(atomicAdd(const_cast<int32_t*>(&items[0].reserved[0]), 1));
+}
+
+// A CTA takes no more units. The last of `ctas` leaves the list as it was when new, for the next launch.
+__device__ __forceinline__ void sched_leave(const SchedItem* items, uint32_t ctas) {
+  int32_t* words = const_cast<int32_t*>(items[0].reserved);
+  if (uint32_t(atomicAdd(words + 1, 1)) == ctas - 1) words[0] = words[1] = 0;
 }
 
 constexpr int kSchedThreads = 1024;

@@ -363,9 +363,8 @@ class ViTMAE3D(nn.Module):
         pos = self.pos_embed
         head = [self.patch_embed.weight, self.patch_embed.bias, wx, pos.weight_y, pos.weight_z, self.cls_token,
                 self.norm.weight, self.norm.bias]
-        for t in head + blocks:
-            if t is not None and (t.dtype != torch.float32 or t.device != wx.device or not t.is_contiguous()):
-                return None
+        if not ops._load_native().plain_params(head + blocks, wx):
+            return None
         patches_per_image = self.coord_grid.shape[1]
         for pt, m in samples:
             if (pt.dtype != torch.float32 or m.dtype != torch.bool or tuple(pt.shape) != (patches_per_image, patch_dim)

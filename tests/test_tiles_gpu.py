@@ -1,12 +1,14 @@
 """The kernels at the edges of their tiles: key and query counts around the 64-column halves and the
 128-row tiles the main kernels work in, one and several of them, against the CPU oracle."""
 
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
 import nanobrain_b200
-from nanobrain_b200 import ops
+from nanobrain_b200 import _lib, ops
 from oracle import attn_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -90,3 +92,24 @@ def test_key_tiles_cut_between_ctas(batch, heads, lq, lk):
         nanobrain_b200.sdpa(qd, kd, vd).backward(d_out.to(DEV))
         ops.check_status()
         check(("dq", "dk", "dv"), (qd.grad, kd.grad, vd.grad), want[2:5])
+
+
+@pytest.mark.parametrize("lengths,heads", [([1], 1), ([130, 0, 64], 2), ([300] * 40 + [2000], 12)])
+def test_work_list_used_again(lengths, heads):
+    # Fewer units than CTAs, and more: every launch over one list does all of its units.
+    total = sum(lengths) + 70  # rows past the last sequence come out as zeros each time
+    g = torch.Generator().manual_seed(total)
+    q, k, v = (torch.randn(total, heads, 64, generator=g).to(DEV, torch.bfloat16) for _ in range(3))
+    cu = torch.tensor([0] + lengths).cumsum(0).to(DEV, torch.int32)
+    want, _ = ops.sdpa_varlen_fwd(q, k, v, cu, cu, max(lengths), max(lengths), 0.125)
+    lib, lse = _lib.load(), torch.empty(heads, total, device=DEV)
+    desc = lambda t: _lib.Tensor(t.data_ptr(), 0, t.stride(0), t.stride(1))
+    shape = _lib.Shape(len(lengths), heads, 64, max(lengths), max(lengths), total, total, cu.data_ptr(), cu.data_ptr(),
+                       0.125)
+    ws = torch.empty(_lib.fwd_workspace_bytes(shape), dtype=torch.uint8, device=DEV)
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for call in (lib.nb_attn_fwd, lib.nb_attn_fwd_again, lib.nb_attn_fwd_again):
+        out = torch.full_like(q, float("nan"))
+        args = _lib.FwdArgs(shape, desc(q), desc(k), desc(v), desc(out), lse.data_ptr(), None, ws.data_ptr(), ws.numel())
+        _lib.check(call(C.byref(args), stream), "nb_attn_fwd")
+        assert torch.equal(out, want)
