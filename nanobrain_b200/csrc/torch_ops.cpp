@@ -12,6 +12,7 @@
 #include <ATen/ATen.h>
 #include <ATen/core/dispatch/Dispatcher.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/autograd_not_implemented_fallback.h>
@@ -160,10 +161,16 @@ nb_attn_tensor packed_desc(const Tensor& t) {
   return {t.data_ptr(), 0, n > 1 ? t.stride(0) : h * kHeadDim, h > 1 ? t.stride(1) : kHeadDim};
 }
 
-// Uninitialised logical [B, H, L, 64] in [B, L, H, 64] memory.
+// Uninitialised tensors on the device of `like`, which is current here: from the caching allocator as
+// at::empty's, without its two dispatched calls (seven tensors per forward + backward).
+Tensor new_tensor(at::IntArrayRef sizes, at::ScalarType type, const Tensor& like) {
+  return at::detail::empty_cuda(sizes, type, like.device(), std::nullopt);
+}
+// Logical [B, H, L, 64] in [B, L, H, 64] memory.
 Tensor new_dense(const Tensor& like) {
   const int64_t b = like.size(0), h = like.size(1), l = like.size(2);
-  return at::empty_strided({b, h, l, kHeadDim}, {l * h * kHeadDim, kHeadDim, h * kHeadDim, 1}, like.options());
+  return at::detail::empty_strided_cuda({b, h, l, kHeadDim}, {l * h * kHeadDim, kHeadDim, h * kHeadDim, 1},
+                                        at::kBFloat16, like.device());
 }
 
 nb_attn_shape dense_shape(const Tensor& q, const Tensor& k, double scale) {
@@ -196,7 +203,7 @@ void launch_fwd(nb_attn_fwd_args& a, const Tensor& q, Tensor& workspace) {
   a.workspace_bytes = a.shape.cu_seqlens_q != nullptr ? nb_attn_fwd_workspace_bytes(&a.shape)  // the work list
                                                       : nb_attn_fwd_split_workspace_bytes(&a.shape);
   if (a.workspace_bytes > 0) {
-    workspace = at::empty({int64_t(a.workspace_bytes)}, q.options().dtype(at::kByte));
+    workspace = new_tensor({int64_t(a.workspace_bytes)}, at::kByte, q);
     a.workspace = workspace.data_ptr();
   }
   check_rc(nb_attn_fwd(&a, at::cuda::getCurrentCUDAStream().stream()), "nb_attn_fwd");
@@ -208,9 +215,10 @@ void launch_bwd(nb_attn_bwd_args& a, const Tensor& q, const Tensor& lse) {
   raise_for_status(word);
   a.lse = lse.data_ptr<float>();
   a.status = const_cast<int32_t*>(word);
-  a.workspace_bytes =
-      std::max(nb_attn_bwd_workspace_bytes(&a.shape), nb_attn_bwd_split_workspace_bytes(&a.shape));
-  Tensor workspace = at::empty({int64_t(a.workspace_bytes)}, q.options().dtype(at::kByte));
+  a.workspace_bytes = nb_attn_bwd_workspace_bytes(&a.shape);
+  if (a.shape.cu_seqlens_q == nullptr)  // room to cut units between CTAs
+    a.workspace_bytes = std::max(a.workspace_bytes, nb_attn_bwd_split_workspace_bytes(&a.shape));
+  Tensor workspace = new_tensor({int64_t(a.workspace_bytes)}, at::kByte, q);
   a.workspace = workspace.data_ptr();
   check_rc(nb_attn_bwd(&a, at::cuda::getCurrentCUDAStream().stream()), "nb_attn_bwd");
   after_launch(word);
@@ -224,7 +232,7 @@ Two sdpa_fwd_cuda(const Tensor& q_, const Tensor& k_, const Tensor& v_, double s
   const c10::cuda::CUDAGuard guard(q_.device());
   const Tensor q = dense_layout(q_), k = dense_layout(k_), v = dense_layout(v_);
   Tensor out = new_dense(q), workspace;
-  Tensor lse = at::empty({b, h, lq}, q.options().dtype(at::kFloat));
+  Tensor lse = new_tensor({b, h, lq}, at::kFloat, q);
   nb_attn_fwd_args a{};
   a.shape = dense_shape(q, k, scale);
   a.q = dense_desc(q), a.k = dense_desc(k), a.v = dense_desc(v), a.o = dense_desc(out);
@@ -261,8 +269,8 @@ Two sdpa_varlen_fwd_cuda(const Tensor& q_, const Tensor& k_, const Tensor& v_, c
   NB_REQUIRE(tq > 0 && k_.size(0) > 0 && max_q > 0 && max_k > 0, "empty tensors are not supported");
   const c10::cuda::CUDAGuard guard(q_.device());
   const Tensor q = packed_layout(q_), k = packed_layout(k_), v = packed_layout(v_);
-  Tensor out = at::empty({tq, h, kHeadDim}, q.options()), workspace;
-  Tensor lse = at::empty({h, tq}, q.options().dtype(at::kFloat));
+  Tensor out = new_tensor({tq, h, kHeadDim}, at::kBFloat16, q), workspace;
+  Tensor lse = new_tensor({h, tq}, at::kFloat, q);
   nb_attn_fwd_args a{};
   a.shape = packed_shape(q, k, cu_q, cu_k, max_q, max_k, scale);
   a.q = packed_desc(q), a.k = packed_desc(k), a.v = packed_desc(v), a.o = packed_desc(out);
@@ -280,8 +288,8 @@ Three sdpa_varlen_bwd_cuda(const Tensor& d_out_, const Tensor& q_, const Tensor&
   const c10::cuda::CUDAGuard guard(q_.device());
   const Tensor q = packed_layout(q_), k = packed_layout(k_), v = packed_layout(v_);
   const Tensor out = packed_layout(out_), d_out = packed_layout(d_out_), lse = lse_.contiguous();
-  Tensor dq = at::empty(q.sizes(), q.options()), dk = at::empty(k.sizes(), k.options()),
-         dv = at::empty(k.sizes(), k.options());
+  Tensor dq = new_tensor(q.sizes(), at::kBFloat16, q), dk = new_tensor(k.sizes(), at::kBFloat16, q),
+         dv = new_tensor(k.sizes(), at::kBFloat16, q);
   nb_attn_bwd_args a{};
   a.shape = packed_shape(q, k, cu_q, cu_k, max_q, max_k, scale);
   a.q = packed_desc(q), a.k = packed_desc(k), a.v = packed_desc(v), a.o = packed_desc(out), a.d_o = packed_desc(d_out);
@@ -328,7 +336,7 @@ bool wants_grad(const Tensor& q, const Tensor& k, const Tensor& v) {
 
 // One node of the autograd graph for both entry points. It is written out instead of derived from
 // torch::autograd::Function because a small call is bound by host work: the wrapper's bookkeeping (maps of
-// saved values, sets of dirty and non-differentiable outputs) was 6 of 77 us of a forward + backward.
+// saved values, sets of dirty and non-differentiable outputs) was 4 of 76 us of a forward + backward.
 struct SdpaNode : public torch::autograd::Node {
   using torch::autograd::Node::Node;
   torch::autograd::SavedVariable q, k, v, out, lse, cu_q, cu_k;  // cu_*: packed calls only
