@@ -105,6 +105,7 @@ constexpr int kFwdPartFloats = kTile * (kHeadDim + 2);  // a cut unit's O (not n
 constexpr int kFwdTmemCols = 256;
 constexpr float kRescaleThreshold = 8.f;                       // log2 units
 constexpr float kFirstPassSumLimit = 1152921504606846976.f;  // 2^60
+constexpr float kPolyLimit = 126.f;                          // log2 units
 
 enum FwdBar : int {
   kFwdQFull = 0,                          // [2]: Q and the unit's descriptor (by descriptor slot)
@@ -194,8 +195,10 @@ __device__ __forceinline__ void chunk_mask(uint32_t (&r)[32], int col0, int vali
 }
 
 // P = exp2(s*scale_log2 - m_scaled) for 32 scores, packed to bf16; four partial row sums kept as
-// two packed fp32 pairs. Packed f32x2 arithmetic halves the issue slots of the FMA and the add.
-__device__ __forceinline__ void chunk_exp(const uint32_t (&r)[32], uint64_t scale2, uint64_t neg_m2,
+// two packed fp32 pairs. Packed f32x2 arithmetic halves the issue slots of the FMA and the add. `top` collects
+// the largest argument that took the polynomial, NaN if one was: its results mean nothing from 2^128 on and
+// do not show a NaN, so the caller has to look.
+__device__ __forceinline__ void chunk_exp(const uint32_t (&r)[32], uint64_t scale2, uint64_t neg_m2, float& top,
                                           uint64_t& l01, uint64_t& l23, uint32_t* pk) {
 #pragma unroll
   for (int j = 0; j < 16; ++j) {
@@ -203,12 +206,17 @@ __device__ __forceinline__ void chunk_exp(const uint32_t (&r)[32], uint64_t scal
     unpack_f32x2(fma_f32x2(pack_f32x2(__uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1])), scale2, neg_m2),
                  x0, x1);
     float p0, p1;
-    // One pair in four takes the polynomial on the FMA pipe: the MUFU unit gives 16 results per clock
-    // and SM, 1024 clocks for a 128 x 128 tile, and the rest of the loop leaves room for about that
-    // much (dense 32 x 8 x 4096: none 1468 us, one in eight 1462, one in four 1455; 24 sequences of
-    // 820 tokens, not power-limited: 13.8, 13.2, 12.7).
-    if ((j & 3) == 3) unpack_f32x2(exp2_poly_f32x2(pack_f32x2(x0, x1)), p0, p1);
-    else p0 = fast_exp2(x0), p1 = fast_exp2(x1);
+    // One pair in eight takes the polynomial on the FMA pipe: the MUFU unit gives 16 results per clock
+    // and SM, 1024 clocks for a 128 x 128 tile. Dense 32 x 8 x 4096, sustained: none 1453 us, one in eight
+    // 1424, one in four 1430; 1 x 12 x 3476, not power-limited: 60.4, 57.5, 56.3. One in four would
+    // double what the polynomial adds to the error of the log-sum-exp (a bias of 5e-7 over many
+    // keys). Without `top`: 1412 and 57.7.
+    if ((j & 7) == 7) {
+      unpack_f32x2(exp2_poly_f32x2(pack_f32x2(x0, x1)), p0, p1);
+      top = max3_nan(top, x0, x1);
+    } else {
+      p0 = fast_exp2(x0), p1 = fast_exp2(x1);
+    }
     if (j & 1) l23 = add_f32x2(l23, pack_f32x2(p0, p1)); else l01 = add_f32x2(l01, pack_f32x2(p0, p1));
     pk[j] = pack_bf16(p0, p1);
   }
@@ -245,7 +253,7 @@ __global__ void __launch_bounds__(256) attn_fwd_combine_kernel(const __grid_cons
       o[j].z = fmaf(a.z, f, o[j].z), o[j].w = fmaf(a.w, f, o[j].w);
     }
   }
-  const float inv_l = l > 0.f ? 1.f / l : 0.f;
+  const float inv_l = 1.f / l;
   const uint32_t seq = p.div_heads.quot(t), h = t - seq * uint32_t(p.heads);
   uint4* dst = reinterpret_cast<uint4*>(p.o + int64_t(seq) * p.o_sb + int64_t(h) * p.o_sh + int64_t(tok) * p.o_st) + g0 / 2;
 #pragma unroll
@@ -460,6 +468,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       const bool safe = meta.safe != 0;
       float m_run = -INFINITY;  // raw (unscaled) offset of the exponent
       float l_run = 0.f;
+      float top = -INFINITY;  // see chunk_exp
       bool s_ok = false;
 #pragma unroll 1
       for (int c0 = 0; c0 < lk; c0 += 64) {  // one half tile: key columns [c0, c0 + 64)
@@ -521,8 +530,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         const float nm = -m_run * p.scale_log2;
         const uint64_t neg_m2 = pack_f32x2(nm, nm);
         uint64_t l01 = 0ull, l23 = 0ull;
-        chunk_exp(ra, scale2, neg_m2, l01, l23, pk);
-        chunk_exp(rb, scale2, neg_m2, l01, l23, pk + 16);
+        chunk_exp(ra, scale2, neg_m2, top, l01, l23, pk);
+        chunk_exp(rb, scale2, neg_m2, top, l01, l23, pk + 16);
         tmem_st32(s_addr + 64 * hf, pk);
         // The next half's scores are usually there already; look while the stores complete.
         if (hf) ++t[1]; else ++t[0];
@@ -546,6 +555,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         mbar_wait(bar(kFwdPvDone + hf), ((hf ? t[1] : t[0]) - 1) & 1, &abort_flag, p.status);
         __syncwarp();
         tc_fence_after();
+        if (!(top < kPolyLimit)) l_run = NAN;
         if (!safe && __any_sync(0xffffffffu, !(l_run <= kFirstPassSumLimit))) {
           // Some exponent ran far above the first half's offset: the unit is walked again.
           if (lane == 0 && atomicExch(&redo_listed[u & 1u], 1) == 0)
@@ -576,7 +586,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         reinterpret_cast<float2*>(part + kTile * kHeadDim)[tid] = make_float2(m_run, l_run);
         store = false;
       } else {
-        const float inv_l = l_run > 0.f ? 1.f / l_run : 0.f;
+        const float inv_l = lk > 0 ? 1.f / l_run : 0.f;
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           uint32_t o[32];

@@ -484,8 +484,16 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   return d;
 }
 
+// The same, NaN if one of them is.
+__device__ __forceinline__ float max3_nan(float a, float b, float c) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
 // exp2 of a packed pair on the FMA and integer pipes instead of the MUFU unit (16 results per clock
-// per SM), for arguments <= ~100: clamp at -126, split x = n + f with n = round(x) by adding
+// per SM), for arguments below 127 (from 128 on the exponent field wraps; NaN gives 2^-126, as everything
+// below -126 does): clamp at -126, split x = n + f with n = round(x) by adding
 // 1.5*2^23, evaluate a degree-3 minimax polynomial for 2^f on [-0.5, 0.5] (relative error 7.5e-5,
 // far below the bf16 rounding the result receives), and add n to the exponent field.
 __device__ __forceinline__ uint64_t exp2_poly_f32x2(uint64_t x2) {

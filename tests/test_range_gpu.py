@@ -1,0 +1,60 @@
+"""The forward on scores and values of unusual size: far above the exponent's offset, infinite, NaN."""
+
+import numpy as np
+import pytest
+import torch
+
+from nanobrain_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def bf16(*shape, seed, mul=1.0):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    return (torch.randn(*shape, generator=g, device=DEV) * mul).to(torch.bfloat16)
+
+
+def exact_forward(q, k, v, scale=0.125):
+    q, k, v = q.double(), k.double(), v.double()
+    s = q @ k.transpose(-1, -2) * scale
+    return torch.softmax(s, -1) @ v, torch.logsumexp(s, -1)
+
+
+@pytest.mark.parametrize("lk", [256, 300])
+@pytest.mark.parametrize("score", [100.0, 200.0, 500.0])
+def test_one_key_far_above_the_first_ones_takes_all_the_weight(lk, score):
+    # One sequence per column at which the dominating key can be: every score is 0 but that one, so the
+    # output is that key's value (exp(-100) of the others), exactly.
+    cols = lk - 64
+    q = torch.zeros(cols, 1, 70, 64, device=DEV, dtype=torch.bfloat16)
+    q[..., 0] = 8.0
+    k = torch.zeros(cols, 1, lk, 64, device=DEV, dtype=torch.bfloat16)
+    k[torch.arange(cols), 0, torch.arange(cols) + 64, 0] = score
+    v = torch.arange(lk, device=DEV, dtype=torch.float32)[None, None, :, None].expand(cols, 1, lk, 64).to(torch.bfloat16)
+    out, lse = ops.sdpa_fwd(q, k, v, 0.125)
+    ops.check_status()
+    want = v[0, 0, 64:, 0][:, None, None, None].expand_as(out)
+    assert torch.equal(out, want), torch.nonzero((out != want).any(-1).any(-1).any(-1)).flatten().tolist()
+    # (fp32 of a score of 722 in log2 units: half a unit in the last place is 3e-5)
+    np.testing.assert_allclose(lse.cpu().numpy(), score, rtol=1e-6, atol=0)
+
+
+def test_a_nan_key_row_shows_in_every_query_row():
+    lk = 200
+    q = bf16(lk, 1, 70, 64, seed=1)
+    k, v = bf16(lk, 1, lk, 64, seed=2), bf16(lk, 1, lk, 64, seed=3)
+    k[torch.arange(lk), 0, torch.arange(lk)] = float("nan")
+    out, lse = ops.sdpa_fwd(q, k, v, 0.125)
+    ops.check_status()
+    seen = torch.isnan(out).all(-1).all(-1).all(-1) & torch.isnan(lse).all(-1).all(-1)
+    assert bool(seen.all()), torch.nonzero(~seen).flatten().tolist()
+
+
+def test_bias_of_the_log_sum_exp():
+    # The polynomial's error is 5.1e-6 on average (7.5e-5 at most), for one key in eight: a bias of 6.4e-7
+    # over many keys, to which the roundings of fp32 sums (unbiased) add little.
+    q, k, v = (bf16(2, 8, 4096, 64, seed=s) for s in (4, 5, 6))
+    lse = ops.sdpa_fwd(q, k, v, 0.125)[1]
+    err = lse.double() - exact_forward(q, k, v)[1]
+    assert abs(float(err.mean())) <= 8.5e-7 and float(err.pow(2).mean().sqrt()) <= 1.1e-6
