@@ -3,7 +3,7 @@
 //
 // A work unit is one 128-row query tile of one (sequence, head), walked over the sequence's keys in
 // 128-row tiles, each in two halves of 64 key columns. CTAs are persistent, two per SM (256
-// tensor-memory columns and 97 KB of shared memory each, so one CTA's softmax overlaps the other's MMAs);
+// tensor-memory columns and 99 KB of shared memory each, so one CTA's softmax overlaps the other's MMAs);
 // the producer warp fetches the units and runs on into the next one -- its descriptor, Q, first K / V
 // tiles and first scores are there before the softmax warps have stored the unit before it. Packed units
 // come from the scheduler's list (sched_kernel.cuh), dense ones by position, and where whole dense units
@@ -14,11 +14,17 @@
 //   warps 0-3 : softmax warpgroup. Thread r owns row r of the tile (tensor-memory lane r). Per half it
 //               pulls its 64 fp32 scores into registers and writes P = exp2(S*scale_log2 - m) as bf16
 //               over the first half of the columns they came from. The offset m is the row max of the
-//               first half tile; later halves compute no max at all: fp32 and bf16 carry exponents up
+//               first tile; later halves compute no max at all: fp32 and bf16 carry exponents up
 //               to 2^127, so scores may rise 60 (in log2 units) above the first ones before anything
 //               has to be rescaled. Only if a row's sum ends above 2^60 (or Inf / NaN) does the CTA list
 //               the unit and walk it a second time, with the running max of every half. At the end of a
-//               unit the warps normalise and store O and the log-sum-exp.
+//               unit the warps normalise and store O and the log-sum-exp. O is divided by the sum of
+//               P as the product sees it, rounded to bf16, which the tensor core forms from 16 columns
+//               of ones behind V: where few keys dominate a row, the rounding of their P then cancels.
+//               Scores of standard deviation 9 and 16 nats, relative error of O against 64 bits: 2.2e-3
+//               and 2.0e-3 divided by the sum before rounding, 1.7e-3 and 1.5e-3 this way (with the running
+//               max as the offset 1.9e-3 and 1.7e-3). The columns cost 1 % (dense 32 x 8 x 4096, sustained:
+//               1428 -> 1442 us), the max of the whole first tile instead of its first half 0.3 %.
 //   warp 4    : one elected thread issues every tcgen05.mma. Q is copied into tensor memory once
 //               per unit (tcgen05.cp), so S = Q K^T takes its A operand from there, as O += P V does. After P of
 //               half h of tile i is complete it issues P V of that half and then S of half h of tile
@@ -35,7 +41,7 @@
 // packed 32 x U[720,920] x 12 heads 130 -> 122 us, 500 sequences of 1..300 tokens 232 -> 179, dense
 // 32 x 8 x 4096 unchanged, 24 sequences of 820 tokens (less than one unit per CTA) 12.7 -> 14.3.
 //
-// Tensor memory (256 columns): S / P [0,128) O [128,192) Q [192,224).
+// Tensor memory (256 columns): S / P [0,128) O [128,192) row sums of P [192,208) Q [208,240).
 #pragma once
 
 #include <type_traits>
@@ -99,9 +105,11 @@ constexpr int kTileBytes = kTile * kHeadDim * 2;  // 16 KB
 constexpr int kFwdThreads = 192;
 constexpr int kFwdQRows = kTile;  // query rows per CTA
 constexpr int kFwdStages = 2;
-constexpr int kFwdSmemBytes = (2 + 2 * kFwdStages) * kTileBytes + 1024;  // Q, K and V rings, O staging
+constexpr int kFwdOnesBytes = 2048;
+// Q, K and V rings, O staging, the block of ones, alignment slack
+constexpr int kFwdSmemBytes = (2 + 2 * kFwdStages) * kTileBytes + kFwdOnesBytes + 1024;
 constexpr int kFwdRedoSlots = 16;
-constexpr int kFwdPartFloats = kTile * (kHeadDim + 2);  // a cut unit's O (not normalised), offsets and sums
+constexpr int kFwdPartFloats = kTile * (kHeadDim + 3);  // a cut unit's O (not normalised), offsets and both sums
 constexpr int kFwdTmemCols = 256;
 constexpr float kRescaleThreshold = 8.f;                       // log2 units
 constexpr float kFirstPassSumLimit = 1152921504606846976.f;  // 2^60
@@ -236,7 +244,7 @@ __global__ void __launch_bounds__(256) attn_fwd_combine_kernel(const __grid_cons
   if (tok >= p.lq) return;
   auto part = [&](uint32_t c) { return p.parts + int64_t(2 * c + (c == b - 1)) * kFwdPartFloats; };
   auto stat = [&](uint32_t c) { return reinterpret_cast<const float2*>(part(c) + kTile * kHeadDim)[row]; };
-  float m = -INFINITY, l = 0.f;
+  float m = -INFINITY, l = 0.f, w = 0.f;
   for (uint32_t c = b - 1; fwd_split_start(p, c) < end; ++c) m = fmaxf(m, stat(c).x);
   float4 o[4];
 #pragma unroll
@@ -246,6 +254,7 @@ __global__ void __launch_bounds__(256) attn_fwd_combine_kernel(const __grid_cons
     const float4* src = reinterpret_cast<const float4*>(part(c)) + g0 * kTile + row;
     const float f = fast_exp2((st.x - m) * p.scale_log2);
     l += st.y * f;
+    w += part(c)[kTile * (kHeadDim + 2) + row] * f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const float4 a = src[j * kTile];
@@ -253,7 +262,7 @@ __global__ void __launch_bounds__(256) attn_fwd_combine_kernel(const __grid_cons
       o[j].z = fmaf(a.z, f, o[j].z), o[j].w = fmaf(a.w, f, o[j].w);
     }
   }
-  const float inv_l = 1.f / l;
+  const float inv_l = 1.f / fmaf(l, 0.f, w);
   const uint32_t seq = p.div_heads.quot(t), h = t - seq * uint32_t(p.heads);
   uint4* dst = reinterpret_cast<uint4*>(p.o + int64_t(seq) * p.o_sb + int64_t(h) * p.o_sh + int64_t(tok) * p.o_st) + g0 / 2;
 #pragma unroll
@@ -286,6 +295,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   auto sK = [&](uint32_t s) { return smem_base + (1 + 2 * s) * kTileBytes; };
   auto sV = [&](uint32_t s) { return smem_base + (2 + 2 * s) * kTileBytes; };
   const uint32_t sO = smem_base + (1 + 2 * kFwdStages) * kTileBytes;
+  const uint32_t sOnes = sO + kTileBytes;
   const uint32_t bar0 = smem_u32(&bars[0]);
   auto bar = [&](uint32_t i) { return bar0 + 8u * i; };
 
@@ -304,6 +314,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   if (warp == 4) {
     tmem_alloc(smem_u32(&tmem_base_slot), kFwdTmemCols);
     tmem_relinquish();
+  } else if (tid < kFwdOnesBytes / 16) {
+    constexpr uint32_t kOnes = 0x3f803f80u;
+    reinterpret_cast<uint4*>(smem_raw + (sOnes - smem_u32(smem_raw)))[tid] = make_uint4(kOnes, kOnes, kOnes, kOnes);
+    fence_proxy_async_smem();
   }
   // Everything this kernel reads may come from the kernel right before it in the stream. (Tensor memory
   // is there for two CTAs per SM, and shared memory admits no more of any kernel that uses it, so what
@@ -314,7 +328,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
-  const uint32_t tm_s = tmem_base, tm_o = tmem_base + 128, tm_q = tmem_base + 192;
+  const uint32_t tm_s = tmem_base, tm_o = tmem_base + 128, tm_q = tmem_base + 208;
 
   if (warp == 5) {
     // ---------------- producer: unit descriptors, Q, K and V ----------------
@@ -374,7 +388,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     // ---------------- MMA issuer ----------------
     if (elect_one()) {
       constexpr uint32_t kIdescS = make_idesc(128, 64, 0, 0);
-      constexpr uint32_t kIdescPV = make_idesc(128, 64, 0, 1);
+      // P V with 16 more columns of B, all ones: the first of them sums up the rows of P as the product
+      // sees it, rounded to bf16. They lie behind V at the descriptor's leading offset, which therefore shrinks by what
+      // the start address grows from K step to K step.
+      constexpr uint32_t kIdescPV = make_idesc(128, 80, 0, 1);
+      constexpr uint64_t kVStep = 128 - (128ull << 16);
       const uint64_t qd = make_sdesc(sQ, 16, 1024);
       uint32_t t = 0;   // key tiles so far
       uint32_t t1 = 0;  // of them with a second half
@@ -419,7 +437,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         for (int i = 0; i < n_kv; ++i, ++t) {
           const uint32_t s = t % kFwdStages, s1 = (t + 1) % kFwdStages;
           mbar_wait(bar(kFwdVFull + s), (t / kFwdStages) & 1, &abort_flag, p.status);
-          const uint64_t vd = make_sdesc(sV(s), 1024, 1024);
+          const uint64_t vd = make_sdesc(sV(s), sOnes - sV(s), 1024);
           const int nh = halves(i), nh1 = i + 1 < n_kv ? halves(i + 1) : 0;
 #pragma unroll 1
           for (int hf = 0; hf < nh; ++hf) {
@@ -431,11 +449,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             if (ksteps == 4) {
 #pragma unroll
               for (int k = 0; k < 4; ++k)
-                mma_ts(tm_o, tm_s + 64 * hf + 8 * k, vd + 512 * hf + 128 * k, kIdescPV, (i | hf | k) > 0);
+                mma_ts(tm_o, tm_s + 64 * hf + 8 * k, vd + kVStep * (4 * hf + k), kIdescPV, (i | hf | k) > 0);
             } else {
 #pragma unroll 1
               for (int k = 0; k < ksteps; ++k)
-                mma_ts(tm_o, tm_s + 64 * hf + 8 * k, vd + 512 * hf + 128 * k, kIdescPV, (i | hf | k) > 0);
+                mma_ts(tm_o, tm_s + 64 * hf + 8 * k, vd + kVStep * (4 * hf + k), kIdescPV, (i | hf | k) > 0);
             }
             tc_commit(bar(kFwdPvDone + hf));
             if (hf == nh - 1) tc_commit(bar(kFwdVEmpty + s));
@@ -503,6 +521,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           float mx0 = -INFINITY, mx1 = -INFINITY, mx2 = -INFINITY, mx3 = -INFINITY;
           chunk_max(ra, mx0, mx1);
           chunk_max(rb, mx2, mx3);
+          if (c0 == 0 && lk > 64) {  // the first offset is the max of the whole tile
+            mbar_wait(bar(kFwdSFull + 1), t[1] & 1, &abort_flag, p.status);
+            __syncwarp();
+            tc_fence_after();
+#pragma unroll 1
+            for (int c = 64; c < 128; c += 32) {
+              uint32_t r[32];
+              tmem_ld32(s_addr + c, r);
+              tmem_wait_ld();
+              if (lk < 128) chunk_mask(r, c, lk);
+              chunk_max(r, mx0, mx1);
+            }
+          }
           const float m_new = fmaxf(m_run, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)));
           const bool need = (m_new - m_run) * p.scale_log2 > kRescaleThreshold;
           if (c0 == 0) {
@@ -517,7 +548,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             if (need) m_run = m_new;
             l_run *= alpha;
 #pragma unroll 1
-            for (int c = 0; c < 4; ++c) {
+            for (int c = 0; c < 5; ++c) {
               uint32_t o[16];
               tmem_ld16(o_addr + c * 16, o);
               tmem_wait_ld();
@@ -566,6 +597,15 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       // Each warp turns its 32 rows into bf16 in a 4 KB staging area and writes them out with eight lanes
       // per 128-byte row, so the stores are whole lines; a warp only reads what it wrote.
       uint8_t* scratch = smem_raw + (sO - smem_u32(smem_raw)) + warp * 4096;
+      // What O is divided by is the sum of the rounded P: the rounding of a key's P then weighs nothing in a row which that
+      // key dominates. The sum before rounding is the one for the log-sum-exp (and carries NaN, see `top`).
+      float w_run = 1.f;
+      if (lk > 0) {
+        uint32_t w[16];
+        tmem_ld16(o_addr + 64, w);
+        tmem_wait_ld();
+        w_run = fmaf(l_run, 0.f, __uint_as_float(w[0]));
+      }
       if (meta.part >= 0) {
         // This CTA's part of a cut unit: O as it is, then offset and sum of every row. O is laid out as 16
         // groups of four columns x 128 rows, so that a warp's stores are whole lines.
@@ -584,9 +624,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         __syncwarp();
         mbar_arrive_if(bar(kFwdOFree), lane0);
         reinterpret_cast<float2*>(part + kTile * kHeadDim)[tid] = make_float2(m_run, l_run);
+        part[kTile * (kHeadDim + 2) + tid] = w_run;
         store = false;
       } else {
-        const float inv_l = lk > 0 ? 1.f / l_run : 0.f;
+        const float inv_l = lk > 0 ? 1.f / w_run : 0.f;
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
           uint32_t o[32];

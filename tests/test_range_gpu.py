@@ -58,3 +58,21 @@ def test_bias_of_the_log_sum_exp():
     lse = ops.sdpa_fwd(q, k, v, 0.125)[1]
     err = lse.double() - exact_forward(q, k, v)[1]
     assert abs(float(err.mean())) <= 8.5e-7 and float(err.pow(2).mean().sqrt()) <= 1.1e-6
+
+
+@pytest.mark.parametrize("shape,mul", [((4, 8, 128), 1.0), ((2, 4, 820), 1.0), ((2, 4, 300), 3.0), ((2, 4, 1000), 4.0), ((1, 2, 3476), 3.0)])
+def test_rounding_of_p_weighs_little_where_one_key_dominates(shape, mul):
+    # P is rounded to bf16 (relative error d_j of key j, independent, 2^-8 at most) and O is divided by the sum of
+    # the same rounded values, so its error is sum_j w_j d_j (v_j - O), plus its own rounding to bf16. A
+    # relative rounding error of a number with evenly spread logarithm has the variance 2^-14 / 12 x 0.541
+    # (spacing 2^-7 at 1, and the mean of 1 / m^2 over its mantissas m).
+    q, k = (bf16(*shape, 64, seed=s, mul=mul) for s in (7, 8))
+    v = bf16(*shape, 64, seed=9)
+    out = ops.sdpa_fwd(q, k, v, 0.125)[0].double()
+    want = exact_forward(q, k, v)[0]
+    w = torch.softmax(q.double() @ k.double().transpose(-1, -2) * 0.125, -1)
+    v = v.double()
+    spread = (w**2) @ v**2 - 2 * ((w**2) @ v) * want + (w**2).sum(-1, keepdim=True) * want**2
+    rounding = (want.to(torch.bfloat16).double() - want) ** 2
+    bound = (spread.sum() * 2.0**-14 / 12 * 0.541 + rounding.sum()).sqrt() / want.norm()
+    assert float((out - want).norm() / want.norm()) <= 1.05 * float(bound)
