@@ -16,8 +16,8 @@
 //               over the first half of the columns they came from. The offset m is the row max of the
 //               first tile; later halves compute no max at all: fp32 and bf16 carry exponents up
 //               to 2^127, so scores may rise 60 (in log2 units) above the first ones before anything
-//               has to be rescaled. Only if a row's sum ends above 2^60 (or Inf / NaN) does the CTA list
-//               the unit and walk it a second time, with the running max of every half. At the end of a
+//               has to be rescaled. Only if a row's sum ends above 2^60 (or Inf / NaN), or above 2^14 with a
+//               P V that is not finite, does the CTA list the unit and walk it a second time, with the running max of every half. At the end of a
 //               unit the warps normalise and store O and the log-sum-exp. O is divided by the sum of
 //               P as the product sees it, rounded to bf16, which the tensor core forms from 16 columns
 //               of ones behind V: where few keys dominate a row, the rounding of their P then cancels.
@@ -113,6 +113,7 @@ constexpr int kFwdPartFloats = kTile * (kHeadDim + 3);  // a cut unit's O (not n
 constexpr int kFwdTmemCols = 256;
 constexpr float kRescaleThreshold = 8.f;                       // log2 units
 constexpr float kFirstPassSumLimit = 1152921504606846976.f;  // 2^60
+constexpr float kPlainSumLimit = 16384.f;
 constexpr float kPolyLimit = 126.f;                          // log2 units
 
 enum FwdBar : int {
@@ -587,11 +588,25 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         __syncwarp();
         tc_fence_after();
         if (!(top < kPolyLimit)) l_run = NAN;
-        if (!safe && __any_sync(0xffffffffu, !(l_run <= kFirstPassSumLimit))) {
-          // Some exponent ran far above the first half's offset: the unit is walked again.
-          if (lane == 0 && atomicExch(&redo_listed[u & 1u], 1) == 0)
-            redo_tokens[uint32_t(atomicAdd(&redo_count, 1)) % kFwdRedoSlots] = meta.token;
-          store = false;
+        if (!safe) {
+          bool again = !(l_run <= kFirstPassSumLimit);
+          if (__any_sync(0xffffffffu, l_run > kPlainSumLimit)) {
+            // P has been far above 1, so P V may have left fp32's range where the result would not.
+#pragma unroll 1
+            for (int c = 0; c < 4; ++c) {
+              uint32_t o[16];
+              tmem_ld16(o_addr + c * 16, o);
+              tmem_wait_ld();
+#pragma unroll
+              for (int j = 0; j < 16; ++j) again |= (o[j] & 0x7f800000u) == 0x7f800000u;
+            }
+          }
+          if (__any_sync(0xffffffffu, again)) {
+            // Some exponent ran far above the first tile's offset: the unit is walked again.
+            if (lane == 0 && atomicExch(&redo_listed[u & 1u], 1) == 0)
+              redo_tokens[uint32_t(atomicAdd(&redo_count, 1)) % kFwdRedoSlots] = meta.token;
+            store = false;
+          }
         }
       }
       // Each warp turns its 32 rows into bf16 in a 4 KB staging area and writes them out with eight lanes

@@ -76,3 +76,17 @@ def test_rounding_of_p_weighs_little_where_one_key_dominates(shape, mul):
     rounding = (want.to(torch.bfloat16).double() - want) ** 2
     bound = (spread.sum() * 2.0**-14 / 12 * 0.541 + rounding.sum()).sqrt() / want.norm()
     assert float((out - want).norm() / want.norm()) <= 1.05 * float(bound)
+
+
+@pytest.mark.parametrize("lk", [512, 4000])  # the second one is cut between CTAs
+@pytest.mark.parametrize("exponent", [60, 90, 112])
+def test_large_values_behind_rising_scores(exponent, lk):
+    # P of the keys 35 nats above the first ones is 2^50: times V that is beyond fp32, the result is not.
+    q = torch.zeros(1, 1, 140, 64, device=DEV, dtype=torch.bfloat16)
+    q[..., 0] = 8.0
+    k = torch.zeros(1, 1, lk, 64, device=DEV, dtype=torch.bfloat16)
+    k[0, 0, 300:302, 0], k[0, 0, 70, 0] = 35.0, 20.0
+    v = torch.full((1, 1, lk, 64), 2.0**exponent, device=DEV).to(torch.bfloat16)
+    out = ops.sdpa_fwd(q, k, v, 0.125)[0]
+    ops.check_status()
+    assert torch.equal(out, v[:, :, :1].expand_as(out))
