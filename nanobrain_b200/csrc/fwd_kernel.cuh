@@ -113,6 +113,7 @@ constexpr int kFwdPartFloats = kTile * (kHeadDim + 3);  // a cut unit's O (not n
 constexpr int kFwdTmemCols = 256;
 constexpr float kRescaleThreshold = 8.f;                       // log2 units
 constexpr float kFirstPassSumLimit = 1152921504606846976.f;  // 2^60
+constexpr float kNoOffset = -1.2676506002282294e30f;  // -2^100
 constexpr float kPlainSumLimit = 16384.f;
 constexpr float kPolyLimit = 126.f;                          // log2 units
 
@@ -538,7 +539,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           const float m_new = fmaxf(m_run, fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)));
           const bool need = (m_new - m_run) * p.scale_log2 > kRescaleThreshold;
           if (c0 == 0) {
-            m_run = m_new;
+            // Where all scores of the tile are -inf, the first walk goes on with that offset: P becomes Inf or NaN, which
+            // leads to the second. There any finite offset makes their P 0.
+            m_run = safe && m_new == -INFINITY ? kNoOffset : m_new;
           } else if (__any_sync(0xffffffffu, need)) {
             // Second time: refresh the offset of the rows that need it, rescale their running sum and
             // their row of the O accumulator (complete up to the previous half).

@@ -90,3 +90,19 @@ def test_large_values_behind_rising_scores(exponent, lk):
     out = ops.sdpa_fwd(q, k, v, 0.125)[0]
     ops.check_status()
     assert torch.equal(out, v[:, :, :1].expand_as(out))
+
+
+@pytest.mark.parametrize("lk,first", [(256, 64), (256, 128), (256, 200), (300, 17), (4096, 128), (4096, 2100)])
+def test_scores_of_minus_infinity_have_no_weight(lk, first):
+    # q.k of the first keys is below fp32's range, all other scores are 0. (4096: cut between CTAs.)
+    q = torch.full((1, 1, 128, 64), 1e30, device=DEV, dtype=torch.bfloat16)
+    k = torch.zeros(1, 1, lk, 64, device=DEV, dtype=torch.bfloat16)
+    k[0, 0, :first] = -1e30
+    v = bf16(1, 1, lk, 64, seed=10)
+    out, lse = ops.sdpa_fwd(q, k, v, 0.125)
+    ops.check_status()
+    want = v[0, 0, first:].double().mean(0)
+    # P = 1 exactly, so O has its own rounding to bf16 alone: half of a spacing of 2^-7 at most
+    assert bool(((out.double() - want).abs() <= 2.0**-8 * 1.001 * want.abs()).all())
+    # the polynomial gives 1 - 7.2e-5 at 0, for at most one in seven of the keys that are left: 1.03e-5
+    np.testing.assert_allclose(lse.cpu().numpy(), np.log(lk - first), rtol=0, atol=1.2e-5)
