@@ -313,22 +313,24 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     }
     fence_mbar_init();
   }
-  if (warp == 4) {
-    tmem_alloc(smem_u32(&tmem_base_slot), kFwdTmemCols);
-    tmem_relinquish();
-  } else if (tid < kFwdOnesBytes / 16) {
+  if (tid < kFwdOnesBytes / 16) {
     constexpr uint32_t kOnes = 0x3f803f80u;
     reinterpret_cast<uint4*>(smem_raw + (sOnes - smem_u32(smem_raw)))[tid] = make_uint4(kOnes, kOnes, kOnes, kOnes);
     fence_proxy_async_smem();
   }
-  // Everything this kernel reads may come from the kernel right before it in the stream. (Tensor memory
-  // is there for two CTAs per SM, and shared memory admits no more of any kernel that uses it, so what
-  // was taken above cannot hold back the kernel that is waited for.)
+  // Everything this kernel reads may come from the kernel right before it in the stream. Tensor memory is taken
+  // behind the wait: the kernel before may be a foreign one (a library GEMM) with blocks that have yet
+  // to take theirs, and neither side's wait would end. For the same reason dependents may start only when this block has
+  // its own.
   pdl_wait();
-  pdl_launch_dependents();
+  if (warp == 4) {
+    tmem_alloc(smem_u32(&tmem_base_slot), kFwdTmemCols);
+    tmem_relinquish();
+  }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  pdl_launch_dependents();
   const uint32_t tmem_base = tmem_base_slot;
   const uint32_t tm_s = tmem_base, tm_o = tmem_base + 128, tm_q = tmem_base + 208;
 

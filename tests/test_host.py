@@ -84,3 +84,19 @@ def test_host_pipeline_refuses_a_cpu_device():
 
     with pytest.raises(RuntimeError, match="CUDA"):
         HostPipeline([10, 20], 2, torch.device("cpu"))
+
+
+def test_tensor_memory_is_taken_after_the_wait_for_the_predecessor():
+    # A block that holds tensor memory while it waits for the kernel before it in the stream can keep that kernel's
+    # last blocks from getting theirs. (The self-test kernels are launched in plain stream order.)
+    from nanobrain_b200 import build
+
+    for name in ("fwd_kernel.cuh", "bwd_kernel.cuh"):
+        source = (build.CSRC / name).read_text()
+        body = source[source.index("extern __shared__ uint8_t smem_raw[];"):]
+        assert body.count("pdl_wait();") == 1 and body.count("tmem_alloc(") == 1, name
+        assert body.index("pdl_wait();") < body.index("tmem_alloc("), name
+    forward = (build.CSRC / "fwd_kernel.cuh").read_text()
+    forward = forward[forward.index("extern __shared__ uint8_t smem_raw[];"):]
+    # (a foreign kernel may follow the forward; what follows the backward's main kernel is its own epilogue)
+    assert forward.index("tmem_alloc(") < forward.index("__syncthreads();") < forward.index("pdl_launch_dependents();")
