@@ -16,9 +16,7 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/autograd_not_implemented_fallback.h>
-#include <torch/csrc/autograd/function.h>
-#include <torch/csrc/autograd/functions/utils.h>
-#include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/autograd/custom_function.h>
 #include <torch/extension.h>
 #include <torch/library.h>
 
@@ -34,6 +32,7 @@
 namespace {
 
 using at::Tensor;
+using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 using Two = std::tuple<Tensor, Tensor>;
 using Three = std::tuple<Tensor, Tensor, Tensor>;
@@ -299,7 +298,7 @@ Three sdpa_varlen_bwd_cuda(const Tensor& d_out_, const Tensor& q_, const Tensor&
 }
 
 // ------------------------------------------------------------------------------------------
-// Autograd. The functions and the node call the ops again below autograd, so dispatch modes (fake tensors, tracing,
+// Autograd. The functions call the ops again below autograd, so dispatch modes (fake tensors, tracing,
 // the FLOP counter) see every forward and backward op.
 // ------------------------------------------------------------------------------------------
 using FwdSig = Two(const Tensor&, const Tensor&, const Tensor&, double);
@@ -334,80 +333,69 @@ bool wants_grad(const Tensor& q, const Tensor& k, const Tensor& v) {
   return at::GradMode::is_enabled() && (q.requires_grad() || k.requires_grad() || v.requires_grad());
 }
 
-// One node of the autograd graph for both entry points. It is written out instead of derived from
-// torch::autograd::Function because a small call is bound by host work: the wrapper's bookkeeping (maps of
-// saved values, sets of dirty and non-differentiable outputs) was 4 of 76 us of a forward + backward.
-struct SdpaNode : public torch::autograd::Node {
-  using torch::autograd::Node::Node;
-  torch::autograd::SavedVariable q, k, v, out, lse, cu_q, cu_k;  // cu_*: packed calls only
-  c10::SymInt max_q, max_k;
-  double scale = 0;
-  bool packed = false, released = false;
+// The gradient of `out`; the log-sum-exp's own gradient is not used (it exists for the backward op).
+Tensor grad_of_out(const variable_list& grads, const Tensor& out) {
+  return grads[0].defined() ? grads[0] : at::zeros_like(out);
+}
 
-  std::string name() const override { return packed ? "SdpaVarlenBackward" : "SdpaBackward"; }
-
-  variable_list apply(variable_list&& grads) override {
-    std::lock_guard<std::mutex> lock(mutex_);
-    TORCH_CHECK(!released, torch::autograd::ERR_BACKWARD_TWICE);
-    const auto self = getptr();
-    const Tensor qt = q.unpack(), kt = k.unpack(), vt = v.unpack(), ot = out.unpack(self), lt = lse.unpack(self);
-    // The log-sum-exp's own gradient is not used (it exists for the backward op).
-    const Tensor g = grads[0].defined() ? grads[0] : at::zeros_like(ot);
-    auto [dq, dk, dv] = packed ? varlen_bwd_op().call(g, qt, kt, vt, ot, lt, cu_q.unpack(), cu_k.unpack(), max_q, max_k, scale)
-                               : bwd_op().call(g, qt, kt, vt, ot, lt, scale);
-    return {std::move(dq), std::move(dk), std::move(dv)};
+struct SdpaFunction : public torch::autograd::Function<SdpaFunction> {
+  static constexpr bool is_traceable = true;  // compiled autograd may trace through backward
+  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, double scale) {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    auto [out, lse] = fwd_op().call(q, k, v, scale);
+    ctx->set_materialize_grads(false);
+    ctx->save_for_backward({q, k, v, out, lse});
+    ctx->saved_data["scale"] = scale;
+    return {out, lse};
   }
-  void release_variables() override {
-    std::lock_guard<std::mutex> lock(mutex_);
-    released = true;
-    for (auto* s : {&q, &k, &v, &out, &lse, &cu_q, &cu_k}) s->reset_data();
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    auto [dq, dk, dv] = bwd_op().call(grad_of_out(grads, s[3]), s[0], s[1], s[2], s[3], s[4],
+                                      ctx->saved_data["scale"].toDouble());
+    return {dq, dk, dv, Tensor()};
   }
 };
 
-// A node over q, k and v; `finish` makes the outputs part of the graph.
-std::shared_ptr<SdpaNode> new_node(const Tensor& q, const Tensor& k, const Tensor& v, double scale) {
-  TORCH_CHECK(!q._fw_grad(0).defined() && !k._fw_grad(0).defined() && !v._fw_grad(0).defined(),
-              "nanobrain_b200.sdpa: forward-mode differentiation is not implemented");
-  std::shared_ptr<SdpaNode> node(new SdpaNode(), torch::autograd::deleteNode);
-  node->set_next_edges(torch::autograd::collect_next_edges(q, k, v));
-  node->q = torch::autograd::SavedVariable(q, false);
-  node->k = torch::autograd::SavedVariable(k, false);
-  node->v = torch::autograd::SavedVariable(v, false);
-  node->scale = scale;
-  return node;
-}
-Two finish(const std::shared_ptr<SdpaNode>& node, Two outputs) {
-  auto& [out, lse] = outputs;
-  torch::autograd::set_history(out, node);
-  torch::autograd::set_history(lse, node);
-  node->out = torch::autograd::SavedVariable(out, true);
-  node->lse = torch::autograd::SavedVariable(lse, true);
-  return outputs;
-}
+struct SdpaVarlenFunction : public torch::autograd::Function<SdpaVarlenFunction> {
+  static constexpr bool is_traceable = true;  // compiled autograd may trace through backward
+  static variable_list forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v,
+                               const Tensor& cu_q, const Tensor& cu_k, c10::SymInt max_q, c10::SymInt max_k,
+                               double scale) {
+    at::AutoDispatchBelowADInplaceOrView guard;
+    auto [out, lse] = varlen_fwd_op().call(q, k, v, cu_q, cu_k, max_q, max_k, scale);
+    ctx->set_materialize_grads(false);
+    ctx->save_for_backward({q, k, v, out, lse, cu_q, cu_k});
+    ctx->saved_data["max_q"] = std::move(max_q);
+    ctx->saved_data["max_k"] = std::move(max_k);
+    ctx->saved_data["scale"] = scale;
+    return {out, lse};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    auto [dq, dk, dv] = varlen_bwd_op().call(grad_of_out(grads, s[3]), s[0], s[1], s[2], s[3], s[4], s[5], s[6],
+                                             ctx->saved_data["max_q"].toSymInt(), ctx->saved_data["max_k"].toSymInt(),
+                                             ctx->saved_data["scale"].toDouble());
+    return {dq, dk, dv, Tensor(), Tensor(), Tensor(), Tensor(), Tensor()};
+  }
+};
 
 Two sdpa_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, double scale) {
-  auto call = [&] {
+  if (!wants_grad(q, k, v)) {
     at::AutoDispatchBelowADInplaceOrView guard;
     return fwd_op().call(q, k, v, scale);
-  };
-  if (!wants_grad(q, k, v)) return call();
-  const auto node = new_node(q, k, v, scale);
-  return finish(node, call());
+  }
+  auto r = SdpaFunction::apply(q, k, v, scale);
+  return {r[0], r[1]};
 }
 
 Two sdpa_varlen_fwd_autograd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu_q, const Tensor& cu_k,
                              c10::SymInt max_q, c10::SymInt max_k, double scale) {
-  auto call = [&] {
+  if (!wants_grad(q, k, v)) {
     at::AutoDispatchBelowADInplaceOrView guard;
     return varlen_fwd_op().call(q, k, v, cu_q, cu_k, max_q, max_k, scale);
-  };
-  if (!wants_grad(q, k, v)) return call();
-  const auto node = new_node(q, k, v, scale);
-  node->packed = true;
-  node->cu_q = torch::autograd::SavedVariable(cu_q, false);
-  node->cu_k = torch::autograd::SavedVariable(cu_k, false);
-  node->max_q = max_q, node->max_k = max_k;
-  return finish(node, call());
+  }
+  auto r = SdpaVarlenFunction::apply(q, k, v, cu_q, cu_k, max_q, max_k, scale);
+  return {r[0], r[1]};
 }
 
 // What Python's sdpa() and sdpa_varlen() call outside of tracing: straight to the dispatcher, without
