@@ -31,6 +31,7 @@ from typing import Optional
 
 import torch
 from torch import Tensor
+from torch.overrides import has_torch_function
 
 from . import _lib
 
@@ -205,8 +206,8 @@ def sdpa(
     _require(not is_causal, "is_causal=True is not supported (the reference's blocks are bidirectional)")
     _require(not enable_gqa, "enable_gqa is not supported")
     scale = 1.0 / math.sqrt(query.shape[-1]) if scale is None else float(scale)
-    if torch.compiler.is_compiling():  # tracing sees the op itself
-        return sdpa_fwd(query, key, value, scale)[0]
+    if torch.compiler.is_compiling() or has_torch_function((query, key, value)):
+        return sdpa_fwd(query, key, value, scale)[0]  # tracing and overrides see the op itself
     return (_native or _load_native()).sdpa(query, key, value, scale)
 
 
@@ -222,7 +223,7 @@ def sdpa_varlen(
 ) -> Tensor:
     """Bidirectional attention over packed ``[T, H, 64]`` tokens addressed by ``cu_seqlens``."""
     scale = 1.0 / math.sqrt(q.shape[-1]) if scale is None else float(scale)
-    if torch.compiler.is_compiling():  # tracing sees the op itself
+    if torch.compiler.is_compiling() or has_torch_function((q, k, v, cu_seqlens_q, cu_seqlens_k)):
         return sdpa_varlen_fwd(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q), int(max_seqlen_k), scale)[0]
     return (_native or _load_native()).sdpa_varlen(q, k, v, cu_seqlens_q, cu_seqlens_k, int(max_seqlen_q),
                                                    int(max_seqlen_k), scale)

@@ -59,3 +59,29 @@ def test_what_is_not_implemented_is_refused():
     q, k, v = dense(requires_grad=False)
     with pytest.raises(RuntimeError):
         torch.func.grad(lambda t: nanobrain_b200.sdpa(t, k, v).float().sum())(q)
+
+
+@pytest.mark.parametrize("case,name", [("dense", "sdpa_fwd"), ("packed", "sdpa_varlen_fwd")])
+def test_torch_function_overrides_see_the_op(case, name):
+    from torch.overrides import TorchFunctionMode
+
+    seen = []
+
+    class Mode(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    class Subclass(torch.Tensor):
+        @classmethod
+        def __torch_function__(cls, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return super().__torch_function__(func, types, args, kwargs or {})
+
+    qkv, call = CASES[case]()
+    with Mode():
+        call(*qkv)
+    assert f"nanobrain_b200.{name}.default" in seen
+    qkv = [t.detach().as_subclass(Subclass) for t in qkv]
+    seen.clear()
+    assert type(call(*qkv)) is Subclass and f"nanobrain_b200.{name}.default" in seen
