@@ -166,8 +166,21 @@ def aggregate(allstats, steps: int):
     }
 
 
+def workloads():
+    """``nanobrain_b200.workloads`` loaded by itself: both arms take their shapes from it, and the reference
+    arm, which is torch alone, must not import the package (its ops bring their native libraries)."""
+    import importlib.util
+
+    name = "bench_workloads"
+    if name not in sys.modules:
+        spec = importlib.util.spec_from_file_location(name, ROOT / "nanobrain_b200" / "workloads.py")
+        sys.modules[name] = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(sys.modules[name])
+    return sys.modules[name]
+
+
 def rank_lengths(args, rank: int, world: int):
-    from nanobrain_b200 import workloads as W
+    W = workloads()
 
     w = W.WORKLOADS[args.workload]
     if args.global_batch:
@@ -183,7 +196,7 @@ def cpu_reference_tflops(lengths, heads, budget_s: float, steps: int = 1, warmup
     batch, n chosen so that (steps + warmup) passes fit the budget. Returns (tflops, info)."""
     import torch
 
-    from nanobrain_b200 import workloads as W
+    W = workloads()
     from oracle import reference_cpu as R
 
     q, k, v, g = W.make_packed_inputs(lengths, heads, seed=0)
@@ -533,7 +546,7 @@ def copy_only_ms(host, host_out, dev, steps: int):
 
 def workload_config(args, w, world: int):
     """The `config` object, computed from shapes alone so that both arms print the same one."""
-    from nanobrain_b200 import workloads as W
+    W = workloads()
 
     per_rank = [rank_lengths(args, r, world)[1] for r in range(world)]
     tokens_all = sum(int(l.sum()) for l in per_rank)

@@ -98,3 +98,25 @@ def test_both_bench_arms_describe_the_same_config():
     strong = argparse.Namespace(workload="vitb_encoder_varlen", global_batch=256, gpus=8)
     cfg = bench.workload_config(strong, W.WORKLOADS["vitb_encoder_varlen"], 8)
     assert cfg["sequences_per_gpu"] == 32 and cfg["global_batch"] == 256
+
+
+def test_the_reference_arm_loads_nothing_of_the_package():
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    code = """
+import sys
+import bench
+from oracle import reference_cpu
+reference_cpu.time_packed_sample = lambda *args: (10.0, 1.0)  # (the computation itself is torch's)
+sys.argv = ["bench.py", "--impl", "reference", "--steps", "1", "--warmup", "1"]
+bench.main()
+assert not [m for m in sys.modules if m.split(".")[0] == "nanobrain_b200"]
+maps = open("/proc/self/maps").read()
+assert "libnb_attn" not in maps and "_nb_torch" not in maps
+"""
+    root = Path(__file__).resolve().parent.parent
+    run = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]
+    assert '"impl": "reference"' in run.stdout
