@@ -27,6 +27,7 @@ import ctypes as C
 import importlib.machinery
 import importlib.util
 import math
+import warnings
 from typing import Optional
 
 import torch
@@ -146,8 +147,11 @@ def _(d_out, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_se
 
 try:
     _load_native()
-except (RuntimeError, OSError, ImportError, AttributeError):
-    pass  # not built yet, or older than these sources: import (to build it) works, the first use raises
+except (RuntimeError, OSError, ImportError, AttributeError) as error:
+    # Not built yet, or older than these sources: import works all the same (to build it), the first use raises.
+    if BINDING_PATH.exists():
+        warnings.warn(f"nanobrain_b200: the native binding could not be loaded ({error}); its ops have no kernels. "
+                      "`python -m nanobrain_b200.build` rebuilds it.")
 
 
 # ------------------------------------------------------------------------------------------

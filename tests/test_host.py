@@ -100,3 +100,18 @@ def test_tensor_memory_is_taken_after_the_wait_for_the_predecessor():
     forward = forward[forward.index("extern __shared__ uint8_t smem_raw[];"):]
     # (a foreign kernel may follow the forward; what follows the backward's main kernel is its own epilogue)
     assert forward.index("tmem_alloc(") < forward.index("__syncthreads();") < forward.index("pdl_launch_dependents();")
+
+
+def test_a_binding_that_cannot_be_loaded_is_reported_at_import(tmp_path):
+    import shutil
+    import subprocess
+    import sys
+    from pathlib import Path
+
+    package = Path(ops.__file__).resolve().parent
+    shutil.copytree(package, tmp_path / package.name, ignore=shutil.ignore_patterns("__pycache__", "csrc", "_nb_torch.so"))
+    (tmp_path / package.name / "_nb_torch.so").write_bytes(b"not a library")
+    code = "import torch, nanobrain_b200; nanobrain_b200.sdpa(*[torch.zeros(1, 1, 4, 64, dtype=torch.bfloat16)] * 3)"
+    run = subprocess.run([sys.executable, "-c", code], cwd=tmp_path, capture_output=True, text=True, timeout=300)
+    assert "UserWarning: nanobrain_b200: the native binding could not be loaded" in run.stderr
+    assert run.returncode != 0 and "ImportError" in run.stderr.splitlines()[-1]
