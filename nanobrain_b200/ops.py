@@ -100,50 +100,52 @@ def _require(cond: bool, msg: str) -> None:
 # ------------------------------------------------------------------------------------------
 # The ops: schemas and fake kernels (same shapes and strides as the real results)
 # ------------------------------------------------------------------------------------------
-_library = torch.library.Library("nanobrain_b200", "DEF")
-for _schema in (
-    "sdpa_fwd(Tensor q, Tensor k, Tensor v, float scale) -> (Tensor, Tensor)",
-    "sdpa_bwd(Tensor d_out, Tensor q, Tensor k, Tensor v, Tensor out, Tensor lse, float scale)"
-    " -> (Tensor, Tensor, Tensor)",
-    "sdpa_varlen_fwd(Tensor q, Tensor k, Tensor v, Tensor cu_seqlens_q, Tensor cu_seqlens_k, SymInt max_seqlen_q,"
-    " SymInt max_seqlen_k, float scale) -> (Tensor, Tensor)",
-    "sdpa_varlen_bwd(Tensor d_out, Tensor q, Tensor k, Tensor v, Tensor out, Tensor lse, Tensor cu_seqlens_q,"
-    " Tensor cu_seqlens_k, SymInt max_seqlen_q, SymInt max_seqlen_k, float scale) -> (Tensor, Tensor, Tensor)",
-):
-    _library.define(_schema, tags=(torch.Tag.pt2_compliant_tag,))
-
-sdpa_fwd = torch.ops.nanobrain_b200.sdpa_fwd.default
-sdpa_bwd = torch.ops.nanobrain_b200.sdpa_bwd.default
-sdpa_varlen_fwd = torch.ops.nanobrain_b200.sdpa_varlen_fwd.default
-sdpa_varlen_bwd = torch.ops.nanobrain_b200.sdpa_varlen_bwd.default
-
-
 def _new_dense(like: Tensor) -> Tensor:
     b, h, l, d = like.shape
     return like.new_empty((b, l, h, d)).transpose(1, 2)
 
 
-@torch.library.register_fake("nanobrain_b200::sdpa_fwd", lib=_library)
-def _(q, k, v, scale):
-    b, h, lq, d = q.shape
-    return _new_dense(q), q.new_empty((b, h, lq), dtype=torch.float32)
+def _define_ops() -> torch.library.Library:
+    library = torch.library.Library("nanobrain_b200", "DEF")
+    for schema in (
+        "sdpa_fwd(Tensor q, Tensor k, Tensor v, float scale) -> (Tensor, Tensor)",
+        "sdpa_bwd(Tensor d_out, Tensor q, Tensor k, Tensor v, Tensor out, Tensor lse, float scale)"
+        " -> (Tensor, Tensor, Tensor)",
+        "sdpa_varlen_fwd(Tensor q, Tensor k, Tensor v, Tensor cu_seqlens_q, Tensor cu_seqlens_k, SymInt max_seqlen_q,"
+        " SymInt max_seqlen_k, float scale) -> (Tensor, Tensor)",
+        "sdpa_varlen_bwd(Tensor d_out, Tensor q, Tensor k, Tensor v, Tensor out, Tensor lse, Tensor cu_seqlens_q,"
+        " Tensor cu_seqlens_k, SymInt max_seqlen_q, SymInt max_seqlen_k, float scale) -> (Tensor, Tensor, Tensor)",
+    ):
+        library.define(schema, tags=(torch.Tag.pt2_compliant_tag,))
+
+    @torch.library.register_fake("nanobrain_b200::sdpa_fwd", lib=library)
+    def _(q, k, v, scale):
+        b, h, lq, d = q.shape
+        return _new_dense(q), q.new_empty((b, h, lq), dtype=torch.float32)
+
+    @torch.library.register_fake("nanobrain_b200::sdpa_bwd", lib=library)
+    def _(d_out, q, k, v, out, lse, scale):
+        return _new_dense(q), _new_dense(k), _new_dense(v)
+
+    @torch.library.register_fake("nanobrain_b200::sdpa_varlen_fwd", lib=library)
+    def _(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, scale):
+        tq, h, d = q.shape
+        return q.new_empty((tq, h, d)), q.new_empty((h, tq), dtype=torch.float32)
+
+    @torch.library.register_fake("nanobrain_b200::sdpa_varlen_bwd", lib=library)
+    def _(d_out, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, scale):
+        return q.new_empty(q.shape), k.new_empty(k.shape), k.new_empty(k.shape)
+
+    return library
 
 
-@torch.library.register_fake("nanobrain_b200::sdpa_bwd", lib=_library)
-def _(d_out, q, k, v, out, lse, scale):
-    return _new_dense(q), _new_dense(k), _new_dense(v)
+if "_library" not in globals():  # (a reload of this module keeps them)
+    _library = _define_ops()
 
-
-@torch.library.register_fake("nanobrain_b200::sdpa_varlen_fwd", lib=_library)
-def _(q, k, v, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, scale):
-    tq, h, d = q.shape
-    return q.new_empty((tq, h, d)), q.new_empty((h, tq), dtype=torch.float32)
-
-
-@torch.library.register_fake("nanobrain_b200::sdpa_varlen_bwd", lib=_library)
-def _(d_out, q, k, v, out, lse, cu_seqlens_q, cu_seqlens_k, max_seqlen_q, max_seqlen_k, scale):
-    return q.new_empty(q.shape), k.new_empty(k.shape), k.new_empty(k.shape)
-
+sdpa_fwd = torch.ops.nanobrain_b200.sdpa_fwd.default
+sdpa_bwd = torch.ops.nanobrain_b200.sdpa_bwd.default
+sdpa_varlen_fwd = torch.ops.nanobrain_b200.sdpa_varlen_fwd.default
+sdpa_varlen_bwd = torch.ops.nanobrain_b200.sdpa_varlen_bwd.default
 
 try:
     _load_native()
@@ -188,7 +190,9 @@ def _register_flop_formulas() -> None:
         return 10 * q.shape[1] * q.shape[2] * _pair_sum(cu_q, cu_k)
 
 
-_register_flop_formulas()
+if not globals().get("_flop_formulas"):
+    _register_flop_formulas()
+    _flop_formulas = True
 
 
 # ------------------------------------------------------------------------------------------

@@ -115,3 +115,19 @@ def test_a_binding_that_cannot_be_loaded_is_reported_at_import(tmp_path):
     run = subprocess.run([sys.executable, "-c", code], cwd=tmp_path, capture_output=True, text=True, timeout=300)
     assert "UserWarning: nanobrain_b200: the native binding could not be loaded" in run.stderr
     assert run.returncode != 0 and "ImportError" in run.stderr.splitlines()[-1]
+
+
+def test_the_ops_module_can_be_reloaded():
+    import subprocess
+    import sys
+
+    code = """
+import importlib, torch, nanobrain_b200
+from nanobrain_b200 import ops
+importlib.reload(ops)
+q = torch.empty(2, 3, 5, 64, dtype=torch.bfloat16, device="meta", requires_grad=True)
+ops.sdpa(q, q, q).sum().backward()
+assert q.grad.shape == q.shape
+"""
+    run = subprocess.run([sys.executable, "-c", code], cwd=W.__file__.rsplit("/", 2)[0], capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-1000:]
