@@ -29,20 +29,45 @@ using OptTensor = std::optional<Tensor>;
 constexpr int kBlockParams = 16;  // norm1 w b, q w b, k w b, v w b, proj w b, norm2 w b, fc1 w b, fc2 w b
 constexpr int64_t kHeadDim = 64;
 
-bool plain_param(const Tensor& t, const Tensor& like) {
-  return t.scalar_type() == at::kFloat && t.device() == like.device() && t.is_contiguous();
+// Can the kernels read this tensor in place: plain contiguous fp32 on one device, 16-byte aligned?
+bool readable(const Tensor& t, const Tensor& like) {
+  return t.scalar_type() == at::kFloat && t.device() == like.device() && t.layout() == at::kStrided &&
+         !t.unsafeGetTensorImpl()->is_python_dispatch() && t.has_storage() && !t.is_neg() && t.is_contiguous() &&
+         (reinterpret_cast<uintptr_t>(t.const_data_ptr()) & 15u) == 0;
 }
 
-// Are these parameters what encode_images takes?
-bool plain_params(const std::vector<OptTensor>& params, const Tensor& like) {
-  for (const OptTensor& t : params)
-    if (t.has_value() && !plain_param(*t, like)) return false;
+// Are these parameters, in the order of encode_images, what it takes? (Anything else is for the modules.)
+bool takes_params(const std::vector<OptTensor>& stem, const std::vector<OptTensor>& blocks) {
+  if (stem.size() != 8 || blocks.empty() || blocks.size() % kBlockParams != 0 || !stem[2].has_value()) return false;
+  const Tensor& like = *stem[2];
+  if (like.dim() != 2) return false;
+  const int64_t dim = like.size(1);
+  for (const auto* list : {&stem, &blocks})
+    for (const OptTensor& t : *list)
+      if (t.has_value() && !readable(*t, like)) return false;
+  auto is = [](const OptTensor& t, at::IntArrayRef sizes) { return t.has_value() && t->sizes() == sizes; };
+  auto absent_or = [&](const OptTensor& t, at::IntArrayRef sizes) { return !t.has_value() || t->sizes() == sizes; };
+  auto matrix = [](const OptTensor& t) { return t.has_value() && t->dim() == 2; };
+  auto norm = [&](const OptTensor& w, const OptTensor& b) { return is(w, {dim}) && is(b, {dim}); };
+  if (!matrix(stem[0]) || stem[0]->size(0) != dim || !absent_or(stem[1], {dim}) || !norm(stem[6], stem[7])) return false;
+  for (int i : {3, 4})
+    if (!matrix(stem[i]) || stem[i]->size(1) != dim) return false;
+  if (stem[5].has_value() && (stem[5]->dim() != 3 || stem[5]->size(0) != 1 || stem[5]->size(2) != dim)) return false;
+  for (size_t at = 0; at < blocks.size(); at += kBlockParams) {
+    const OptTensor* b = blocks.data() + at;
+    for (int i : {2, 4, 6, 8})
+      if (!is(b[i], {dim, dim}) || !absent_or(b[i + 1], {dim})) return false;
+    if (b[3].has_value() != b[5].has_value() || b[3].has_value() != b[7].has_value()) return false;
+    if (!norm(b[0], b[1]) || !norm(b[10], b[11]) || !matrix(b[12])) return false;
+    const int64_t hidden = b[12]->size(0);
+    if (hidden % 8 != 0 || !is(b[12], {hidden, dim}) || !absent_or(b[13], {hidden})) return false;
+    if (!is(b[14], {dim, hidden}) || !absent_or(b[15], {dim})) return false;
+  }
   return true;
 }
 
 void check_param(const Tensor& t, const Tensor& like) {
-  TORCH_CHECK(plain_param(t, like) && (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0,
-              "nanobrain_b200 encoder: parameters must be contiguous float32 on one device");
+  TORCH_CHECK(readable(t, like), "nanobrain_b200 encoder: parameters must be contiguous float32 on one device");
 }
 
 // bf16 copies of fp32 parameters in one buffer, cast together.
@@ -284,7 +309,7 @@ std::tuple<Tensor, std::vector<Tensor>> encode_images(const std::vector<Tensor>&
 namespace nbt {
 
 void bind_encoder(pybind11::module_& m) {
-  m.def("plain_params", &plain_params);
+  m.def("takes_params", &takes_params);
   m.def("encode_images", &encode_images, pybind11::call_guard<pybind11::gil_scoped_release>());
 }
 

@@ -357,24 +357,30 @@ class ViTMAE3D(nn.Module):
                 return None
             heads = attn.num_heads
             for m in (n1, *linears[:4], n2, *linears[4:]):
-                blocks += [m._parameters["weight"], m._parameters["bias"]]
+                blocks += [m._parameters.get("weight"), m._parameters.get("bias")]
             eps += [n1.eps, n2.eps]
         eps.append(self.norm.eps)
-        pos = self.pos_embed
-        head = [self.patch_embed.weight, self.patch_embed.bias, wx, pos.weight_y, pos.weight_z, self.cls_token,
-                self.norm.weight, self.norm.bias]
-        if not ops._load_native().plain_params(head + blocks, wx):
+        pos, cls = self.pos_embed, self.cls_token
+        head = [self.patch_embed._parameters.get("weight"), self.patch_embed._parameters.get("bias"), wx, pos.weight_y,
+                pos.weight_z, cls, self.norm._parameters.get("weight"), self.norm._parameters.get("bias")]
+        if not ops._load_native().takes_params(head, blocks):
+            return None
+        tables = (wx, pos.weight_y, pos.weight_z)
+        if any(t.shape[0] < size // p for t, size, p in zip(tables, self.grid_size, self.patch_size)):
+            return None
+        if dim != self.embed_dim or (cls.shape[1] if cls is not None else 0) != self.class_tokens:
             return None
         patches_per_image = self.coord_grid.shape[1]
         for pt, m in samples:
             if (pt.dtype != torch.float32 or m.dtype != torch.bool or tuple(pt.shape) != (patches_per_image, patch_dim)
-                    or m.numel() != patches_per_image):
+                    or tuple(m.shape) != (patches_per_image,)):
                 return None
         return head, blocks, eps, heads
 
     def _embed_native(self, samples, return_dense, head, blocks, eps, heads) -> List[dict]:
         device = head[2].device
         patches = [pt.to(device).contiguous() for pt, _ in samples]
+        patches = [pt if pt.data_ptr() % 16 == 0 else pt.clone() for pt in patches]  # the gather reads 16 bytes at a time
         masks = [m.to(device).contiguous() for _, m in samples]
         means, dense = ops._load_native().encode_images(patches, masks, self.coord_grid[0].contiguous(), head, blocks,
                                                         eps, heads, return_dense)

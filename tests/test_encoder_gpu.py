@@ -94,3 +94,61 @@ def test_gelu_of_every_bf16_value(copies):
     want = torch.nn.functional.gelu(v)
     nan = torch.isnan(want)
     assert torch.equal(torch.isnan(got), nan) and torch.equal(got[~nan], want[~nan])
+
+
+def alone(model, samples):
+    """The reference's loop: one dense forward of the modules per image."""
+    out = []
+    for patches, mask in samples:
+        with torch.inference_mode(), torch.autocast("cuda", dtype=torch.bfloat16):
+            tokens = model.forward_encoder(patches[mask][None], model.coord_grid[:, mask])[0, model.class_tokens:].float()
+        out.append(tokens.mean(0))
+    return out
+
+
+def flat_parameters(model, offset):
+    """Every parameter a view of one buffer, `offset` elements past a 16-byte boundary."""
+    params = [p for p in model.parameters()]
+    flat = torch.empty(sum((p.numel() + 3) // 4 * 4 for p in params) + 4, device=DEV)
+    at = offset
+    for p in params:
+        view = flat[at:at + p.numel()].view_as(p)
+        view.copy_(p.data)
+        p.data = view
+        at += (p.numel() + 3) // 4 * 4
+
+
+def without(model, names):
+    for name in names:
+        model.blocks[1].get_submodule(name.rsplit(".", 1)[0]).register_parameter(name.rsplit(".", 1)[1], None)
+
+
+@pytest.mark.parametrize("change,native", [
+    (lambda m: None, True),
+    (lambda m: flat_parameters(m, 0), True),
+    (lambda m: flat_parameters(m, 1), False),
+    (lambda m: without(m, ["norm1.weight", "norm1.bias"]), False),
+    (lambda m: without(m, ["norm2.bias"]), False),
+    (lambda m: without(m, ["attn.k.bias"]), False),
+    (lambda m: setattr(m.blocks[0], "mlp", M.Mlp(128, mlp_ratio=2.7, bias=True).to(DEV)), False),  # 345 columns
+])
+@pytest.mark.parametrize("counts", [[31, 40], [30, 41, 1]])
+def test_parameters_that_the_kernels_do_not_take(change, native, counts):
+    model = build(2, 1)
+    change(model)
+    samples = images(model, counts)
+    assert (model._native_encoder(samples) is not None) == native
+    got = model.embed_packed(samples)
+    ops.check_status()
+    for a, b in zip(got, alone(model, samples)):
+        assert (a["global_embedding"] - b).abs().max() <= 3e-2 * b.abs().max()
+
+
+@pytest.mark.parametrize("offset", [1, 2, 4])
+def test_patches_that_start_anywhere(offset):
+    model = build(2, 1)
+    samples = images(model, [31, 40])
+    want = model.embed_packed(samples)
+    moved = [(torch.empty(p.numel() + offset, device=DEV)[offset:].view_as(p).copy_(p), m) for p, m in samples]
+    for a, b in zip(model.embed_packed(moved), want):
+        assert torch.equal(a["global_embedding"], b["global_embedding"])
