@@ -33,7 +33,7 @@ from torch import Tensor
 
 from . import ops
 from . import token_prep as T
-from .modules import Attention, Block, LayerNorm, Mlp, SeparablePosEmbed3D
+from .modules import Attention, Block, DropPath, LayerNorm, Mlp, SeparablePosEmbed3D
 
 
 def patchify3d(x: Tensor, patch_size: int = 8) -> Tensor:
@@ -329,12 +329,16 @@ class ViTMAE3D(nn.Module):
     def _native_encoder(self, samples):
         """The encoder's parameters as ``csrc/torch_encoder.cpp`` takes them, or None where that does
         not apply: CPU, other types than fp32 parameters and patches, modules that are not the ones this
-        file builds (or carry hooks), active stochastic depth."""
-        stem = (self.patch_embed, self.pos_embed, self.norm)
-        wx = self.pos_embed.weight_x if type(self.pos_embed) is SeparablePosEmbed3D else None
-        if wx is None or not wx.is_cuda or len(samples) == 0 or len(self.blocks) == 0 or self.pos_embed.unit != 1.0:
+        file builds or that someone has changed or watches (``_plain``), active stochastic depth."""
+        if _global_hooks() or any(cls.forward is not forward for cls, forward in _FORWARDS.items()):
             return None
-        if type(self.patch_embed) is not nn.Linear or type(self.norm) is not nn.LayerNorm or _hooked(self, *stem):
+        if type(self).forward_encoder_packed is not _FORWARD_ENCODER_PACKED or "forward_encoder_packed" in vars(self):
+            return None
+        if not (_plain(self.patch_embed, nn.Linear) and _plain(self.pos_embed, SeparablePosEmbed3D)
+                and _plain(self.norm, nn.LayerNorm)):
+            return None
+        wx = self.pos_embed.weight_x
+        if not wx.is_cuda or len(samples) == 0 or len(self.blocks) == 0 or self.pos_embed.unit != 1.0:
             return None
         dim, patch_dim = wx.shape[1], self.patch_embed.in_features
         if dim % 64 or dim > 1024 or patch_dim % 4:
@@ -342,19 +346,17 @@ class ViTMAE3D(nn.Module):
         blocks, eps = [], []
         heads = None
         for blk in self.blocks:
-            sub = blk._modules
-            n1, attn, n2, mlp = sub.get("norm1"), sub.get("attn"), sub.get("norm2"), sub.get("mlp")
-            if (type(blk) is not Block or type(attn) is not Attention or type(mlp) is not Mlp or blk.training and
-                    not (type(blk.drop_path1) is nn.Identity and type(blk.drop_path2) is nn.Identity)):
+            if not (_plain(blk, Block) and _plain(blk.attn, Attention) and _plain(blk.mlp, Mlp)):
                 return None
-            am, mm = attn._modules, mlp._modules
-            linears = (am["q"], am["k"], am["v"], am["proj"], mm["fc1"], mm["fc2"])
-            if type(mm["act"]) is not nn.GELU or mm["act"].approximate != "none":
+            n1, attn, n2, mlp, act = blk.norm1, blk.attn, blk.norm2, blk.mlp, blk.mlp.act
+            linears = (attn.q, attn.k, attn.v, attn.proj, mlp.fc1, mlp.fc2)
+            if not (all(_plain(m, nn.Linear) for m in linears) and _plain(n1, nn.LayerNorm) and _plain(n2, nn.LayerNorm)):
                 return None
-            if any(type(m) is not nn.Linear for m in linears) or type(n1) is not nn.LayerNorm or type(n2) is not nn.LayerNorm:
+            if not _plain(act, nn.GELU) or act.approximate != "none" or heads not in (None, attn.num_heads):
                 return None
-            if _hooked(blk, n1, attn, n2, mlp, mm["act"], *linears) or heads not in (None, attn.num_heads):
-                return None
+            for drop in (blk.drop_path1, blk.drop_path2):
+                if not (_plain(drop, nn.Identity) or _plain(drop, DropPath) and not (drop.training and drop.drop_prob)):
+                    return None
             heads = attn.num_heads
             for m in (n1, *linears[:4], n2, *linears[4:]):
                 blocks += [m._parameters.get("weight"), m._parameters.get("bias")]
@@ -395,7 +397,18 @@ class ViTMAE3D(nn.Module):
         return outputs
 
 
-def _hooked(*modules: nn.Module) -> bool:
-    """Does any forward hook want to see one of these modules run?"""
-    return bool(nn.modules.module._global_forward_hooks or nn.modules.module._global_forward_pre_hooks) or any(
-        m._forward_hooks or m._forward_pre_hooks for m in modules)
+# What the native encoder stands for.
+_FORWARDS = {cls: cls.forward for cls in (Block, Attention, Mlp, DropPath, SeparablePosEmbed3D, nn.Linear, nn.LayerNorm,
+                                          nn.GELU, nn.Identity)}
+_FORWARD_ENCODER_PACKED = ViTMAE3D.forward_encoder_packed
+
+
+def _plain(module: nn.Module, cls: type) -> bool:
+    """Is this a ``cls`` that runs the class's own forward, with no forward hooks around it and not compiled?"""
+    state = vars(module)
+    return (type(module) is cls and "forward" not in state and not state["_forward_hooks"]
+            and not state["_forward_pre_hooks"] and state.get("_compiled_call_impl") is None)
+
+
+def _global_hooks() -> bool:
+    return bool(nn.modules.module._global_forward_hooks or nn.modules.module._global_forward_pre_hooks)

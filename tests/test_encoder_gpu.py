@@ -152,3 +152,58 @@ def test_patches_that_start_anywhere(offset):
     moved = [(torch.empty(p.numel() + offset, device=DEV)[offset:].view_as(p).copy_(p), m) for p, m in samples]
     for a, b in zip(model.embed_packed(moved), want):
         assert torch.equal(a["global_embedding"], b["global_embedding"])
+
+
+class Halved(torch.nn.Module):
+    def forward(self, x):
+        return x * 0.5
+
+
+class Subclass(M.ViTMAE3D):
+    def forward_encoder_packed(self, *args, **kwargs):
+        x, *rest = super().forward_encoder_packed(*args, **kwargs)
+        return (x * 0.5, *rest)
+
+
+def replaced_forward(module):
+    original = module.forward
+    module.forward = lambda *args, **kwargs: original(*args, **kwargs) * 0.5
+
+
+@pytest.mark.parametrize("change", [
+    lambda m: replaced_forward(m.blocks[1].attn),
+    lambda m: replaced_forward(m.blocks[1].mlp.fc2),
+    lambda m: replaced_forward(m.norm),
+    lambda m: setattr(m.blocks[0], "drop_path2", Halved()),
+    lambda m: setattr(m, "__class__", Subclass),
+], ids=["attn.forward", "fc2.forward", "norm.forward", "drop_path2", "subclass"])
+def test_changed_modules_are_run(change):
+    model = build(2, 1)
+    samples = images(model, [31, 40])
+    before = model.embed_packed(samples)
+    change(model)
+    assert model._native_encoder(samples) is None
+    got = [o["global_embedding"] for o in model.embed_packed(samples)]
+    # (alone() goes through forward_encoder, which the subclass does not change)
+    want = [o["global_embedding"] * 0.5 for o in before] if type(model) is Subclass else alone(model, samples)
+    for a, b, c in zip(got, want, before):
+        assert (a - b).abs().max() <= 3e-2 * b.abs().max()
+        assert (a - c["global_embedding"]).norm() > 0.05 * a.norm()
+
+
+def test_compiled_and_watched_blocks_are_run():
+    model = build(2, 1)
+    samples = images(model, [31, 40])
+    ran = []
+    model.blocks[0].compile(backend=lambda graph, inputs: lambda *args: ran.append(1) or graph(*args))
+    assert model._native_encoder(samples) is None
+    model.embed_packed(samples)
+    assert ran
+    model = build(2, 1)
+    handle = model.blocks[1].drop_path1.register_forward_hook(lambda *args: ran.append(2))
+    model.embed_packed(samples)
+    handle.remove()
+    assert 2 in ran and model._native_encoder(samples) is not None
+    drops = M.ViTMAE3D(grid_size=(24, 16, 20), patch_size=4, depth=2, embed_dim=128, num_heads=2, decoder_depth=0,
+                       decoder_embed_dim=64, decoder_num_heads=1, drop_path_rate=0.5).to(DEV)
+    assert drops.train()._native_encoder(samples) is None and drops.eval()._native_encoder(samples) is not None
