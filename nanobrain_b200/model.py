@@ -30,6 +30,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 from torch import Tensor
+from torch.utils._device import DeviceContext
 
 from . import ops
 from . import token_prep as T
@@ -329,8 +330,9 @@ class ViTMAE3D(nn.Module):
     def _native_encoder(self, samples):
         """The encoder's parameters as ``csrc/torch_encoder.cpp`` takes them, or None where that does
         not apply: CPU, other types than fp32 parameters and patches, modules that are not the ones this
-        file builds or that someone has changed or watches (``_plain``), active stochastic depth."""
-        if _global_hooks() or any(cls.forward is not forward for cls, forward in _FORWARDS.items()):
+        file builds or that someone has changed or watches (``_plain``), active stochastic depth, a mode or a
+        tracer that is to see the operations."""
+        if _observed() or _global_hooks() or any(cls.forward is not forward for cls, forward in _FORWARDS.items()):
             return None
         if type(self).forward_encoder_packed is not _FORWARD_ENCODER_PACKED or "forward_encoder_packed" in vars(self):
             return None
@@ -412,3 +414,11 @@ def _plain(module: nn.Module, cls: type) -> bool:
 
 def _global_hooks() -> bool:
     return bool(nn.modules.module._global_forward_hooks or nn.modules.module._global_forward_pre_hooks)
+
+
+def _observed() -> bool:
+    """Is there a mode (FLOP counter, fake tensors, logging, ...), a tracer or a compiler that sees torch's operations?
+    (``with torch.device(...)`` is a mode that only places new tensors.)"""
+    modes = torch.overrides._get_current_function_mode_stack()
+    return (torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack() > 0
+            or any(not isinstance(mode, DeviceContext) for mode in modes))

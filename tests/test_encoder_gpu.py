@@ -207,3 +207,27 @@ def test_compiled_and_watched_blocks_are_run():
     drops = M.ViTMAE3D(grid_size=(24, 16, 20), patch_size=4, depth=2, embed_dim=128, num_heads=2, decoder_depth=0,
                        decoder_embed_dim=64, decoder_num_heads=1, drop_path_rate=0.5).to(DEV)
     assert drops.train()._native_encoder(samples) is None and drops.eval()._native_encoder(samples) is not None
+
+
+def test_modes_see_the_operations():
+    from torch.overrides import TorchFunctionMode
+    from torch.utils.flop_counter import FlopCounterMode
+
+    model = build(2, 1)
+    samples = images(model, [31, 40])
+    with FlopCounterMode(display=False) as counter:
+        model.embed_packed(samples)
+    rows, pairs = 31 + 40 + 2, 32 ** 2 + 41 ** 2
+    assert counter.get_total_flops() == 2 * 71 * 64 * 128 + 2 * (2 * rows * 12 * 128 ** 2 + 4 * 128 * pairs)
+    seen = []
+
+    class Mode(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(func)
+            return func(*args, **(kwargs or {}))
+
+    with Mode():
+        model.embed_packed(samples)
+    assert torch.nn.functional.layer_norm in seen
+    with torch.device(DEV):  # only places new tensors
+        assert model._native_encoder(samples) is not None
