@@ -15,6 +15,7 @@
 #include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <exception>
 #include <optional>
 #include <vector>
 
@@ -99,10 +100,12 @@ struct Casts {
     }
     return s;
   }
-  void run(const Tensor& like, cudaStream_t stream) {
+  void allocate(const Tensor& like) {
     buffer = at::empty({total}, like.options().dtype(at::kBFloat16));
     auto* base = static_cast<at::BFloat16*>(buffer.data_ptr());
     for (size_t i = 0; i < items.size(); ++i) items[i].dst = base + offsets[i];
+  }
+  void run(cudaStream_t stream) const {
     nbt::check_rc(nb_enc_cast(items.data(), int(items.size()), stream), "nb_enc_cast");
   }
   Tensor view(int64_t offset, at::IntArrayRef sizes, at::IntArrayRef strides) const {
@@ -110,6 +113,15 @@ struct Casts {
                                                         buffer.key_set(), buffer.dtype());
     t.unsafeGetTensorImpl()->set_sizes_and_strides(sizes, strides, offset);
     return t;
+  }
+};
+
+// Waits for a stream at the end of a scope that is left by an exception.
+struct Finished {
+  cudaStream_t stream;
+  const int exceptions = std::uncaught_exceptions();
+  ~Finished() {
+    if (std::uncaught_exceptions() > exceptions) cudaStreamSynchronize(stream);
   }
 };
 
@@ -171,25 +183,7 @@ std::tuple<Tensor, std::vector<Tensor>> encode_images(const std::vector<Tensor>&
   }
   const bool has_cls = stem[5].has_value();
   const int class_tokens = has_cls ? int(stem[5]->size(-2)) : 0;
-  Tensor ids = at::empty({n_images, n_patches}, i32), rank = at::empty({n_images, n_patches}, i32);
-  Tensor counts = at::empty({n_images}, i32), cu = at::empty({n_images + 1}, i32), cu_r = at::empty({n_images + 1}, i32);
-  Tensor host_counts = at::empty({n_images}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
-  auto chunks = [&](auto f) {
-    for (int64_t at = 0; at < n_images; at += NB_ENC_MAX_IMAGES)
-      f(int(at), int(std::min<int64_t>(NB_ENC_MAX_IMAGES, n_images - at)));
-  };
-  chunks([&](int first, int n) {
-    nbt::check_rc(nb_enc_select(mask_ptrs.data() + first, first, n, int(n_patches), ids.data_ptr<int32_t>(),
-                                rank.data_ptr<int32_t>(), counts.data_ptr<int32_t>(), stream),
-                  "nb_enc_select");
-  });
-  nbt::check_rc(nb_enc_offsets(counts.data_ptr<int32_t>(), int(n_images), class_tokens, cu.data_ptr<int32_t>(),
-                               cu_r.data_ptr<int32_t>(), host_counts.data_ptr<int32_t>(), stream),
-                "nb_enc_offsets");
-  at::cuda::CUDAEvent counted;
-  counted.record(at::cuda::getCurrentCUDAStream());
-
-  // bf16 weights, cast while the host waits for the counts.
+  // What can be wrong with the parameters is found before anything is launched.
   Casts casts;
   const auto w_patch = casts.add({&stem[0]}, table_x), b_patch = casts.add({&stem[1]}, table_x);
   std::vector<BlockWeights> weights(depth);
@@ -207,7 +201,7 @@ std::tuple<Tensor, std::vector<Tensor>> encode_images(const std::vector<Tensor>&
   norms.push_back(make_norm(stem[6], stem[7], eps[2 * depth], table_x));
   for (int i : {2, 3, 4}) check_param(*stem[i], table_x);
   if (has_cls) check_param(*stem[5], table_x);
-  casts.run(table_x, stream);
+  casts.allocate(table_x);
   const Product patch_product(casts, w_patch, b_patch);
   std::vector<Product> products;
   products.reserve(4 * depth);
@@ -217,6 +211,28 @@ std::tuple<Tensor, std::vector<Tensor>> encode_images(const std::vector<Tensor>&
     products.emplace_back(casts, w.w1, w.b1);
     products.emplace_back(casts, w.w2, w.b2);
   }
+
+  Tensor ids = at::empty({n_images, n_patches}, i32), rank = at::empty({n_images, n_patches}, i32);
+  Tensor counts = at::empty({n_images}, i32), cu = at::empty({n_images + 1}, i32), cu_r = at::empty({n_images + 1}, i32);
+  // A kernel writes the counts into pinned host memory, which the caching host allocator may hand out again as soon as
+  // the tensor is gone: whichever way this function is left, the write has happened before that.
+  Tensor host_counts = at::empty({n_images}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+  const Finished counts_written{stream};
+  auto chunks = [&](auto f) {
+    for (int64_t at = 0; at < n_images; at += NB_ENC_MAX_IMAGES)
+      f(int(at), int(std::min<int64_t>(NB_ENC_MAX_IMAGES, n_images - at)));
+  };
+  chunks([&](int first, int n) {
+    nbt::check_rc(nb_enc_select(mask_ptrs.data() + first, first, n, int(n_patches), ids.data_ptr<int32_t>(),
+                                rank.data_ptr<int32_t>(), counts.data_ptr<int32_t>(), stream),
+                  "nb_enc_select");
+  });
+  nbt::check_rc(nb_enc_offsets(counts.data_ptr<int32_t>(), int(n_images), class_tokens, cu.data_ptr<int32_t>(),
+                               cu_r.data_ptr<int32_t>(), host_counts.data_ptr<int32_t>(), stream),
+                "nb_enc_offsets");
+  at::cuda::CUDAEvent counted;
+  counted.record(at::cuda::getCurrentCUDAStream());
+  casts.run(stream);  // while the host waits for the counts
 
   counted.synchronize();
   const int32_t* n_tokens = host_counts.data_ptr<int32_t>();

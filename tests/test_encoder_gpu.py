@@ -231,3 +231,21 @@ def test_modes_see_the_operations():
     assert torch.nn.functional.layer_norm in seen
     with torch.device(DEV):  # only places new tensors
         assert model._native_encoder(samples) is not None
+
+
+def test_refused_parameters_leave_no_write_behind():
+    # A refusal comes before anything is launched: the pinned words for the patch counts go back to their
+    # allocator, and the next owner must not see a kernel write to them.
+    model = build(2, 1)
+    samples = images(model, [31, 40, 5])
+    head, blocks, eps, heads = model._native_encoder(samples)
+    coord = model.coord_grid[0].contiguous()
+    patches, masks = [p for p, _ in samples], [m for _, m in samples]
+    blocks = list(blocks)
+    blocks[-6] = None  # norm2.weight of the last block
+    torch.cuda._sleep(20_000_000)  # about 10 ms: what is launched now runs later
+    with torch.inference_mode(), pytest.raises(RuntimeError, match="LayerNorm"):
+        ops._load_native().encode_images(patches, masks, coord, head, blocks, eps, heads, False)
+    words = [torch.full((3,), -7, dtype=torch.int32).pin_memory() for _ in range(4)]
+    torch.cuda.synchronize()
+    assert all(w.tolist() == [-7] * 3 for w in words)
