@@ -627,7 +627,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         uint32_t w[16];
         tmem_ld16(o_addr + 64, w);
         tmem_wait_ld();
-        w_run = fmaf(l_run, 0.f, __uint_as_float(w[0]));
+        // (A sequence of one tile has its max as the offset, whose P is exactly 1: nothing to gain there.)
+        w_run = lk <= kTile && meta.part < 0 ? l_run : fmaf(l_run, 0.f, __uint_as_float(w[0]));
       }
       if (meta.part >= 0) {
         // This CTA's part of a cut unit: O as it is, then offset and sum of every row. O is laid out as 16
