@@ -118,3 +118,49 @@ def test_many_short_units_per_persistent_cta_match_the_oracle():
         assert np.isfinite(err).all(), name
         assert err.max() <= MAX_ABS * max(1.0, np.abs(b).max()) and err.mean() <= MEAN_ABS, (name, err.max(), err.mean())
 
+
+
+@pytest.mark.parametrize("lengths,spare", [
+    ([820], 0), ([127, 129, 256, 1, 0, 700], 0), ([200] * 30 + [2000], 70),
+    (torch.randint(0, 1500, (400,), generator=torch.Generator().manual_seed(2)).tolist(), 300),
+])
+def test_the_lists_that_the_calls_build(lengths, spare):
+    # What a forward and a backward leave in their workspaces: every tile once, most expensive first, in one cost class
+    # the full tiles before the ragged ones, the first entry's counters as in a new list (forward).
+    import ctypes as C
+
+    heads, total = 2, sum(lengths) + spare
+    g = torch.Generator(device=DEV).manual_seed(len(lengths))
+    q, k, v, d_out = (torch.randn(total, heads, 64, generator=g, device=DEV).to(torch.bfloat16) for _ in range(4))
+    out, dq, dk, dv = (torch.empty_like(q) for _ in range(4))
+    lse = torch.empty(heads, total, device=DEV)
+    cu = torch.tensor([0] + lengths).cumsum(0).to(DEV, torch.int32)
+    shape = _lib.Shape(len(lengths), heads, 64, max(lengths), max(lengths), total, total, cu.data_ptr(), cu.data_ptr(), 0.125)
+    fwd_ws = torch.empty(_lib.fwd_workspace_bytes(shape), dtype=torch.uint8, device=DEV)
+    bwd_ws = torch.empty(_lib.bwd_workspace_bytes(shape), dtype=torch.uint8, device=DEV)
+    d = lambda t: _lib.Tensor(t.data_ptr(), 0, t.stride(0), t.stride(1))
+    lib, stream = _lib.load(), C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    fwd = _lib.FwdArgs(shape, d(q), d(k), d(v), d(out), lse.data_ptr(), None, fwd_ws.data_ptr(), fwd_ws.numel())
+    bwd = _lib.BwdArgs(shape, d(q), d(k), d(v), d(out), d(d_out), d(dq), d(dk), d(dv), lse.data_ptr(), bwd_ws.data_ptr(),
+                       bwd_ws.numel(), None, None, None)
+    _lib.check(lib.nb_attn_fwd(C.byref(fwd), stream), "nb_attn_fwd")
+    _lib.check(lib.nb_attn_bwd(C.byref(bwd), stream), "nb_attn_bwd")
+    torch.cuda.synchronize()
+    n = schedule.capacity(total, len(lengths))
+    lists_ = [fwd_ws.view(torch.int32).reshape(-1, 8), bwd_ws[-n * 32:].view(torch.int32).reshape(-1, 8)]
+    starts = cu.tolist()
+    own = list(lengths) + [spare]
+    cost = [(length + 127) // 128 for length in lengths] + [0]
+    want = [(i, t) for i, length in enumerate(own) for t in range((length + 127) // 128)]
+    for items in lists_:
+        rows = items.cpu().tolist()
+        used = [r for r in rows if r[0] >= 0]
+        assert rows[:len(used)] == used and len(rows) == n             # unused entries at the end
+        assert sorted((r[0], r[1]) for r in used) == want              # every tile, once
+        for seq, _, own_begin, own_len, other_begin, other_len, *_ in used:
+            assert (own_begin, own_len) == (starts[seq], own[seq])
+            assert seq == len(lengths) or (other_begin, other_len) == (starts[seq], lengths[seq])
+        order = [(-cost[r[0]], r[1] == own[r[0]] // 128) for r in used]  # (cost class, ragged)
+        assert order == sorted(order)
+        assert all(r[6:] == [0, 0] for r in rows[1:])
+    assert lists_[0][0, 6:].tolist() == [0, 0]

@@ -15,6 +15,10 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
+def dense_shape(batch, heads, lq, lk):
+    return _lib.Shape(batch, heads, 64, lq, lk, batch * lq, batch * lk, None, None, 0.125)
+
+
 def check(names, got, want):
     for name, a, b in zip(names, got, want):
         b = np.asarray(b, dtype=np.float32)
@@ -62,6 +66,7 @@ def test_second_pass_over_the_keys(lk):
 def test_query_tiles_cut_between_ctas(batch, heads, lq, lk, rising):
     # Few query tiles and many keys: the dense forward gives every CTA an equal run of key tiles and
     # puts the parts of a query tile together afterwards; `rising` scores need the second walk as well.
+    assert _lib.load().nb_attn_fwd_split_workspace_bytes(C.byref(dense_shape(batch, heads, lq, lk))) > 0
     g = torch.Generator().manual_seed(lq + lk)
     q = torch.randn(batch, heads, lq, 64, generator=g)
     k, v = (torch.randn(batch, heads, lk, 64, generator=g) for _ in range(2))
@@ -78,11 +83,12 @@ def test_query_tiles_cut_between_ctas(batch, heads, lq, lk, rising):
 
 
 @pytest.mark.parametrize("batch,heads,lq,lk", [
-    (1, 1, 600, 130), (1, 1, 1000, 1), (2, 1, 1537, 300), (1, 2, 4096, 64), (1, 12, 900, 1500), (2, 12, 820, 820),
+    (1, 1, 900, 130), (1, 1, 1000, 1), (2, 1, 1537, 300), (1, 2, 4096, 64), (1, 6, 900, 1500), (2, 12, 820, 820),
 ])
 def test_key_tiles_cut_between_ctas(batch, heads, lq, lk):
     # Few key tiles and many queries: the dense backward gives every CTA an equal run of query tiles and
     # the epilogue adds up the parts of a key tile's dK and dV.
+    assert _lib.load().nb_attn_bwd_split_workspace_bytes(C.byref(dense_shape(batch, heads, lq, lk))) > 0
     g = torch.Generator().manual_seed(lq + lk)
     q, d_out = (torch.randn(batch, heads, lq, 64, generator=g).to(torch.bfloat16) for _ in range(2))
     k, v = (torch.randn(batch, heads, lk, 64, generator=g).to(torch.bfloat16) for _ in range(2))
