@@ -250,7 +250,10 @@ int builtin_scratch_address(void** out) {
 // has the SM for itself is only a little faster) x tiles; cut ones take an equal share plus about four
 // tiles' time for the parts and the kernel that puts them together. An eighth has to be gained, because
 // at the power limit SMs that wait let the others run faster (1024 units of 32 tiles: 186 us whole, 189
-// cut; the image: 68 whole, 57 cut). A CTA gets at least four tiles.
+// cut; the image: 73.5 whole, 58.5 cut). A CTA gets at least four tiles. Where every unit has an SM for itself
+// but its parts would share SMs, whole units take 5.2 us + 1.05 per tile and cut ones 12 us + 1.55 per tile of
+// their share: 1 x 8 x 2048 22.3 whole, 24.1 cut; x 1800 20.9 and 21.7; x 1500 18.1 and 17.2; 1 x 4 x 2000 22.0
+// and 17.8.
 struct FwdSplit {
   unsigned ctas = 0;  // 0: whole units
   size_t bytes = 0;
@@ -264,7 +267,9 @@ FwdSplit fwd_split(const nb_attn_shape& s) {
   const int64_t ctas = steps / 4 < slots ? steps / 4 : slots;
   if (ctas < 2 || steps > INT32_MAX) return r;
   const int64_t k = (units + slots / 2 - 1) / (slots / 2);
-  if ((k / 2 * 10 + (k & 1) * 9) * n_kt * 8 <= 90 * ((steps + ctas - 1) / ctas + 4)) return r;
+  const int64_t share = (steps + ctas - 1) / ctas;
+  if ((k / 2 * 10 + (k & 1) * 9) * n_kt * 8 <= 90 * (share + 4)) return r;
+  if (k == 1 && ctas > slots / 2 && 10 * n_kt < 60 + 15 * share) return r;
   r.ctas = unsigned(ctas);
   r.bytes = 2 * size_t(ctas) * nb::kFwdPartFloats * sizeof(float);
   return r;

@@ -119,3 +119,9 @@ def test_work_list_used_again(lengths, heads):
         args = _lib.FwdArgs(shape, desc(q), desc(k), desc(v), desc(out), lse.data_ptr(), None, ws.data_ptr(), ws.numel())
         _lib.check(call(C.byref(args), stream), "nb_attn_fwd")
         assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("heads,length,cut", [(8, 1500, True), (8, 1800, False), (8, 2048, False), (4, 2000, True)])
+def test_query_tiles_with_an_sm_each_are_cut_where_that_is_faster(heads, length, cut):
+    shape = dense_shape(1, heads, length, length)
+    assert (_lib.load().nb_attn_fwd_split_workspace_bytes(C.byref(shape)) > 0) == cut
