@@ -35,9 +35,10 @@
  *    lengths in cu_seqlens (they size tensor maps and the work list); the kernels verify this on
  *    the device and report NB_ATTN_STATUS_BAD_SEQLENS instead of dropping tiles.
  *  - Varlen scheduling: every call turns cu_seqlens into a work list of (sequence, 128-row tile)
- *    items on the device, most expensive items first and ragged last tiles at the end; persistent CTAs
- *    (two per SM in the forward, one in the backward) take the (item, head) pairs in list order. The
- *    list lives in the call's workspace.
+ *    items on the device, most expensive items first, ragged last tiles behind the full ones of their cost
+ *    class; persistent CTAs (two per SM in the forward, one in the backward) take the (item, head) pairs in
+ *    list order. The list lives in the call's workspace; the reserved words of its first entry count the
+ *    units taken and the CTAs done, and a finished forward leaves them at 0.
  *  - Varlen padding: cu_seqlens[batch] may be smaller than total_q / total_k (tokens packed into
  *    a buffer of fixed capacity). The rows past the last sequence belong to no sequence; the
  *    kernels write zeros to them in o, dq, dk and dv (and -inf in lse), so every output row is
@@ -113,8 +114,8 @@ typedef struct nb_attn_fwd_args {
 int nb_attn_fwd(const nb_attn_fwd_args* args, void* stream);
 
 /* The same for further calls with the shape, cu_seqlens and `workspace` of an nb_attn_fwd call that comes
- * before it in the order of `stream` (the layers of a network): the work list in `workspace` is used again
- * instead of built again. Calls that share a workspace must not run at the same time. */
+ * before it in the order of `stream` (the layers of a network): the work list in `workspace`, which nothing
+ * else may have written to since, is used again instead of built again. Calls that share a workspace must not run at the same time. */
 int nb_attn_fwd_again(const nb_attn_fwd_args* args, void* stream);
 
 /* Scratch bytes nb_attn_fwd needs: the work list of query tiles in varlen mode, 0 in dense mode. */
@@ -122,7 +123,8 @@ size_t nb_attn_fwd_workspace_bytes(const nb_attn_shape* shape);
 
 /* Scratch bytes that let a dense nb_attn_fwd divide few query tiles evenly over the SMs of the current
  * device (a tile's keys are then walked by more than one CTA and the parts added up); 0 where that would
- * not pay. Optional: with less scratch the call gives the same results from whole tiles. */
+ * not pay. Optional: with less scratch the call computes whole tiles, with results that are
+ * the same up to the order of fp32 additions. */
 size_t nb_attn_fwd_split_workspace_bytes(const nb_attn_shape* shape);
 
 /* Backward: replaces the autograd backward of the same call (reached from
@@ -223,7 +225,7 @@ typedef struct nb_attn_sched_item {
   int32_t own_len;      /* its length there */
   int32_t other_begin;  /* the same on the side the item's inner loop walks */
   int32_t other_len;
-  int32_t reserved[2];
+  int32_t reserved[2];  /* 0 in a new list; a call's own list counts units in the first entry's */
 } nb_attn_sched_item;
 
 int64_t nb_attn_schedule_capacity(int64_t total_tokens, int32_t batch);

@@ -4,7 +4,8 @@
 //                              clears the fp32 dQ accumulator. HBM-bound.
 //   attn_bwd_kernel          : a work unit is one 128-row K/V tile of one (sequence, head), walked
 //                              over the sequence's queries in 128-row steps. Everything is computed
-//                              transposed so that a thread owns a key row (tensor-memory lane):
+//                              transposed (a tensor-memory lane is a key row; a compute thread holds
+//                              four key rows x 16 query columns of a step):
 //                                S^T  = K Q^T                       (A = K from tensor memory)
 //                                dP^T = V dO^T                      (A = V from tensor memory)
 //                                P^T  = exp2(S^T*scale_log2 - lse)  (recomputed from the saved LSE)
@@ -14,7 +15,7 @@
 //                                dQ   = dS K                        (A = dS from shared memory)
 //                              What bounds it: the SM's shared-memory port (operand reads of the MMAs,
 //                              128 B per clock), the compute warps' dependent chain and the board's
-//                              power limit (at 1 kW the SMs run at 1.65-1.75 GHz of 1.965). So operands
+//                              power limit (at 1 kW, on long sequences, the SMs run at 1.47-1.6 GHz of 1.965). So operands
 //                              come from tensor memory wherever they can: K and V are copied there once
 //                              per work unit (tcgen05.cp) and P^T and dS^T are written over the scores
 //                              they came from; only dQ reads both operands from shared memory. Per step
@@ -24,8 +25,8 @@
 //                              because every K/V tile of a sequence contributes to every dQ row.
 //                              CTAs are persistent (one per SM): each walks its share of the work
 //                              units and the step pipeline runs on through the boundary between
-//                              two units -- K is double-buffered, V is reloaded as soon as the
-//                              unit's last dP^T MMA has read it, dV / dK leave through the drain
+//                              two units -- K is double-buffered, V is reloaded as soon as it
+//                              has been copied into tensor memory, dV / dK leave through the drain
 //                              warps while the next unit's first steps run -- so a unit's start-up
 //                              and tail (a third of a CTA's life on ~800-token sequences) overlap
 //                              its neighbours' steps.
@@ -85,7 +86,7 @@ struct BwdParams {
   float* dq_accum;  // fp32 [total_q][heads][64]
   const int32_t* cu_q;
   const int32_t* cu_k;
-  const SchedItem* items;  // packed mode: work list of key tiles; CTA x runs entry x / heads for head x % heads
+  const SchedItem* items;  // packed mode: work list of key tiles; a unit is an entry and a head
   SchedParams sched;      // packed mode: what block 0 of the prologue builds (items == NULL: nothing)
   int32_t batch, heads;
   int32_t lq, lk;
@@ -388,8 +389,8 @@ enum BwdCtrl : uint32_t {
 };
 
 // The compute warps' role: for every step of the CTA, P^T from S^T, then dS^T from dP^T.
-// Not inlined on purpose: compiled by itself the step body keeps its instruction schedule (it sits
-// at the compute warps' 168-register cap, and inlined into the kernel it came out 10-60 % slower
+// Not inlined on purpose: compiled by itself the step body keeps its instruction schedule (it needs
+// 144 of the compute warps' 152 registers, and inlined into the kernel it came out 10-60 % slower
 // whenever the code around it changed).
 __device__ __noinline__ void bwd_compute_role(const uint32_t bar0, int* abort_flag, int32_t* status,
                                               const uint32_t tmem_base, const float* sLse, const float* sDelta,
@@ -616,8 +617,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     setmaxnreg_dec<kBwdLoaderRegs>();
     if (warp == 16) {
       // ---------------- TMA producer (one lane) ----------------
-      // K of the next item goes into the other K buffer; V is reloaded as soon as the item's last
-      // dP^T MMA has read it; Q/dO tiles run through the ring without regard to item boundaries.
+      // K of the next item goes into the other K buffer; V is reloaded as soon as it has been
+      // copied into tensor memory; Q/dO tiles run through the ring without regard to item boundaries.
       if (lane == 0) {
         BwdStepPos pos;
         uint32_t ni = 0;  // items with queries so far

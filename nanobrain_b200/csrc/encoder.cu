@@ -476,7 +476,7 @@ int nb_enc_gelu(void* v, int64_t n, void* stream) {
   if (!aligned16(v)) return NB_ATTN_ERR_ALIGN;
   if (n <= 0 || n % 8 != 0) return NB_ATTN_ERR_SHAPE;
   const int64_t blocks = (n / 8 + 511) / 512;
-  const bool table = n >= kGeluTableMin;  // four resident blocks per SM then walk the array
+  const bool table = n >= kGeluTableMin;  // four resident blocks on each of 148 SMs then walk the array
   launch(table ? gelu_kernel<true> : gelu_kernel<false>, dim3(unsigned(table ? (blocks < 592 ? blocks : 592) : blocks)),
          dim3(512), stream, static_cast<__nv_bfloat16*>(v), n);
   return launched();

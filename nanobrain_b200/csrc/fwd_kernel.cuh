@@ -16,9 +16,11 @@
 //               over the first half of the columns they came from. The offset m is the row max of the
 //               first tile; later halves compute no max at all: fp32 and bf16 carry exponents up
 //               to 2^127, so scores may rise 60 (in log2 units) above the first ones before anything
-//               has to be rescaled. Only if a row's sum ends above 2^60 (or Inf / NaN), or above 2^14 with a
-//               P V that is not finite, does the CTA list the unit and walk it a second time, with the running max of every half. At the end of a
-//               unit the warps normalise and store O and the log-sum-exp. O is divided by the sum of
+//               has to be rescaled. Only if a row's sum ends above 2^60 (or Inf / NaN), or above 2^14
+//               with a P V that is not finite, or the polynomial met an argument beyond its range,
+//               does the CTA list the unit and walk it a second time, with the running max of every
+//               half. At the end of a unit the warps normalise and store O and the log-sum-exp. O is
+//               divided (where there is more than one tile) by the sum of
 //               P as the product sees it, rounded to bf16, which the tensor core forms from 16 columns
 //               of ones behind V: where few keys dominate a row, the rounding of their P then cancels.
 //               Scores of standard deviation 9 and 16 nats, relative error of O against 64 bits: 2.2e-3
@@ -37,9 +39,12 @@
 // What bounds it: the instructions of the softmax warps and the board's power limit (at 1 kW the SMs
 // run at 1.65-1.8 GHz of 1.965). Measured on dense 32 x 8 x 4096, repeated for 0.3 s: with a score tile
 // and P of 128 columns each, Q from shared memory and P handed over once per tile 1550 us (1540 clocks
-// per 128 x 128 tile and SM); this form 1455 us (1363 clocks). Persistent CTAs against one CTA per unit:
-// packed 32 x U[720,920] x 12 heads 130 -> 122 us, 500 sequences of 1..300 tokens 232 -> 179, dense
-// 32 x 8 x 4096 unchanged, 24 sequences of 820 tokens (less than one unit per CTA) 12.7 -> 14.3.
+// per 128 x 128 tile and SM); this form 1402 us before `top`, the columns of ones and the first tile's max,
+// 1448 with them (exact scores and NaN cost 1.5 %, precision 1.4 %). Against the form before it, in GPU time between
+// unrelated kernels: packed 32 x U[720,920] x 12 heads 138 -> 113 us, 500 sequences of 1..300 tokens 258 -> 165,
+// 1 x 12 x 3476 77 -> 58, 2 x 12 x 820 15.7 -> 15.4. Calls of at most 300 tokens lose 1 to 2 us (1 x 12 x 128: 4.5 -> 6.4,
+// 1 x 12 x 300: 7.2 -> 8.1): a block that has one unit runs through twice the code once, cold. Loads issued before the
+// tensor memory is there (6.3) and a rolled epilogue (6.3, 500 short sequences 165 -> 169) were not worth their code.
 //
 // Tensor memory (256 columns): S / P [0,128) O [128,192) row sums of P [192,208) Q [208,240).
 #pragma once
@@ -77,7 +82,7 @@ struct FwdParams {
   float* lse;
   const int32_t* cu_q;  // NULL => dense
   const int32_t* cu_k;
-  const SchedItem* items;  // packed mode: the scheduler's work list; CTA x runs entry x / heads for head x % heads
+  const SchedItem* items;  // packed mode: the scheduler's work list; a unit is an entry and a head
   int32_t batch, heads;
   int32_t lq, lk;  // dense lengths (max_seqlen in varlen mode)
   int64_t total_q, total_k;

@@ -131,7 +131,7 @@ int check_shape(const nb_attn_shape& s) {
       return NB_ATTN_ERR_SHAPE;
   } else {
     if (s.total_q > INT32_MAX || s.total_k > INT32_MAX) return NB_ATTN_ERR_SHAPE;
-    // The grid is items x heads.
+    // Units (items x heads) are counted in 32 bits.
     if (nb::sched_capacity(s.total_q, s.batch) * s.heads > INT32_MAX ||
         nb::sched_capacity(s.total_k, s.batch) * s.heads > INT32_MAX)
       return NB_ATTN_ERR_SHAPE;
@@ -377,7 +377,7 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
       p.split_base = steps / ctas, p.split_extra = steps % ctas;
     }
   } else {
-    // Block 0 of the prologue builds the list of key tiles; the main kernel runs items x heads CTAs.
+    // Block 0 of the prologue builds the list of key tiles; units are items x heads.
     const int64_t n_items = nb::sched_capacity(s.total_k, s.batch);
     nb::SchedItem* items =
         reinterpret_cast<nb::SchedItem*>(static_cast<unsigned char*>(workspace) + bwd_items_offset(s));
@@ -395,7 +395,8 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t rows = s.total_q * s.heads;
   const int64_t want_blocks = (rows * 8 + 255) / 256;
-  const int aux_blocks = int(want_blocks < 148 * 16 ? want_blocks : 148 * 16);
+  const int64_t most_blocks = 16 * int64_t(device_sm_count());
+  const int aux_blocks = int(want_blocks < most_blocks ? want_blocks : most_blocks);
   p.row_blocks = aux_blocks;
   const int combine_blocks = p.parts != nullptr ? 4 * (int(ctas) - 1) : 0;
   bool ok = launch(nb::attn_bwd_prologue_kernel, dim3(aux_blocks), dim3(256), 0, st, p) == cudaSuccess;

@@ -22,7 +22,7 @@
 //     owns rows [cu_seqlens[batch], total) and has nothing on the other side: its items make the
 //     kernels write zeros there, so every row of every output is defined;
 //   * the list has a host-known capacity of floor(total / 128) + batch + 1 entries; unused entries
-//     have seq = -1 and their CTAs exit at once;
+//     have seq = -1 and end a CTA's work;
 //   * an entry carries the sequence's offsets and lengths on both sides, so a CTA learns all it
 //     needs about its work from one 32-byte read instead of a chain of dependent loads.
 //
