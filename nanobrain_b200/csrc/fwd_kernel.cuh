@@ -347,7 +347,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       uint32_t redo = 0;  // units walked again so far
       const bool packed = p.cu_q != nullptr;
       auto wait_done = [&](uint32_t v) {  // unit v is finished
-        mbar_wait(bar(kFwdUnitDone + (v & 1u)), (v >> 1) & 1u, &abort_flag, p.status);
+        mbar_wait(bar(kFwdUnitDone + (v & 1u)), (v >> 1) & 1u, &abort_flag);
       };
       uint32_t token = packed ? sched_next(p.items) : p.parts != nullptr ? 0u : blockIdx.x;
 #pragma unroll 1
@@ -365,7 +365,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           w.safe = 1;
         }
         if (u >= 2) wait_done(u - 2);  // the descriptor slot's last user
-        if (u >= 1) mbar_wait(bar(kFwdQEmpty), (u - 1) & 1u, &abort_flag, p.status);
+        if (u >= 1) mbar_wait(bar(kFwdQEmpty), (u - 1) & 1u, &abort_flag);
         units[u & 1u] = w;
         redo_listed[u & 1u] = 0;
         if (w.lk == 0) {
@@ -379,10 +379,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll 1
         for (int row = 0; row < w.lk; row += kTile, ++t) {
           const uint32_t s = t % kFwdStages, ph = ((t / kFwdStages) - 1) & 1;
-          if (t >= uint32_t(kFwdStages)) mbar_wait(bar(kFwdKEmpty + s), ph, &abort_flag, p.status);
+          if (t >= uint32_t(kFwdStages)) mbar_wait(bar(kFwdKEmpty + s), ph, &abort_flag);
           mbar_arrive_expect_tx(bar(kFwdKFull + s), kTileBytes);
           tma_load_4d(sK(s), &tmap_k, bar(kFwdKFull + s), 0, w.k_begin + row, w.h, w.bcoord);
-          if (t >= uint32_t(kFwdStages)) mbar_wait(bar(kFwdVEmpty + s), ph, &abort_flag, p.status);
+          if (t >= uint32_t(kFwdStages)) mbar_wait(bar(kFwdVEmpty + s), ph, &abort_flag);
           mbar_arrive_expect_tx(bar(kFwdVFull + s), kTileBytes);
           tma_load_4d(sV(s), &tmap_v, bar(kFwdVFull + s), 0, w.k_begin + row, w.h, w.bcoord);
         }
@@ -411,7 +411,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       uint32_t uo = 0;  // units with keys so far
 #pragma unroll 1
       for (uint32_t u = 0;; ++u) {
-        if (!mbar_wait(bar(kFwdQFull + (u & 1u)), (u >> 1) & 1u, &abort_flag, p.status)) break;
+        if (!mbar_wait(bar(kFwdQFull + (u & 1u)), (u >> 1) & 1u, &abort_flag)) break;
         const int lk = reinterpret_cast<volatile FwdUnit*>(units)[u & 1u].lk;
         if (lk < 0) break;
         if (lk == 0) {
@@ -436,24 +436,24 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 #pragma unroll
         for (int k = 0; k < 4; ++k) tmem_copy_128x256b(tm_q + 8 * k, qd + 2 * k);
         tc_commit(bar(kFwdQEmpty));
-        mbar_wait(bar(kFwdKFull + t % kFwdStages), (t / kFwdStages) & 1, &abort_flag, p.status);
+        mbar_wait(bar(kFwdKFull + t % kFwdStages), (t / kFwdStages) & 1, &abort_flag);
         tc_fence_after();
         const int nh0 = halves(0);
         issue_s(0, t, 0);
         if (nh0 > 1) issue_s(0, t, 1);
         tc_commit(bar(kFwdKEmpty + t % kFwdStages));
         // O of the previous unit has to be out of tensor memory before the first P V product.
-        if (uo > 0) mbar_wait(bar(kFwdOFree), (uo - 1) & 1u, &abort_flag, p.status);
+        if (uo > 0) mbar_wait(bar(kFwdOFree), (uo - 1) & 1u, &abort_flag);
         ++uo;
 #pragma unroll 1
         for (int i = 0; i < n_kv; ++i, ++t) {
           const uint32_t s = t % kFwdStages, s1 = (t + 1) % kFwdStages;
-          mbar_wait(bar(kFwdVFull + s), (t / kFwdStages) & 1, &abort_flag, p.status);
+          mbar_wait(bar(kFwdVFull + s), (t / kFwdStages) & 1, &abort_flag);
           const uint64_t vd = make_sdesc(sV(s), sOnes - sV(s), 1024);
           const int nh = halves(i), nh1 = i + 1 < n_kv ? halves(i + 1) : 0;
 #pragma unroll 1
           for (int hf = 0; hf < nh; ++hf) {
-            mbar_wait(bar(kFwdPFull + hf), (hf ? t1 : t) & 1, &abort_flag, p.status);
+            mbar_wait(bar(kFwdPFull + hf), (hf ? t1 : t) & 1, &abort_flag);
             tc_fence_after();
             // P of this half times V (the softmax warps have cleared the V rows between the last live
             // key and the next multiple of 16).
@@ -471,7 +471,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             if (hf == nh - 1) tc_commit(bar(kFwdVEmpty + s));
             if (hf < nh1) {
               if (hf == 0) {
-                mbar_wait(bar(kFwdKFull + s1), ((t + 1) / kFwdStages) & 1, &abort_flag, p.status);
+                mbar_wait(bar(kFwdKFull + s1), ((t + 1) / kFwdStages) & 1, &abort_flag);
                 tc_fence_after();
               }
               issue_s(i + 1, t + 1, hf);
@@ -491,7 +491,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     uint32_t t[2] = {0, 0};  // first and second halves so far
 #pragma unroll 1
     for (uint32_t u = 0;; ++u) {
-      if (!mbar_wait(bar(kFwdQFull + (u & 1u)), (u >> 1) & 1u, &abort_flag, p.status)) break;
+      if (!mbar_wait(bar(kFwdQFull + (u & 1u)), (u >> 1) & 1u, &abort_flag)) break;
       const volatile FwdUnit& meta = reinterpret_cast<volatile FwdUnit*>(units)[u & 1u];
       const int lk = meta.lk;
       if (lk < 0) break;
@@ -505,7 +505,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         const int hf = (c0 >> 6) & 1;
         const int valid = lk - c0;  // live columns, if below 64
         const uint32_t th = hf ? t[1] : t[0];
-        if (!s_ok) mbar_wait(bar(kFwdSFull + hf), th & 1, &abort_flag, p.status);
+        if (!s_ok) mbar_wait(bar(kFwdSFull + hf), th & 1, &abort_flag);
         __syncwarp();
         tc_fence_after();
         uint32_t ra[32], rb[32], pk[32];
@@ -521,7 +521,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             // cleared before P is handed to the MMA warp. (The swizzle only permutes 16-byte chunks
             // inside a 128-byte row: whole rows are contiguous.)
             const uint32_t tile = hf ? t[0] - 1 : t[0], st = tile % kFwdStages;
-            mbar_wait(bar(kFwdVFull + st), (tile / kFwdStages) & 1, &abort_flag, p.status);
+            mbar_wait(bar(kFwdVFull + st), (tile / kFwdStages) & 1, &abort_flag);
             uint8_t* v_rows = smem_raw + (sV(st) - smem_u32(smem_raw)) + hf * (kTileBytes / 2);
             for (int c = valid * 8 + lane; c < ((valid + 15) & ~15) * 8; c += 32)
               reinterpret_cast<uint4*>(v_rows)[c] = make_uint4(0, 0, 0, 0);
@@ -534,7 +534,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           chunk_max(ra, mx0, mx1);
           chunk_max(rb, mx2, mx3);
           if (c0 == 0 && lk > 64) {  // the first offset is the max of the whole tile
-            mbar_wait(bar(kFwdSFull + 1), t[1] & 1, &abort_flag, p.status);
+            mbar_wait(bar(kFwdSFull + 1), t[1] & 1, &abort_flag);
             __syncwarp();
             tc_fence_after();
 #pragma unroll 1
@@ -555,7 +555,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           } else if (__any_sync(0xffffffffu, need)) {
             // Second time: refresh the offset of the rows that need it, rescale their running sum and
             // their row of the O accumulator (complete up to the previous half).
-            mbar_wait(bar(kFwdPvDone + (hf ^ 1)), ((hf ? t[0] : t[1]) - 1) & 1, &abort_flag, p.status);
+            mbar_wait(bar(kFwdPvDone + (hf ^ 1)), ((hf ? t[0] : t[1]) - 1) & 1, &abort_flag);
             __syncwarp();
             tc_fence_after();
             const float alpha = need ? fast_exp2((m_run - m_new) * p.scale_log2) : 1.f;
@@ -597,7 +597,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       bool store = true;
       if (lk > 0) {
         const int hf = ((lk - 1) >> 6) & 1;  // the last half; MMAs complete in order
-        mbar_wait(bar(kFwdPvDone + hf), ((hf ? t[1] : t[0]) - 1) & 1, &abort_flag, p.status);
+        mbar_wait(bar(kFwdPvDone + hf), ((hf ? t[1] : t[0]) - 1) & 1, &abort_flag);
         __syncwarp();
         tc_fence_after();
         if (!(top < kPolyLimit)) l_run = NAN;
@@ -710,6 +710,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) report_abort(&abort_flag, p.status);
   if (warp == 4) {
     __syncwarp();
     tc_fence_after();

@@ -3,9 +3,9 @@
 // (tcgen05.alloc / ld / st) and the 5th-generation tensor-core MMA (tcgen05.mma).
 //
 // Every wait in this file is bounded: after roughly two seconds without progress a
-// waiter raises a CTA-wide abort flag in shared memory, records a code in the caller's
-// status word in global memory and returns; later waits see the flag and return at once,
-// so a kernel always runs to its end and frees its tensor memory.
+// waiter raises a CTA-wide abort flag in shared memory and returns; later waits see the flag and
+// return at once, so a kernel always runs to its end, where it records a code in the caller's status word in
+// global memory (report_abort) and frees its tensor memory.
 #pragma once
 
 #include <cuda.h>
@@ -112,11 +112,14 @@ constexpr uint64_t kWaitLimitNs = 2000000000ull;  // about two seconds
 // Bounded wait. `abort_flag` lives in shared memory and is shared by the whole CTA. The attention
 // kernels use the default limit (a compile-time constant); the wait self-test passes its own
 // (at most 4 s: the clock is the low word of the nanosecond timer).
-// The loop is kept as small as it can be -- 32-bit timer arithmetic, the flag and the status word
-// touched with plain state-space stores: the warp-specialised kernels have dozens of wait sites,
-// every one of them inlined, and their hot code has to fit the SM's instruction cache (with a
+// The loop is kept as small as it can be -- 32-bit timer arithmetic, the flag touched with plain
+// state-space accesses, the status word left to the kernel's end: the warp-specialised kernels have dozens of
+// wait sites, every one of them inlined, and their hot code has to fit the SM's instruction cache (with a
 // larger loop the backward kernel's instruction-cache hit rate was 92 % at best and instruction
-// fetch was its top stall).
+// fetch was its top stall). The status word's store at every site was 3 of the backward kernel's 54 KB; without it the
+// backward of 500 sequences of 1..300 tokens takes 555 instead of 568 us, of 32 x 12 x 820 328 instead of 333. A smaller site
+// yet, polls counted instead of timed, saved another 2 KB and cost 5 % (32 x 8 x 4096: 3392 -> 3552 us): the
+// timer's latency keeps the waiters from polling too often.
 __device__ __forceinline__ uint32_t globaltimer_lo() {
   uint32_t t;
   asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
@@ -124,7 +127,7 @@ __device__ __forceinline__ uint32_t globaltimer_lo() {
 }
 
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          int* status_word, uint64_t limit_ns = kWaitLimitNs) {
+                                          uint64_t limit_ns = kWaitLimitNs) {
   if (mbar_try_wait(bar, parity)) return true;
   const uint32_t flag_addr = smem_u32(const_cast<int*>(abort_flag));
   const uint32_t limit = uint32_t(limit_ns);
@@ -138,9 +141,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     if (globaltimer_lo() - t0 > limit) break;
   }
   asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(flag_addr), "r"(1) : "memory");
-  if (status_word)
-    asm volatile("st.volatile.global.u32 [%0], %1;" ::"l"(status_word), "r"((int)kStatusWaitTimeout) : "memory");
   return false;
+}
+
+// At the end of a kernel, by one thread behind a block-wide barrier: says whether a wait of this block gave up.
+__device__ __forceinline__ void report_abort(volatile int* abort_flag, int* status_word) {
+  if (*abort_flag != 0 && status_word != nullptr) *static_cast<volatile int*>(status_word) = int(kStatusWaitTimeout);
 }
 
 // One look at a barrier that never suspends the thread.
@@ -371,11 +377,11 @@ __device__ __forceinline__ void setmaxnreg_dec() {
 
 // Waits for two barriers with the two polls in flight together (their latencies overlap).
 __device__ __forceinline__ bool mbar_wait2(uint32_t bar_a, uint32_t par_a, uint32_t bar_b, uint32_t par_b,
-                                           volatile int* abort_flag, int* status_word) {
+                                           volatile int* abort_flag) {
   const bool a = mbar_try_wait(bar_a, par_a);
   const bool b = mbar_try_wait(bar_b, par_b);
-  if (!a && !mbar_wait(bar_a, par_a, abort_flag, status_word)) return false;
-  return b || mbar_wait(bar_b, par_b, abort_flag, status_word);
+  if (!a && !mbar_wait(bar_a, par_a, abort_flag)) return false;
+  return b || mbar_wait(bar_b, par_b, abort_flag);
 }
 
 // ----------------------------------------------------------------------------------------

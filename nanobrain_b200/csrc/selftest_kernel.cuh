@@ -89,7 +89,7 @@ mma_selftest_kernel(int mode, const __nv_bfloat16* __restrict__ A, const __nv_bf
     tc_commit(smem_u32(&bar));
   }
   __syncwarp();
-  mbar_wait(smem_u32(&bar), 0, &abort_flag, status);
+  mbar_wait(smem_u32(&bar), 0, &abort_flag);
   tc_fence_after();
   const int ncols = mode == 0 ? 128 : 64;
   for (int c = 0; c < ncols / 32; ++c) {
@@ -100,6 +100,7 @@ mma_selftest_kernel(int mode, const __nv_bfloat16* __restrict__ A, const __nv_bf
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) report_abort(&abort_flag, status);
   if (warp == 0) {
     tc_fence_after();
     tmem_dealloc(tmem_base, 256);
@@ -108,7 +109,7 @@ mma_selftest_kernel(int mode, const __nv_bfloat16* __restrict__ A, const __nv_bf
 
 // Self-test of the bounded wait: one CTA allocates tensor memory, then all its warps wait on an
 // mbarrier that nothing will ever arrive on, with the caller's limit instead of the kernels' two
-// seconds. The wait gives up, the status word receives kStatusWaitTimeout, the tensor memory is
+// seconds. The wait gives up, the status word receives kStatusWaitTimeout at the kernel's end, the tensor memory is
 // freed and the kernel returns -- what every attention kernel does if one of its waits runs out.
 // out[0] = 1 if the first wait returned "gave up", out[1] = 1 if a later wait returned at once
 // because of the CTA-wide abort flag.
@@ -130,10 +131,10 @@ __global__ void __launch_bounds__(128) wait_selftest_kernel(uint64_t limit_ns, i
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const bool first = mbar_wait(smem_u32(&bar), 0, &abort_flag, status, limit_ns);
+  const bool first = mbar_wait(smem_u32(&bar), 0, &abort_flag, limit_ns);
   __syncthreads();
   const uint64_t t0 = globaltimer_ns();
-  const bool second = mbar_wait(smem_u32(&bar), 0, &abort_flag, status, limit_ns);
+  const bool second = mbar_wait(smem_u32(&bar), 0, &abort_flag, limit_ns);
   const uint64_t waited = globaltimer_ns() - t0;
   if (tid == 0 && out != nullptr) {
     out[0] = first ? 0 : 1;
@@ -141,6 +142,7 @@ __global__ void __launch_bounds__(128) wait_selftest_kernel(uint64_t limit_ns, i
   }
   tc_fence_before();
   __syncthreads();
+  if (tid == 0) report_abort(&abort_flag, status);
   if (warp == 0) {
     __syncwarp();
     tc_fence_after();
