@@ -30,17 +30,16 @@
 //                              warps while the next unit's first steps run -- so a unit's start-up
 //                              and tail (a third of a CTA's life on ~800-token sequences) overlap
 //                              its neighbours' steps.
-//                              Warp roles (640 threads): warps 0-7 are two compute warpgroups that
+//                              Warp roles (512 threads): warps 0-7 are two compute warpgroups that
 //                              split the 128 query columns of a step (64 each); warps 8, 10, 11 are
 //                              three MMA issuers (dV and the next S^T; dK and the next dP^T; dQ: one
 //                              elected thread each, so that a wait of one does not hold back the
-//                              others); warps 12-15 drain the dQ tiles (one tensor-memory lane
-//                              quadrant each) into the accumulator and, at the end of a unit, dV
-//                              and dK into their tensors; warp 16 drives TMA; warp 17 stages the
-//                              steps' LSE/delta rows and control words (warps 18-19 only complete
-//                              its warpgroup for the register re-partitioning). Warp 16 fetches the
-//                              units and publishes them to warp 17 and the drain warps; the compute
-//                              warps and the issuers learn about a step from its control word alone.
+//                              others); warp 9 fetches the units, drives TMA and stages the steps'
+//                              LSE/delta rows and control words; warps 12-15 drain the dQ tiles (one
+//                              tensor-memory lane quadrant each) into the accumulator and, at the end
+//                              of a unit, dV and dK into their tensors. Warp 9 publishes the units to
+//                              the drain warps; the compute warps and the issuers learn about a step
+//                              from its control word alone.
 //                              Code size is a first-order concern here: five roles' loops run at
 //                              the same time and have to share the SM's instruction cache (at
 //                              67 KB of code its hit rate was 68 % and instruction fetch was the
@@ -237,7 +236,7 @@ __global__ void __launch_bounds__(256) attn_bwd_epilogue_kernel(const BwdParams 
 // ----------------------------------------------------------------------------------------
 // Main backward kernel
 // ----------------------------------------------------------------------------------------
-constexpr int kBwdThreads = 640;
+constexpr int kBwdThreads = 512;
 constexpr int kBwdStages = 3;  // Q/dO ring
 constexpr int kBwdOutStageBytes = 8192;  // dK/dV read-out: 2 KB per drain warp
 // K (two buffers), V, 3x(Q, dO), dS (two 64-column halves), fp32 dQ staging (two 32-column halves),
@@ -246,19 +245,19 @@ constexpr int kBwdSmemBytes =
     (3 + 2 * kBwdStages + 4) * kTileBytes + kBwdOutStageBytes + kBwdStages * 2 * kTile * 4 + 64 + 1024;
 // Tensor memory: S^T 0 (P^T over it), dP^T 128 (dS^T over it), dV 256, dK 320, dQ 384, K 448, V 480
 constexpr int kBwdTmemCols = 512;
-// Register re-partitioning. The CTA launches with 640 threads x 96 registers (the most the
-// register file allows); setmaxnreg only moves registers inside that allocation, so the budget
-// must balance exactly or the growing warps would wait for ever:
-//   2 compute warpgroups x 128 x 152 + issuers 128 x 64 + drainers 128 x 64 + loader group 128 x 48
-//   = 38912 + 8192 + 8192 + 6144 = 61440 = 640 x 96 (the compute role needs 144).
-// Every warp of an aligned warpgroup executes the same setmaxnreg instruction.
-constexpr int kBwdLaunchRegs = 96;
+// Register re-partitioning. The CTA launches with 512 threads x 128 registers (the whole register file); setmaxnreg
+// only moves registers inside that allocation, so the budget must balance exactly or the growing warps would
+// wait for ever. Every warp of an aligned warpgroup executes the same setmaxnreg instruction. The compute role needs 144.
+// With 640 threads x 96 registers (TMA and LSE/delta rows in a warpgroup of their own; drain 64, loaders 48) ptxas
+// spilled 40 to 72 bytes in the other roles' step loops: whole backward of 2 x 12 x 820 32.9 us, now 30.8; 1 x 12 x 3476 132.0 and
+// 128.4; 32 x 12 x 820 328 and 317; 256 sequences of 720..920 tokens 2555 and 2500. (Many sequences of two tiles lose: 300 of 200
+// tokens 368 -> 384, where the one warp's reads of list and rows follow each other.)
+constexpr int kBwdLaunchRegs = 128;
 constexpr int kBwdComputeRegs = 152;
-constexpr int kBwdIssuerRegs = 64;
-constexpr int kBwdDrainRegs = 64;
-constexpr int kBwdLoaderRegs = 48;
-static_assert(256 * kBwdComputeRegs + 128 * (kBwdIssuerRegs + kBwdDrainRegs + kBwdLoaderRegs) ==
-                  kBwdThreads * kBwdLaunchRegs, "register budget");
+constexpr int kBwdIssuerRegs = 104;  // issuers and loader
+constexpr int kBwdDrainRegs = 104;
+static_assert(256 * kBwdComputeRegs + 128 * (kBwdIssuerRegs + kBwdDrainRegs) == kBwdThreads * kBwdLaunchRegs,
+              "register budget");
 
 constexpr int kBwdWorkSlots = 4;
 
@@ -283,7 +282,7 @@ enum BwdBar : int {
   kBarDvOut,    // 4: the drain warps have read the item's dV accumulator
   kBarDkOut,    // 4
   kBarWorkFull,                                  // [kBwdWorkSlots] the ring of published units
-  kBarWorkEmpty = kBarWorkFull + kBwdWorkSlots,  // [kBwdWorkSlots], 5: LSE/delta warp and drain warps
+  kBarWorkEmpty = kBarWorkFull + kBwdWorkSlots,  // [kBwdWorkSlots], 4: drain warps
   kBwdNumBars = kBarWorkEmpty + kBwdWorkSlots
 };
 
@@ -567,7 +566,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   const uint32_t bar0 = smem_u32(&bars[0]);
   auto bar = [&](int i) { return bar0 + 8u * uint32_t(i); };
 
-  if (tid == 16 * 32) {
+  if (tid == 9 * 32) {
     tma_prefetch_desc(&tmap_k);
     tma_prefetch_desc(&tmap_q);
     tma_prefetch_desc(&tmap_v);
@@ -579,7 +578,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       if (i >= kBarQdoEmpty && i < kBarQdoEmpty + kBwdStages) count = 2;
       if (i >= kBarPFull && i < kBarDsFull + 2) count = 4;
       if (i == kBarDqFree || i == kBarDvOut || i == kBarDkOut) count = 4;
-      if (i >= kBarWorkEmpty) count = 5;
+      if (i >= kBarWorkEmpty) count = 4;
       mbar_init(bar(i), count);
     }
     fence_mbar_init();
@@ -612,115 +611,95 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     return w;
   };
 
-  if (warp >= 16) {
-    setmaxnreg_dec<kBwdLoaderRegs>();
-    if (warp == 16) {
-      // ---------------- TMA producer (one lane) ----------------
-      // K of the next item goes into the other K buffer; V is reloaded as soon as it has been
-      // copied into tensor memory; Q/dO tiles run through the ring without regard to item boundaries.
+  if (warp >= 8 && warp < 12) setmaxnreg_dec<kBwdIssuerRegs>();
+  if (warp == 9) {
+    // ---------------- loader: units, TMA (lane 0), LSE/delta rows and the steps' control words ----------------
+    // K of the next item goes into the other K buffer; V is reloaded as soon as it has been
+    // copied into tensor memory; Q/dO tiles run through the ring without regard to item boundaries.
+    // A step's LSE/delta rows are requested before the wait for a free stage, so that this latency does not
+    // sit between a stage becoming free and becoming full again. They are staged negated: -lse in
+    // the log2 domain and -delta. Rows past the end of the sequence get -lse = -inf, which makes
+    // their P^T column 0.
+    BwdStepPos pos;
+    uint32_t ni = 0;  // items with queries so far
+    auto next_token = [&](uint32_t g) {
+      if (!packed) return kCut ? g + 1 : g + gridDim.x;
+      uint32_t token = 0;
+      if (lane == 0) token = sched_next(p.items);
+      return __shfl_sync(0xffffffffu, token, 0);
+    };
+    uint32_t g = packed ? next_token(0) : kCut ? 0u : blockIdx.x;
+#pragma unroll 1
+    for (uint32_t round = 0;; ++round) {
+      const BwdWorkOf<kCut> wk = bwd_work<kCut>(p, g);
+      const uint32_t slot = round % kBwdWorkSlots, kb = ni & 1u;
+      const int krow = wk.k_begin + wk.kt * kTile;
       if (lane == 0) {
-        BwdStepPos pos;
-        uint32_t ni = 0;  // items with queries so far
-        uint32_t g = packed ? sched_next(p.items) : kCut ? 0u : blockIdx.x;
-#pragma unroll 1
-        for (uint32_t round = 0;; ++round) {
-          const BwdWorkOf<kCut> wk = bwd_work<kCut>(p, g);
-          const uint32_t slot = round % kBwdWorkSlots;
-          if (round >= uint32_t(kBwdWorkSlots))
-            mbar_wait(bar(kBarWorkEmpty + slot), ((round / kBwdWorkSlots) - 1) & 1, &abort_flag);
-          work_ring[slot] = wk;
-          mbar_arrive(bar(kBarWorkFull + slot));
-          if (wk.n_q < 0) break;
-          const uint32_t kb = ni & 1u;
-          const int krow = wk.k_begin + wk.kt * kTile;
-          if (wk.n_q > 0) {
-            if (ni >= 2) mbar_wait(bar(kBarKFree + kb), ((ni >> 1) - 1) & 1, &abort_flag);
-            mbar_arrive_expect_tx(bar(kBarKFull + kb), kTileBytes);
-            tma_load_4d(sK(kb), &tmap_k, bar(kBarKFull + kb), 0, krow, wk.h, wk.bcoord);
-          }
-          int jt = bwd_start(wk);
-#pragma unroll 1
-          for (int j = 0; j < wk.n_q; ++j) {
-            if (pos.s >= uint32_t(kBwdStages))
-              mbar_wait(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u, &abort_flag);
-            mbar_arrive_expect_tx(bar(kBarQdoFull + pos.qs), 2 * kTileBytes);
-            tma_load_4d(sQ(pos.qs), &tmap_q, bar(kBarQdoFull + pos.qs), 0, wk.q_begin + jt * kTile, wk.h, wk.bcoord);
-            tma_load_4d(sDO(pos.qs), &tmap_do, bar(kBarQdoFull + pos.qs), 0, wk.q_begin + jt * kTile, wk.h,
-                        wk.bcoord);
-            if (j == 0) {
-              if (ni >= 1) mbar_wait(bar(kBarVFree), (ni - 1) & 1, &abort_flag);
-              mbar_arrive_expect_tx(bar(kBarVFull), kTileBytes);
-              tma_load_4d(sV, &tmap_v, bar(kBarVFull), 0, krow, wk.h, wk.bcoord);
-            }
-            pos.advance();
-            jt = jt + 1 == bwd_tiles(wk) ? 0 : jt + 1;
-          }
-          if (wk.n_q > 0) ++ni;
-          // The next unit is taken as late as can be: this thread is about three steps ahead of the MMAs,
-          // which covers the counter's and the list's latency, and a unit taken earlier would wait behind a
-          // long one while other CTAs run dry.
-          g = packed ? sched_next(p.items) : kCut ? g + 1 : g + gridDim.x;
+        if (round >= uint32_t(kBwdWorkSlots))
+          mbar_wait(bar(kBarWorkEmpty + slot), ((round / kBwdWorkSlots) - 1) & 1, &abort_flag);
+        work_ring[slot] = wk;
+        mbar_arrive(bar(kBarWorkFull + slot));
+        if (wk.n_q > 0) {
+          if (ni >= 2) mbar_wait(bar(kBarKFree + kb), ((ni >> 1) - 1) & 1, &abort_flag);
+          mbar_arrive_expect_tx(bar(kBarKFull + kb), kTileBytes);
+          tma_load_4d(sK(kb), &tmap_k, bar(kBarKFull + kb), 0, krow, wk.h, wk.bcoord);
         }
-        // One more stage carries the stop mark (no data).
-        if (pos.s >= uint32_t(kBwdStages)) mbar_wait(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u, &abort_flag);
-        mbar_arrive(bar(kBarQdoFull + pos.qs));
       }
-    } else if (warp == 17) {
-      // ---------------- LSE/delta staging and the steps' control words ----------------
-      // A step's rows are requested before the wait for a free stage, so that this latency does not
-      // sit between a stage becoming free and becoming full again. They are staged negated: -lse in
-      // the log2 domain and -delta. Rows past the end of the sequence get -lse = -inf, which makes
-      // their P^T column 0.
-      BwdStepPos pos;
-      uint32_t ni = 0;
+      if (wk.n_q < 0) break;
+      const int rows_live = min(wk.lk - wk.kt * kTile, kTile);
+      const int64_t stat_base =
+          packed ? int64_t(wk.h) * p.total_q + wk.q_begin : (int64_t(wk.b) * p.heads + wk.h) * p.lq;
+      int jt = bwd_start(wk);
 #pragma unroll 1
-      for (uint32_t round = 0;; ++round) {
-        const BwdWorkOf<kCut> wk = next_work(round);
-        if (wk.n_q < 0) break;
-        if (wk.n_q == 0) continue;
-        const int rows_live = min(wk.lk - wk.kt * kTile, kTile);
-        const int64_t stat_base =
-            packed ? int64_t(wk.h) * p.total_q + wk.q_begin : (int64_t(wk.b) * p.heads + wk.h) * p.lq;
-        int jt = bwd_start(wk);
-#pragma unroll 1
-        for (int j = 0; j < wk.n_q; ++j) {
-          float l2[4], dl[4];
+      for (int j = 0; j < wk.n_q; ++j) {
+        float l2[4], dl[4];  // (as they are: arithmetic on them here would wait for them before the TMA loads are issued)
 #pragma unroll
-          for (int r4 = 0; r4 < 4; ++r4) {
-            const int r = jt * kTile + r4 * 32 + lane;
-            l2[r4] = -INFINITY, dl[r4] = 0.f;
-            if (r < wk.lq) {
-              l2[r4] = p.lse[stat_base + r] * -1.4426950408889634f;
-              dl[r4] = -p.delta[stat_base + r];
-            }
-          }
-          if (pos.s >= uint32_t(kBwdStages) && lane == 0)
-            mbar_wait(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u, &abort_flag);
-          __syncwarp();
-#pragma unroll
-          for (int r4 = 0; r4 < 4; ++r4) {
-            sLse[pos.qs * kTile + r4 * 32 + lane] = l2[r4];
-            sDelta[pos.qs * kTile + r4 * 32 + lane] = dl[r4];
-          }
-          if (lane == 0) {
-            const uint32_t ctrl = (j == 0 ? kCtrlFirst : 0u) | (j == wk.n_q - 1 ? kCtrlLast : 0u) |
-                                  ((ni & 1u) ? kCtrlKb : 0u) | (uint32_t(rows_live) << 8);
-            sCtrl[pos.qs] = ctrl;
-            sCtrlQ[pos.s & 7u] = ctrl;
-          }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar(kBarQdoFull + pos.qs));
-          pos.advance();
-          jt = jt + 1 == bwd_tiles(wk) ? 0 : jt + 1;
+        for (int r4 = 0; r4 < 4; ++r4) {
+          const int r = jt * kTile + r4 * 32 + lane;
+          l2[r4] = INFINITY, dl[r4] = 0.f;
+          if (r < wk.lq) l2[r4] = p.lse[stat_base + r], dl[r4] = p.delta[stat_base + r];
         }
-        ++ni;
+        if (lane == 0) {
+          if (pos.s >= uint32_t(kBwdStages)) mbar_wait(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u, &abort_flag);
+          mbar_arrive_expect_tx(bar(kBarQdoFull + pos.qs), 2 * kTileBytes);
+          tma_load_4d(sQ(pos.qs), &tmap_q, bar(kBarQdoFull + pos.qs), 0, wk.q_begin + jt * kTile, wk.h, wk.bcoord);
+          tma_load_4d(sDO(pos.qs), &tmap_do, bar(kBarQdoFull + pos.qs), 0, wk.q_begin + jt * kTile, wk.h, wk.bcoord);
+          const uint32_t ctrl = (j == 0 ? kCtrlFirst : 0u) | (j == wk.n_q - 1 ? kCtrlLast : 0u) | (kb ? kCtrlKb : 0u) |
+                                (uint32_t(rows_live) << 8);
+          sCtrl[pos.qs] = ctrl;
+          sCtrlQ[pos.s & 7u] = ctrl;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int r4 = 0; r4 < 4; ++r4) {
+          sLse[pos.qs * kTile + r4 * 32 + lane] = l2[r4] * -1.4426950408889634f;
+          sDelta[pos.qs * kTile + r4 * 32 + lane] = -dl[r4];
+        }
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(bar(kBarQdoFull + pos.qs));
+          if (j == 0) {
+            if (ni >= 1) mbar_wait(bar(kBarVFree), (ni - 1) & 1, &abort_flag);
+            mbar_arrive_expect_tx(bar(kBarVFull), kTileBytes);
+            tma_load_4d(sV, &tmap_v, bar(kBarVFull), 0, krow, wk.h, wk.bcoord);
+          }
+        }
+        pos.advance();
+        jt = jt + 1 == bwd_tiles(wk) ? 0 : jt + 1;
       }
-      if (lane == 0) {
-        if (pos.s >= uint32_t(kBwdStages)) mbar_wait(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u, &abort_flag);
-        sCtrl[pos.qs] = kCtrlStop;
-        sCtrlQ[pos.s & 7u] = kCtrlStop;
-        mbar_arrive(bar(kBarQdoFull + pos.qs));
-      }
+      if (wk.n_q > 0) ++ni;
+      // The next unit is taken as late as can be: this warp is about three steps ahead of the MMAs,
+      // which covers the counter's and the list's latency, and a unit taken earlier would wait behind a
+      // long one while other CTAs run dry.
+      g = next_token(g);
+    }
+    // One more stage carries the stop mark (no data).
+    if (lane == 0) {
+      if (pos.s >= uint32_t(kBwdStages)) mbar_wait(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u, &abort_flag);
+      sCtrl[pos.qs] = kCtrlStop;
+      sCtrlQ[pos.s & 7u] = kCtrlStop;
+      mbar_arrive(bar(kBarQdoFull + pos.qs));
+      mbar_arrive(bar(kBarQdoFull + pos.qs));
     }
   } else if (warp >= 12) {
     // ---------------- drain warps: dQ tiles every step, dV and dK once per item ----------------
@@ -875,14 +854,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     }
     if (lane == 0) bulk_wait_group_read0();  // the staging rows must outlive the TMA engine's reads
   } else if (warp >= 8) {
-    setmaxnreg_dec<kBwdIssuerRegs>();
     // Three issuers, one elected thread each, that walk the CTA's steps by their control words. The two
     // halves of a step's query columns (one per compute warpgroup) run half a step apart, so one
     // warpgroup's exponentials overlap the other's dS arithmetic and the MMAs of both. P^T takes the
     // columns of the S^T it came from and dS^T those of its dP^T, so the next S^T (dP^T) may only be
     // written after the dV (dK) MMAs have read them: each pair is issued by one thread in that order, and
     // MMAs of one thread execute in order.
-    if (warp != 9 && elect_one()) {
+    if (elect_one()) {
       BwdStepPos pos;
       uint32_t ni = 0;  // items started
       volatile uint32_t* ctrl_ring = sCtrl;
