@@ -288,7 +288,7 @@ enum BwdBar : int {
 
 // One unit of a CTA's work: a 128-row K/V tile of one (sequence, head).
 struct BwdWork {
-  int n_q;  // query tiles to walk; 0: keys without queries (dK = dV = 0); -1: no more work
+  int n_q;  // query tiles to walk; 0: keys without queries (dK = dV = 0, not published); -1: no more work
   int kt, h, b, bcoord;
   int k_begin, lk, q_begin, lq;
 };
@@ -629,11 +629,26 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       return __shfl_sync(0xffffffffu, token, 0);
     };
     uint32_t g = packed ? next_token(0) : kCut ? 0u : blockIdx.x;
+    uint32_t round = 0;  // units published
 #pragma unroll 1
-    for (uint32_t round = 0;; ++round) {
+    for (;;) {
       const BwdWorkOf<kCut> wk = bwd_work<kCut>(p, g);
       const uint32_t slot = round % kBwdWorkSlots, kb = ni & 1u;
       const int krow = wk.k_begin + wk.kt * kTile;
+      const int rows_live = min(wk.lk - wk.kt * kTile, kTile);
+      if (!kCut && wk.n_q == 0) {
+        // Keys without queries: dK = dV = 0, written here. Such units have no step, and the drain warps hold a unit until
+        // the issuers have seen the next step: published, a few of them in a row would fill the ring and nothing would move.
+        auto clear = [&](__nv_bfloat16* rows, int64_t st) {
+#pragma unroll 1
+          for (int c = lane; c < rows_live * 8; c += 32)
+            *reinterpret_cast<uint4*>(rows + int64_t(c >> 3) * st + (c & 7) * 8) = make_uint4(0, 0, 0, 0);
+        };
+        clear(p.dv + (int64_t(wk.bcoord) * p.dv_sb + int64_t(wk.h) * p.dv_sh + krow * p.dv_st), p.dv_st);
+        clear(p.dk + (int64_t(wk.bcoord) * p.dk_sb + int64_t(wk.h) * p.dk_sh + krow * p.dk_st), p.dk_st);
+        g = next_token(g);
+        continue;
+      }
       if (lane == 0) {
         if (round >= uint32_t(kBwdWorkSlots))
           mbar_wait(bar(kBarWorkEmpty + slot), ((round / kBwdWorkSlots) - 1) & 1, &abort_flag);
@@ -645,8 +660,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           tma_load_4d(sK(kb), &tmap_k, bar(kBarKFull + kb), 0, krow, wk.h, wk.bcoord);
         }
       }
+      ++round;
       if (wk.n_q < 0) break;
-      const int rows_live = min(wk.lk - wk.kt * kTile, kTile);
       const int64_t stat_base =
           packed ? int64_t(wk.h) * p.total_q + wk.q_begin : (int64_t(wk.b) * p.heads + wk.h) * p.lq;
       int jt = bwd_start(wk);
@@ -687,7 +702,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         pos.advance();
         jt = jt + 1 == bwd_tiles(wk) ? 0 : jt + 1;
       }
-      if (wk.n_q > 0) ++ni;
+      ++ni;
       // The next unit is taken as late as can be: this warp is about three steps ahead of the MMAs,
       // which covers the counter's and the list's latency, and a unit taken earlier would wait behind a
       // long one while other CTAs run dry.
@@ -732,17 +747,6 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       const int out_row = wk.k_begin + wk.kt * kTile + quad * 32, bcoord = wk.bcoord;
       auto dv_rows = [&] { return p.dv + (int64_t(bcoord) * p.dv_sb + int64_t(h) * p.dv_sh + out_row * p.dv_st); };
       auto dk_rows = [&] { return p.dk + (int64_t(bcoord) * p.dk_sb + int64_t(h) * p.dk_sh + out_row * p.dk_st); };
-      if (n_q == 0) {
-        // No queries at all: dK = dV = 0.
-        if (lane < rows_live) {
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            reinterpret_cast<uint4*>(dv_rows() + int64_t(lane) * p.dv_st)[c] = make_uint4(0, 0, 0, 0);
-            reinterpret_cast<uint4*>(dk_rows() + int64_t(lane) * p.dk_st)[c] = make_uint4(0, 0, 0, 0);
-          }
-        }
-        continue;
-      }
       const int n_qt = bwd_tiles(wk), part = bwd_part(wk);
       int row = (packed ? 0 : wk.b * p.lq) + wk.q_begin + quad * 32 + bwd_start(wk) * kTile;
       const int row_end = (packed ? 0 : wk.b * p.lq) + wk.q_begin + quad * 32 + n_qt * kTile;
