@@ -454,7 +454,7 @@ __device__ __noinline__ void bwd_compute_role(const uint32_t bar0, int* abort_fl
     if (ctrl & kCtrlStop) {
       // The dQ issuer learns of the end here -- once it has seen the step before (a barrier must never
       // run two phases ahead of a waiter that tests by parity).
-      if (s > 0) mbar_wait(bar(kBarDsFree), (s - 1) & 1, abort_flag);
+      if (s > 0) mbar_wait_inline(bar(kBarDsFree), (s - 1) & 1, abort_flag);
       __syncwarp();
       mbar_arrive_if(bar(kBarDsFull + w), lane0);
       break;
@@ -492,7 +492,7 @@ __device__ __noinline__ void bwd_compute_role(const uint32_t bar0, int* abort_fl
       const float2 v = dl2[4 * i];
       nd[i] = pack_f32x2(v.x, v.y);
     }
-    if (!dp_ok) mbar_wait(bar(kBarDpFull + w), s & 1, abort_flag);
+    if (!dp_ok) mbar_wait_inline(bar(kBarDpFull + w), s & 1, abort_flag);
     __syncwarp();
     tc_fence_after();
     tmem_ld_16x256b_x8(tm_dp, ra[0]);
@@ -515,7 +515,7 @@ __device__ __noinline__ void bwd_compute_role(const uint32_t bar0, int* abort_fl
     tc_fence_before();
     __syncwarp();
     mbar_arrive_if(bar(kBarDstFull + w), lane0);
-    if (!ds_ok) mbar_wait(bar(kBarDsFree), (s - 1) & 1, abort_flag);
+    if (!ds_ok) mbar_wait_inline(bar(kBarDsFree), (s - 1) & 1, abort_flag);
     __syncwarp();  // lanes leave a wait one by one; the aligned instructions below need the whole warp
 #pragma unroll
     for (int half = 0; half < 2; ++half)
@@ -605,7 +605,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const uint32_t slot = round % kBwdWorkSlots;
     BwdWorkOf<kCut> w;
     w.n_q = -1;
-    if (mbar_wait(bar(kBarWorkFull + slot), (round / kBwdWorkSlots) & 1, &abort_flag)) w = work_ring[slot];
+    if (mbar_wait_inline(bar(kBarWorkFull + slot), (round / kBwdWorkSlots) & 1, &abort_flag)) w = work_ring[slot];
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(kBarWorkEmpty + slot));
     return w;
@@ -651,11 +651,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       if (lane == 0) {
         if (round >= uint32_t(kBwdWorkSlots))
-          mbar_wait(bar(kBarWorkEmpty + slot), ((round / kBwdWorkSlots) - 1) & 1, &abort_flag);
+          mbar_wait_inline(bar(kBarWorkEmpty + slot), ((round / kBwdWorkSlots) - 1) & 1, &abort_flag);
         work_ring[slot] = wk;
         mbar_arrive(bar(kBarWorkFull + slot));
         if (wk.n_q > 0) {
-          if (ni >= 2) mbar_wait(bar(kBarKFree + kb), ((ni >> 1) - 1) & 1, &abort_flag);
+          if (ni >= 2) mbar_wait_inline(bar(kBarKFree + kb), ((ni >> 1) - 1) & 1, &abort_flag);
           mbar_arrive_expect_tx(bar(kBarKFull + kb), kTileBytes);
           tma_load_4d(sK(kb), &tmap_k, bar(kBarKFull + kb), 0, krow, wk.h, wk.bcoord);
         }
@@ -675,7 +675,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           if (r < wk.lq) l2[r4] = p.lse[stat_base + r], dl[r4] = p.delta[stat_base + r];
         }
         if (lane == 0) {
-          if (pos.s >= uint32_t(kBwdStages)) mbar_wait(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u, &abort_flag);
+          if (pos.s >= uint32_t(kBwdStages)) mbar_wait_inline(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u, &abort_flag);
           mbar_arrive_expect_tx(bar(kBarQdoFull + pos.qs), 2 * kTileBytes);
           tma_load_4d(sQ(pos.qs), &tmap_q, bar(kBarQdoFull + pos.qs), 0, wk.q_begin + jt * kTile, wk.h, wk.bcoord);
           tma_load_4d(sDO(pos.qs), &tmap_do, bar(kBarQdoFull + pos.qs), 0, wk.q_begin + jt * kTile, wk.h, wk.bcoord);
@@ -694,7 +694,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (lane == 0) {
           mbar_arrive(bar(kBarQdoFull + pos.qs));
           if (j == 0) {
-            if (ni >= 1) mbar_wait(bar(kBarVFree), (ni - 1) & 1, &abort_flag);
+            if (ni >= 1) mbar_wait_inline(bar(kBarVFree), (ni - 1) & 1, &abort_flag);
             mbar_arrive_expect_tx(bar(kBarVFull), kTileBytes);
             tma_load_4d(sV, &tmap_v, bar(kBarVFull), 0, krow, wk.h, wk.bcoord);
           }
@@ -710,7 +710,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     }
     // One more stage carries the stop mark (no data).
     if (lane == 0) {
-      if (pos.s >= uint32_t(kBwdStages)) mbar_wait(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u, &abort_flag);
+      if (pos.s >= uint32_t(kBwdStages)) mbar_wait_inline(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u, &abort_flag);
       sCtrl[pos.qs] = kCtrlStop;
       sCtrlQ[pos.s & 7u] = kCtrlStop;
       mbar_arrive(bar(kBarQdoFull + pos.qs));
@@ -755,7 +755,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       for (int e = 0; e < n_q + 2; ++e) {
         if (e == n_q - 1 || e == n_q + 1) {
           const bool is_dk = e > n_q;
-          mbar_wait(bar(is_dk ? kBarDkDone : kBarDvDone), ni & 1, &abort_flag);
+          mbar_wait_inline(bar(is_dk ? kBarDkDone : kBarDvDone), ni & 1, &abort_flag);
           tc_fence_after();
           const uint32_t tm_acc = (is_dk ? tm_dk : tm_dv) + lane_off;
           const float out_scale = is_dk ? p.scale : 1.f;
@@ -819,7 +819,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           }
           continue;
         }
-        mbar_wait(bar(kBarDqFull), s & 1, &abort_flag);
+        mbar_wait_inline(bar(kBarDqFull), s & 1, &abort_flag);
         tc_fence_after();
         if (lane == 0) bulk_wait_group_read0();  // the previous reductions have read the staging rows
         __syncwarp();
@@ -876,7 +876,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         auto copy_k = [&](uint32_t c) {
           const uint32_t kb = (c & kCtrlKb) ? 1u : 0u;
           const uint64_t kd = make_sdesc(sK(kb), 16, 1024);
-          mbar_wait(bar(kBarKFull + kb), (ni >> 1) & 1, &abort_flag);
+          mbar_wait_inline(bar(kBarKFull + kb), (ni >> 1) & 1, &abort_flag);
           ++ni;
 #pragma unroll 1
           for (int k = 0; k < 4; ++k) tmem_copy_128x256b(tm_k + 8 * k, kd + 2 * k);
@@ -887,7 +887,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           for (int k = 0; k < 4; ++k) mma_ts(tm_s + 64 * h, tm_k + 8 * k, qd + 2 * k, kIdescSH, k > 0);
           tc_commit(bar(kBarSFull + h));
         };
-        mbar_wait(bar(kBarQdoFull), 0, &abort_flag);
+        mbar_wait_inline(bar(kBarQdoFull), 0, &abort_flag);
         ctrl = ctrl_ring[0];
         if (!(ctrl & kCtrlStop)) {
           copy_k(ctrl);
@@ -902,23 +902,23 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           BwdStepPos next = pos;
           next.advance();
           // The previous item's dV has to be out of tensor memory before this one's first MMA.
-          if (first && ni > 1) mbar_wait(bar(kBarDvOut), (ni - 2) & 1, &abort_flag);
+          if (first && ni > 1) mbar_wait_inline(bar(kBarDvOut), (ni - 2) & 1, &abort_flag);
           const uint64_t gd_mn = make_sdesc(sDO(pos.qs), 1024, 1024);
           uint32_t next_ctrl = 0;
 #pragma unroll 1
           for (int h = 0; h < 2; ++h) {
-            if (!mbar_wait(bar(kBarPFull + h), pos.s & 1, &abort_flag)) next_ctrl = kCtrlStop;
+            if (!mbar_wait_inline(bar(kBarPFull + h), pos.s & 1, &abort_flag)) next_ctrl = kCtrlStop;
             tc_fence_after();
 #pragma unroll
             for (int k = 0; k < 4; ++k)  // A: P^T of query columns [64h + 16k, +16)
               mma_ts(tm_dv, tm_s + 64 * h + 8 * k, gd_mn + 512 * h + 128 * k, kIdescKN, !first || (h + k > 0));
             if (h == 0) {
               if (pos.s == 0) issue_s(0, 1);  // the second half starts later: see above
-              mbar_wait(bar(kBarQdoFull + next.qs), next.qph, &abort_flag);
+              mbar_wait_inline(bar(kBarQdoFull + next.qs), next.qph, &abort_flag);
               next_ctrl |= ctrl_ring[next.qs];
               if ((next_ctrl & (kCtrlFirst | kCtrlStop)) == kCtrlFirst) {
                 // The MMAs that read the previous item's K must be complete.
-                mbar_wait(bar(kBarSFull + 1), pos.s & 1, &abort_flag);
+                mbar_wait_inline(bar(kBarSFull + 1), pos.s & 1, &abort_flag);
                 tc_fence_after();
                 copy_k(next_ctrl);
               }
@@ -938,7 +938,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         // ---------------- dP^T = V dO^T of step s+1 after dK += dS^T Q of step s, half by half ----------------
         const uint64_t vd = make_sdesc(sV, 16, 1024);
         auto copy_v = [&] {
-          mbar_wait(bar(kBarVFull), ni & 1, &abort_flag);
+          mbar_wait_inline(bar(kBarVFull), ni & 1, &abort_flag);
           ++ni;
 #pragma unroll 1
           for (int k = 0; k < 4; ++k) tmem_copy_128x256b(tm_v + 8 * k, vd + 2 * k);
@@ -950,7 +950,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           for (int k = 0; k < 4; ++k) mma_ts(tm_dp + 64 * h, tm_v + 8 * k, gd + 2 * k, kIdescSH, k > 0);
           tc_commit(bar(kBarDpFull + h));
         };
-        mbar_wait(bar(kBarQdoFull), 0, &abort_flag);
+        mbar_wait_inline(bar(kBarQdoFull), 0, &abort_flag);
         ctrl = ctrl_ring[0];
         if (!(ctrl & kCtrlStop)) {
           copy_v();
@@ -962,22 +962,22 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           const bool first = (ctrl & kCtrlFirst) != 0;
           BwdStepPos next = pos;
           next.advance();
-          if (first && ni > 1) mbar_wait(bar(kBarDkOut), (ni - 2) & 1, &abort_flag);
+          if (first && ni > 1) mbar_wait_inline(bar(kBarDkOut), (ni - 2) & 1, &abort_flag);
           const uint64_t qd_mn = make_sdesc(sQ(pos.qs), 1024, 1024);
           uint32_t next_ctrl = 0;
 #pragma unroll 1
           for (int h = 0; h < 2; ++h) {
-            if (!mbar_wait(bar(kBarDstFull + h), pos.s & 1, &abort_flag)) next_ctrl = kCtrlStop;
+            if (!mbar_wait_inline(bar(kBarDstFull + h), pos.s & 1, &abort_flag)) next_ctrl = kCtrlStop;
             tc_fence_after();
 #pragma unroll
             for (int k = 0; k < 4; ++k)  // A: dS^T of query columns [64h + 16k, +16)
               mma_ts(tm_dk, tm_dp + 64 * h + 8 * k, qd_mn + 512 * h + 128 * k, kIdescKN, !first || (h + k > 0));
             if (h == 0) {
-              mbar_wait(bar(kBarQdoFull + next.qs), next.qph, &abort_flag);
+              mbar_wait_inline(bar(kBarQdoFull + next.qs), next.qph, &abort_flag);
               next_ctrl |= ctrl_ring[next.qs];
               if ((next_ctrl & (kCtrlFirst | kCtrlStop)) == kCtrlFirst) {
                 // The MMAs that read the previous item's V must be complete.
-                mbar_wait(bar(kBarDpFull + 1), pos.s & 1, &abort_flag);
+                mbar_wait_inline(bar(kBarDpFull + 1), pos.s & 1, &abort_flag);
                 tc_fence_after();
                 copy_v();
               }
@@ -1002,16 +1002,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           // again is the tightest in the pipeline), so it reads a copy of the control word from a ring of
           // eight: the word of step s+8 is written after step s+5 has freed its stage, hence after the
           // dQ MMAs of step s+3. The compute warps have seen the word before they arrive here.
-          if (!mbar_wait(bar(kBarDsFull), pos.s & 1, &abort_flag)) break;
+          if (!mbar_wait_inline(bar(kBarDsFull), pos.s & 1, &abort_flag)) break;
           ctrl = (reinterpret_cast<volatile uint32_t*>(sCtrlQ))[pos.s & 7u];
           if (ctrl & kCtrlStop) break;
           if (ctrl & kCtrlFirst) {
             kb = (ctrl & kCtrlKb) ? 1u : 0u;
             kd_mn = make_sdesc(sK(kb), 1024, 1024);
-            mbar_wait(bar(kBarKFull + kb), (ni >> 1) & 1, &abort_flag);
+            mbar_wait_inline(bar(kBarKFull + kb), (ni >> 1) & 1, &abort_flag);
           }
-          if (pos.s > 0) mbar_wait(bar(kBarDqFree), (pos.s - 1) & 1, &abort_flag);
-          mbar_wait(bar(kBarDsFull + 1), pos.s & 1, &abort_flag);
+          if (pos.s > 0) mbar_wait_inline(bar(kBarDqFree), (pos.s - 1) & 1, &abort_flag);
+          mbar_wait_inline(bar(kBarDsFull + 1), pos.s & 1, &abort_flag);
           tc_fence_after();
 #pragma unroll
           for (int k = 0; k < 8; ++k) mma_ss(tm_dq, ds_mn + 128 * k, kd_mn + 128 * k, kIdescNN, k > 0);

@@ -114,7 +114,7 @@ constexpr uint64_t kWaitLimitNs = 2000000000ull;  // about two seconds
 // (at most 4 s: the clock is the low word of the nanosecond timer).
 // The loop is kept as small as it can be -- 32-bit timer arithmetic, the flag touched with plain
 // state-space accesses, the status word left to the kernel's end: the warp-specialised kernels have dozens of
-// wait sites, every one of them inlined, and their hot code has to fit the SM's instruction cache (with a
+// wait sites, and their hot code has to fit the SM's instruction cache (with a
 // larger loop the backward kernel's instruction-cache hit rate was 92 % at best and instruction
 // fetch was its top stall). The status word's store at every site was 3 of the backward kernel's 54 KB; without it the
 // backward of 500 sequences of 1..300 tokens takes 555 instead of 568 us, of 32 x 12 x 820 328 instead of 333. A smaller site
@@ -126,11 +126,7 @@ __device__ __forceinline__ uint32_t globaltimer_lo() {
   return t;
 }
 
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
-                                          uint64_t limit_ns = kWaitLimitNs) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint32_t flag_addr = smem_u32(const_cast<int*>(abort_flag));
-  const uint32_t limit = uint32_t(limit_ns);
+__device__ __forceinline__ bool mbar_wait_loop(uint32_t bar, uint32_t parity, uint32_t flag_addr, uint32_t limit) {
   const uint32_t t0 = globaltimer_lo();
 #pragma unroll 1
   for (;;) {
@@ -142,6 +138,21 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
   asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(flag_addr), "r"(1) : "memory");
   return false;
+}
+// A site that has to wait calls the loop (112 bytes a site instead of 300): the forward, 48 -> 44 KB, takes 36.2 instead of 37.0
+// us on one sequence of 2000 tokens among thirty of 200, 942 instead of 961 on 256 of 720..920, 1 % less on most others.
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, uint32_t flag_addr, uint32_t limit) {
+  return mbar_wait_loop(bar, parity, flag_addr, limit);
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+                                          uint64_t limit_ns = kWaitLimitNs) {
+  if (mbar_try_wait(bar, parity)) return true;
+  return mbar_wait_slow(bar, parity, smem_u32(const_cast<int*>(abort_flag)), uint32_t(limit_ns));
+}
+// The same without a call, for code that fills its registers and for code that is short enough.
+__device__ __forceinline__ bool mbar_wait_inline(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (mbar_try_wait(bar, parity)) return true;
+  return mbar_wait_loop(bar, parity, smem_u32(const_cast<int*>(abort_flag)), uint32_t(kWaitLimitNs));
 }
 
 // At the end of a kernel, by one thread behind a block-wide barrier: says whether a wait of this block gave up.
@@ -233,6 +244,28 @@ __device__ __forceinline__ void bulk_commit_group() { asm volatile("cp.async.bul
 // Waits until the shared-memory sources of all committed bulk groups have been read.
 __device__ __forceinline__ void bulk_wait_group_read0() {
   asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+
+// Waits until all but the kPending newest bulk groups of the thread are complete: their writes to global memory
+// done, not only their sources read.
+template <int kPending>
+__device__ __forceinline__ void bulk_wait_group() {
+  asm volatile("cp.async.bulk.wait_group %0;" ::"n"(kPending) : "memory");
+}
+// Plain bulk copies of contiguous bytes (addresses and size multiples of 16).
+__device__ __forceinline__ void bulk_load(uint32_t smem_dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_dst),
+               "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_store(void* dst, uint32_t smem_src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_src), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_reduce_add(float* dst, uint32_t smem_src, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;" ::"l"(dst), "r"(smem_src),
+               "r"(bytes)
+               : "memory");
 }
 
 // ----------------------------------------------------------------------------------------
@@ -380,8 +413,8 @@ __device__ __forceinline__ bool mbar_wait2(uint32_t bar_a, uint32_t par_a, uint3
                                            volatile int* abort_flag) {
   const bool a = mbar_try_wait(bar_a, par_a);
   const bool b = mbar_try_wait(bar_b, par_b);
-  if (!a && !mbar_wait(bar_a, par_a, abort_flag)) return false;
-  return b || mbar_wait(bar_b, par_b, abort_flag);
+  if (!a && !mbar_wait_inline(bar_a, par_a, abort_flag)) return false;
+  return b || mbar_wait_inline(bar_b, par_b, abort_flag);
 }
 
 // ----------------------------------------------------------------------------------------
