@@ -153,7 +153,8 @@ int nb_attn_bwd(const nb_attn_bwd_args* args, void* stream);
 size_t nb_attn_bwd_workspace_bytes(const nb_attn_shape* shape);
 
 /* The larger workspace with which a dense nb_attn_bwd divides few key tiles evenly over the SMs of the
- * current device (see nb_attn_fwd_split_workspace_bytes); 0 where that would not pay. Optional. */
+ * current device (see nb_attn_fwd_split_workspace_bytes), or a packed one keeps the dQ tiles of the sequences
+ * that one block works off in scratch of that block's; 0 where neither would pay. Optional. */
 size_t nb_attn_bwd_split_workspace_bytes(const nb_attn_shape* shape);
 
 /* Backward for callers that cannot allocate device memory (no counterpart in the reference).

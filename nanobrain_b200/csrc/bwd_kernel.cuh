@@ -52,6 +52,14 @@
 //                              3.82 ms; this form 3.37 ms.
 //   attn_bwd_epilogue_kernel : dQ = bf16(scale * accumulator). HBM-bound.
 //
+// Packed calls with many (sequence, head) pairs of not too many tiles have a second kind of unit, a run: one
+// CTA works off all key tiles of a pair and keeps its dQ in tiles of its own (see BwdRun). Clearing the accumulator in
+// the prologue and reading it again in the epilogue is 16 % of the backward of such a call; for a run both fall away
+// and delta is all that the prologue computes. Whole backward, us, without and with runs: 256 sequences of 720..920
+// tokens x 12 heads 2505 -> 2230, 500 of 1..300 563 -> 427, 300 of 200 398 -> 295, 128 of 720..920 1082 -> 969, 64 of them 534 -> 499.
+// The form of the main kernel that knows runs is an instantiation of its own: its code is 2 KB larger, and
+// with its waits inlined like the others' 7 KB, which made it 5 to 20 % slower on calls without any run.
+//
 // Packed mode: block 0 of the prologue also builds the scheduler's work list of key tiles
 // (sched_kernel.cuh); the main kernel's work units are list entries x heads (the heads of one entry
 // adjacent), taken by the CTAs in the list's order of decreasing cost.
@@ -98,7 +106,14 @@ struct BwdParams {
   uint32_t split_base, split_extra;  // CTA c starts at step c * base + min(c, extra)
   int32_t n_qt;                      // dense mode: query tiles per sequence
   FastDiv div_n_qt;
+  FastDiv div_lq;
+  int32_t rows32;      // (token, head) rows can be counted in 31 bits
   int32_t row_blocks;  // blocks of the epilogue that convert dQ; the ones after them add up parts
+  // Runs: units that stand for all key tiles of a (sequence, head). Their dQ is summed up in the CTA's own
+  // tiles and leaves as bf16 with the last key tile, so the accumulator and the epilogue are for the others.
+  float* own;         // [CTAs][own_tiles][128 x 64]
+  int32_t own_tiles;  // query tiles per CTA
+  int32_t* rest;      // packed mode with runs: see sched_write_rest; NULL: every sequence is single tiles
   int64_t total_q, total_k;
   float scale, scale_log2;
   int32_t* status;
@@ -107,34 +122,110 @@ struct BwdParams {
 // ----------------------------------------------------------------------------------------
 // Prologue: one quarter-warp (8 lanes x 16 bytes) per (token, head) row.
 // ----------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) attn_bwd_prologue_kernel(const BwdParams p) {
+constexpr int kAuxThreads = 256;
+
+// Token, head and (dense mode) sequence and position of a (token, head) row. 64-bit divisions are routines of some
+// hundred instructions, so rows that fit 31 bits are divided by multiply-high. In packed mode b = 0 and tok = t.
+struct AuxRow {
+  int64_t t, b, tok;
+  int h;
+  __device__ __forceinline__ AuxRow(const BwdParams& p, int64_t row) {
+    b = 0;
+    if (p.rows32) {
+      const uint32_t t32 = p.div_heads.quot(uint32_t(row));
+      t = tok = t32, h = int(uint32_t(row) - t32 * uint32_t(p.heads));
+      if (p.cu_q == nullptr) {
+        const uint32_t b32 = p.div_lq.quot(t32);
+        b = b32, tok = t32 - b32 * uint32_t(p.lq);
+      }
+    } else {
+      t = tok = row / p.heads, h = int(row - t * p.heads);
+      if (p.cu_q == nullptr) b = t / p.lq, tok = t - b * p.lq;
+    }
+  }
+};
+// A block's part of `n_rows` rows where it takes consecutive ones: an equal share each.
+__device__ __forceinline__ int64_t aux_begin(int64_t n_rows, uint32_t blocks, uint32_t block) {
+  return min(int64_t(block) * ((n_rows + blocks - 1) / blocks), n_rows);
+}
+
+struct BwdPrologueShared {
+  SchedRunShared runs;
+  int end[kSchedRunSeqs + 1];  // last query row of each sequence + 1, and of the rows past the last one; bit 31: a run
+  int first;                   // the sequence in which the block's rows start
+};
+
+template <bool kRuns>
+__global__ void __launch_bounds__(kAuxThreads) attn_bwd_prologue_kernel(const BwdParams p) {
   __shared__ SchedShared sched_sm;
+  __shared__ std::conditional_t<kRuns, BwdPrologueShared, int> sm;
   pdl_wait();  // O comes from the forward kernel, dO from whatever ran before this call
   pdl_launch_dependents();
-  if (blockIdx.x == 0 && p.sched.items != nullptr) sched_build<256>(p.sched, sched_sm);
   const int64_t n_rows = p.total_q * p.heads;
   const int lane8 = threadIdx.x & 7;
-  int64_t row = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 3;
-  const int64_t row_step = (int64_t(gridDim.x) * blockDim.x) >> 3;
+  int64_t first = int64_t(blockIdx.x) * (kAuxThreads / 8), step = int64_t(gridDim.x) * (kAuxThreads / 8), end = n_rows;
+  SchedRuns rule = {-1, 0};
+  // With runs every block finds out by itself which sequences are: their accumulator needs no clearing.
+  if constexpr (kRuns) rule = sched_runs<kAuxThreads>(p.sched, sm.runs);
+  if (blockIdx.x == 0 && p.sched.items != nullptr) {
+    sched_build<kAuxThreads>(p.sched, sched_sm, rule);
+    if constexpr (kRuns) sched_write_rest<kAuxThreads>(p.sched, rule, sm.runs);
+  }
+  int seq = 0;
+  if constexpr (kRuns) {
+    // (The first block has the list to build, which the main kernel waits for: the others share its rows.)
+    const uint32_t others = gridDim.x - 1;
+    if (others > 0 && blockIdx.x == 0) return;
+    const uint32_t part = others > 0 ? blockIdx.x - 1 : 0, parts = others > 0 ? others : 1;
+    first = aux_begin(n_rows, parts, part), end = aux_begin(n_rows, parts, part + 1), step = kAuxThreads / 8;
+    const int tok = int(min(first, n_rows - 1) / p.heads);
+    if (threadIdx.x == 0) sm.first = 0;
+    __syncthreads();
+#pragma unroll 1
+    for (int i = threadIdx.x; i <= p.batch; i += kAuxThreads) {
+      int begin = 0, stop = int(p.total_q);
+      bool run = false;
+      if (!sm.runs.bad) {
+        begin = p.cu_q[i];
+        if (i < p.batch) {
+          stop = p.cu_q[i + 1];
+          const int keys = p.cu_k[i + 1] - p.cu_k[i], cost = sm.runs.cost[i];
+          run = keys > kTile ? i < rule.below && cost > 0 && cost <= rule.max_cost : keys > 0 && stop > begin;
+        }
+      }
+      sm.end[i] = stop | (run ? int(0x80000000u) : 0);
+      if (begin <= tok && tok < stop) sm.first = i;
+    }
+    __syncthreads();
+    seq = sm.first;
+  }
 #if NB_BWD_L2_HINTS
   const uint64_t keep = l2_policy_evict_last();
 #endif
-  for (; row < n_rows; row += row_step) {
-    const int64_t t = row / p.heads;
-    const int h = int(row - t * p.heads);
-    int64_t b = 0, tok = t, didx;
+  struct Loaded {
+    uint4 o, g;
+    int64_t row, didx;
+    bool clear;
+  };
+  auto load = [&](int64_t row, Loaded& l) {
+    const AuxRow w(p, row);
+    l.row = row, l.clear = true;
     if (p.cu_q == nullptr) {
-      b = t / p.lq;
-      tok = t - b * p.lq;
-      didx = (b * p.heads + h) * p.lq + tok;
+      l.didx = (w.b * p.heads + w.h) * p.lq + w.tok;
     } else {
-      didx = int64_t(h) * p.total_q + t;
+      l.didx = int64_t(w.h) * p.total_q + w.tok;
+      if constexpr (kRuns) {
+        int stop = sm.end[seq];
+        while (w.tok >= (stop & 0x7fffffff) && seq < p.batch) stop = sm.end[++seq];
+        l.clear = stop >= 0;
+      }
     }
-    const uint4 ov = *reinterpret_cast<const uint4*>(p.o + b * p.o_sb + tok * p.o_st + h * p.o_sh + lane8 * 8);
-    const uint4 gv =
-        *reinterpret_cast<const uint4*>(p.d_o + b * p.do_sb + tok * p.do_st + h * p.do_sh + lane8 * 8);
-    const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&ov);
-    const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&gv);
+    l.o = *reinterpret_cast<const uint4*>(p.o + w.b * p.o_sb + w.tok * p.o_st + w.h * p.o_sh + lane8 * 8);
+    l.g = *reinterpret_cast<const uint4*>(p.d_o + w.b * p.do_sb + w.tok * p.do_st + w.h * p.do_sh + lane8 * 8);
+  };
+  auto finish = [&](const Loaded& l) {
+    const __nv_bfloat162* o2 = reinterpret_cast<const __nv_bfloat162*>(&l.o);
+    const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&l.g);
     float acc = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -143,11 +234,13 @@ __global__ void __launch_bounds__(256) attn_bwd_prologue_kernel(const BwdParams 
       acc = fmaf(a.x, g.x, acc);
       acc = fmaf(a.y, g.y, acc);
     }
-    acc += __shfl_xor_sync(0xffffffffu, acc, 4);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
-    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
-    if (lane8 == 0) p.delta[didx] = acc;
-    float4* acc_row = reinterpret_cast<float4*>(p.dq_accum + row * kHeadDim);
+    const uint32_t group = 0xffu << (threadIdx.x & 24);
+    acc += __shfl_xor_sync(group, acc, 4);
+    acc += __shfl_xor_sync(group, acc, 2);
+    acc += __shfl_xor_sync(group, acc, 1);
+    if (lane8 == 0) p.delta[l.didx] = acc;
+    if (!l.clear) return;
+    float4* acc_row = reinterpret_cast<float4*>(p.dq_accum + l.row * kHeadDim);
     const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
 #if NB_BWD_L2_HINTS
     st_global_v4_hint(acc_row + lane8 * 2, z, keep);
@@ -156,6 +249,26 @@ __global__ void __launch_bounds__(256) attn_bwd_prologue_kernel(const BwdParams 
     acc_row[lane8 * 2] = z;
     acc_row[lane8 * 2 + 1] = z;
 #endif
+  };
+  if constexpr (kRuns) {
+    // Two rows at a time, so that twice the bytes are in flight: the stores keep the compiler from requesting the second
+    // row before the first is done. (Where every row is cleared too, the writes are more than half of the traffic and
+    // one row at a time is as fast.)
+#pragma unroll 1
+    for (int64_t row = first + (threadIdx.x >> 3); row < end; row += 2 * step) {
+      Loaded l0, l1;
+      load(row, l0);
+      const bool two = row + step < end;
+      if (two) load(row + step, l1);
+      finish(l0);
+      if (two) finish(l1);
+    }
+  } else {
+    for (int64_t row = first + (threadIdx.x >> 3); row < end; row += step) {
+      Loaded l;
+      load(row, l);
+      finish(l);
+    }
   }
 }
 
@@ -199,26 +312,47 @@ __device__ __forceinline__ void bwd_combine(const BwdParams& p, uint32_t block) 
 // ----------------------------------------------------------------------------------------
 // Epilogue: dQ = bf16(scale * accumulator), 8 lanes per (token, head) row; dK and dV of cut units.
 // ----------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) attn_bwd_epilogue_kernel(const BwdParams p) {
+template <bool kRuns>
+__global__ void __launch_bounds__(kAuxThreads) attn_bwd_epilogue_kernel(const BwdParams p) {
+  __shared__ SchedRest rest_sm[kRuns ? kSchedRunSeqs + 1 : 1];
+  __shared__ int first_sm;
   pdl_wait();  // the accumulator is complete when the main kernel is
   pdl_launch_dependents();
   if (int(blockIdx.x) >= p.row_blocks) return bwd_combine(p, blockIdx.x - uint32_t(p.row_blocks));
 #if NB_BWD_L2_HINTS
   const uint64_t drop = l2_policy_evict_first();
 #endif
-  const int64_t n_rows = p.total_q * p.heads;
   const int lane8 = threadIdx.x & 7;
-  int64_t row = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 3;
-  const int64_t row_step = (int64_t(p.row_blocks) * blockDim.x) >> 3;
-  for (; row < n_rows; row += row_step) {
-    const int64_t t = row / p.heads;
-    const int h = int(row - t * p.heads);
-    int64_t b = 0, tok = t;
-    if (p.cu_q == nullptr) {
-      b = t / p.lq;
-      tok = t - b * p.lq;
+  int64_t first = int64_t(blockIdx.x) * (kAuxThreads / 8), step = int64_t(p.row_blocks) * (kAuxThreads / 8),
+          end = p.total_q * p.heads;
+  int seq = 0;
+  if constexpr (kRuns) {
+    const int64_t n_rows = int64_t(p.rest[0]) * p.heads;
+    first = aux_begin(n_rows, uint32_t(p.row_blocks), blockIdx.x);
+    end = aux_begin(n_rows, uint32_t(p.row_blocks), blockIdx.x + 1), step = kAuxThreads / 8;
+    if (first >= end) return;  // the whole block
+    const int tok = int(first / p.heads);
+    const SchedRest* rest = reinterpret_cast<const SchedRest*>(p.rest + 4);
+#pragma unroll 1
+    for (int i = threadIdx.x; i <= p.batch; i += kAuxThreads) {
+      const SchedRest r = rest[i];
+      rest_sm[i] = r;
+      if (tok < r.end && (i == 0 || tok >= rest[i - 1].end)) first_sm = i;
     }
-    const float4* acc_row = reinterpret_cast<const float4*>(p.dq_accum + row * kHeadDim);
+    __syncthreads();
+    seq = first_sm;
+  }
+  for (int64_t row = first + (threadIdx.x >> 3); row < end; row += step) {
+    const AuxRow w(p, row);
+    const int64_t b = w.b;
+    const int h = w.h;
+    int64_t tok = w.tok, at = row;
+    if constexpr (kRuns) {
+      while (tok >= rest_sm[seq].end) ++seq;
+      tok += rest_sm[seq].shift;
+      at = tok * p.heads + h;
+    }
+    const float4* acc_row = reinterpret_cast<const float4*>(p.dq_accum + at * kHeadDim);
 #if NB_BWD_L2_HINTS
     const float4 x = ld_global_v4_hint(acc_row + lane8 * 2, drop), y = ld_global_v4_hint(acc_row + lane8 * 2 + 1, drop);
 #else
@@ -251,7 +385,7 @@ constexpr int kBwdTmemCols = 512;
 // With 640 threads x 96 registers (TMA and LSE/delta rows in a warpgroup of their own; drain 64, loaders 48) ptxas
 // spilled 40 to 72 bytes in the other roles' step loops: whole backward of 2 x 12 x 820 32.9 us, now 30.8; 1 x 12 x 3476 132.0 and
 // 128.4; 32 x 12 x 820 328 and 317; 256 sequences of 720..920 tokens 2555 and 2500. (Many sequences of two tiles lose: 300 of 200
-// tokens 368 -> 384, where the one warp's reads of list and rows follow each other.)
+// tokens 368 -> 384, where the one warp's reads of list and rows follow each other; as runs they take 295.)
 constexpr int kBwdLaunchRegs = 128;
 constexpr int kBwdComputeRegs = 152;
 constexpr int kBwdIssuerRegs = 104;  // issuers and loader
@@ -281,7 +415,8 @@ enum BwdBar : int {
   kBarDkDone,
   kBarDvOut,    // 4: the drain warps have read the item's dV accumulator
   kBarDkOut,    // 4
-  kBarWorkFull,                                  // [kBwdWorkSlots] the ring of published units
+  kBarOwnFull,  // [4]: a drain warp's part of the CTA's own dQ tile has been read back
+  kBarWorkFull = kBarOwnFull + 4,                // [kBwdWorkSlots] the ring of published units
   kBarWorkEmpty = kBarWorkFull + kBwdWorkSlots,  // [kBwdWorkSlots], 4: drain warps
   kBwdNumBars = kBarWorkEmpty + kBwdWorkSlots
 };
@@ -292,6 +427,15 @@ struct BwdWork {
   int kt, h, b, bcoord;
   int k_begin, lk, q_begin, lq;
 };
+
+// Key tiles of a run go one after the other through the same CTA, each in the order of query tiles that it has as a
+// unit of its own (so dK and dV are the same either way). dQ of the first key tile is stored into the CTA's own
+// tiles, that of the others added to them, and the last one's leaves as bf16 together with what is there. So the accumulator of a run is neither
+// cleared nor read by a pass of its own, and 148 x own_tiles x 32 KB stay in the L2 from run to run.
+enum BwdRun : int { kRunTile = 1, kRunFirst = 2, kRunLast = 4 };
+// Most query tiles of a run: 148 CTAs' own tiles, Q and dO then take 148 x 8 x 64 KB = 78 of the L2's 126 MB. (With 18, 16
+// sequences of 1700..2140 tokens took 1118 us where single tiles took 953.)
+constexpr int kBwdRunTiles = 8;
 
 // Query tile an item starts at. Concurrent CTAs work on the key tiles of one (sequence, head) and
 // all add into the same dQ tiles, so they start at different ones: key tile kt at query tile kt,
@@ -308,24 +452,35 @@ struct BwdCutWork : BwdWork {
   int jt0, n_qt;  // first query tile of the walk, query tiles of the sequence
   int part;       // >= 0: the unit is cut; where this CTA's dV and dK go
 };
+// And where there may be runs.
+struct BwdRunWork : BwdWork {
+  int run;  // a key tile of a run: BwdRun bits; 0: a unit of its own
+};
+// The kernel's forms.
+enum BwdMode : int { kBwdWhole, kBwdCut, kBwdRuns };
+__device__ __forceinline__ int bwd_run(const BwdWork&) { return 0; }
+__device__ __forceinline__ int bwd_run(const BwdRunWork& w) { return w.run; }
 __device__ __forceinline__ int bwd_start(const BwdWork& w) { return bwd_first_tile(w.kt, w.n_q); }
 __device__ __forceinline__ int bwd_start(const BwdCutWork& w) { return w.jt0; }
 __device__ __forceinline__ int bwd_tiles(const BwdWork& w) { return w.n_q; }
 __device__ __forceinline__ int bwd_tiles(const BwdCutWork& w) { return w.n_qt; }
 __device__ __forceinline__ int bwd_part(const BwdWork&) { return -1; }
 __device__ __forceinline__ int bwd_part(const BwdCutWork& w) { return w.part; }
-template <bool kCut>
-using BwdWorkOf = std::conditional_t<kCut, BwdCutWork, BwdWork>;
+template <int kMode>
+using BwdWorkOf = std::conditional_t<kMode == kBwdCut, BwdCutWork, std::conditional_t<kMode == kBwdRuns, BwdRunWork, BwdWork>>;
 
 // Unit g of the call; n_q = -1 past the last one. The loader fetches a CTA's units and publishes them to
 // the other roles through a small ring. Dense units all cost the same: CTA c of G takes c, G + c, ...
 // Packed units are taken from the list's counter, most expensive first. Where whole dense units would
 // leave CTAs idle, CTA c takes an equal run of (unit, query tile) steps; g then counts the units that run
-// touches, and at most two of them are cut: the one the run starts in and the one it ends in.
-template <bool kCut>
-__device__ __forceinline__ BwdWorkOf<kCut> bwd_work(const BwdParams& p, uint32_t g) {
-  BwdWorkOf<kCut> w;
+// touches, and at most two of them are cut: the one that run starts in and the one it ends in.
+// kt = -1: all key tiles of the (sequence, head), a run.
+template <int kMode>
+__device__ __forceinline__ BwdWorkOf<kMode> bwd_work(const BwdParams& p, uint32_t g) {
+  constexpr bool kCut = kMode == kBwdCut, kRuns = kMode == kBwdRuns;
+  BwdWorkOf<kMode> w;
   w.n_q = -1, w.kt = 0, w.h = 0, w.b = 0, w.bcoord = 0, w.k_begin = 0, w.lk = 0, w.q_begin = 0, w.lq = 0;
+  if constexpr (kRuns) w.run = 0;
   if constexpr (kCut) {
     w.jt0 = w.n_qt = 0, w.part = -1;
     const int s0 = int(bwd_split_start(p, blockIdx.x)), s1 = int(bwd_split_start(p, blockIdx.x + 1));
@@ -340,7 +495,7 @@ __device__ __forceinline__ BwdWorkOf<kCut> bwd_work(const BwdParams& p, uint32_t
   } else if (g >= uint32_t(p.n_work)) {
     return w;
   }
-  if (!kCut && p.cu_q != nullptr) {
+  if (kRuns || (!kCut && p.cu_q != nullptr)) {
     // One 32-byte read tells all about the item (the sequence index `batch` stands for the rows past
     // the last sequence: keys without queries). Unused entries sit at the end of the list.
     const uint32_t idx = p.div_heads.quot(g);
@@ -529,7 +684,7 @@ __device__ __noinline__ void bwd_compute_role(const uint32_t bar0, int* abort_fl
   }
 }
 
-template <bool kCut>
+template <int kMode>
 __global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                 const __grid_constant__ CUtensorMap tmap_v, const __grid_constant__ CUtensorMap tmap_do,
@@ -538,7 +693,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   __shared__ __align__(8) uint64_t bars[kBwdNumBars];
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
-  __shared__ BwdWorkOf<kCut> work_ring[kBwdWorkSlots];
+  constexpr bool kCut = kMode == kBwdCut, kRuns = kMode == kBwdRuns;
+  __shared__ BwdWorkOf<kMode> work_ring[kBwdWorkSlots];
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -565,6 +721,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
   const uint32_t bar0 = smem_u32(&bars[0]);
   auto bar = [&](int i) { return bar0 + 8u * uint32_t(i); };
+  // In the form with runs a wait's loop is called instead of inlined, 5 KB less code: 256 sequences of 720..920 tokens 2316 -> 2247 us.
+  // The others, small enough, do not gain (2 x 12 x 820: 31.7 -> 32.6).
+  auto wait = [&](uint32_t b, uint32_t parity) {
+    return kRuns ? mbar_wait(b, parity, &abort_flag) : mbar_wait_inline(b, parity, &abort_flag);
+  };
 
   if (tid == 9 * 32) {
     tma_prefetch_desc(&tmap_k);
@@ -598,14 +759,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   constexpr uint32_t kIdescSH = make_idesc(128, 64, 0, 0);   // K-major x K-major, N = 64
   constexpr uint32_t kIdescKN = make_idesc(128, 64, 0, 1);   // A K-major / tensor memory, B MN-major
   constexpr uint32_t kIdescNN = make_idesc(128, 64, 1, 1);   // A MN-major, B MN-major
-  const bool packed = !kCut && p.cu_q != nullptr;
+  const bool packed = kRuns || (!kCut && p.cu_q != nullptr);
 
   // The CTA's unit number `round`, read by a whole warp from the loader's ring.
   auto next_work = [&](uint32_t round) {
     const uint32_t slot = round % kBwdWorkSlots;
-    BwdWorkOf<kCut> w;
+    BwdWorkOf<kMode> w;
     w.n_q = -1;
-    if (mbar_wait_inline(bar(kBarWorkFull + slot), (round / kBwdWorkSlots) & 1, &abort_flag)) w = work_ring[slot];
+    if (wait(bar(kBarWorkFull + slot), (round / kBwdWorkSlots) & 1)) w = work_ring[slot];
     __syncwarp();
     if (lane == 0) mbar_arrive(bar(kBarWorkEmpty + slot));
     return w;
@@ -622,17 +783,23 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     // their P^T column 0.
     BwdStepPos pos;
     uint32_t ni = 0;  // items with queries so far
-    auto next_token = [&](uint32_t g) {
+    auto next_unit = [&](uint32_t g) {
       if (!packed) return kCut ? g + 1 : g + gridDim.x;
       uint32_t token = 0;
       if (lane == 0) token = sched_next(p.items);
       return __shfl_sync(0xffffffffu, token, 0);
     };
-    uint32_t g = packed ? next_token(0) : kCut ? 0u : blockIdx.x;
+    uint32_t g = packed ? next_unit(0) : kCut ? 0u : blockIdx.x;
+    BwdWorkOf<kMode> wk;
+    int kt_end = 0;  // of a run
     uint32_t round = 0;  // units published
 #pragma unroll 1
     for (;;) {
-      const BwdWorkOf<kCut> wk = bwd_work<kCut>(p, g);
+      if (kt_end == 0) wk = bwd_work<kMode>(p, g);
+      if constexpr (kRuns) {
+        if (wk.kt < 0) kt_end = (wk.lk + kTile - 1) / kTile, wk.kt = 0;
+        if (kt_end > 0) wk.run = kRunTile | (wk.kt == 0 ? kRunFirst : 0) | (wk.kt == kt_end - 1 ? kRunLast : 0);
+      }
       const uint32_t slot = round % kBwdWorkSlots, kb = ni & 1u;
       const int krow = wk.k_begin + wk.kt * kTile;
       const int rows_live = min(wk.lk - wk.kt * kTile, kTile);
@@ -646,16 +813,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         };
         clear(p.dv + (int64_t(wk.bcoord) * p.dv_sb + int64_t(wk.h) * p.dv_sh + krow * p.dv_st), p.dv_st);
         clear(p.dk + (int64_t(wk.bcoord) * p.dk_sb + int64_t(wk.h) * p.dk_sh + krow * p.dk_st), p.dk_st);
-        g = next_token(g);
+        g = next_unit(g);
         continue;
       }
       if (lane == 0) {
         if (round >= uint32_t(kBwdWorkSlots))
-          mbar_wait_inline(bar(kBarWorkEmpty + slot), ((round / kBwdWorkSlots) - 1) & 1, &abort_flag);
+          wait(bar(kBarWorkEmpty + slot), ((round / kBwdWorkSlots) - 1) & 1);
         work_ring[slot] = wk;
         mbar_arrive(bar(kBarWorkFull + slot));
         if (wk.n_q > 0) {
-          if (ni >= 2) mbar_wait_inline(bar(kBarKFree + kb), ((ni >> 1) - 1) & 1, &abort_flag);
+          if (ni >= 2) wait(bar(kBarKFree + kb), ((ni >> 1) - 1) & 1);
           mbar_arrive_expect_tx(bar(kBarKFull + kb), kTileBytes);
           tma_load_4d(sK(kb), &tmap_k, bar(kBarKFull + kb), 0, krow, wk.h, wk.bcoord);
         }
@@ -675,7 +842,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           if (r < wk.lq) l2[r4] = p.lse[stat_base + r], dl[r4] = p.delta[stat_base + r];
         }
         if (lane == 0) {
-          if (pos.s >= uint32_t(kBwdStages)) mbar_wait_inline(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u, &abort_flag);
+          if (pos.s >= uint32_t(kBwdStages)) wait(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u);
           mbar_arrive_expect_tx(bar(kBarQdoFull + pos.qs), 2 * kTileBytes);
           tma_load_4d(sQ(pos.qs), &tmap_q, bar(kBarQdoFull + pos.qs), 0, wk.q_begin + jt * kTile, wk.h, wk.bcoord);
           tma_load_4d(sDO(pos.qs), &tmap_do, bar(kBarQdoFull + pos.qs), 0, wk.q_begin + jt * kTile, wk.h, wk.bcoord);
@@ -694,7 +861,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (lane == 0) {
           mbar_arrive(bar(kBarQdoFull + pos.qs));
           if (j == 0) {
-            if (ni >= 1) mbar_wait_inline(bar(kBarVFree), (ni - 1) & 1, &abort_flag);
+            if (ni >= 1) wait(bar(kBarVFree), (ni - 1) & 1);
             mbar_arrive_expect_tx(bar(kBarVFull), kTileBytes);
             tma_load_4d(sV, &tmap_v, bar(kBarVFull), 0, krow, wk.h, wk.bcoord);
           }
@@ -703,14 +870,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         jt = jt + 1 == bwd_tiles(wk) ? 0 : jt + 1;
       }
       ++ni;
+      if constexpr (kRuns) {
+        if (++wk.kt < kt_end) continue;
+        kt_end = 0;
+      }
       // The next unit is taken as late as can be: this warp is about three steps ahead of the MMAs,
       // which covers the counter's and the list's latency, and a unit taken earlier would wait behind a
-      // long one while other CTAs run dry.
-      g = next_token(g);
+      // long one while other CTAs run dry. (Taken before the wait for the last step's stage: 300 sequences of 200 tokens 294 -> 300 us.)
+      g = next_unit(g);
     }
     // One more stage carries the stop mark (no data).
     if (lane == 0) {
-      if (pos.s >= uint32_t(kBwdStages)) mbar_wait_inline(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u, &abort_flag);
+      if (pos.s >= uint32_t(kBwdStages)) wait(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u);
       sCtrl[pos.qs] = kCtrlStop;
       sCtrlQ[pos.s & 7u] = kCtrlStop;
       mbar_arrive(bar(kBarQdoFull + pos.qs));
@@ -733,13 +904,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     const uint32_t lane_off = uint32_t(quad * 32) << 16;
     uint8_t* stage = sDQ_ptr + quad * 4096;
     uint8_t* ostage = sOut_ptr + quad * (kBwdOutStageBytes / 4);
-    uint32_t s = 0, ni = 0;
+    uint32_t s = 0, ni = 0, own_phase = 0;
 #if NB_BWD_L2_HINTS
     const uint64_t keep = l2_policy_evict_last();
 #endif
 #pragma unroll 1
     for (uint32_t round = 0;; ++round) {
-      const BwdWorkOf<kCut> wk = next_work(round);
+      const BwdWorkOf<kMode> wk = next_work(round);
       const int n_q = wk.n_q;
       if (n_q < 0) break;
       const int h = wk.h;
@@ -750,15 +921,48 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       const int n_qt = bwd_tiles(wk), part = bwd_part(wk);
       int row = (packed ? 0 : wk.b * p.lq) + wk.q_begin + quad * 32 + bwd_start(wk) * kTile;
       const int row_end = (packed ? 0 : wk.b * p.lq) + wk.q_begin + quad * 32 + n_qt * kTile;
+      // A run: this warp's part of the CTA's own dQ tiles, and reading one of them back into the staging rows.
+      const int run = bwd_run(wk);
+      float* const own0 = p.own + (int64_t(blockIdx.x) * p.own_tiles * 4 + quad) * 2048;
+      int jt = kRuns && run ? bwd_start(wk) : 0;
+      // Key tile kt starts one query tile behind the key tile before it, so a query tile's turns are n_q - 1
+      // steps apart, or further; where there are more key than query tiles they may be neighbours.
+      const bool far_apart = n_q > 2 && wk.kt < n_q;
+      const bool read_back = kRuns && (run & (kRunFirst | kRunLast)) == kRunLast;
+      // Waits until what was done to the own tile that is next, n_q - 1 steps ago or earlier, is complete.
+      auto own_order = [&] {
+        if (!far_apart) bulk_wait_group<0>();
+        else if (n_q < 5) bulk_wait_group<1>();
+        else if (n_q < 7) bulk_wait_group<3>();
+        else bulk_wait_group<5>();
+      };
+      auto own_load = [&] {
+        const float* own = own0 + jt * 8192;
+        mbar_arrive_expect_tx(bar(kBarOwnFull + quad), 8192);
+        bulk_load(smem_u32(stage), own, 4096, bar(kBarOwnFull + quad));
+        bulk_load(smem_u32(stage + kTileBytes), own + 1024, 4096, bar(kBarOwnFull + quad));
+      };
+      if (read_back && lane == 0) {
+        // (The last addition may still read the staging rows.)
+        bulk_wait_group_read0();
+        own_order();
+        own_load();
+      }
       // Events of an item, in order: the dQ tiles of steps 0 .. n_q-2, dV, the last dQ tile, dK.
 #pragma unroll 1
       for (int e = 0; e < n_q + 2; ++e) {
-        if (e == n_q - 1 || e == n_q + 1) {
-          const bool is_dk = e > n_q;
-          mbar_wait_inline(bar(is_dk ? kBarDkDone : kBarDvDone), ni & 1, &abort_flag);
+        const bool is_out = e == n_q - 1 || e == n_q + 1, is_dk = e > n_q;
+        const bool is_dq = kRuns && !is_out;
+        if (is_out || (is_dq && (run & kRunLast))) {
+          wait(bar(is_dq ? kBarDqFull : is_dk ? kBarDkDone : kBarDvDone), (is_dq ? s : ni) & 1);
           tc_fence_after();
-          const uint32_t tm_acc = (is_dk ? tm_dk : tm_dv) + lane_off;
-          const float out_scale = is_dk ? p.scale : 1.f;
+          const uint32_t tm_acc = (is_dq ? tm_dq : is_dk ? tm_dk : tm_dv) + lane_off;
+          const float out_scale = is_dk || is_dq ? p.scale : 1.f;
+          const bool add = is_dq && read_back;
+          if (add) {
+            wait(bar(kBarOwnFull + quad), own_phase);
+            own_phase ^= 1u;
+          }
           // The whole 64-column row of this lane becomes 32 packed registers (four 16-column loads)
           // and the accumulator is handed back at once. The rows then go out 32 columns at a time
           // through a 2 KB scratch area, four lanes per 64-byte half row (a row per lane straight
@@ -789,16 +993,40 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             uint32_t r[16];
             tmem_ld16(tm_acc + 16 * q4, r);
             tmem_wait_ld();
+            if (kRuns && add) {
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                const float4 a = *reinterpret_cast<const float4*>(stage + (q4 >> 1) * kTileBytes +
+                                                                  swz128(lane, (q4 & 1) * 4 + c));
+                r[4 * c] = __float_as_uint(__uint_as_float(r[4 * c]) + a.x);
+                r[4 * c + 1] = __float_as_uint(__uint_as_float(r[4 * c + 1]) + a.y);
+                r[4 * c + 2] = __float_as_uint(__uint_as_float(r[4 * c + 2]) + a.z);
+                r[4 * c + 3] = __float_as_uint(__uint_as_float(r[4 * c + 3]) + a.w);
+              }
+            }
 #pragma unroll
             for (int i = 0; i < 8; ++i)
               pk[8 * q4 + i] =
                   pack_bf16(__uint_as_float(r[2 * i]) * out_scale, __uint_as_float(r[2 * i + 1]) * out_scale);
           }
           tc_fence_before();
+          if (kRuns && add) fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) mbar_arrive(bar(is_dk ? kBarDkOut : kBarDvOut));  // the accumulator is free
+          if (lane == 0) mbar_arrive(bar(is_dq ? kBarDqFree : is_dk ? kBarDkOut : kBarDvOut));  // the accumulator is free
           __nv_bfloat16* out = is_dk ? dk_rows() : dv_rows();
-          const int64_t out_st = is_dk ? p.dk_st : p.dv_st;
+          int64_t out_st = is_dk ? p.dk_st : p.dv_st;
+          int out_live = rows_live;
+          if (kRuns && is_dq) {
+            out = p.dq + (int64_t(bcoord) * p.dq_sb + int64_t(h) * p.dq_sh + (wk.q_begin + jt * kTile + quad * 32) * p.dq_st);
+            out_st = p.dq_st;
+            out_live = wk.lq - jt * kTile - quad * 32;
+            ++s;
+            jt = jt + 1 == n_q ? 0 : jt + 1;
+            if (add && e < n_q && lane == 0) {  // the next one (the last is event n_q)
+              bulk_wait_group<0>();
+              own_load();
+            }
+          }
 #pragma unroll
           for (int half = 0; half < 2; ++half) {
             // Row `lane` of the scratch holds 32 bf16 = four 16-byte chunks, XOR-ed with the row
@@ -813,15 +1041,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
             for (int it = 0; it < 4; ++it) {
               const int rloc = it * 8 + (lane >> 2), c = lane & 3;
               const uint4 v = *reinterpret_cast<const uint4*>(ostage + rloc * 64 + ((c ^ ((rloc >> 1) & 3)) << 4));
-              if (rloc < rows_live) *reinterpret_cast<uint4*>(out + int64_t(rloc) * out_st + half * 32 + c * 8) = v;
+              if (rloc < out_live) *reinterpret_cast<uint4*>(out + int64_t(rloc) * out_st + half * 32 + c * 8) = v;
             }
             __syncwarp();
           }
           continue;
         }
-        mbar_wait_inline(bar(kBarDqFull), s & 1, &abort_flag);
+        wait(bar(kBarDqFull), s & 1);
         tc_fence_after();
-        if (lane == 0) bulk_wait_group_read0();  // the previous reductions have read the staging rows
+        if (lane == 0) {
+          bulk_wait_group_read0();  // the previous reductions have read the staging rows
+          // Additions to an own tile have to find the ones before them done.
+          if (kRuns && run) own_order();
+        }
         __syncwarp();
 #pragma unroll 1
         for (int half = 0; half < 2; ++half) {
@@ -840,7 +1072,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) {
+        if (kRuns && run) {
+          if (lane == 0) {
+            float* own = own0 + jt * 8192;
+            if (run & kRunFirst) {
+              bulk_store(own, smem_u32(stage), 4096);
+              bulk_store(own + 1024, smem_u32(stage + kTileBytes), 4096);
+            } else {
+              bulk_reduce_add(own, smem_u32(stage), 4096);
+              bulk_reduce_add(own + 1024, smem_u32(stage + kTileBytes), 4096);
+            }
+            bulk_commit_group();
+          }
+          jt = jt + 1 == n_q ? 0 : jt + 1;
+        } else if (lane == 0) {
 #if NB_BWD_L2_HINTS
           tma_reduce_add_3d_hint(&tmap_dq, smem_u32(stage), 0, row, h, keep);
           tma_reduce_add_3d_hint(&tmap_dq, smem_u32(stage + kTileBytes), 32, row, h, keep);
@@ -876,7 +1121,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         auto copy_k = [&](uint32_t c) {
           const uint32_t kb = (c & kCtrlKb) ? 1u : 0u;
           const uint64_t kd = make_sdesc(sK(kb), 16, 1024);
-          mbar_wait_inline(bar(kBarKFull + kb), (ni >> 1) & 1, &abort_flag);
+          wait(bar(kBarKFull + kb), (ni >> 1) & 1);
           ++ni;
 #pragma unroll 1
           for (int k = 0; k < 4; ++k) tmem_copy_128x256b(tm_k + 8 * k, kd + 2 * k);
@@ -887,7 +1132,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           for (int k = 0; k < 4; ++k) mma_ts(tm_s + 64 * h, tm_k + 8 * k, qd + 2 * k, kIdescSH, k > 0);
           tc_commit(bar(kBarSFull + h));
         };
-        mbar_wait_inline(bar(kBarQdoFull), 0, &abort_flag);
+        wait(bar(kBarQdoFull), 0);
         ctrl = ctrl_ring[0];
         if (!(ctrl & kCtrlStop)) {
           copy_k(ctrl);
@@ -902,23 +1147,23 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           BwdStepPos next = pos;
           next.advance();
           // The previous item's dV has to be out of tensor memory before this one's first MMA.
-          if (first && ni > 1) mbar_wait_inline(bar(kBarDvOut), (ni - 2) & 1, &abort_flag);
+          if (first && ni > 1) wait(bar(kBarDvOut), (ni - 2) & 1);
           const uint64_t gd_mn = make_sdesc(sDO(pos.qs), 1024, 1024);
           uint32_t next_ctrl = 0;
 #pragma unroll 1
           for (int h = 0; h < 2; ++h) {
-            if (!mbar_wait_inline(bar(kBarPFull + h), pos.s & 1, &abort_flag)) next_ctrl = kCtrlStop;
+            if (!wait(bar(kBarPFull + h), pos.s & 1)) next_ctrl = kCtrlStop;
             tc_fence_after();
 #pragma unroll
             for (int k = 0; k < 4; ++k)  // A: P^T of query columns [64h + 16k, +16)
               mma_ts(tm_dv, tm_s + 64 * h + 8 * k, gd_mn + 512 * h + 128 * k, kIdescKN, !first || (h + k > 0));
             if (h == 0) {
               if (pos.s == 0) issue_s(0, 1);  // the second half starts later: see above
-              mbar_wait_inline(bar(kBarQdoFull + next.qs), next.qph, &abort_flag);
+              wait(bar(kBarQdoFull + next.qs), next.qph);
               next_ctrl |= ctrl_ring[next.qs];
               if ((next_ctrl & (kCtrlFirst | kCtrlStop)) == kCtrlFirst) {
                 // The MMAs that read the previous item's K must be complete.
-                mbar_wait_inline(bar(kBarSFull + 1), pos.s & 1, &abort_flag);
+                wait(bar(kBarSFull + 1), pos.s & 1);
                 tc_fence_after();
                 copy_k(next_ctrl);
               }
@@ -938,7 +1183,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         // ---------------- dP^T = V dO^T of step s+1 after dK += dS^T Q of step s, half by half ----------------
         const uint64_t vd = make_sdesc(sV, 16, 1024);
         auto copy_v = [&] {
-          mbar_wait_inline(bar(kBarVFull), ni & 1, &abort_flag);
+          wait(bar(kBarVFull), ni & 1);
           ++ni;
 #pragma unroll 1
           for (int k = 0; k < 4; ++k) tmem_copy_128x256b(tm_v + 8 * k, vd + 2 * k);
@@ -950,7 +1195,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           for (int k = 0; k < 4; ++k) mma_ts(tm_dp + 64 * h, tm_v + 8 * k, gd + 2 * k, kIdescSH, k > 0);
           tc_commit(bar(kBarDpFull + h));
         };
-        mbar_wait_inline(bar(kBarQdoFull), 0, &abort_flag);
+        wait(bar(kBarQdoFull), 0);
         ctrl = ctrl_ring[0];
         if (!(ctrl & kCtrlStop)) {
           copy_v();
@@ -962,22 +1207,22 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           const bool first = (ctrl & kCtrlFirst) != 0;
           BwdStepPos next = pos;
           next.advance();
-          if (first && ni > 1) mbar_wait_inline(bar(kBarDkOut), (ni - 2) & 1, &abort_flag);
+          if (first && ni > 1) wait(bar(kBarDkOut), (ni - 2) & 1);
           const uint64_t qd_mn = make_sdesc(sQ(pos.qs), 1024, 1024);
           uint32_t next_ctrl = 0;
 #pragma unroll 1
           for (int h = 0; h < 2; ++h) {
-            if (!mbar_wait_inline(bar(kBarDstFull + h), pos.s & 1, &abort_flag)) next_ctrl = kCtrlStop;
+            if (!wait(bar(kBarDstFull + h), pos.s & 1)) next_ctrl = kCtrlStop;
             tc_fence_after();
 #pragma unroll
             for (int k = 0; k < 4; ++k)  // A: dS^T of query columns [64h + 16k, +16)
               mma_ts(tm_dk, tm_dp + 64 * h + 8 * k, qd_mn + 512 * h + 128 * k, kIdescKN, !first || (h + k > 0));
             if (h == 0) {
-              mbar_wait_inline(bar(kBarQdoFull + next.qs), next.qph, &abort_flag);
+              wait(bar(kBarQdoFull + next.qs), next.qph);
               next_ctrl |= ctrl_ring[next.qs];
               if ((next_ctrl & (kCtrlFirst | kCtrlStop)) == kCtrlFirst) {
                 // The MMAs that read the previous item's V must be complete.
-                mbar_wait_inline(bar(kBarDpFull + 1), pos.s & 1, &abort_flag);
+                wait(bar(kBarDpFull + 1), pos.s & 1);
                 tc_fence_after();
                 copy_v();
               }
@@ -1002,16 +1247,16 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           // again is the tightest in the pipeline), so it reads a copy of the control word from a ring of
           // eight: the word of step s+8 is written after step s+5 has freed its stage, hence after the
           // dQ MMAs of step s+3. The compute warps have seen the word before they arrive here.
-          if (!mbar_wait_inline(bar(kBarDsFull), pos.s & 1, &abort_flag)) break;
+          if (!wait(bar(kBarDsFull), pos.s & 1)) break;
           ctrl = (reinterpret_cast<volatile uint32_t*>(sCtrlQ))[pos.s & 7u];
           if (ctrl & kCtrlStop) break;
           if (ctrl & kCtrlFirst) {
             kb = (ctrl & kCtrlKb) ? 1u : 0u;
             kd_mn = make_sdesc(sK(kb), 1024, 1024);
-            mbar_wait_inline(bar(kBarKFull + kb), (ni >> 1) & 1, &abort_flag);
+            wait(bar(kBarKFull + kb), (ni >> 1) & 1);
           }
-          if (pos.s > 0) mbar_wait_inline(bar(kBarDqFree), (pos.s - 1) & 1, &abort_flag);
-          mbar_wait_inline(bar(kBarDsFull + 1), pos.s & 1, &abort_flag);
+          if (pos.s > 0) wait(bar(kBarDqFree), (pos.s - 1) & 1);
+          wait(bar(kBarDsFull + 1), pos.s & 1);
           tc_fence_after();
 #pragma unroll
           for (int k = 0; k < 8; ++k) mma_ss(tm_dq, ds_mn + 128 * k, kd_mn + 128 * k, kIdescNN, k > 0);

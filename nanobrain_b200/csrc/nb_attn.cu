@@ -85,9 +85,11 @@ int ensure_device_ready() {
     rc = NB_ATTN_ERR_DEVICE;
   } else if (cudaFuncSetAttribute(nb::attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   nb::kFwdSmemBytes) != cudaSuccess ||
-             cudaFuncSetAttribute(nb::attn_bwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+             cudaFuncSetAttribute(nb::attn_bwd_kernel<nb::kBwdWhole>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   nb::kBwdSmemBytes) != cudaSuccess ||
-             cudaFuncSetAttribute(nb::attn_bwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+             cudaFuncSetAttribute(nb::attn_bwd_kernel<nb::kBwdCut>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  nb::kBwdSmemBytes) != cudaSuccess ||
+             cudaFuncSetAttribute(nb::attn_bwd_kernel<nb::kBwdRuns>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   nb::kBwdSmemBytes) != cudaSuccess ||
              cudaFuncSetAttribute(nb::mma_selftest_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   nb::kSelftestSmemBytes) != cudaSuccess) {
@@ -210,6 +212,7 @@ nb::SchedParams make_sched(const nb_attn_shape& s, int side, nb::SchedItem* item
   sp.n_items = int32_t(n_items);
   sp.status = status;
   sp.merged = 0;
+  sp.run_tiles = 0, sp.heads = s.heads, sp.sms = 1, sp.rest = nullptr;
   return sp;
 }
 
@@ -297,6 +300,32 @@ BwdSplit bwd_split(const nb_attn_shape& s) {
   return r;
 }
 
+// May sequences of a packed backward be runs (see BwdRun)? Which of them are the device decides (sched_runs), and every
+// block of the prologue has to look at all sequences for it (1-2 us). It takes four rounds of (sequence, head) pairs
+// over the SMs for runs to fill most of the SMs' time in whole rounds: 64 sequences of 720..920 tokens and 12 heads (5.2 rounds)
+// 534 us without runs, 499 with; 32 of them (2.6 rounds) 268 and 274; 30 of 200 tokens and one of 2000 (2.5) 82 and 91. Where the
+// sequences have more than eight tiles on average few could be runs.
+struct BwdRuns {
+  int tiles = 0;  // SchedParams::run_tiles
+  int own_tiles = 0;
+  size_t rest_offset = 0, own_offset = 0, bytes = 0;  // of the whole workspace; bytes = 0: no
+};
+BwdRuns bwd_runs(const nb_attn_shape& s) {
+  BwdRuns r;
+  const int64_t pairs = int64_t(s.batch) * s.heads, sms = device_sm_count();
+  const int n_qt = ceil_div(s.max_seqlen_q, nb::kTile), n_kt = ceil_div(s.max_seqlen_k, nb::kTile);
+  if (s.cu_seqlens_q == nullptr || s.batch > nb::kSchedRunSeqs || pairs < 4 * sms ||
+      s.total_q > int64_t(s.batch) * nb::kBwdRunTiles * nb::kTile)
+    return r;
+  r.tiles = n_kt == 1 ? -1 : n_qt < nb::kBwdRunTiles ? n_qt : nb::kBwdRunTiles;
+  r.own_tiles = n_kt == 1 ? 0 : r.tiles;
+  r.rest_offset =
+      align_up(bwd_items_offset(s) + size_t(nb::sched_capacity(s.total_k, s.batch)) * sizeof(nb::SchedItem), 256);
+  r.own_offset = align_up(r.rest_offset + nb::sched_rest_bytes(s.batch), 256);
+  r.bytes = r.own_offset + size_t(sms) * r.own_tiles * nb::kTile * nb::kHeadDim * sizeof(float);
+  return r;
+}
+
 // Everything about a backward call that can be checked without touching CUDA.
 int validate_bwd(const nb_attn_bwd_args* a) {
   if (a == nullptr) return NB_ATTN_ERR_NULL;
@@ -365,6 +394,11 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
   p.n_qt = ceil_div(s.max_seqlen_q, nb::kTile);
   p.parts = nullptr;
   unsigned ctas = unsigned(device_sm_count());
+  const BwdRuns runs = bwd_runs(s);
+  const bool use_runs = runs.bytes > 0 && workspace_bytes >= runs.bytes;
+  p.own = use_runs ? reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + runs.own_offset) : nullptr;
+  p.own_tiles = runs.own_tiles;
+  p.rest = nullptr;
   if (dense) {
     p.items = nullptr;
     p.sched = nb::SchedParams{};
@@ -384,9 +418,15 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
     p.items = items;
     p.sched = make_sched(s, 1, items, n_items, a->status);
     p.sched.merged = 1;
+    if (use_runs) {
+      p.rest = reinterpret_cast<int32_t*>(static_cast<unsigned char*>(workspace) + runs.rest_offset);
+      p.sched.run_tiles = runs.tiles, p.sched.sms = int32_t(ctas), p.sched.rest = p.rest;
+    }
     n_work = n_items * s.heads;
   }
   p.n_work = int32_t(n_work);
+  p.rows32 = s.total_q * s.heads <= INT32_MAX;
+  p.div_lq = nb::make_fast_div(uint32_t(s.max_seqlen_q));
   p.div_heads = nb::make_fast_div(uint32_t(s.heads));
   p.div_n_kt = nb::make_fast_div(uint32_t(p.n_kt));
   p.div_n_qt = nb::make_fast_div(uint32_t(p.n_qt));
@@ -395,16 +435,20 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t rows = s.total_q * s.heads;
   const int64_t want_blocks = (rows * 8 + 255) / 256;
-  const int64_t most_blocks = 16 * int64_t(device_sm_count());
+  // (With runs a block first looks at all sequences and takes consecutive rows: no more blocks than are resident.)
+  const int64_t most_blocks = (p.rest != nullptr ? 8 : 16) * int64_t(device_sm_count());
   const int aux_blocks = int(want_blocks < most_blocks ? want_blocks : most_blocks);
   p.row_blocks = aux_blocks;
   const int combine_blocks = p.parts != nullptr ? 4 * (int(ctas) - 1) : 0;
-  bool ok = launch(nb::attn_bwd_prologue_kernel, dim3(aux_blocks), dim3(256), 0, st, p) == cudaSuccess;
+  const auto main = p.parts != nullptr ? nb::attn_bwd_kernel<nb::kBwdCut>
+                    : use_runs           ? nb::attn_bwd_kernel<nb::kBwdRuns>
+                                         : nb::attn_bwd_kernel<nb::kBwdWhole>;
+  bool ok = launch(use_runs ? nb::attn_bwd_prologue_kernel<true> : nb::attn_bwd_prologue_kernel<false>, dim3(aux_blocks), dim3(256), 0, st, p) == cudaSuccess;
   if (a->event_main_begin) cudaEventRecord(static_cast<cudaEvent_t>(a->event_main_begin), st);
-  ok = ok && launch(p.parts != nullptr ? nb::attn_bwd_kernel<true> : nb::attn_bwd_kernel<false>, grid, dim3(nb::kBwdThreads), nb::kBwdSmemBytes, st, tq, tk, tv, tg, tdq, p) ==
+  ok = ok && launch(main, grid, dim3(nb::kBwdThreads), nb::kBwdSmemBytes, st, tq, tk, tv, tg, tdq, p) ==
                  cudaSuccess;
   if (a->event_main_end) cudaEventRecord(static_cast<cudaEvent_t>(a->event_main_end), st);
-  ok = ok && launch(nb::attn_bwd_epilogue_kernel, dim3(aux_blocks + combine_blocks), dim3(256), 0, st, p) == cudaSuccess;
+  ok = ok && launch(use_runs ? nb::attn_bwd_epilogue_kernel<true> : nb::attn_bwd_epilogue_kernel<false>, dim3(aux_blocks + combine_blocks), dim3(256), 0, st, p) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();  // leave no sticky "last error" behind for the caller's own checks
     return NB_ATTN_ERR_LAUNCH;
@@ -527,7 +571,8 @@ size_t nb_attn_bwd_workspace_bytes(const nb_attn_shape* shape) {
 
 size_t nb_attn_bwd_split_workspace_bytes(const nb_attn_shape* shape) {
   if (shape == nullptr || check_shape(*shape) != NB_ATTN_OK || ensure_device_ready() != NB_ATTN_OK) return 0;
-  return bwd_split(*shape).bytes;
+  const size_t split = bwd_split(*shape).bytes, runs = bwd_runs(*shape).bytes;
+  return split > runs ? split : runs;
 }
 
 size_t nb_attn_fwd_workspace_bytes(const nb_attn_shape* shape) {

@@ -42,7 +42,7 @@ namespace nb {
 // One work item; mirrors nb_attn_sched_item in include/nb_attn.h.
 struct __align__(16) SchedItem {
   int32_t seq;          // sequence index; `batch` = the rows past the last sequence; -1 = unused entry
-  int32_t tile;         // 128-row tile on the own side
+  int32_t tile;         // 128-row tile on the own side; -1: all of them (see SchedRuns)
   int32_t own_begin;    // first packed row of the sequence on the own side
   int32_t own_len;      // its length there
   int32_t other_begin;  // the same on the side the item's inner loop walks
@@ -92,6 +92,11 @@ struct SchedParams {
   int32_t n_items;  // capacity, >= sched_capacity(total_own, batch)
   int32_t* status;
   int32_t merged;  // ragged tiles at the end of their cost class instead of after all full tiles
+  // Runs (see SchedRuns) have at most this many tiles on the other side. -1: no sequence has more than one tile on the
+  // own side.
+  int32_t run_tiles;
+  int32_t heads, sms;
+  int32_t* rest;  // where the list of the sequences that are no runs goes
 };
 
 // Exclusive prefix sum over one value per thread of a block of kThreads threads (returns the
@@ -131,12 +136,31 @@ struct SchedSeq {
   int ragged;  // 1 if a partial last tile exists
   int bucket;  // 0 = most expensive
   bool ok;
+  bool run;  // one item stands for all tiles
   int own_begin, own_len, other_begin, other_len;
 };
 
+// Which sequences are runs: one item, all of whose tiles the CTA that takes it works off one after the other.
+// A sequence with something on both sides is one if it has a single tile on the own side, or if its
+// index is below `below`, it has at most run_tiles tiles on the other side and a cost (steps of all its tiles) of at
+// most max_cost. below = -1: there are none.
+struct SchedRuns {
+  int below, max_cost;
+};
+__host__ __device__ inline int sched_tiles(int len) { return len / kSchedTile + (len % kSchedTile != 0); }
+// Steps of the sequence as a run; 0 if it is none.
+__host__ __device__ inline int sched_run_cost(const SchedParams& p, const SchedSeq& s, int i, const SchedRuns& r) {
+  if (r.below < 0 || !s.ok || s.own_len <= 0 || s.other_len <= 0) return 0;
+  const int own = sched_tiles(s.own_len), other = sched_tiles(s.other_len);
+  if (own == 1) return other;
+  // (One tile on the other side that several own tiles add to: no step in between for an addition to complete.)
+  if (i >= r.below || other > p.run_tiles || other == 1 || own > r.max_cost / other) return 0;
+  return own * other;
+}
+
 __host__ __device__ inline SchedItem sched_item(const SchedSeq& s, int seq, int tile) {
   SchedItem it;
-  it.seq = seq, it.tile = tile;
+  it.seq = seq, it.tile = s.run ? -1 : tile;
   it.own_begin = s.own_begin, it.own_len = s.own_len, it.other_begin = s.other_begin, it.other_len = s.other_len;
   it.reserved[0] = it.reserved[1] = 0;
   return it;
@@ -150,8 +174,12 @@ __host__ __device__ inline SchedItem sched_no_item() {
 }
 
 // i in [0, batch]: i == batch is the pseudo-sequence of the rows past the last sequence.
+__host__ __device__ inline int sched_bucket(int steps) {
+  return kSchedBuckets - 1 - (steps < kSchedBuckets - 1 ? steps : kSchedBuckets - 1);
+}
 __host__ __device__ inline SchedSeq sched_classify(const SchedParams& p, int i) {
   SchedSeq s;
+  s.run = false;
   int64_t len, steps_len;
   if (i == p.batch) {
     len = p.total_own - int64_t(p.cu_own[i]);
@@ -174,9 +202,117 @@ __host__ __device__ inline SchedSeq sched_classify(const SchedParams& p, int i) 
   s.full = len > 0 ? int(len / kSchedTile) : 0;
   s.ragged = len > 0 && (len % kSchedTile) != 0;
   const int steps = steps_len > 0 ? int((steps_len + kSchedTile - 1) / kSchedTile) : 0;
-  const int clipped = steps < kSchedBuckets - 1 ? steps : kSchedBuckets - 1;
-  s.bucket = kSchedBuckets - 1 - clipped;
+  s.bucket = sched_bucket(steps);
   return s;
+}
+// The same with runs: a run is one full tile of the run's cost.
+__host__ __device__ inline SchedSeq sched_classify(const SchedParams& p, int i, const SchedRuns& r) {
+  SchedSeq s = sched_classify(p, i);
+  if (const int cost = sched_run_cost(p, s, i, r)) s.run = true, s.full = 1, s.ragged = 0, s.bucket = sched_bucket(cost);
+  return s;
+}
+
+// ---- runs ---------------------------------------------------------------------------------
+constexpr int kSchedRunSeqs = 2048;  // packings of more sequences have no runs (their ends are kept in shared memory)
+
+template <int kThreads>
+__device__ __forceinline__ unsigned long long block_sum(unsigned long long v, unsigned long long* scratch) {
+#pragma unroll
+  for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = 0;
+#pragma unroll
+  for (int w = 0; w < kThreads / 32; ++w) v += scratch[w];
+  __syncthreads();  // scratch may be reused
+  return v;
+}
+
+struct SchedRunShared {
+  unsigned long long sum[32];
+  int scratch[32];
+  int most, below, bad;
+  int cost[kSchedRunSeqs];  // steps of the sequence as a run of several tiles, 0: it can be none
+};
+
+// The rule for this packing; every block that calls it comes to the same one. A run must not outlast a CTA's share of
+// all steps; and runs of the most expensive one's cost shall fill whole rounds over the SMs: what is left over
+// for a round that would not be full stays single tiles, which fill the gaps. (32 sequences of seven
+// tiles and 12 heads are 2.6 rounds of runs: 24 of the 32 become runs.)
+template <int kThreads>
+__device__ __forceinline__ SchedRuns sched_runs(const SchedParams& p, SchedRunShared& sm) {
+  if (threadIdx.x == 0) sm.most = 0, sm.below = p.batch, sm.bad = 0;
+  __syncthreads();
+  unsigned long long steps = 0;
+#pragma unroll 1
+  for (int i = threadIdx.x; i <= p.batch; i += kThreads) {
+    const SchedSeq s = sched_classify(p, i);
+    if (!s.ok) sm.bad = 1;
+    if (!s.ok || i == p.batch) continue;
+    steps += (unsigned long long)sched_tiles(s.own_len) * unsigned(sched_tiles(s.other_len));
+    sm.cost[i] = s.own_len > kSchedTile ? sched_run_cost(p, s, i, {p.batch, 0x7fffffff}) : 0;
+  }
+  steps = block_sum<kThreads>(steps, sm.sum);
+  if (sm.bad) return {-1, 0};
+  if (p.run_tiles < 0) return {0, 0};
+  const unsigned long long share = steps * unsigned(p.heads) / unsigned(p.sms);
+  const SchedRuns all = {p.batch, share < 0x7fffffffull ? int(share) : 0x7fffffff};
+  unsigned long long total = 0;
+  int most = 0;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < p.batch; i += kThreads) {
+    const int cost = sm.cost[i];
+    if (cost <= all.max_cost) total += unsigned(cost), most = max(most, cost);
+  }
+  if (most > 0) atomicMax(&sm.most, most);
+  total = block_sum<kThreads>(total, sm.sum);
+  most = sm.most;
+  if (most == 0) return {0, 0};
+  const unsigned long long budget = share / unsigned(most) * unsigned(most) * unsigned(p.sms) / unsigned(p.heads);
+  if (total <= budget) return all;
+  unsigned long long before = 0;
+#pragma unroll 1
+  for (int base = 0; base < p.batch && before <= budget; base += kThreads) {
+    const int i = base + threadIdx.x;
+    int cost = i < p.batch ? sm.cost[i] : 0;
+    if (cost > all.max_cost) cost = 0;
+    int sum = 0;
+    const int excl = block_exclusive_scan<kThreads>(cost, sm.scratch, &sum);
+    if (cost > 0 && before + unsigned(excl) + unsigned(cost) > budget) atomicMin(&sm.below, i);
+    before += unsigned(sum);
+  }
+  __syncthreads();
+  return {sm.below, all.max_cost};
+}
+
+// The sequences that are no runs, as the epilogue reads them: word 0 counts the rows on the other side that
+// belong to them; row x of these (in the order of the sequences) is row x + shift of the whole, shift from the first
+// entry whose `end` exceeds x. One entry per sequence and one for the rows past the last one.
+struct SchedRest {
+  int end, shift;
+};
+__host__ __device__ inline size_t sched_rest_bytes(int32_t batch) { return 16 + (size_t(batch) + 1) * sizeof(SchedRest); }
+template <int kThreads>
+__device__ __forceinline__ void sched_write_rest(const SchedParams& p, const SchedRuns& r, SchedRunShared& sm) {
+  SchedRest* rest = reinterpret_cast<SchedRest*>(p.rest + 4);
+  int before = 0;
+#pragma unroll 1
+  for (int base = 0; base <= p.batch; base += kThreads) {
+    const int i = base + threadIdx.x;
+    int begin = 0, rows = 0;
+    if (sm.bad) {  // not a packing: all rows
+      rows = i == 0 ? int(p.total_other) : 0;
+    } else if (i <= p.batch) {
+      begin = p.cu_other[i];
+      rows = (i < p.batch ? p.cu_other[i + 1] : int(p.total_other)) - begin;
+      if (sched_run_cost(p, sched_classify(p, i), i, r) > 0) rows = 0;
+    }
+    int sum = 0;
+    const int at = before + block_exclusive_scan<kThreads>(rows, sm.scratch, &sum);
+    if (i <= p.batch) rest[i] = {at + rows, begin - at};
+    before += sum;
+  }
+  if (threadIdx.x == 0) p.rest[0] = before;
 }
 
 // Shared-memory state of one list build.
@@ -189,7 +325,7 @@ struct SchedShared {
 
 // Builds the list with one block of kThreads threads (every thread of the block must call it).
 template <int kThreads>
-__device__ __forceinline__ void sched_build(const SchedParams& p, SchedShared& sm) {
+__device__ __forceinline__ void sched_build(const SchedParams& p, SchedShared& sm, const SchedRuns runs = {-1, 0}) {
   static_assert(kSchedBuckets % kThreads == 0, "each thread owns a run of consecutive buckets");
   constexpr int kPer = kSchedBuckets / kThreads;
   const int tid = threadIdx.x;
@@ -201,7 +337,7 @@ __device__ __forceinline__ void sched_build(const SchedParams& p, SchedShared& s
   __syncthreads();
 
   for (int i = tid; i <= p.batch; i += kThreads) {
-    const SchedSeq s = sched_classify(p, i);
+    const SchedSeq s = sched_classify(p, i, runs);
     if (!s.ok) {
       sm.bad = 1;
     } else {
@@ -237,7 +373,7 @@ __device__ __forceinline__ void sched_build(const SchedParams& p, SchedShared& s
   __syncthreads();
 
   for (int i = tid; i <= p.batch; i += kThreads) {
-    const SchedSeq s = sched_classify(p, i);
+    const SchedSeq s = sched_classify(p, i, runs);
     if (s.full) {
       const int at = atomicAdd(&sm.full_pos[s.bucket], s.full);
       for (int t = 0; t < s.full; ++t) p.items[at + t] = sched_item(s, i, t);

@@ -214,9 +214,8 @@ void launch_bwd(nb_attn_bwd_args& a, const Tensor& q, const Tensor& lse) {
   raise_for_status(word);
   a.lse = lse.data_ptr<float>();
   a.status = const_cast<int32_t*>(word);
-  a.workspace_bytes = nb_attn_bwd_workspace_bytes(&a.shape);
-  if (a.shape.cu_seqlens_q == nullptr)  // room to cut units between CTAs
-    a.workspace_bytes = std::max(a.workspace_bytes, nb_attn_bwd_split_workspace_bytes(&a.shape));
+  // With room to cut units between CTAs or for their own dQ tiles.
+  a.workspace_bytes = std::max(nb_attn_bwd_workspace_bytes(&a.shape), nb_attn_bwd_split_workspace_bytes(&a.shape));
   Tensor workspace = new_tensor({int64_t(a.workspace_bytes)}, at::kByte, q);
   a.workspace = workspace.data_ptr();
   check_rc(nb_attn_bwd(&a, at::cuda::getCurrentCUDAStream().stream()), "nb_attn_bwd");

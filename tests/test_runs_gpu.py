@@ -1,0 +1,57 @@
+"""The backward where one CTA takes all key tiles of a (sequence, head) and sums dQ up in tiles of its
+own, next to sequences whose key tiles are spread over the CTAs, against the CPU oracle."""
+
+import numpy as np
+import pytest
+import torch
+
+import nanobrain_b200
+from nanobrain_b200 import ops
+from oracle import attn_oracle as O
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def check(names, got, want):
+    # bf16 results of bf16 products with fp32 accumulation, as for every other configuration
+    for name, a, b in zip(names, got, want):
+        b = np.asarray(b, dtype=np.float32)
+        err = np.abs(a.detach().float().cpu().numpy() - b)
+        assert np.isfinite(err).all(), name
+        assert err.max() <= 2e-2 * max(1.0, np.abs(b).max()) and err.mean() <= 2e-3 * max(1.0, np.abs(b).max()), name
+
+
+@pytest.mark.parametrize("lengths_q,lengths_k,heads,spare", [
+    ([200] * 14 + [700], None, 45, 0),                       # two query tiles: neighbouring additions to a tile
+    ([130, 0, 256, 257, 1, 128, 140, 500] * 3, None, 25, 70),  # all kinds, and rows past the last sequence
+    ([300] * 5, None, 120, 1),                               # 4.05 rounds over the SMs: the last sequence is single tiles
+    ([64, 1, 128, 0, 100], None, 120, 30),                   # one tile at most
+    ([300, 100, 0, 260, 128] * 4, [50, 400, 200, 0, 129] * 4, 30, 5),
+    ([140] * 3, [1000, 1024, 513], 200, 0),                  # more key than query tiles
+    ([1100, 900, 1024], [140, 130, 129], 200, 0),            # more query tiles than a CTA keeps
+])
+def test_packed_runs(lengths_q, lengths_k, heads, spare):
+    lengths_k = lengths_q if lengths_k is None else lengths_k
+    assert len(lengths_q) * heads >= 4 * 148  # fewer pairs of sequence and head are always spread over the CTAs
+    g = torch.Generator().manual_seed(sum(lengths_q))
+    tq, tk = sum(lengths_q) + spare, sum(lengths_k) + spare
+    q, d_out = (torch.randn(tq, heads, 64, generator=g).to(torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(tk, heads, 64, generator=g).to(torch.bfloat16) for _ in range(2))
+    cu_q, cu_k = (torch.tensor([0] + list(x)).cumsum(0).to(DEV, torch.int32) for x in (lengths_q, lengths_k))
+    want = [np.zeros((n, heads, 64), np.float32) for n in (tq, tk, tk)]
+    at_q = at_k = 0
+    for nq, nk in zip(lengths_q, lengths_k):
+        if nq and nk:
+            sq, sk = slice(at_q, at_q + nq), slice(at_k, at_k + nk)
+            one = lambda t, s: t[s].float().numpy().transpose(1, 0, 2)[None]
+            grads = O.sdpa_fwd_bwd(one(q, sq), one(k, sk), one(v, sk), one(d_out, sq))[2:5]
+            for w, s, x in zip(want, (sq, sk, sk), grads):
+                w[s] = x[0].transpose(1, 0, 2)
+        at_q, at_k = at_q + nq, at_k + nk
+    for _ in range(2):
+        qd, kd, vd = (t.to(DEV).requires_grad_(True) for t in (q, k, v))
+        out = nanobrain_b200.sdpa_varlen(qd, kd, vd, cu_q, cu_k, max(lengths_q), max(lengths_k))
+        out.backward(d_out.to(DEV))
+        ops.check_status()
+        check(("dq", "dk", "dv"), (qd.grad, kd.grad, vd.grad), want)
