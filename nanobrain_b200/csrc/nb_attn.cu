@@ -301,10 +301,12 @@ BwdSplit bwd_split(const nb_attn_shape& s) {
 }
 
 // May sequences of a packed backward be runs (see BwdRun)? Which of them are the device decides (sched_runs), and every
-// block of the prologue has to look at all sequences for it (1-2 us). It takes four rounds of (sequence, head) pairs
-// over the SMs for runs to fill most of the SMs' time in whole rounds: 64 sequences of 720..920 tokens and 12 heads (5.2 rounds)
-// 534 us without runs, 499 with; 32 of them (2.6 rounds) 268 and 274; 30 of 200 tokens and one of 2000 (2.5) 82 and 91. Where the
-// sequences have more than eight tiles on average few could be runs.
+// block of the prologue has to look at all sequences for it, 3 us or so. So there have to be two rounds of (sequence, head)
+// pairs over the SMs, or most of the work stays single tiles anyway, and thirty steps per SM, about 40 us, to save from:
+// 32 sequences of 720..920 tokens and 12 heads (2.6 rounds, 106 steps) 259.9 us without runs, 255.8 with; 40 of them 326.7 and
+// 306.7; 45 of 400 (3.6, 36) 155.4 and 142.5; 300 of 200 (24, 59) 398 and 282; but 45 of 200 (3.6, 9) 55.9 and 60.0. Where the
+// sequences have more than eight tiles on average few could be runs. Sequences of one key tile are runs without
+// more ado (100 of 128 tokens x 8 heads 42.9 and 41.6), from four rounds on.
 struct BwdRuns {
   int tiles = 0;  // SchedParams::run_tiles
   int own_tiles = 0;
@@ -314,9 +316,11 @@ BwdRuns bwd_runs(const nb_attn_shape& s) {
   BwdRuns r;
   const int64_t pairs = int64_t(s.batch) * s.heads, sms = device_sm_count();
   const int n_qt = ceil_div(s.max_seqlen_q, nb::kTile), n_kt = ceil_div(s.max_seqlen_k, nb::kTile);
-  if (s.cu_seqlens_q == nullptr || s.batch > nb::kSchedRunSeqs || pairs < 4 * sms ||
+  if (s.cu_seqlens_q == nullptr || s.batch > nb::kSchedRunSeqs || pairs < (n_kt == 1 ? 4 : 2) * sms ||
       s.total_q > int64_t(s.batch) * nb::kBwdRunTiles * nb::kTile)
     return r;
+  const double steps = double(s.total_q) / nb::kTile * (double(s.total_k) / nb::kTile) * s.heads / s.batch;  // or more
+  if (n_kt > 1 && steps < 30. * double(sms)) return r;
   r.tiles = n_kt == 1 ? -1 : n_qt < nb::kBwdRunTiles ? n_qt : nb::kBwdRunTiles;
   r.own_tiles = n_kt == 1 ? 0 : r.tiles;
   r.rest_offset =
@@ -435,8 +439,9 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t rows = s.total_q * s.heads;
   const int64_t want_blocks = (rows * 8 + 255) / 256;
-  // (With runs a block first looks at all sequences and takes consecutive rows: no more blocks than are resident.)
-  const int64_t most_blocks = (p.rest != nullptr ? 8 : 16) * int64_t(device_sm_count());
+  // (With runs a block first looks at all sequences and takes consecutive rows: no more blocks than are resident. 300 sequences of
+  // 200 tokens: 282 us with four per SM, 286 with eight.)
+  const int64_t most_blocks = (p.rest != nullptr ? 4 : 16) * int64_t(device_sm_count());
   const int aux_blocks = int(want_blocks < most_blocks ? want_blocks : most_blocks);
   p.row_blocks = aux_blocks;
   const int combine_blocks = p.parts != nullptr ? 4 * (int(ctas) - 1) : 0;

@@ -23,19 +23,20 @@ def check(names, got, want):
 
 
 @pytest.mark.parametrize("lengths_q,lengths_k,heads,spare", [
-    ([200] * 14 + [700], None, 45, 0),                       # two query tiles: neighbouring additions to a tile
-    ([130, 0, 256, 257, 1, 128, 140, 500] * 3, None, 25, 70),  # all kinds, and rows past the last sequence
-    ([300] * 5, None, 120, 1),                               # 4.05 rounds over the SMs: the last sequence is single tiles
-    ([64, 1, 128, 0, 100], None, 120, 30),                   # one tile at most
-    ([300, 100, 0, 260, 128] * 4, [50, 400, 200, 0, 129] * 4, 30, 5),
-    ([140] * 3, [1000, 1024, 513], 200, 0),                  # more key than query tiles
-    ([1100, 900, 1024], [140, 130, 129], 200, 0),            # more query tiles than a CTA keeps
+    ([200] * 14 + [700], None, 100, 0),                       # two query tiles: neighbouring additions to a tile
+    ([130, 0, 256, 257, 1, 128, 140, 500] * 3, None, 100, 70),  # all kinds, and rows past the last sequence
+    ([300] * 5, None, 170, 1),                                # 5.7 rounds over the SMs: the last sequence is single tiles
+    ([64, 1, 128, 0, 100], None, 120, 30),                    # one tile at most
+    ([300, 100, 0, 260, 128] * 4, [50, 400, 200, 0, 129] * 4, 150, 5),
+    ([140] * 3, [1000, 1024, 513], 210, 0),                   # more key than query tiles
+    ([1100, 900, 1024], [140, 130, 129], 200, 0),             # more query tiles than a CTA keeps
 ])
 def test_packed_runs(lengths_q, lengths_k, heads, spare):
     lengths_k = lengths_q if lengths_k is None else lengths_k
-    assert len(lengths_q) * heads >= 4 * 148  # fewer pairs of sequence and head are always spread over the CTAs
     g = torch.Generator().manual_seed(sum(lengths_q))
     tq, tk = sum(lengths_q) + spare, sum(lengths_k) + spare
+    # Calls of fewer steps are spread over the CTAs altogether.
+    assert max(lengths_k) <= 128 or tq * tk * heads >= 30 * 148 * 128 ** 2 * len(lengths_q)
     q, d_out = (torch.randn(tq, heads, 64, generator=g).to(torch.bfloat16) for _ in range(2))
     k, v = (torch.randn(tk, heads, 64, generator=g).to(torch.bfloat16) for _ in range(2))
     cu_q, cu_k = (torch.tensor([0] + list(x)).cumsum(0).to(DEV, torch.int32) for x in (lengths_q, lengths_k))
