@@ -162,6 +162,11 @@ def bwd_workspace_bytes(shape: Shape) -> int:
     return int(load().nb_attn_bwd_workspace_bytes(C.byref(shape)))
 
 
+def bwd_full_workspace_bytes(shape: Shape) -> int:
+    """Scratch bytes with which ``nb_attn_bwd`` runs at its best on the current GPU: at least what it needs."""
+    return max(bwd_workspace_bytes(shape), int(load().nb_attn_bwd_split_workspace_bytes(C.byref(shape))))
+
+
 def check(code: int, what: str) -> None:
     """Raise RuntimeError for a non-zero return code of the library."""
     if code != 0:
