@@ -308,12 +308,22 @@ __global__ void __launch_bounds__(512) gelu_kernel(__nv_bfloat16* v, int64_t n) 
     if (kTable && at < kGeluCodes) return table[at + (code >> 15) * kGeluCodes];
     return gelu_bits(code);
   };
-  for (int64_t i = (int64_t(blockIdx.x) * 512 + threadIdx.x) * 8; i < n; i += int64_t(gridDim.x) * 512 * 8) {
-    uint4 u = *reinterpret_cast<const uint4*>(v + i);
+  auto eight = [&](uint4 u) {
     uint32_t* w = reinterpret_cast<uint32_t*>(&u);
 #pragma unroll
     for (int k = 0; k < 4; ++k) w[k] = one(w[k] & 0xffffu) | one(w[k] >> 16) << 16;
-    *reinterpret_cast<uint4*>(v + i) = u;
+    return u;
+  };
+  // Two pieces at a time: the second one's load is under way while the first is looked up.
+  const int64_t step = int64_t(gridDim.x) * 512 * 8;
+#pragma unroll 1
+  for (int64_t i = (int64_t(blockIdx.x) * 512 + threadIdx.x) * 8; i < n; i += 2 * step) {
+    const bool two = i + step < n;
+    const uint4 a = *reinterpret_cast<const uint4*>(v + i);
+    uint4 b = make_uint4(0, 0, 0, 0);
+    if (two) b = *reinterpret_cast<const uint4*>(v + i + step);
+    *reinterpret_cast<uint4*>(v + i) = eight(a);
+    if (two) *reinterpret_cast<uint4*>(v + i + step) = eight(b);
   }
 }
 
