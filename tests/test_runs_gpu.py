@@ -56,3 +56,19 @@ def test_packed_runs(lengths_q, lengths_k, heads, spare):
         out.backward(d_out.to(DEV))
         ops.check_status()
         check(("dq", "dk", "dv"), (qd.grad, kd.grad, vd.grad), want)
+
+
+def test_an_invalid_packing_is_reported_and_nothing_runs():
+    # The rule for runs is looked for before the packing is known to be one.
+    heads, n = 200, 8
+    t = torch.randn(n * 300, heads, 64, device=DEV).to(torch.bfloat16)
+    good = torch.arange(0, n * 300 + 1, 300, dtype=torch.int32, device=DEV)
+    bad = good.clone()
+    bad[3], bad[4] = 1300, 900
+    out, lse = ops.sdpa_varlen_fwd(t, t, t, good, good, 300, 300, 0.125)
+    dq, _, _ = ops.sdpa_varlen_bwd(t, t, t, t, out, lse, bad, bad, 400, 400, 0.125)
+    with pytest.raises(RuntimeError, match="cu_seqlens"):
+        ops.check_status()
+    assert int(dq.count_nonzero()) == 0
+    ops.sdpa_varlen_bwd(t, t, t, t, out, lse, good, good, 300, 300, 0.125)
+    ops.check_status()
