@@ -21,6 +21,7 @@
 //     capacity to avoid a device-to-host sync) form one more pseudo-sequence, index `batch`, that
 //     owns rows [cu_seqlens[batch], total) and has nothing on the other side: its items make the
 //     kernels write zeros there, so every row of every output is defined;
+//   * the backward's list may have runs (SchedRuns): one item for all key tiles of a sequence, for one CTA per head;
 //   * the list has a host-known capacity of floor(total / 128) + batch + 1 entries; unused entries
 //     have seq = -1 and end a CTA's work;
 //   * an entry carries the sequence's offsets and lengths on both sides, so a CTA learns all it
