@@ -433,9 +433,10 @@ struct BwdWork {
 // tiles, that of the others added to them, and the last one's leaves as bf16 together with what is there. So the accumulator of a run is neither
 // cleared nor read by a pass of its own, and 148 x own_tiles x 32 KB stay in the L2 from run to run.
 enum BwdRun : int { kRunTile = 1, kRunFirst = 2, kRunLast = 4 };
-// Most query tiles of a run: 148 CTAs' own tiles, Q and dO then take 148 x 8 x 64 KB = 78 of the L2's 126 MB. (With 18, 16
-// sequences of 1700..2140 tokens took 1118 us where single tiles took 953.)
-constexpr int kBwdRunTiles = 8;
+// Most query tiles of a run: 148 CTAs' own tiles, Q and dO then take 148 x 10 x 64 KB = 97 of the L2's 126 MB. 64 sequences of
+// 1030..1150 tokens (nine tiles) x 12 heads take 781 us instead of 854, of 1160..1280 972 instead of 1020; but with twelve tiles 64 of
+// 1400..1536 take 1646 instead of 1409. (The tenth tile pays from five rounds of pairs on, see bwd_runs in nb_attn.cu.)
+constexpr int kBwdRunTiles = 10;
 
 // Query tile an item starts at. Concurrent CTAs work on the key tiles of one (sequence, head) and
 // all add into the same dQ tiles, so they start at different ones: key tile kt at query tile kt,

@@ -305,7 +305,8 @@ BwdSplit bwd_split(const nb_attn_shape& s) {
 // pairs over the SMs, or most of the work stays single tiles anyway, and thirty steps per SM, about 40 us, to save from:
 // 32 sequences of 720..920 tokens and 12 heads (2.6 rounds, 106 steps) 259.9 us without runs, 255.8 with; 40 of them 326.7 and
 // 306.7; 45 of 400 (3.6, 36) 155.4 and 142.5; 300 of 200 (24, 59) 398 and 282; but 45 of 200 (3.6, 9) 55.9 and 60.0. Where the
-// sequences have more than eight tiles on average few could be runs. Sequences of one key tile are runs without
+// sequences have more tiles on average than a run few could be. Ten tiles are allowed from five rounds on: 32 sequences of
+// 1160..1280 tokens and 16 heads (3.5) take 679 us without runs, 687 with; 64 of them and 12 heads (5.2) 1020 and 972. Sequences of one key tile are runs without
 // more ado (100 of 128 tokens x 8 heads 42.9 and 41.6), from four rounds on.
 struct BwdRuns {
   int tiles = 0;  // SchedParams::run_tiles
@@ -316,12 +317,13 @@ BwdRuns bwd_runs(const nb_attn_shape& s) {
   BwdRuns r;
   const int64_t pairs = int64_t(s.batch) * s.heads, sms = device_sm_count();
   const int n_qt = ceil_div(s.max_seqlen_q, nb::kTile), n_kt = ceil_div(s.max_seqlen_k, nb::kTile);
+  const int most = pairs < 5 * sms ? nb::kBwdRunTiles - 1 : nb::kBwdRunTiles;
   if (s.cu_seqlens_q == nullptr || s.batch > nb::kSchedRunSeqs || pairs < (n_kt == 1 ? 4 : 2) * sms ||
-      s.total_q > int64_t(s.batch) * nb::kBwdRunTiles * nb::kTile)
+      s.total_q > int64_t(s.batch) * most * nb::kTile)
     return r;
   const double steps = double(s.total_q) / nb::kTile * (double(s.total_k) / nb::kTile) * s.heads / s.batch;  // or more
   if (n_kt > 1 && steps < 30. * double(sms)) return r;
-  r.tiles = n_kt == 1 ? -1 : n_qt < nb::kBwdRunTiles ? n_qt : nb::kBwdRunTiles;
+  r.tiles = n_kt == 1 ? -1 : n_qt < most ? n_qt : most;
   r.own_tiles = n_kt == 1 ? 0 : r.tiles;
   r.rest_offset =
       align_up(bwd_items_offset(s) + size_t(nb::sched_capacity(s.total_k, s.batch)) * sizeof(nb::SchedItem), 256);

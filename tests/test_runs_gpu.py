@@ -25,11 +25,12 @@ def check(names, got, want):
 @pytest.mark.parametrize("lengths_q,lengths_k,heads,spare", [
     ([200] * 14 + [700], None, 100, 0),                       # two query tiles: neighbouring additions to a tile
     ([130, 0, 256, 257, 1, 128, 140, 500] * 3, None, 100, 70),  # all kinds, and rows past the last sequence
+    ([1153, 1100], [150, 129], 400, 0),                       # nine and ten
     ([300] * 5, None, 170, 1),                                # 5.7 rounds over the SMs: the last sequence is single tiles
     ([64, 1, 128, 0, 100], None, 120, 30),                    # one tile at most
     ([300, 100, 0, 260, 128] * 4, [50, 400, 200, 0, 129] * 4, 150, 5),
     ([140] * 3, [1000, 1024, 513], 210, 0),                   # more key than query tiles
-    ([1100, 900, 1024], [140, 130, 129], 200, 0),             # more query tiles than a CTA keeps
+    ([1300, 900, 1024], [140, 130, 129], 200, 0),             # more query tiles than a CTA keeps, and as many
 ])
 def test_packed_runs(lengths_q, lengths_k, heads, spare):
     lengths_k = lengths_q if lengths_k is None else lengths_k
