@@ -153,6 +153,7 @@ struct BwdPrologueShared {
   SchedRunShared runs;
   int end[kSchedRunSeqs + 1];  // last query row of each sequence + 1, and of the rows past the last one; bit 31: a run
   int first;                   // the sequence in which the block's rows start
+  int lead;                    // rows before the first sequence
 };
 
 template <bool kRuns>
@@ -171,7 +172,7 @@ __global__ void __launch_bounds__(kAuxThreads) attn_bwd_prologue_kernel(const Bw
     sched_build<kAuxThreads>(p.sched, sched_sm, rule);
     if constexpr (kRuns) sched_write_rest<kAuxThreads>(p.sched, rule, sm.runs);
   }
-  int seq = 0;
+  int seq = 0, lead = 0;
   if constexpr (kRuns) {
     // (The first block has the list to build, which the main kernel waits for: the others share its rows.)
     const uint32_t others = gridDim.x - 1;
@@ -195,9 +196,10 @@ __global__ void __launch_bounds__(kAuxThreads) attn_bwd_prologue_kernel(const Bw
       }
       sm.end[i] = stop | (run ? int(0x80000000u) : 0);
       if (begin <= tok && tok < stop) sm.first = i;
+      if (i == 0) sm.lead = begin;
     }
     __syncthreads();
-    seq = sm.first;
+    seq = sm.first, lead = sm.lead;
   }
 #if NB_BWD_L2_HINTS
   const uint64_t keep = l2_policy_evict_last();
@@ -217,7 +219,7 @@ __global__ void __launch_bounds__(kAuxThreads) attn_bwd_prologue_kernel(const Bw
       if constexpr (kRuns) {
         int stop = sm.end[seq];
         while (w.tok >= (stop & 0x7fffffff) && seq < p.batch) stop = sm.end[++seq];
-        l.clear = stop >= 0;
+        l.clear = stop >= 0 || w.tok < lead;
       }
     }
     l.o = *reinterpret_cast<const uint4*>(p.o + w.b * p.o_sb + w.tok * p.o_st + w.h * p.o_sh + lane8 * 8);

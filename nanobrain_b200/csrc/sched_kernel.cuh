@@ -293,7 +293,8 @@ __device__ __forceinline__ SchedRuns sched_runs(const SchedParams& p, SchedRunSh
 
 // The sequences that are no runs, as the epilogue reads them: word 0 counts the rows on the other side that
 // belong to them; row x of these (in the order of the sequences) is row x + shift of the whole, shift from the first
-// entry whose `end` exceeds x. One entry per sequence and one for the rows past the last one.
+// entry whose `end` exceeds x. One entry per sequence, the first one's with the rows before it, and one for the rows past
+// the last one.
 struct SchedRest {
   int end, shift;
 };
@@ -309,9 +310,10 @@ __device__ __forceinline__ void sched_write_rest(const SchedParams& p, const Sch
     if (sm.bad) {  // not a packing: all rows
       rows = i == 0 ? int(p.total_other) : 0;
     } else if (i <= p.batch) {
-      begin = p.cu_other[i];
+      // (Rows before the first sequence are nobody's: the first entry has them, also in front of a run.)
+      begin = i > 0 ? p.cu_other[i] : 0;
       rows = (i < p.batch ? p.cu_other[i + 1] : int(p.total_other)) - begin;
-      if (sched_run_cost(p, sched_classify(p, i), i, r) > 0) rows = 0;
+      if (sched_run_cost(p, sched_classify(p, i), i, r) > 0) rows = i > 0 ? 0 : p.cu_other[0];
     }
     int sum = 0;
     const int at = before + block_exclusive_scan<kThreads>(rows, sm.scratch, &sum);

@@ -1,12 +1,14 @@
 """The backward where one CTA takes all key tiles of a (sequence, head) and sums dQ up in tiles of its
 own, next to sequences whose key tiles are spread over the CTAs, against the CPU oracle."""
 
+import ctypes as C
+
 import numpy as np
 import pytest
 import torch
 
 import nanobrain_b200
-from nanobrain_b200 import ops
+from nanobrain_b200 import _lib, ops
 from oracle import attn_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -73,3 +75,36 @@ def test_an_invalid_packing_is_reported_and_nothing_runs():
     assert int(dq.count_nonzero()) == 0
     ops.sdpa_varlen_bwd(t, t, t, t, out, lse, good, good, 300, 300, 0.125)
     ops.check_status()
+
+
+def backward(lengths_q, lengths_k, heads, lead=0, spare=0, full=True):
+    """Forward and backward of random packed sequences through the C ABI, ``lead`` rows before the first and ``spare`` behind
+    the last, with the larger workspace or the one that a call has to have. dQ, dK and dV start as NaN."""
+    cu_q, cu_k = (torch.tensor([lead] + list(x)).cumsum(0).to(DEV, torch.int32) for x in (lengths_q, lengths_k))
+    tq, tk = lead + sum(lengths_q) + spare, lead + sum(lengths_k) + spare
+    g = torch.Generator(device=DEV).manual_seed(tq + tk)
+    q, d_out = (torch.randn(tq, heads, 64, generator=g, device=DEV).to(torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(tk, heads, 64, generator=g, device=DEV).to(torch.bfloat16) for _ in range(2))
+    out, lse = ops.sdpa_varlen_fwd(q, k, v, cu_q, cu_k, max(lengths_q), max(lengths_k), 0.125)
+    dq, dk, dv = (torch.full_like(t, float("nan")) for t in (q, k, v))
+    shape = _lib.Shape(len(lengths_q), heads, 64, max(lengths_q), max(lengths_k), tq, tk, cu_q.data_ptr(), cu_k.data_ptr(),
+                       0.125)
+    least, most = _lib.bwd_workspace_bytes(shape), _lib.bwd_full_workspace_bytes(shape)
+    assert most > least  # the larger one is for runs
+    ws = torch.empty(most if full else least, dtype=torch.uint8, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    d = lambda t: _lib.Tensor(t.data_ptr(), 0, t.stride(0), t.stride(1))
+    args = _lib.BwdArgs(shape, d(q), d(k), d(v), d(out), d(d_out), d(dq), d(dk), d(dv), lse.data_ptr(), ws.data_ptr(),
+                        ws.numel(), status.data_ptr(), None, None)
+    _lib.check(_lib.load().nb_attn_bwd(C.byref(args), C.c_void_p(torch.cuda.current_stream().cuda_stream)), "nb_attn_bwd")
+    assert int(status.item()) == 0
+    return dq, dk, dv
+
+
+@pytest.mark.parametrize("lengths", [[200] * 14 + [700], [1500] + [200] * 20])  # the first one is a run, or single tiles
+def test_dq_of_rows_before_the_first_sequence_is_zero(lengths):
+    for full in (False, True):
+        dq, dk, dv = backward(lengths, lengths, 100, lead=70, spare=33, full=full)
+        assert int(dq[:70].count_nonzero()) == 0 and int(dq[-33:].count_nonzero()) == 0
+        assert torch.isfinite(dq.float()).all()
+        assert torch.isfinite(dk[70:].float()).all() and torch.isfinite(dv[70:].float()).all()
