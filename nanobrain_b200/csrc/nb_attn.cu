@@ -99,7 +99,8 @@ int ensure_device_ready() {
   return rc;
 }
 
-// SM count of the current device (after ensure_device_ready succeeded on it).
+// SM count of the current device (after ensure_device_ready succeeded on it). An entry point asks once and hands the
+// number on to the rules: asked for by each of them a dense backward took the lock eight times (0.1 us of 14).
 int device_sm_count() {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return 1;
@@ -261,12 +262,12 @@ struct FwdSplit {
   unsigned ctas = 0;  // 0: whole units
   size_t bytes = 0;
 };
-FwdSplit fwd_split(const nb_attn_shape& s) {
+FwdSplit fwd_split(const nb_attn_shape& s, int sms) {
   FwdSplit r;
   if (s.cu_seqlens_q != nullptr) return r;
   const int64_t n_kt = ceil_div(s.max_seqlen_k, nb::kTile);
   const int64_t units = int64_t(ceil_div(s.max_seqlen_q, nb::kFwdQRows)) * s.heads * s.batch;
-  const int64_t slots = 2 * int64_t(device_sm_count()), steps = units * n_kt;
+  const int64_t slots = 2 * int64_t(sms), steps = units * n_kt;
   const int64_t ctas = steps / 4 < slots ? steps / 4 : slots;
   if (ctas < 2 || steps > INT32_MAX) return r;
   const int64_t k = (units + slots / 2 - 1) / (slots / 2);
@@ -285,12 +286,12 @@ struct BwdSplit {
   unsigned ctas = 0;
   size_t parts_offset = 0, bytes = 0;  // of the whole workspace
 };
-BwdSplit bwd_split(const nb_attn_shape& s) {
+BwdSplit bwd_split(const nb_attn_shape& s, int64_t sms) {
   BwdSplit r;
   if (s.cu_seqlens_q != nullptr) return r;
   const int64_t n_qt = ceil_div(s.max_seqlen_q, nb::kTile);
   const int64_t units = int64_t(ceil_div(s.max_seqlen_k, nb::kTile)) * s.heads * s.batch;
-  const int64_t sms = device_sm_count(), steps = units * n_qt;
+  const int64_t steps = units * n_qt;
   const int64_t ctas = steps / 2 < sms ? steps / 2 : sms;
   if (ctas < 2 || steps > INT32_MAX) return r;
   if ((units + sms - 1) / sms * n_qt * 12 <= 13 * ((steps + ctas - 1) / ctas + 3)) return r;
@@ -313,12 +314,13 @@ struct BwdRuns {
   int own_tiles = 0;
   size_t rest_offset = 0, own_offset = 0, bytes = 0;  // of the whole workspace; bytes = 0: no
 };
-BwdRuns bwd_runs(const nb_attn_shape& s) {
+BwdRuns bwd_runs(const nb_attn_shape& s, int64_t sms) {
   BwdRuns r;
-  const int64_t pairs = int64_t(s.batch) * s.heads, sms = device_sm_count();
+  if (s.cu_seqlens_q == nullptr) return r;
+  const int64_t pairs = int64_t(s.batch) * s.heads;
   const int n_qt = ceil_div(s.max_seqlen_q, nb::kTile), n_kt = ceil_div(s.max_seqlen_k, nb::kTile);
   const int most = pairs < 5 * sms ? nb::kBwdRunTiles - 1 : nb::kBwdRunTiles;
-  if (s.cu_seqlens_q == nullptr || s.batch > nb::kSchedRunSeqs || pairs < (n_kt == 1 ? 4 : 2) * sms ||
+  if (s.batch > nb::kSchedRunSeqs || pairs < (n_kt == 1 ? 4 : 2) * sms ||
       s.total_q > int64_t(s.batch) * most * nb::kTile)
     return r;
   const double steps = double(s.total_q) / nb::kTile * (double(s.total_k) / nb::kTile) * s.heads / s.batch;  // or more
@@ -399,8 +401,9 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
   p.n_kt = ceil_div(s.max_seqlen_k, nb::kTile);
   p.n_qt = ceil_div(s.max_seqlen_q, nb::kTile);
   p.parts = nullptr;
-  unsigned ctas = unsigned(device_sm_count());
-  const BwdRuns runs = bwd_runs(s);
+  const int sms = device_sm_count();
+  unsigned ctas = unsigned(sms);
+  const BwdRuns runs = bwd_runs(s, sms);
   const bool use_runs = runs.bytes > 0 && workspace_bytes >= runs.bytes;
   p.own = use_runs ? reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + runs.own_offset) : nullptr;
   p.own_tiles = runs.own_tiles;
@@ -409,7 +412,7 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
     p.items = nullptr;
     p.sched = nb::SchedParams{};
     n_work = int64_t(p.n_kt) * s.heads * s.batch;
-    const BwdSplit split = bwd_split(s);
+    const BwdSplit split = bwd_split(s, sms);
     if (split.ctas > 0 && workspace_bytes >= split.bytes) {
       const uint32_t steps = uint32_t(n_work * p.n_qt);
       p.parts = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + split.parts_offset);
@@ -443,7 +446,7 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
   const int64_t want_blocks = (rows * 8 + 255) / 256;
   // (With runs a block first looks at all sequences and takes consecutive rows: no more blocks than are resident. 300 sequences of
   // 200 tokens: 282 us with four per SM, 286 with eight.)
-  const int64_t most_blocks = (p.rest != nullptr ? 4 : 16) * int64_t(device_sm_count());
+  const int64_t most_blocks = (p.rest != nullptr ? 4 : 16) * int64_t(sms);
   const int aux_blocks = int(want_blocks < most_blocks ? want_blocks : most_blocks);
   p.row_blocks = aux_blocks;
   const int combine_blocks = p.parts != nullptr ? 4 * (int(ctas) - 1) : 0;
@@ -509,9 +512,10 @@ int run_fwd(const nb_attn_fwd_args* a, bool listed, void* stream) {
   p.n_qt = ceil_div(s.max_seqlen_q, nb::kFwdQRows);
   p.n_kt = ceil_div(s.max_seqlen_k, nb::kTile);
   int64_t n_units = int64_t(p.n_qt) * s.heads * s.batch;
-  unsigned slots = 2 * unsigned(device_sm_count());  // CTAs are persistent, two per SM
+  const int sms = device_sm_count();
+  unsigned slots = 2 * unsigned(sms);  // CTAs are persistent, two per SM
   if (dense) {
-    const FwdSplit split = fwd_split(s);
+    const FwdSplit split = fwd_split(s, sms);
     if (split.ctas > 0 && a->workspace != nullptr && a->workspace_bytes >= split.bytes &&
         (reinterpret_cast<uintptr_t>(a->workspace) & 255u) == 0) {
       const uint32_t steps = uint32_t(n_units * p.n_kt);
@@ -578,8 +582,8 @@ size_t nb_attn_bwd_workspace_bytes(const nb_attn_shape* shape) {
 
 size_t nb_attn_bwd_split_workspace_bytes(const nb_attn_shape* shape) {
   if (shape == nullptr || check_shape(*shape) != NB_ATTN_OK || ensure_device_ready() != NB_ATTN_OK) return 0;
-  const size_t split = bwd_split(*shape).bytes, runs = bwd_runs(*shape).bytes;
-  return split > runs ? split : runs;
+  const int sms = device_sm_count();
+  return shape->cu_seqlens_q == nullptr ? bwd_split(*shape, sms).bytes : bwd_runs(*shape, sms).bytes;
 }
 
 size_t nb_attn_fwd_workspace_bytes(const nb_attn_shape* shape) {
@@ -589,7 +593,7 @@ size_t nb_attn_fwd_workspace_bytes(const nb_attn_shape* shape) {
 
 size_t nb_attn_fwd_split_workspace_bytes(const nb_attn_shape* shape) {
   if (shape == nullptr || check_shape(*shape) != NB_ATTN_OK || ensure_device_ready() != NB_ATTN_OK) return 0;
-  return fwd_split(*shape).bytes;
+  return fwd_split(*shape, device_sm_count()).bytes;
 }
 
 int nb_attn_fwd(const nb_attn_fwd_args* a, void* stream) { return run_fwd(a, false, stream); }
