@@ -391,8 +391,8 @@ constexpr int kBwdTmemCols = 512;
 // wait for ever. Every warp of an aligned warpgroup executes the same setmaxnreg instruction. The compute role needs 144.
 // With 640 threads x 96 registers (TMA and LSE/delta rows in a warpgroup of their own; drain 64, loaders 48) ptxas
 // spilled 40 to 72 bytes in the other roles' step loops: whole backward of 2 x 12 x 820 32.9 us, now 30.8; 1 x 12 x 3476 132.0 and
-// 128.4; 32 x 12 x 820 328 and 317; 256 sequences of 720..920 tokens 2555 and 2500. (Many sequences of two tiles lose: 300 of 200
-// tokens 368 -> 384, where the one warp's reads of list and rows follow each other; as runs they take 295.)
+// 128.4; 32 x 12 x 820 328 and 317; 256 sequences of 720..920 tokens 2555 and 2500. (Many sequences of two tiles, 300 of 200
+// tokens, gain nothing: the one warp's reads of list and rows follow each other.)
 constexpr int kBwdLaunchRegs = 128;
 constexpr int kBwdComputeRegs = 152;
 constexpr int kBwdIssuerRegs = 104;  // issuers and loader
@@ -828,6 +828,22 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         g = next_unit(g);
         continue;
       }
+      const int64_t stat_base =
+          packed ? int64_t(wk.h) * p.total_q + wk.q_begin : (int64_t(wk.b) * p.heads + wk.h) * p.lq;
+      int jt = bwd_start(wk);
+      float l2[4], dl[4];  // (as they are: arithmetic on them here would wait for them before the TMA loads are issued)
+      auto rows = [&] {
+#pragma unroll
+        for (int r4 = 0; r4 < 4; ++r4) {
+          const int r = jt * kTile + r4 * 32 + lane;
+          l2[r4] = INFINITY, dl[r4] = 0.f;
+          if (r < wk.lq) l2[r4] = p.lse[stat_base + r], dl[r4] = p.delta[stat_base + r];
+        }
+      };
+      // The first step's rows are requested before the waits for a slot, the K buffer and a stage, or on short sequences
+      // their latency would come on top of the list's: 2100 sequences of 200 tokens x 2 heads 468 us without, 437 with;
+      // 300 x 12 heads 412 and 382. (As runs, whose units are longer, these take 291 us without and 295 with.)
+      if (!kRuns && wk.n_q > 0) rows();
       if (lane == 0) {
         if (round >= uint32_t(kBwdWorkSlots))
           wait(bar(kBarWorkEmpty + slot), ((round / kBwdWorkSlots) - 1) & 1);
@@ -841,18 +857,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
       ++round;
       if (wk.n_q < 0) break;
-      const int64_t stat_base =
-          packed ? int64_t(wk.h) * p.total_q + wk.q_begin : (int64_t(wk.b) * p.heads + wk.h) * p.lq;
-      int jt = bwd_start(wk);
 #pragma unroll 1
       for (int j = 0; j < wk.n_q; ++j) {
-        float l2[4], dl[4];  // (as they are: arithmetic on them here would wait for them before the TMA loads are issued)
-#pragma unroll
-        for (int r4 = 0; r4 < 4; ++r4) {
-          const int r = jt * kTile + r4 * 32 + lane;
-          l2[r4] = INFINITY, dl[r4] = 0.f;
-          if (r < wk.lq) l2[r4] = p.lse[stat_base + r], dl[r4] = p.delta[stat_base + r];
-        }
+        if (kRuns || j > 0) rows();
         if (lane == 0) {
           if (pos.s >= uint32_t(kBwdStages)) wait(bar(kBarQdoEmpty + pos.qs), pos.qph ^ 1u);
           mbar_arrive_expect_tx(bar(kBarQdoFull + pos.qs), 2 * kTileBytes);
