@@ -818,8 +818,10 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       if (!kCut && wk.n_q == 0) {
         // Keys without queries: dK = dV = 0, written here. Such units have no step, and the drain warps hold a unit until
         // the issuers have seen the next step: published, a few of them in a row would fill the ring and nothing would move.
+        // (One warp writes what four did: one 512-byte store at a time, 63 sequences of 300 keys without queries x 12 heads take
+        // 48.8 us, four at a time 37.2; 56 of 64 sequences of 800 keys 158 and 136.)
         auto clear = [&](__nv_bfloat16* rows, int64_t st) {
-#pragma unroll 1
+#pragma unroll 4
           for (int c = lane; c < rows_live * 8; c += 32)
             *reinterpret_cast<uint4*>(rows + int64_t(c >> 3) * st + (c & 7) * 8) = make_uint4(0, 0, 0, 0);
         };
