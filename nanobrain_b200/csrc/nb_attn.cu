@@ -302,13 +302,21 @@ BwdSplit bwd_split(const nb_attn_shape& s, int64_t sms) {
 }
 
 // May sequences of a packed backward be runs (see BwdRun)? Which of them are the device decides (sched_runs), and every
-// block of the prologue has to look at all sequences for it, 3 us or so. So there have to be two rounds of (sequence, head)
-// pairs over the SMs, or most of the work stays single tiles anyway, and thirty steps per SM, about 40 us, to save from:
-// 32 sequences of 720..920 tokens and 12 heads (2.6 rounds, 106 steps) 259.9 us without runs, 255.8 with; 40 of them 326.7 and
-// 306.7; 45 of 400 (3.6, 36) 155.4 and 142.5; 300 of 200 (24, 59) 398 and 282; but 45 of 200 (3.6, 9) 55.9 and 60.0. Where the
-// sequences have more tiles on average than a run few could be. Ten tiles are allowed from five rounds on: 32 sequences of
-// 1160..1280 tokens and 16 heads (3.5) take 679 us without runs, 687 with; 64 of them and 12 heads (5.2) 1020 and 972. Sequences of one key tile are runs without
-// more ado (100 of 128 tokens x 8 heads 42.9 and 41.6), from four rounds on.
+// block of the prologue has to look at all sequences for it, 3 to 5 us. So there have to be
+//   * two rounds of (sequence, head) pairs over the SMs, or most of the work stays single tiles anyway. 12 heads, us without
+//     and with runs: 16 x 820 tokens (1.3 rounds) 138.8 and 143.1, 20 (1.6) 172.0 and 172.2, 24 (1.95) 209.8 and 203.1, 26
+//     (2.1) 223.6 and 212.9, 32 of 720..920 (2.6) 277 and 257, 25 of 500..1100 (2.03) 203.1 and 205.4;
+//   * 21 steps per SM, about 30 us, to save from, by the mean length (skewed lengths have more, but spread over fewer
+//     units: 30 of 200 and one of 2000, 10.2 by the mean and 30.5 in fact, 75.4 and 84.9). 50 x 200 (9.9 steps) 59.5 and 64.2,
+//     60 x 200 (11.9) 73.3 and 72.8, 35 x 300 (15.6) 75.3 and 80.2, 80 x 200 (15.8) 98.8 and 91.5, 40 x 300 (17.8) 86.4 and
+//     86.2, 26 x 400 (20.6) 88.5 and 90.2, 110 x 200 (21.8) 137.2 and 119.4, 50 x 300 (22.3) 108.5 and 104.1, 40 x 400 (31.7)
+//     136.5 and 129.2, 170 x 200 (33.7) 212.9 and 172.2;
+//   * no more tiles per sequence on average than a run has at most, or few could be one. Ten are allowed from five rounds
+//     on, where they make no difference beyond what runs of one side differ by (64 of 1160..1280 tokens, 5.2 rounds: 1152 us
+//     without, 1144 with nine, 1162 with ten); below, ten lose more often than not: 32 (2.6) 529, 533 and 572, 44 (3.6) 772,
+//     756 and 805, 50 (4.05) 888, 910 and 875, 56 (4.5) 1017, 997 and 1061.
+// Sequences of one key tile are runs without more ado, which pays from four rounds on: x 128 tokens x 8 heads, 40 (2.2)
+// 24.1 and 25.9 to 27.6, 60 (3.2) 30.7 and 30.7 to 34.1, 80 (4.3) 37.8 and 35.8 to 37.2, 200 (10.8) 76.4 and 62.3.
 struct BwdRuns {
   int tiles = 0;  // SchedParams::run_tiles
   int own_tiles = 0;
@@ -320,11 +328,13 @@ BwdRuns bwd_runs(const nb_attn_shape& s, int64_t sms) {
   const int64_t pairs = int64_t(s.batch) * s.heads;
   const int n_qt = ceil_div(s.max_seqlen_q, nb::kTile), n_kt = ceil_div(s.max_seqlen_k, nb::kTile);
   const int most = pairs < 5 * sms ? nb::kBwdRunTiles - 1 : nb::kBwdRunTiles;
-  if (s.batch > nb::kSchedRunSeqs || pairs < (n_kt == 1 ? 4 : 2) * sms ||
-      s.total_q > int64_t(s.batch) * most * nb::kTile)
+  // (Rows past the last sequence, of a buffer with room to spare, are no work.)
+  const int64_t most_q = int64_t(s.batch) * s.max_seqlen_q, most_k = int64_t(s.batch) * s.max_seqlen_k;
+  const int64_t rows_q = s.total_q < most_q ? s.total_q : most_q, rows_k = s.total_k < most_k ? s.total_k : most_k;
+  if (s.batch > nb::kSchedRunSeqs || pairs < (n_kt == 1 ? 4 : 2) * sms || rows_q > int64_t(s.batch) * most * nb::kTile)
     return r;
-  const double steps = double(s.total_q) / nb::kTile * (double(s.total_k) / nb::kTile) * s.heads / s.batch;  // or more
-  if (n_kt > 1 && steps < 30. * double(sms)) return r;
+  const double steps = double(rows_q) / nb::kTile * (double(rows_k) / nb::kTile) * s.heads / s.batch;  // or more
+  if (n_kt > 1 && steps < 21. * double(sms)) return r;
   r.tiles = n_kt == 1 ? -1 : n_qt < most ? n_qt : most;
   r.own_tiles = n_kt == 1 ? 0 : r.tiles;
   r.rest_offset =

@@ -108,3 +108,17 @@ def test_dq_of_rows_before_the_first_sequence_is_zero(lengths):
         assert int(dq[:70].count_nonzero()) == 0 and int(dq[-33:].count_nonzero()) == 0
         assert torch.isfinite(dq.float()).all()
         assert torch.isfinite(dk[70:].float()).all() and torch.isfinite(dv[70:].float()).all()
+
+
+@pytest.mark.parametrize("lengths,heads,spare,runs", [
+    ([200] * 45, 12, 9000, False),     # nine steps per SM, 36 if the spare rows were sequences
+    ([200] * 45, 12, 0, False),
+    ([200] * 140, 12, 14000, True),    # 28 steps per SM, 63 if they were
+    ([200] * 300, 12, 0, True),
+    ([200] * 300, 12, 400000, True),   # eleven tiles per sequence if they were
+])
+def test_spare_rows_do_not_decide_about_runs(lengths, heads, spare, runs):
+    total = sum(lengths) + spare
+    cu = torch.zeros(len(lengths) + 1, dtype=torch.int32, device=DEV)
+    shape = _lib.Shape(len(lengths), heads, 64, max(lengths), max(lengths), total, total, cu.data_ptr(), cu.data_ptr(), 0.125)
+    assert (_lib.load().nb_attn_bwd_split_workspace_bytes(C.byref(shape)) > 0) == runs
