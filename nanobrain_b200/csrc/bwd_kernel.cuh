@@ -52,13 +52,13 @@
 //                              3.82 ms; this form 3.37 ms.
 //   attn_bwd_epilogue_kernel : dQ = bf16(scale * accumulator). HBM-bound.
 //
-// Packed calls with many (sequence, head) pairs of not too many tiles have a second kind of unit, a run: one
-// CTA works off all key tiles of a pair and keeps its dQ in tiles of its own (see BwdRun). Clearing the accumulator in
-// the prologue and reading it again in the epilogue is 16 % of the backward of such a call; for a run both fall away
-// and delta is all that the prologue computes. Whole backward, us, without and with runs: 256 sequences of 720..920
-// tokens x 12 heads 2505 -> 2230, 500 of 1..300 563 -> 427, 300 of 200 398 -> 295, 128 of 720..920 1082 -> 969, 64 of them 534 -> 499.
-// The form of the main kernel that knows runs is an instantiation of its own: its code is 2 KB larger, and
-// with its waits inlined like the others' 7 KB, which made it 5 to 20 % slower on calls without any run.
+// Packed calls with many (sequence, head) pairs of not too many tiles have a second kind of unit, a run: one CTA works
+// off all key tiles of a pair and keeps its dQ in tiles of its own (see BwdRun). Clearing the accumulator in the
+// prologue and reading it again in the epilogue is 16 % of the backward of such a call; for a run both fall away and
+// delta is all that the prologue computes. Whole backward, us, without and with runs: 256 sequences of 720..920 tokens
+// x 12 heads 2204 and 1932, 128 of them 1088 and 983, 64 537 and 507, 32 270 and 262; 500 of 1..300 490 and 383; 300 of
+// 200 372 and 292. The form of the main kernel that knows runs is an instantiation of its own: its code is 2 KB larger,
+// and with its waits inlined like the others' 7 KB, which made it 5 to 20 % slower on calls without any run.
 //
 // Packed mode: block 0 of the prologue also builds the scheduler's work list of key tiles
 // (sched_kernel.cuh); the main kernel's work units are list entries x heads (the heads of one entry
@@ -119,9 +119,10 @@ struct BwdParams {
   int32_t* status;
   int32_t pad[2];  // see below
 };
-// The host needs 1.9 us to launch a kernel whose parameters leave a remainder of 24 or 32 bytes by 64, and 2.2 to 2.3 us with
-// any other remainder (an empty kernel, sizes of 200..1144 bytes). It is these bytes for the prologue and epilogue, these and five
-// tensor maps of 128 bytes for the main kernel: a backward's host time is 12.6 us with 24 and 13.4 us with 16.
+// The host needs 1.9 us to launch a kernel whose parameters leave a remainder of 24 or 32 bytes by 64, and 2.2 to 2.3
+// us with any other remainder (an empty kernel, sizes of 200..1144 bytes). It is these bytes for the prologue and
+// epilogue, these and five tensor maps of 128 bytes for the main kernel: a backward's host time is 12.6 us with 24 and
+// 13.4 us with 16.
 static_assert(sizeof(BwdParams) % 64 == 24 || sizeof(BwdParams) % 64 == 32, "choose the size of `pad`");
 
 // ----------------------------------------------------------------------------------------
@@ -387,12 +388,13 @@ constexpr int kBwdSmemBytes =
 // Tensor memory: S^T 0 (P^T over it), dP^T 128 (dS^T over it), dV 256, dK 320, dQ 384, K 448, V 480
 constexpr int kBwdTmemCols = 512;
 // Register re-partitioning. The CTA launches with 512 threads x 128 registers (the whole register file); setmaxnreg
-// only moves registers inside that allocation, so the budget must balance exactly or the growing warps would
-// wait for ever. Every warp of an aligned warpgroup executes the same setmaxnreg instruction. The compute role needs 144.
-// With 640 threads x 96 registers (TMA and LSE/delta rows in a warpgroup of their own; drain 64, loaders 48) ptxas
-// spilled 40 to 72 bytes in the other roles' step loops: whole backward of 2 x 12 x 820 32.9 us, now 30.8; 1 x 12 x 3476 132.0 and
-// 128.4; 32 x 12 x 820 328 and 317; 256 sequences of 720..920 tokens 2555 and 2500. (Many sequences of two tiles, 300 of 200
-// tokens, gain nothing: the one warp's reads of list and rows follow each other.)
+// only moves registers inside that allocation, so the budget must balance exactly or the growing warps would wait for
+// ever. Every warp of an aligned warpgroup executes the same setmaxnreg instruction. The compute role needs 144. With
+// 640 threads x 96 registers (TMA and LSE/delta rows in a warpgroup of their own; drain 64, loaders 48) ptxas spilled
+// 40 to 72 bytes in the other roles' step loops (8 bytes are left in the form of whole units, none in the others): the
+// change was worth 6 % of the whole backward of 2 x 12 x 820, 3 % of 1 x 12 x 3476 and 32 x 12 x 820, 2 % of 256
+// sequences of 720..920 tokens. (Many sequences of two tiles, 300 of 200 tokens, gain nothing: the one warp's reads of
+// list and rows follow each other.)
 constexpr int kBwdLaunchRegs = 128;
 constexpr int kBwdComputeRegs = 152;
 constexpr int kBwdIssuerRegs = 104;  // issuers and loader
@@ -437,13 +439,15 @@ struct BwdWork {
 };
 
 // Key tiles of a run go one after the other through the same CTA, each in the order of query tiles that it has as a
-// unit of its own (so dK and dV are the same either way). dQ of the first key tile is stored into the CTA's own
-// tiles, that of the others added to them, and the last one's leaves as bf16 together with what is there. So the accumulator of a run is neither
-// cleared nor read by a pass of its own, and 148 x own_tiles x 32 KB stay in the L2 from run to run.
+// unit of its own (so dK and dV are the same either way). dQ of the first key tile is stored into the CTA's own tiles,
+// that of the others added to them, and the last one's leaves as bf16 together with what is there. So the accumulator
+// of a run is neither cleared nor read by a pass of its own, and 148 x own_tiles x 32 KB stay in the L2 from run to
+// run.
 enum BwdRun : int { kRunTile = 1, kRunFirst = 2, kRunLast = 4 };
-// Most query tiles of a run: 148 CTAs' own tiles, Q and dO then take 148 x 10 x 64 KB = 97 of the L2's 126 MB. 64 sequences of
-// 1030..1150 tokens (nine tiles) x 12 heads take 781 us instead of 854, of 1160..1280 972 instead of 1020; but with twelve tiles 64 of
-// 1400..1536 take 1646 instead of 1409. (The tenth tile pays from five rounds of pairs on, see bwd_runs in nb_attn.cu.)
+// Most query tiles of a run: 148 CTAs' own tiles, Q and dO then take 148 x 10 x 64 KB = 97 of the L2's 126 MB. 64
+// sequences of 1030..1150 tokens (nine tiles) x 12 heads take 814 us instead of 863, of 1160..1280 1017 instead of
+// 1041; but with twelve tiles 64 of 1400..1536 take 1646 instead of 1409. (The tenth tile is allowed from five rounds of
+// pairs on, see bwd_runs in nb_attn.cu.)
 constexpr int kBwdRunTiles = 10;
 
 // Query tile an item starts at. Concurrent CTAs work on the key tiles of one (sequence, head) and
@@ -476,7 +480,8 @@ __device__ __forceinline__ int bwd_tiles(const BwdCutWork& w) { return w.n_qt; }
 __device__ __forceinline__ int bwd_part(const BwdWork&) { return -1; }
 __device__ __forceinline__ int bwd_part(const BwdCutWork& w) { return w.part; }
 template <int kMode>
-using BwdWorkOf = std::conditional_t<kMode == kBwdCut, BwdCutWork, std::conditional_t<kMode == kBwdRuns, BwdRunWork, BwdWork>>;
+using BwdWorkOf = std::conditional_t<kMode == kBwdCut, BwdCutWork,
+                                     std::conditional_t<kMode == kBwdRuns, BwdRunWork, BwdWork>>;
 
 // Unit g of the call; n_q = -1 past the last one. The loader fetches a CTA's units and publishes them to
 // the other roles through a small ring. Dense units all cost the same: CTA c of G takes c, G + c, ...
@@ -555,9 +560,9 @@ enum BwdCtrl : uint32_t {
 // Not inlined on purpose: compiled by itself the step body keeps its instruction schedule (it needs
 // 144 of the compute warps' 152 registers, and inlined into the kernel it came out 10-60 % slower
 // whenever the code around it changed).
-__device__ __noinline__ void bwd_compute_role(const uint32_t bar0, int* abort_flag, const uint32_t tmem_base, const float* sLse, const float* sDelta,
-                                              const volatile uint32_t* sCtrl, const uint32_t ds_smem,
-                                              const float scale_log2) {
+__device__ __noinline__ void bwd_compute_role(const uint32_t bar0, int* abort_flag, const uint32_t tmem_base,
+                                              const float* sLse, const float* sDelta, const volatile uint32_t* sCtrl,
+                                              const uint32_t ds_smem, const float scale_log2) {
   const int warp = threadIdx.x >> 5;
   const int w = warp >> 2;                       // warpgroup: query columns [64w, 64w+64)
   const int t = threadIdx.x & 31, quad = warp & 3;
@@ -730,8 +735,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
 
   const uint32_t bar0 = smem_u32(&bars[0]);
   auto bar = [&](int i) { return bar0 + 8u * uint32_t(i); };
-  // In the form with runs a wait's loop is called instead of inlined, 5 KB less code: 256 sequences of 720..920 tokens 2316 -> 2247 us.
-  // The others, small enough, do not gain (2 x 12 x 820: 31.7 -> 32.6).
+  // In the form with runs a wait's loop is called instead of inlined, 5 KB less code: 3 % of 256 sequences of 720..920
+  // tokens. The others, small enough, do not gain (2 x 12 x 820: 31.7 -> 32.6).
   auto wait = [&](uint32_t b, uint32_t parity) {
     return kRuns ? mbar_wait(b, parity, &abort_flag) : mbar_wait_inline(b, parity, &abort_flag);
   };
@@ -818,8 +823,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       if (!kCut && wk.n_q == 0) {
         // Keys without queries: dK = dV = 0, written here. Such units have no step, and the drain warps hold a unit until
         // the issuers have seen the next step: published, a few of them in a row would fill the ring and nothing would move.
-        // (One warp writes what four did: one 512-byte store at a time, 63 sequences of 300 keys without queries x 12 heads take
-        // 48.8 us, four at a time 37.2; 56 of 64 sequences of 800 keys 158 and 136.)
+        // (One warp writes what four did: one 512-byte store at a time, 63 sequences of 300 keys without queries x 12
+        // heads take 48.8 us, four at a time 37.2; 56 of 64 sequences of 800 keys 158 and 136.)
         auto clear = [&](__nv_bfloat16* rows, int64_t st) {
 #pragma unroll 4
           for (int c = lane; c < rows_live * 8; c += 32)
@@ -895,9 +900,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         if (++wk.kt < kt_end) continue;
         kt_end = 0;
       }
-      // The next unit is taken as late as can be: this warp is about three steps ahead of the MMAs,
-      // which covers the counter's and the list's latency, and a unit taken earlier would wait behind a
-      // long one while other CTAs run dry. (Taken before the wait for the last step's stage: 300 sequences of 200 tokens 294 -> 300 us.)
+      // The next unit is taken as late as can be: this warp is about three steps ahead of the MMAs, which covers the
+      // counter's and the list's latency, and a unit taken earlier would wait behind a long one while other CTAs run
+      // dry. (Taken before the wait for the last step's stage: 300 sequences of 200 tokens lose 2 %.)
       g = next_unit(g);
     }
     // One more stage carries the stop mark (no data).
@@ -1038,7 +1043,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
           int64_t out_st = is_dk ? p.dk_st : p.dv_st;
           int out_live = rows_live;
           if (kRuns && is_dq) {
-            out = p.dq + (int64_t(bcoord) * p.dq_sb + int64_t(h) * p.dq_sh + (wk.q_begin + jt * kTile + quad * 32) * p.dq_st);
+            out = p.dq + (int64_t(bcoord) * p.dq_sb + int64_t(h) * p.dq_sh +
+                          (wk.q_begin + jt * kTile + quad * 32) * p.dq_st);
             out_st = p.dq_st;
             out_live = wk.lq - jt * kTile - quad * 32;
             ++s;

@@ -303,20 +303,19 @@ BwdSplit bwd_split(const nb_attn_shape& s, int64_t sms) {
 
 // May sequences of a packed backward be runs (see BwdRun)? Which of them are the device decides (sched_runs), and every
 // block of the prologue has to look at all sequences for it, 3 to 5 us. So there have to be
-//   * two rounds of (sequence, head) pairs over the SMs, or most of the work stays single tiles anyway. 12 heads, us without
-//     and with runs: 16 x 820 tokens (1.3 rounds) 138.8 and 143.1, 20 (1.6) 172.0 and 172.2, 24 (1.95) 209.8 and 203.1, 26
-//     (2.1) 223.6 and 212.9, 32 of 720..920 (2.6) 277 and 257, 25 of 500..1100 (2.03) 203.1 and 205.4;
+//   * two rounds of (sequence, head) pairs over the SMs, or most of the work stays single tiles anyway. 12 heads, us
+//     without and with runs: 20 x 820 tokens (1.6 rounds) 178.6 and 180.0, 24 (1.95) 212.0 and 210.0, 26 (2.1) 227.9 and
+//     220.3, 32 of 720..920 (2.6) 270.4 and 261.6; 25 of 500..1100 (2.03) still 209.7 and 213.2;
 //   * 21 steps per SM, about 30 us, to save from, by the mean length (skewed lengths have more, but spread over fewer
-//     units: 30 of 200 and one of 2000, 10.2 by the mean and 30.5 in fact, 75.4 and 84.9). 50 x 200 (9.9 steps) 59.5 and 64.2,
-//     60 x 200 (11.9) 73.3 and 72.8, 35 x 300 (15.6) 75.3 and 80.2, 80 x 200 (15.8) 98.8 and 91.5, 40 x 300 (17.8) 86.4 and
-//     86.2, 26 x 400 (20.6) 88.5 and 90.2, 110 x 200 (21.8) 137.2 and 119.4, 50 x 300 (22.3) 108.5 and 104.1, 40 x 400 (31.7)
-//     136.5 and 129.2, 170 x 200 (33.7) 212.9 and 172.2;
+//     units: 30 of 200 and one of 2000, 10.2 by the mean and 30.5 in fact, 79.2 and 88.4). 35 x 300 (15.6 steps) 79.8 and
+//     85.1, 80 x 200 (15.8) 101.5 and 96.3, 40 x 300 (17.8) 90.7 and 91.8, 26 x 400 (20.6) 93.9 and 96.4, 110 x 200 (21.8)
+//     139.7 and 125.3, 50 x 300 (22.3) 112.1 and 109.6, 40 x 400 (31.7) 142.0 and 135.5;
 //   * no more tiles per sequence on average than a run has at most, or few could be one. Ten are allowed from five rounds
-//     on, where they make no difference beyond what runs of one side differ by (64 of 1160..1280 tokens, 5.2 rounds: 1152 us
-//     without, 1144 with nine, 1162 with ten); below, ten lose more often than not: 32 (2.6) 529, 533 and 572, 44 (3.6) 772,
-//     756 and 805, 50 (4.05) 888, 910 and 875, 56 (4.5) 1017, 997 and 1061.
+//     on: sequences of 1160..1280 tokens, without and with ten, 32 (2.6 rounds) 518.8 and 537.9, 44 (3.6) 713 and 737, 50
+//     (4.05) 811 and 787, 56 (4.5) 908 and 929, 60 (4.9) 976 and 1000, 64 (5.2) 1041 and 1017, 72 (5.8) 1170 and 1185, 80
+//     (6.5) 1305 and 1295: it is the part of a round left over that decides, and it weighs less the more rounds there are.
 // Sequences of one key tile are runs without more ado, which pays from four rounds on: x 128 tokens x 8 heads, 40 (2.2)
-// 24.1 and 25.9 to 27.6, 60 (3.2) 30.7 and 30.7 to 34.1, 80 (4.3) 37.8 and 35.8 to 37.2, 200 (10.8) 76.4 and 62.3.
+// 23.4 and 24.3, 60 (3.2) 29.7 and 29.1, 80 (4.3) 36.2 and 34.0, 100 (5.4) 42.1 and 39.3.
 struct BwdRuns {
   int tiles = 0;  // SchedParams::run_tiles
   int own_tiles = 0;
@@ -454,8 +453,8 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int64_t rows = s.total_q * s.heads;
   const int64_t want_blocks = (rows * 8 + 255) / 256;
-  // (With runs a block first looks at all sequences and takes consecutive rows: no more blocks than are resident. 300 sequences of
-  // 200 tokens: 282 us with four per SM, 286 with eight.)
+  // (With runs a block first looks at all sequences and takes consecutive rows: no more blocks than are resident. 300
+  // sequences of 200 tokens gain 4 us by four per SM instead of eight.)
   const int64_t most_blocks = (p.rest != nullptr ? 4 : 16) * int64_t(sms);
   const int aux_blocks = int(want_blocks < most_blocks ? want_blocks : most_blocks);
   p.row_blocks = aux_blocks;
@@ -463,12 +462,14 @@ int launch_bwd(const nb_attn_bwd_args* a, void* workspace, size_t workspace_byte
   const auto main = p.parts != nullptr ? nb::attn_bwd_kernel<nb::kBwdCut>
                     : use_runs           ? nb::attn_bwd_kernel<nb::kBwdRuns>
                                          : nb::attn_bwd_kernel<nb::kBwdWhole>;
-  bool ok = launch(use_runs ? nb::attn_bwd_prologue_kernel<true> : nb::attn_bwd_prologue_kernel<false>, dim3(aux_blocks), dim3(256), 0, st, p) == cudaSuccess;
+  const auto prologue = use_runs ? nb::attn_bwd_prologue_kernel<true> : nb::attn_bwd_prologue_kernel<false>;
+  const auto epilogue = use_runs ? nb::attn_bwd_epilogue_kernel<true> : nb::attn_bwd_epilogue_kernel<false>;
+  bool ok = launch(prologue, dim3(aux_blocks), dim3(nb::kAuxThreads), 0, st, p) == cudaSuccess;
   if (a->event_main_begin) cudaEventRecord(static_cast<cudaEvent_t>(a->event_main_begin), st);
   ok = ok && launch(main, grid, dim3(nb::kBwdThreads), nb::kBwdSmemBytes, st, tq, tk, tv, tg, tdq, p) ==
                  cudaSuccess;
   if (a->event_main_end) cudaEventRecord(static_cast<cudaEvent_t>(a->event_main_end), st);
-  ok = ok && launch(use_runs ? nb::attn_bwd_epilogue_kernel<true> : nb::attn_bwd_epilogue_kernel<false>, dim3(aux_blocks + combine_blocks), dim3(256), 0, st, p) == cudaSuccess;
+  ok = ok && launch(epilogue, dim3(aux_blocks + combine_blocks), dim3(nb::kAuxThreads), 0, st, p) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();  // leave no sticky "last error" behind for the caller's own checks
     return NB_ATTN_ERR_LAUNCH;

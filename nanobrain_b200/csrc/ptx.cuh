@@ -112,14 +112,13 @@ constexpr uint64_t kWaitLimitNs = 2000000000ull;  // about two seconds
 // Bounded wait. `abort_flag` lives in shared memory and is shared by the whole CTA. The attention
 // kernels use the default limit (a compile-time constant); the wait self-test passes its own
 // (at most 4 s: the clock is the low word of the nanosecond timer).
-// The loop is kept as small as it can be -- 32-bit timer arithmetic, the flag touched with plain
-// state-space accesses, the status word left to the kernel's end: the warp-specialised kernels have dozens of
-// wait sites, and their hot code has to fit the SM's instruction cache (with a
-// larger loop the backward kernel's instruction-cache hit rate was 92 % at best and instruction
-// fetch was its top stall). The status word's store at every site was 3 of the backward kernel's 54 KB; without it the
-// backward of 500 sequences of 1..300 tokens takes 555 instead of 568 us, of 32 x 12 x 820 328 instead of 333. A smaller site
-// yet, polls counted instead of timed, saved another 2 KB and cost 5 % (32 x 8 x 4096: 3392 -> 3552 us): the
-// timer's latency keeps the waiters from polling too often.
+// The loop is kept as small as it can be -- 32-bit timer arithmetic, the flag touched with plain state-space accesses,
+// the status word left to the kernel's end: the warp-specialised kernels have dozens of wait sites, and their hot code
+// has to fit the SM's instruction cache (with a larger loop the backward kernel's instruction-cache hit rate was 92 %
+// at best and instruction fetch was its top stall). The status word's store at every site was 3 of the backward
+// kernel's 54 KB; without it the backward of 500 sequences of 1..300 tokens takes 555 instead of 568 us, of 32 x 12 x
+// 820 328 instead of 333. A smaller site yet, polls counted instead of timed, saved another 2 KB and cost 5 % (32 x 8 x
+// 4096: 3392 -> 3552 us): the timer's latency keeps the waiters from polling too often.
 __device__ __forceinline__ uint32_t globaltimer_lo() {
   uint32_t t;
   asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
@@ -139,8 +138,9 @@ __device__ __forceinline__ bool mbar_wait_loop(uint32_t bar, uint32_t parity, ui
   asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(flag_addr), "r"(1) : "memory");
   return false;
 }
-// A site that has to wait calls the loop (112 bytes a site instead of 300): the forward, 48 -> 44 KB, takes 36.2 instead of 37.0
-// us on one sequence of 2000 tokens among thirty of 200, 942 instead of 961 on 256 of 720..920, 1 % less on most others.
+// A site that has to wait calls the loop (112 bytes a site instead of 300): the forward, 48 -> 44 KB, takes 36.2
+// instead of 37.0 us on one sequence of 2000 tokens among thirty of 200, 942 instead of 961 on 256 of 720..920, 1 %
+// less on most others.
 static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, uint32_t flag_addr, uint32_t limit) {
   return mbar_wait_loop(bar, parity, flag_addr, limit);
 }
