@@ -41,7 +41,7 @@ NOMINAL_BF16_TFLOPS = 2250.0
 FALLBACK_PEAKS = {"hbm_gbs": 6650.0, "bf16_tflops": 1590.0, "bf16_tflops_sustained": 1400.0}
 # dram__bytes_read.sum + dram__bytes_write.sum of one attn_bwd_kernel launch, from an ncu capture of
 # this workload (only known for that workload; not measured by the run itself).
-NCU_DRAM_BYTES_BWD_MAIN = {"vitb_encoder_varlen": 412.3e6}
+NCU_DRAM_BYTES_BWD_MAIN = {"vitb_encoder_varlen": 370.3e6}
 
 
 def parse_args():
@@ -696,7 +696,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
                                           "frac": oprob.bwd_flops / (o_main * 1e-3) / 1e12 / peak, "unit": UNIT},
                 }
                 if name == "mae_decoder_dense" and not args.skip_comparators:
-                    line["gpu_comparators"] = gpu_comparators(prob, oprob, steps=5)
+                    line["gpu_comparators"] = gpu_comparators(prob, oprob, steps=o_steps)
                 del oprob
                 torch.cuda.empty_cache()
             line["other_workloads"] = other
