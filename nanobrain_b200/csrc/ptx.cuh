@@ -155,9 +155,16 @@ __device__ __forceinline__ bool mbar_wait_inline(uint32_t bar, uint32_t parity, 
   return mbar_wait_loop(bar, parity, smem_u32(const_cast<int*>(abort_flag)), uint32_t(kWaitLimitNs));
 }
 
-// At the end of a kernel, by one thread behind a block-wide barrier: says whether a wait of this block gave up.
+// At the end of a kernel, by one thread behind a block-wide barrier: says whether a wait of this block gave up. Then nobody
+// has waited for the TMA loads still under way, and they must not arrive in shared memory that belongs to the next block
+// by then: the thread keeps the block for a tenth of a millisecond, a hundred times what a load takes.
+constexpr uint32_t kAbortDrainNs = 100000;
 __device__ __forceinline__ void report_abort(volatile int* abort_flag, int* status_word) {
-  if (*abort_flag != 0 && status_word != nullptr) *static_cast<volatile int*>(status_word) = int(kStatusWaitTimeout);
+  if (*abort_flag == 0) return;
+  const uint32_t t0 = globaltimer_lo();
+#pragma unroll 1
+  for (int i = 0; i < (1 << 20) && globaltimer_lo() - t0 < kAbortDrainNs; ++i) __nanosleep(200);
+  if (status_word != nullptr) *static_cast<volatile int*>(status_word) = int(kStatusWaitTimeout);
 }
 
 // One look at a barrier that never suspends the thread.

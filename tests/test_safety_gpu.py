@@ -146,6 +146,21 @@ def test_a_wait_that_cannot_complete_gives_up_and_frees_tensor_memory():
     assert torch.isfinite(out.float()).all() and torch.isfinite(t.grad.float()).all()
 
 
+def test_a_block_whose_wait_gave_up_stays_until_its_copies_are_over():
+    # 2 ms of waiting and 0.1 ms for loads that may still be under way, on the device's clock.
+    schedule.selftest_wait(2_000_000, torch.device(DEV))
+    begin, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    status = torch.zeros(1, dtype=torch.int32).pin_memory()
+    out = torch.zeros(2, dtype=torch.int32, device=DEV)
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    begin.record()
+    _lib.check(_lib.load().nb_attn_selftest_wait(2_000_000, status.data_ptr(), out.data_ptr(), stream), "selftest_wait")
+    end.record()
+    torch.cuda.synchronize()
+    assert int(status[0]) == _lib.STATUS_WAIT_TIMEOUT and out.tolist() == [1, 1]
+    assert begin.elapsed_time(end) >= 2.09
+
+
 def test_a_reported_status_surfaces_at_the_next_call_without_a_sync():
     word = ops._status_word(torch.device(DEV, torch.cuda.current_device()))
     word[0] = _lib.STATUS_WAIT_TIMEOUT      # what a kernel would have written
